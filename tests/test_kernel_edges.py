@@ -26,3 +26,16 @@ def test_gemm_f32_tiles(M, N, K):
     one = torch.empty(1, N, device=DEV)
     ops().gemm_f32(a[M - 1:].contiguous(), w, one)
     assert torch.equal(one[0], out[M - 1])               # whichever tile made the row
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,I,group", [(1, 8, 0), (3, 4096, 0), (5, 12, 0), (2, 7, 0), (3, 64, 8), (3, 64, 16), (5, 36, 4), (7, 48, 24)])
+def test_silu_mul_layouts(T, I, group, dtype):
+    gu = (torch.randn(T, 2 * I, device=DEV) * 4).to(dtype)
+    out = torch.empty(T, I, device=DEV, dtype=dtype)
+    ops().silu_mul(gu, out, group=group)
+    parts = gu.double().view(T, -1, 2, group or I)
+    g, u = parts[:, :, 0].reshape(T, I), parts[:, :, 1].reshape(T, I)
+    ref = g / (1 + torch.exp(-g)) * u
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6      # one rounding / a handful of them
+    assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())

@@ -8,35 +8,6 @@
 // The arithmetic is float32; input and output are in the activation dtype.
 #include "common.cuh"
 
-template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total, int group) {
-    pdl_launch_dependents();
-    pdl_wait();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    const size_t t = idx / I;
-    const int i = (int)(idx - t * I);
-    const size_t gi = group > 0 ? (size_t)2 * group * (i / group) + i % group : (size_t)i;
-    const float g = to_f32(gu[t * 2 * (size_t)I + gi]);
-    const float u = to_f32(gu[t * 2 * (size_t)I + gi + (group > 0 ? group : I)]);
-    out[idx] = from_f32<T>(g / (1.0f + expf(-g)) * u);
-}
-
-extern "C" int vl_silu_mul(const void* gu, void* out, int dtype, int T, int I, int group, void* stream) {
-    if (T <= 0 || I <= 0) return VL_OK;
-    if (group < 0 || (group > 0 && I % group)) return VL_ERR_ARGUMENT;
-    const size_t total = (size_t)T * I;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
-    cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == VL_F32)
-        return vl_launch(silu_mul_kernel<float>, dim3(blocks), dim3(256), 0, s, (const float*)gu, (float*)out, I, total, group);
-    else if (dtype == VL_BF16)
-        return vl_launch(silu_mul_kernel<bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total, group);
-    else
-        return VL_ERR_UNSUPPORTED;
-    return vl_launch_status();
-}
-
 // Gated activations of other feed-forwards, on the same [T, 2I] layouts:  out = f(gate, up)
 //   VL_ACT_SILU          silu(g) * u
 //   VL_ACT_RELU          max(g, 0) * u
@@ -75,9 +46,10 @@ __global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, 
     out[idx] = from_f32<T>(r);
 }
 
-// The plain-halves layout (group 0) with I a multiple of 8: eight outputs a thread, 16-byte accesses.
+// I a multiple of 8, and so is the group if there is one: eight outputs a thread, 16-byte accesses.  A pass over memory
+// (or over what L2 still holds of the product): 536 x 12,288 bfloat16 outputs 8.9 us, 27.4 us one by one.
 template <typename T>
-__global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total8, int act,
+__global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total8, int group, int act,
                                      float alpha, float limit, float shift, const float* __restrict__ bias) {
     pdl_launch_dependents();
     pdl_wait();
@@ -86,12 +58,13 @@ __global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ o
     const int per_row = I / 8;
     const size_t t = idx / per_row;
     const int i = (int)(idx - t * per_row) * 8;
+    const int gi = group > 0 ? 2 * group * (i / group) + i % group : i, ui = gi + (group > 0 ? group : I);
     float g[8], u[8], r[8];
-    load8(gu + t * 2 * (size_t)I + i, g);
-    load8(gu + t * 2 * (size_t)I + I + i, u);
+    load8(gu + t * 2 * (size_t)I + gi, g);
+    load8(gu + t * 2 * (size_t)I + ui, u);
     if (bias) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { g[e] += bias[i + e]; u[e] += bias[I + i + e]; }
+        for (int e = 0; e < 8; ++e) { g[e] += bias[gi + e]; u[e] += bias[ui + e]; }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -115,14 +88,14 @@ extern "C" int vl_gated_act(const void* gu, void* out, int dtype, int T, int I, 
     const size_t total = (size_t)T * I;
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (group == 0 && I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
+    if (group % 8 == 0 && I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
         const size_t total8 = total / 8;
         const unsigned b8 = (unsigned)((total8 + 255) / 256);
         if (dtype == VL_F32)
-            return vl_launch(gated_act_vec_kernel<float>, dim3(b8), dim3(256), 0, s, (const float*)gu, (float*)out, I, total8, act,
+            return vl_launch(gated_act_vec_kernel<float>, dim3(b8), dim3(256), 0, s, (const float*)gu, (float*)out, I, total8, group, act,
                              alpha, limit, shift, bias);
         if (dtype == VL_BF16)
-            return vl_launch(gated_act_vec_kernel<bf16>, dim3(b8), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total8, act,
+            return vl_launch(gated_act_vec_kernel<bf16>, dim3(b8), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total8, group, act,
                              alpha, limit, shift, bias);
     }
     if (dtype == VL_F32)
@@ -132,6 +105,10 @@ extern "C" int vl_gated_act(const void* gu, void* out, int dtype, int T, int I, 
         return vl_launch(gated_act_kernel<bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total, group,
                          act, alpha, limit, shift, bias);
     return VL_ERR_UNSUPPORTED;
+}
+
+extern "C" int vl_silu_mul(const void* gu, void* out, int dtype, int T, int I, int group, void* stream) {
+    return vl_gated_act(gu, out, dtype, T, I, group, VL_ACT_SILU, 1.f, 0.f, 0.f, nullptr, stream);
 }
 
 // A function of one argument, element by element in float32: act 16 = the square of max(v, 0), 17 = tanh(v), 18 = gelu(v) =
