@@ -142,6 +142,10 @@ gemm_tc5_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         }
     } else {                                                 // ---- epilogue: warps 2..5 ----
         const int quarter = warp & 3;                        // the TMEM lanes this warp may read
+        // A lane owns a row, so a store of two bytes costs the warp as much as one of sixteen: eight activations a store
+        // where the rows of C allow it (2,048 tokens x top 4 over 32 experts, 2,048 x 2,048 a gate/up: 173 us with stores of two bytes,
+        // which kept the tensor cores waiting for the epilogue, 98 with these).
+        const bool wide = ldc % 8 == 0 && ((uintptr_t)C & 15) == 0;
         int local = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
             int m0, n0;
@@ -182,10 +186,16 @@ gemm_tc5_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 #pragma unroll
                     for (int blk = 0; blk < 2; ++blk) {
                         if (n0 + c0 + 16 * blk + 16 <= N) {
+                            float o[8];
 #pragma unroll
                             for (int i = 0; i < 8; ++i)
-                                dst[8 * blk + i] = from_f32<TO>(gated(__uint_as_float(v[16 * blk + i]),
-                                                                      __uint_as_float(v[16 * blk + 8 + i]), act, alpha, limit, shift));
+                                o[i] = gated(__uint_as_float(v[16 * blk + i]), __uint_as_float(v[16 * blk + 8 + i]), act, alpha, limit, shift);
+                            if (wide) {
+                                store8(dst + 8 * blk, o);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) dst[8 * blk + i] = from_f32<TO>(o[i]);
+                            }
                         }
                     }
                 }
