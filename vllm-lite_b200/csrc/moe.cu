@@ -155,14 +155,21 @@ moe_align_kernel(const int* __restrict__ ids, int npairs, int E, int bm, int cap
     for (int r = tid; r < cap; r += 1024) sorted_rows[r] = -1;
     for (int y = tid; y < max_tiles; y += 1024) tile_group[y] = -1;
     __syncthreads();
-    if (tid == 0) {
+    // One warp: where every expert's tiles begin, 32 experts at a time (one thread, expert after expert: 17 us for 8,192 pairs over
+    // 32 experts and 7.6 for 32 pairs; now 8.6 and 3.0).
+    if (tid < 32) {
         int at = 0;
-        for (int e = 0; e < E; ++e) {
-            s_start[e] = at;
-            const int tiles = (s_count[e] + bm - 1) / bm;
-            for (int y = 0; y < tiles; ++y) tile_group[at / bm + y] = e;
-            at += tiles * bm;
-            s_count[e] = 0;                              // now the cursor of the expert's rows
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + tid, tiles = e < E ? (s_count[e] + bm - 1) / bm : 0;
+            int x = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (tid >= o) x += y; }
+            if (e < E) {
+                s_start[e] = (at + x - tiles) * bm;
+                for (int y = 0; y < tiles; ++y) tile_group[at + x - tiles + y] = e;
+                s_count[e] = 0;                          // now the cursor of the expert's rows
+            }
+            at += __shfl_sync(0xffffffffu, x, 31);
         }
     }
     __syncthreads();
