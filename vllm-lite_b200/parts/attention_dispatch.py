@@ -51,6 +51,10 @@ def _decode(ops, args, step, spec, group, num_tokens, max_context, token_index=N
         # 64 x 16 heads, window 1,024 of 4,096: 19 us with chunks of 256 against 29 with chunks of 1,024).
         reach = min(int(max_context), int(spec.window)) if spec.window else int(max_context)
         chunk = 256 if reach <= 1024 else (512 if reach <= 2048 else 1024)
+        # Few tokens: such chunks leave SMs idle, and a block's own pace is what bounds the launch (8 tokens of 900 to 2,400 keys x
+        # 16 heads on a row of 256, bound 4,096: 32 us with 32 blocks of 1,024 keys, 13 with chunks of 128)
+        while chunk > 128 and num_tokens * -(-spec.num_heads // 16) * -(-reach // chunk) < 2 * ops.sm_pairs():
+            chunk //= 2
         own_merge = False
     S, n_acc, n_ml = ops.decode_attention_scratch(num_tokens, spec.num_heads, spec.head_dim, max_context, chunk)
     part_acc = step.workspace.get(step.tag + "attn.part_acc", (n_acc,), torch.float32)
