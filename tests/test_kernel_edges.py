@@ -39,3 +39,66 @@ def test_silu_mul_layouts(T, I, group, dtype):
     ref = g / (1 + torch.exp(-g)) * u
     rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6      # one rounding / a handful of them
     assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())
+
+
+def decayed_memory(r, k, v, w, u, S):
+    """float64, one request: r, k, w [T, H, D], v [T, H, P], u [H, D], S [H, D, P]; (outputs [T, H, P], the state behind them)."""
+    out = torch.empty(v.shape, dtype=torch.float64, device=DEV)
+    for t in range(r.shape[0]):
+        kv = k[t][:, :, None] * v[t][:, None]
+        out[t] = torch.einsum("hdp,hd->hp", S + u[:, :, None] * kv, r[t])
+        S = w[t][:, :, None] * S + kv
+    return out, S
+
+
+# portions on both sides of 96 tokens and of whole chunks, heads of one tile and two, decays from nothing kept to all kept, a state carried over
+@pytest.mark.parametrize("H,D,P", [(1, 4, 4), (2, 12, 20), (2, 64, 64), (3, 64, 36), (2, 128, 128), (1, 100, 68)])
+@pytest.mark.parametrize("lengths", [[96], [95, 128, 97], [129, 1, 200], [7, 191]])
+@pytest.mark.parametrize("decays", ["mixed", "strong", "zeros"])
+def test_decay_chunks(H, D, P, lengths, decays):
+    gen = torch.Generator(device=DEV).manual_seed(D * 7 + sum(lengths))
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    T, B, eps = sum(lengths), len(lengths), 1e-5
+    cu = torch.tensor([sum(lengths[:i]) for i in range(B + 1)], dtype=torch.int32, device=DEV)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32, device=DEV)
+    u, norm = rnd(H * D) * 0.5, 1 + 0.1 * rnd(H * P)
+    state = torch.zeros(B + 1, ops().decay_state_floats(H, D, P) + 4, device=DEV)
+    S = [torch.zeros(H, D, P, dtype=torch.float64, device=DEV) for _ in lengths]
+    for turn in range(2):                                # the second portions start from what the first ones left
+        r, k, v, gate = rnd(T, H * D + 4), rnd(T, H * D), rnd(T, H * P), rnd(T, H * P + 8).to(torch.bfloat16)
+        w = {"mixed": torch.exp(-torch.exp(2 * rnd(T, H * D) - 2)), "strong": torch.exp(-torch.exp(rnd(T, H * D) + 2)),
+             "zeros": (rnd(T, H * D) > 0).float()}[decays]
+        out = torch.full((T, H * P), float("nan"), device=DEV, dtype=torch.bfloat16)
+        o = torch.empty(T, H * P, device=DEV)
+        scan = (r, 4), (k, 0), (v, 0), (w, 0), u, state, 4, cu, slots
+        walked = state.clone()
+        ops().decay_scan(*scan[:5], walked, *scan[6:], o, H, D, P)       # the walk over everything, beside it
+        if min(lengths) < ops().DECAY_MIN_CHUNK:
+            o2 = torch.empty(T, H * P, device=DEV)
+            ops().decay_scan(*scan, o2, H, D, P, longest=ops().DECAY_MIN_CHUNK - 1)
+        chunks = ops().decay_chunks_of(lengths)
+        scratch = torch.full((ops().decay_chunk_floats(chunks, H, D, P),), float("nan"), device=DEV)
+        ops().decay_chunks(*scan, chunks, scratch, gate, 8, norm, eps, out, H, D, P)
+        for b, n in enumerate(lengths):
+            at = slice(int(cu[b]), int(cu[b]) + n)
+            heads = lambda x, m: x[at].double().view(n, H, m)
+            want, S[b] = decayed_memory(heads(r[:, 4:].contiguous(), D), heads(k, D), heads(v, P), heads(w, D), u.double().view(H, D), S[b])
+            if n < ops().DECAY_MIN_CHUNK:
+                assert torch.equal(o2[at], o[at]) and out[at].isnan().all()
+                continue
+            y = want / torch.sqrt((want * want).mean(-1, keepdim=True) + eps) * norm.double().view(H, P)
+            y = y * torch.nn.functional.silu(heads(gate[:, 8:].contiguous(), P))
+            assert float((heads(out, P) - y).norm() / y.norm()) <= 2.0 ** -8      # the result's rounding
+        # float32 inside: the states as near to 64 bits as the walk's, up to a small factor
+        native = lambda st, b: st[int(slots[b]), 4:]
+        for b in range(B):
+            err = [float((state_of(native(st, b), H, D, P) - S[b]).norm() / S[b].norm()) for st in (state, walked)]
+            assert err[0] <= 2 * err[1] + 3e-7, (b, err)
+            assert torch.equal(state[:, :4], walked[:, :4])
+
+
+def state_of(flat, H, D, P):
+    """decay_scan's state of one request as [H, D, P] in float64."""
+    rows, lanes, cols, tiles = ops().decay_scan_shape(D, P)
+    x = flat.double().view(H, tiles, rows, cols, lanes)              # element (row l rows + i, column z cols + col)
+    return x.permute(0, 4, 2, 1, 3).reshape(H, lanes * rows, tiles * cols)[:, :D, :P]

@@ -77,8 +77,10 @@ def _mixer_width(mixer) -> int:
         return (2 * hd + 2 * hp + 2 * mixer.num_heads) + 2 * hp + hp
     if hasattr(mixer, "decay_rank") and not hasattr(mixer, "gate_rank"):
         # time mixing: five mixes of the input, r, k, v and the raw decay in float32, the gate, the scan's result, the gated rows
+        # ... and, in chunks of 64 tokens (a portion's last one may be short), per head two states, two rows a token and one
         hd = mixer.num_heads * mixer.dim
-        return 5 * mixer.hidden_size + 8 * hd + hd + 2 * mixer.decay_rank + 2 * hd + hd
+        chunks = 2 * 2 * mixer.num_heads * (2 * mixer.dim * mixer.dim // 64 + 2 * mixer.dim + mixer.dim // 64 + 1)
+        return 5 * mixer.hidden_size + 8 * hd + hd + 2 * mixer.decay_rank + 2 * hd + hd + chunks
     if hasattr(mixer, "unit_eps") and not hasattr(mixer, "decay_rank"):
         # delta rule with one decay per head: one product (with the gate, two numbers a head and up to 7 rows of padding), its
         # convolved float32 copy, the scan's float32 result, the gated rows

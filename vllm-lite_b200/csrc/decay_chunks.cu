@@ -1,0 +1,356 @@
+// The recurrence of `vl_decay_scan` (csrc/recurrent.cu) over long portions, with the norm per head and the gate behind it:
+//     o_t = (S + diag(u) k_t v_t^T)^T r_t,   S <- diag(w_t) S + k_t v_t^T,   out = rms_head(o) * norm * silu(gate)
+// (S: D x P a head, D, P up to 128 and multiples of 4; w in (0, 1) per head and key channel), float32 throughout.
+//
+// Walked token by token one request keeps few warps busy with a chain of 2,048 steps.  Here a portion is cut into chunks of 64
+// tokens that are worked off all at once, but for the state's way from chunk to chunk, which is one multiply-add an element:
+//   (1) per chunk and head: the 64 x 64 matrix A_ts = sum_d r_td k_sd prod_{s<j<t} w_jd (t > s), A_tt = sum_d r_td u_d k_td; the part of
+//       the outputs that stays inside the chunk, A V; what the chunk adds to the state, sum_s (k_s prod_{j>s} w_j) v_s^T; r_t times the
+//       decays since the chunk's start;
+//   (2) per head: S at every chunk's start, S <- diag(prod w) S + what the chunk added;
+//   (3) per chunk and head: A V + (decayed r) S, normed and gated.
+// No decay is ever divided by: for a pair of tokens in different halves of a run of 64, 32 or 16 tokens the product splits at
+// the middle into one factor of r_t and one of k_s, both running products of numbers below 1, as the walk's own; pairs within 8 tokens
+// multiply their few decays directly.  The products (2,016 pairs x D in a chunk, then 64 x 64 x P, 64 x D x P twice) are plain
+// multiply-adds on tiles in shared memory, which is what bounds (1) and (3).
+// One request of 2,048 tokens, 32 heads of 64 x 64: 137 us with the norm and the gate (89 + 15 + 32), against 413 for the walk and the norm's
+// kernel behind it; 128 x 128: 401 against 1,191; 512 tokens: 37 against 107; 64 tokens: 27 against 18, and of 32 requests of 64 tokens
+// 168 against 230: a lone portion wins from about 100 tokens on.
+#include "common.cuh"
+#include "chunk_index.cuh"
+
+#define CT 64                          // tokens of a chunk
+#define DCH_MIN 96                     // portions of fewer tokens are walked
+#define DCH_MAX 128                    // most rows and columns of a head's state
+
+__device__ __forceinline__ float4 dc_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void dc_st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void dc_fma(float4& a, float x, float4 v) { a.x += x * v.x; a.y += x * v.y; a.z += x * v.z; a.w += x * v.w; }
+__device__ __forceinline__ float dc_at(const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
+
+struct DecayRows { const float* p; int ld, col; };                // rows [T, ld], the first column
+
+// acc (rows 4 ty .., columns 4 tx ..) += a b over k in [0, n), a[row][k], b[k][column]
+__device__ __forceinline__ void dc_product(float4 (&acc)[4], const float* a, int lda, const float* b, int ldb, int n) {
+    for (int k = 0; k < n; k += 4) {
+        float4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x[i] = dc_ld4(a + i * lda + k);
+            y[i] = dc_ld4(b + (k + i) * ldb);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dc_fma(acc[i], dc_at(x[i], e), y[e]);
+    }
+}
+
+// A running product of decays over `n` tokens (a multiple of 8), first to last (DOWN) or last to first, of one channel: put(t, x[t] times the decays of the tokens passed
+// before t); returns the product of all.  Eight tokens' numbers are on their way from shared memory together.
+template <bool DOWN, typename Put>
+__device__ __forceinline__ float dc_chain(const float* x, const float* w, int ld, int t0, int n, Put put) {
+    float f = 1.f;
+    for (int i = 0; i < n; i += 8) {
+        float a[8], g[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int t = DOWN ? t0 + i + e : t0 + n - 1 - i - e;
+            a[e] = x[t * ld]; g[e] = w[t * ld];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { put(DOWN ? t0 + i + e : t0 + n - 1 - i - e, a[e] * f); f *= g[e]; }
+    }
+    return f;
+}
+
+#define DCH_LDA (CT + 4)
+// Buffers of chunk and head number i = chunk * H + head: added [D][P], start [D][P] (S at the chunk's start), rdec [64][D], inner [64][P],
+// keep [D].
+__global__ void __launch_bounds__(256)
+decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const float* __restrict__ u, const int* __restrict__ cu, int B,
+                  float* __restrict__ added, float* __restrict__ rdec, float* __restrict__ inner, float* __restrict__ keep, int H, int D, int P) {
+    extern __shared__ __align__(16) float sm[];
+    pdl_launch_dependents();
+    pdl_wait();
+    int b, c;
+    if (!ci_find(cu, B, CT, DCH_MIN, blockIdx.x, &b, &c)) return;
+    const int h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int row0 = cu[b] + c * CT, m = min(CT, cu[b + 1] - row0);
+    const int LD = D + 4, D4 = D >> 2;
+    const size_t ch = (size_t)blockIdx.x * H + h;
+    float* R = sm;                                                // [64][LD], later the values [64][68]
+    float* K = R + CT * (LD > DCH_LDA ? LD : DCH_LDA);
+    float* W = K + CT * LD;
+    float* X = W + CT * LD;                                       // r or k times one level's decays
+    float* A = X + CT * LD;                                       // [64][68]
+    for (int i = tid; i < CT * D4; i += 256) {                    // (tokens behind the portion: nothing added, nothing decayed)
+        const int t = i / D4, d = 4 * (i - t * D4);
+        const size_t row = row0 + t, at = (size_t)h * D + d;
+        const bool in = t < m;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+        dc_st4(R + t * LD + d, in ? dc_ld4(r.p + row * r.ld + r.col + at) : z);
+        dc_st4(K + t * LD + d, in ? dc_ld4(k.p + row * k.ld + k.col + at) : z);
+        dc_st4(W + t * LD + d, in ? dc_ld4(w.p + row * w.ld + w.col + at) : one);
+    }
+    for (int i = tid; i < CT * DCH_LDA / 4; i += 256) dc_st4(A + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+    __syncthreads();
+    // pairs in different halves of a run of 2 `half` tokens
+#pragma unroll
+    for (int half = 32; half >= 8; half >>= 1) {
+        for (int i = tid; i < (CT / half) * D; i += 256) {        // a run of `half` tokens of one channel
+            const int seg = i / D, d = i - seg * D, t0 = seg * half;
+            auto put = [&](int t, float v) { X[t * LD + d] = v; };
+            if (seg & 1) dc_chain<true>(R + d, W + d, LD, t0, half, put);      // behind the middle: r times the decays from there on
+            else dc_chain<false>(K + d, W + d, LD, t0, half, put);             // before it: k times the decays behind the token
+        }
+        __syncthreads();
+        // 32 half pairs: a thread takes `each` neighbouring s for one or two t
+        if (half == 32) {
+            const float* a = X + (32 + ty) * LD;
+            const float* q = X + tx * LD;
+            float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+            for (int d = 0; d < D; d += 4) {
+                const float4 a0 = dc_ld4(a + d), a1 = dc_ld4(a + 16 * LD + d), b0 = dc_ld4(q + d), b1 = dc_ld4(q + 16 * LD + d);
+                s[0][0] += a0.x * b0.x; s[0][0] += a0.y * b0.y; s[0][0] += a0.z * b0.z; s[0][0] += a0.w * b0.w;
+                s[0][1] += a0.x * b1.x; s[0][1] += a0.y * b1.y; s[0][1] += a0.z * b1.z; s[0][1] += a0.w * b1.w;
+                s[1][0] += a1.x * b0.x; s[1][0] += a1.y * b0.y; s[1][0] += a1.z * b0.z; s[1][0] += a1.w * b0.w;
+                s[1][1] += a1.x * b1.x; s[1][1] += a1.y * b1.y; s[1][1] += a1.z * b1.z; s[1][1] += a1.w * b1.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) A[(32 + ty + 16 * i) * DCH_LDA + tx + 16 * j] = s[i][j];
+        } else {
+            const int per = half * half, lh = half == 16 ? 4 : 3;
+            for (int i = tid; i < 32 * half; i += 256) {
+                const int seg = i / per, e = i - seg * per, t = seg * 2 * half + half + (e >> lh), s = seg * 2 * half + (e & (half - 1));
+                float x = 0.f, y = 0.f;
+                for (int d = 0; d < D; d += 4) {
+                    const float4 a = dc_ld4(X + t * LD + d), q = dc_ld4(X + s * LD + d);
+                    x += a.x * q.x; y += a.y * q.y; x += a.z * q.z; y += a.w * q.w;
+                }
+                A[t * DCH_LDA + s] = x + y;
+            }
+        }
+        __syncthreads();
+    }
+    // pairs within 8 tokens and the tokens themselves: a warp a run, four channels a lane, everything in registers
+    {
+        const int t0 = 8 * (tid >> 5), d = 4 * (tid & 31);
+        const bool on = d < D;
+        float4 rr[8], ww[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            rr[e] = on ? dc_ld4(R + (t0 + e) * LD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            ww[e] = on ? dc_ld4(W + (t0 + e) * LD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const float4 uu = on ? dc_ld4(u + (size_t)h * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            float4 q = on ? dc_ld4(K + (t0 + s) * LD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float sum[8];
+            sum[s] = (rr[s].x * (uu.x * q.x) + rr[s].y * (uu.y * q.y)) + (rr[s].z * (uu.z * q.z) + rr[s].w * (uu.w * q.w));
+#pragma unroll
+            for (int t = s + 1; t < 8; ++t) {
+                sum[t] = (rr[t].x * q.x + rr[t].y * q.y) + (rr[t].z * q.z + rr[t].w * q.w);
+                q.x *= ww[t].x; q.y *= ww[t].y; q.z *= ww[t].z; q.w *= ww[t].w;
+            }
+#pragma unroll
+            for (int t = s; t < 8; ++t) {
+                const float v = warp_sum(sum[t]);
+                if ((tid & 31) == t) A[(t0 + t) * DCH_LDA + t0 + s] = v;
+            }
+        }
+    }
+    // r times the decays since the chunk's start (to memory); k times those up to its end (X); the chunk's own decay
+    __syncthreads();
+    for (int i = tid; i < 2 * D; i += 256) {
+        const int d = i < D ? i : i - D;
+        if (i < D) keep[ch * D + d] = dc_chain<true>(R + d, W + d, LD, 0, CT, [&](int t, float v) { rdec[(ch * CT + t) * D + d] = v; });
+        else dc_chain<false>(K + d, W + d, LD, 0, CT, [&](int t, float v) { X[t * LD + d] = v; });
+    }
+    for (int p0 = 0; p0 < P; p0 += 64) {                          // 64 columns of the values at a time, in the place of r
+        __syncthreads();
+        for (int i = tid; i < CT * 16; i += 256) {
+            const int t = i >> 4, p = 4 * (i & 15);
+            dc_st4(R + t * DCH_LDA + p, t < m && p0 + p < P ? dc_ld4(v.p + (size_t)(row0 + t) * v.ld + v.col + (size_t)h * P + p0 + p)
+                                                             : make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+        __syncthreads();
+        const bool cols = p0 + 4 * tx < P;
+        float4 acc[4] = {};
+        for (int d0 = 4 * ty; d0 < D; d0 += 64) {                 // (the values of a step of four tokens serve both products)
+            float4 sum[4] = {};
+#pragma unroll 2
+            for (int k = 0; k < CT; k += 4) {
+                float4 y[4], x[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { y[i] = dc_ld4(R + (k + i) * DCH_LDA + 4 * tx); x[i] = dc_ld4(X + (k + i) * LD + d0); }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dc_fma(sum[i], dc_at(x[e], i), y[e]);
+                if (d0 < 64 && k <= 4 * ty) {                     // (A is zero above the diagonal)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = dc_ld4(A + (4 * ty + i) * DCH_LDA + k);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) dc_fma(acc[i], dc_at(x[i], e), y[e]);
+                }
+            }
+            if (cols) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dc_st4(added + (ch * D + d0 + i) * P + p0 + 4 * tx, sum[i]);
+            }
+        }
+        if (4 * ty >= D) dc_product(acc, A + 4 * ty * DCH_LDA, DCH_LDA, R + 4 * tx, DCH_LDA, 4 * ty + 4);   // (rows of the state there are none)
+        if (cols) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dc_st4(inner + (ch * CT + 4 * ty + i) * P + p0 + 4 * tx, acc[i]);
+        }
+    }
+}
+
+// The state of a request lies as vl_decay_scan keeps it: row d and column p of head h at scan_at(h, d, p).
+struct ScanLayout { int rows, L, cols, tiles; };
+__device__ __forceinline__ size_t scan_at(const ScanLayout& y, int h, int d, int p) {
+    const int z = p / y.cols, col = p - z * y.cols, l = d / y.rows, i = d - l * y.rows;
+    return (((size_t)h * y.tiles + z) * y.rows + i) * (y.cols * y.L) + col * y.L + l;
+}
+__global__ void __launch_bounds__(256)
+decay_chain_kernel(const float* __restrict__ added, const float* __restrict__ keep, float* __restrict__ start, float* __restrict__ state,
+                   long long state_stride, const int* __restrict__ cu, const int* __restrict__ slots, ScanLayout lay, int H, int D, int P) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int b = blockIdx.y, n = cu[b + 1] - cu[b];
+    if (n < DCH_MIN) return;
+    const int first = ci_first(cu, b, CT, DCH_MIN), chunks = (n + CT - 1) / CT;
+    const int idx = blockIdx.x * 256 + threadIdx.x, per = D * (P >> 2), h = idx / per;
+    if (h >= H) return;
+    const int e = idx - h * per, d = e / (P >> 2), p = 4 * (e - d * (P >> 2));
+    float* S = state + (long long)slots[b] * state_stride;
+    float4 s = make_float4(S[scan_at(lay, h, d, p)], S[scan_at(lay, h, d, p + 1)], S[scan_at(lay, h, d, p + 2)], S[scan_at(lay, h, d, p + 3)]);
+    const size_t at = (size_t)(first * H + h) * D + d, step = (size_t)H * D;
+#pragma unroll 8
+    for (int c = 0; c < chunks; ++c) {                            // (the reads of eight chunks are on their way together)
+        const float4 x = dc_ld4(added + (at + c * step) * P + p);
+        const float g = keep[at + c * step];
+        dc_st4(start + (at + c * step) * P + p, s);
+        s.x = g * s.x + x.x; s.y = g * s.y + x.y; s.z = g * s.z + x.z; s.w = g * s.w + x.w;
+    }
+    S[scan_at(lay, h, d, p)] = s.x; S[scan_at(lay, h, d, p + 1)] = s.y;
+    S[scan_at(lay, h, d, p + 2)] = s.z; S[scan_at(lay, h, d, p + 3)] = s.w;
+}
+
+template <typename TP, int NC>                                    // NC: 64 columns of the values a step
+__global__ void __launch_bounds__(256)
+decay_out_kernel(const float* __restrict__ rdec, const float* __restrict__ start, const float* __restrict__ inner,
+                 const TP* __restrict__ gate, int ld, int gate_col, const float* __restrict__ norm, float eps, const int* __restrict__ cu,
+                 int B, TP* __restrict__ out, int H, int D, int P) {
+    extern __shared__ __align__(16) float sm[];
+    pdl_launch_dependents();
+    pdl_wait();
+    int b, c;
+    if (!ci_find(cu, B, CT, DCH_MIN, blockIdx.x, &b, &c)) return;
+    const int h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int row0 = cu[b] + c * CT, m = min(CT, cu[b + 1] - row0);
+    const size_t ch = (size_t)blockIdx.x * H + h;
+    const int LD = D + 4, LDP = 64 * NC + 4, D4 = D >> 2;
+    float* R = sm;                                                // [64][LD]
+    float* S = R + CT * LD;                                       // [D][LDP]
+    for (int i = tid; i < CT * D4; i += 256) {
+        const int t = i / D4, d = 4 * (i - t * D4);
+        dc_st4(R + t * LD + d, dc_ld4(rdec + ch * CT * D + 4 * i));
+    }
+    for (int i = tid; i < D * 16 * NC; i += 256) {
+        const int d = i / (16 * NC), p = 4 * (i - d * 16 * NC);
+        dc_st4(S + d * LDP + p, p < P ? dc_ld4(start + (ch * D + d) * P + p) : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    float4 acc[NC][4];
+#pragma unroll
+    for (int e = 0; e < NC; ++e)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            acc[e][i] = 64 * e + 4 * tx < P ? dc_ld4(inner + (ch * CT + 4 * ty + i) * P + 64 * e + 4 * tx) : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < NC; ++e) dc_product(acc[e], R + 4 * ty * LD, LD, S + 64 * e + 4 * tx, LDP, D);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = 4 * ty + i;
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < NC; ++e) ss += acc[e][i].x * acc[e][i].x + acc[e][i].y * acc[e][i].y + acc[e][i].z * acc[e][i].z + acc[e][i].w * acc[e][i].w;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);      // (columns behind P are zero)
+        const float inv = 1.f / sqrtf(ss / (float)P + eps);
+        if (t >= m) continue;
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+            const int p = 64 * e + 4 * tx;
+            if (p >= P) continue;
+            const float4 a = acc[e][i], w = dc_ld4(norm + (size_t)h * P + p), z = Quad<TP>::load(gate + (size_t)(row0 + t) * ld + gate_col + (size_t)h * P + p);
+            Quad<TP>::store(out + (size_t)(row0 + t) * H * P + (size_t)h * P + p,
+                            make_float4(a.x * inv * w.x * (z.x / (1.f + expf(-z.x))), a.y * inv * w.y * (z.y / (1.f + expf(-z.y))),
+                                        a.z * inv * w.z * (z.z / (1.f + expf(-z.z))), a.w * inv * w.w * (z.w / (1.f + expf(-z.w)))));
+        }
+    }
+}
+
+extern "C" int vl_decay_min_chunk() { return DCH_MIN; }
+// Floats of scratch for a launch of up to `chunks` chunks.
+extern "C" long long vl_decay_chunk_floats(int chunks, int H, int D, int P) {
+    return (long long)chunks * H * (2ll * D * P + (long long)CT * (D + P) + D);
+}
+
+// r, k, v, w: columns rc .. of rows ldr wide and so on (float32).  `chunks`: at least the chunks of all portions of DCH_MIN tokens and
+// more; requests that bring fewer are left alone.  state rows as vl_decay_scan's, described by lay_* (vl_decay_scan: rows a lane, lanes a
+// column, columns a block, blocks a head); gate and out of `dtype`, norm float32 [H * P].
+extern "C" int vl_decay_chunks(const float* rp, int ldr, int rc, const float* kp, int ldk, int kc, const float* vp, int ldv, int vc,
+                               const float* wp, int ldw, int wc, const float* u, float* state, long long state_stride, int lay_rows,
+                               int lay_lanes, int lay_cols, int lay_tiles, const int* cu, const int* slots, int B, int chunks, float* scratch,
+                               const void* gate, int dtype, int ldg, int gate_col, const float* norm, float eps, void* out, int H, int D,
+                               int P, void* stream) {
+    if (B <= 0 || chunks <= 0) return VL_OK;
+    if (H <= 0 || D <= 0 || P <= 0 || D > DCH_MAX || P > DCH_MAX || D % 4 || P % 4) return VL_ERR_UNSUPPORTED;
+    if (rc < 0 || kc < 0 || vc < 0 || wc < 0 || gate_col < 0 || rc + H * D > ldr || kc + H * D > ldk || vc + H * P > ldv || wc + H * D > ldw ||
+        gate_col + H * P > ldg || !gate || !norm || !scratch || lay_rows <= 0 || lay_lanes <= 0 || lay_cols <= 0 || lay_tiles <= 0 ||
+        lay_rows * lay_lanes < D || lay_cols * lay_tiles < P || H > 65535 || B > 65535)
+        return VL_ERR_ARGUMENT;
+    if (((ldr | rc | ldk | kc | ldv | vc | ldw | wc | ldg | gate_col) & 3) ||
+        (((uintptr_t)rp | (uintptr_t)kp | (uintptr_t)vp | (uintptr_t)wp | (uintptr_t)u | (uintptr_t)scratch | (uintptr_t)gate | (uintptr_t)norm |
+          (uintptr_t)out) & 15))
+        return VL_ERR_UNSUPPORTED;
+    const size_t n = (size_t)chunks * H;
+    float* added = scratch;
+    float* start = added + n * D * P;
+    float* rdec = start + n * D * P;
+    float* inner = rdec + n * CT * D;
+    float* keep = inner + n * CT * P;
+    const int LD = D + 4;
+    const ScanLayout lay = {lay_rows, lay_lanes, lay_cols, lay_tiles};
+    cudaStream_t s = (cudaStream_t)stream;
+    const size_t prep = sizeof(float) * CT * ((size_t)3 * LD + (LD > DCH_LDA ? LD : DCH_LDA) + DCH_LDA);
+    cudaError_t e = cudaFuncSetAttribute(decay_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
+    if (e != cudaSuccess) return (int)e;
+    int rcode = vl_launch(decay_prep_kernel, dim3(chunks, H), dim3(256), prep, s, DecayRows{rp, ldr, rc}, DecayRows{kp, ldk, kc}, DecayRows{vp, ldv, vc},
+                          DecayRows{wp, ldw, wc}, u, cu, B, added, rdec, inner, keep, H, D, P);
+    if (rcode) return rcode;
+    rcode = vl_launch(decay_chain_kernel, dim3((H * D * (P / 4) + 255) / 256, B), dim3(256), 0, s, (const float*)added, (const float*)keep, start,
+                      state, state_stride, cu, slots, lay, H, D, P);
+    if (rcode) return rcode;
+    auto outputs = [&](auto kernel, auto* g, auto* o, int nc) {
+        const size_t smem = sizeof(float) * ((size_t)CT * LD + (size_t)D * (64 * nc + 4));
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err != cudaSuccess) return (int)err;
+        return vl_launch(kernel, dim3(chunks, H), dim3(256), smem, s, (const float*)rdec, (const float*)start, (const float*)inner, g, ldg, gate_col,
+                         norm, eps, cu, B, o, H, D, P);
+    };
+    if (dtype == VL_BF16)
+        return P <= 64 ? outputs(decay_out_kernel<bf16, 1>, (const bf16*)gate, (bf16*)out, 1) : outputs(decay_out_kernel<bf16, 2>, (const bf16*)gate, (bf16*)out, 2);
+    if (dtype == VL_F32)
+        return P <= 64 ? outputs(decay_out_kernel<float, 1>, (const float*)gate, (float*)out, 1) : outputs(decay_out_kernel<float, 2>, (const float*)gate, (float*)out, 2);
+    return VL_ERR_UNSUPPORTED;
+}

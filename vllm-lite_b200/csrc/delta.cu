@@ -22,6 +22,7 @@
 // L is summed in double precision and kept as two floats, so that differences of it are exact however far it has fallen.
 // The order of every sum depends on the sizes and on the place in the portion alone, not on what else the launch holds.
 #include "tc5.cuh"
+#include "chunk_index.cuh"
 
 #define DC 64                         // tokens of a chunk
 #define DELTA_MIN_CHUNK 16            // portions of fewer tokens are walked token by token
@@ -274,40 +275,8 @@ extern "C" int vl_delta_step(const float* qkv, int C, const void* proj, int dtyp
 }
 
 // ------------------------------------------------------------------------------------------ chunks: which is whose
-__device__ __forceinline__ int dl_chunks_of(const int* cu, int b, int B) {
-    const int n = b < B ? cu[b + 1] - cu[b] : 0;
-    return n >= DELTA_MIN_CHUNK ? (n + DC - 1) / DC : 0;
-}
-// Chunk number `idx` of the launch: request b and its chunk c.  Called by whole warps; false beyond the last chunk.
-__device__ __forceinline__ bool dl_find(const int* cu, int B, int idx, int* b, int* c) {
-    const int lane = threadIdx.x & 31;
-    int base = 0;
-    for (int b0 = 0; b0 < B; b0 += 32) {
-        const int k = dl_chunks_of(cu, b0 + lane, B);
-        int x = k;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, x, 31);
-        if (idx < base + total) {
-            const int src = __ffs(__ballot_sync(0xffffffffu, base + x > idx)) - 1;
-            *b = b0 + src;
-            *c = idx - base - __shfl_sync(0xffffffffu, x - k, src);
-            return true;
-        }
-        base += total;
-    }
-    return false;
-}
-__device__ __forceinline__ int dl_first_chunk(const int* cu, int b) {       // chunks of the requests before b; by whole warps
-    int k = 0;
-    for (int i = threadIdx.x & 31; i < b; i += 32) k += dl_chunks_of(cu, i, b);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-    return k;
-}
+__device__ __forceinline__ bool dl_find(const int* cu, int B, int idx, int* b, int* c) { return ci_find(cu, B, DC, DELTA_MIN_CHUNK, idx, b, c); }
+__device__ __forceinline__ int dl_first_chunk(const int* cu, int b) { return ci_first(cu, b, DC, DELTA_MIN_CHUNK); }
 // Buffers of a chunk and head (number i = chunk * H + head): Wt [D][64], Ut [P][64] (right sides solved, token index last),
 // M [64][64], rows [3][64] (factor of q rows, factor of k rows, e^(L_64) in the first place), S0 [D][P].
 #define DL_ROWS 3

@@ -66,7 +66,10 @@ _SIGNATURES = {
                                             c_void_p, c_int, c_int, c_int, c_void_p],
     ("recurrent", "vl_decay_scan"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                      c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int,
-                                     c_int, c_int, c_void_p],
+                                     c_int, c_int, c_int, c_void_p],
+    ("decay_chunks", "vl_decay_chunks"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+                                          c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                                          c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     ("recurrent", "vl_decay_from_raw"): [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
     ("rope_cache", "vl_conv_rows_norm_rope_write"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p,
                                                      c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float,
@@ -1748,10 +1751,11 @@ def decay_from_raw(z, col, w0):
     return z
 
 
-def decay_scan(r, k, v, w, u, state, state_off, cu, slots, o, H, D, P):
+def decay_scan(r, k, v, w, u, state, state_off, cu, slots, o, H, D, P, longest=None):
     """Per head a memory S [D, P] with a decay per key channel: o_t = (S + diag(u) k_t v_t^T)^T r_t, then
     S <- diag(w_t) S + k_t v_t^T.  r, k, w: (tensor [T, ld], first column) with H*D columns, v likewise with H*P, all of
-    one dtype; u float32 [H*D] (the bonus of the current token); o float32 [T, H*P]; the state as `decay_state_floats(H, D, P)`."""
+    one dtype; u float32 [H*D] (the bonus of the current token); o float32 [T, H*P]; the state as `decay_state_floats(H, D, P)`.
+    `longest`: requests that bring more tokens are left alone."""
     (rt, rc), (kt, kc), (vt, vc), (wt, wc) = r, k, v, w
     for t, n in ((rt, "r"), (kt, "k"), (vt, "v"), (wt, "w")):
         _need(t, rt.dtype, n, 2)
@@ -1763,8 +1767,52 @@ def decay_scan(r, k, v, w, u, state, state_off, cu, slots, o, H, D, P):
     sp, stride = _state_args(state, state_off, decay_state_floats(H, D, P))
     _check(_fn("recurrent", "vl_decay_scan")(_ptr(rt), rt.shape[1], int(rc), _ptr(kt), kt.shape[1], int(kc), _ptr(vt), vt.shape[1],
                                              int(vc), _ptr(wt), wt.shape[1], int(wc), dtype_code(rt.dtype), _ptr(u), sp,
-                                             stride, _ptr(cu), _ptr(slots), B, _ptr(o), H, D, P, _stream()), "vl_decay_scan")
+                                             stride, _ptr(cu), _ptr(slots), B, _ptr(o), H, D, P, int(longest or 0), _stream()), "vl_decay_scan")
     return o
+
+
+DECAY_CHUNK, DECAY_MIN_CHUNK, DECAY_MAX = 64, 96, 128
+
+
+def decay_chunks_ok(D, P) -> bool:
+    """Whether `decay_chunks` takes states of D x P numbers a head."""
+    return 0 < D <= DECAY_MAX and 0 < P <= DECAY_MAX and D % 4 == 0 and P % 4 == 0
+
+
+def decay_chunks_of(counts) -> int:
+    """Chunks of 64 tokens of the requests that bring DECAY_MIN_CHUNK tokens or more (`counts`: tokens per request)."""
+    return sum(-(-n // DECAY_CHUNK) for n in counts if n >= DECAY_MIN_CHUNK)
+
+
+def decay_chunk_floats(chunks, H, D, P) -> int:
+    """Floats of `decay_chunks`' scratch."""
+    return chunks * H * (2 * D * P + DECAY_CHUNK * (D + P) + D)
+
+
+def decay_chunks(r, k, v, w, u, state, state_off, cu, slots, chunks, scratch, gate, gate_col, norm, eps, out, H, D, P):
+    """What `decay_scan` and then `gate_norm` (parts of P columns, a silu gate behind the norm) do, for the requests that bring
+    DECAY_MIN_CHUNK tokens or more, in chunks of 64 tokens; the others' rows and states are left alone.  r, k, v, w float32;
+    `chunks`: at least `decay_chunks_of` the step; scratch float32 [decay_chunk_floats]; gate and out of one dtype."""
+    (rt, rc), (kt, kc), (vt, vc), (wt, wc) = r, k, v, w
+    for t, n in ((rt, "r"), (kt, "k"), (vt, "v"), (wt, "w")):
+        _need(t, torch.float32, n, 2)
+    _need(u, torch.float32, "u", 1); _need(norm, torch.float32, "norm", 1); _need(scratch, torch.float32, "scratch", 1)
+    _need(gate, None, "gate", 2); _need(out, gate.dtype, "out", 2)
+    T = rt.shape[0]
+    if any(t.shape[0] != T for t in (kt, vt, wt, gate)) or out.shape != (T, H * P) or u.shape[0] != H * D or norm.shape[0] != H * P:
+        raise KernelError("decay_chunks: shapes disagree")
+    if not decay_chunks_ok(D, P) or scratch.numel() < decay_chunk_floats(chunks, H, D, P):
+        raise KernelError(f"decay_chunks: heads of {D} x {P} not taken, or too little scratch for {chunks} chunks")
+    B = _seg_args(cu, slots)
+    rows, lanes, cols, tiles = decay_scan_shape(D, P)
+    sp, stride = _state_args(state, state_off, decay_state_floats(H, D, P))
+    _check(_fn("decay_chunks", "vl_decay_chunks")(
+        _ptr(rt), rt.shape[1], int(rc), _ptr(kt), kt.shape[1], int(kc), _ptr(vt), vt.shape[1], int(vc), _ptr(wt), wt.shape[1], int(wc),
+        _ptr(u), sp, stride, rows, lanes, cols, tiles, _ptr(cu), _ptr(slots), B, int(chunks), _ptr(scratch), _ptr(gate),
+        dtype_code(gate.dtype), gate.shape[1], int(gate_col), _ptr(norm), float(eps), _ptr(out), H, D, P, _stream()), "vl_decay_chunks")
+    global launch_count
+    launch_count += 2             # three launches
+    return out
 
 
 GATES = {None: 0, "silu": 1, "sigmoid": 2}

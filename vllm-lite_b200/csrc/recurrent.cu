@@ -1016,13 +1016,13 @@ __global__ void __launch_bounds__(DS_THREADS)
 decay_scan_kernel(const TP* __restrict__ rp, int ldr, int rc, const TP* __restrict__ kp, int ldk, int kc, const TP* __restrict__ vp,
                   int ldv, int vc, const TP* __restrict__ wp, int ldw, int wc, const float* __restrict__ u,
                   float* __restrict__ state, long long state_stride, const int* __restrict__ cu,
-                  const int* __restrict__ slots, float* __restrict__ o, int H, int D, int P, int chunk, int DP) {
+                  const int* __restrict__ slots, float* __restrict__ o, int H, int D, int P, int chunk, int DP, int longest) {
     extern __shared__ __align__(16) float sm[];
     pdl_launch_dependents();
     pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y;
     const int s0 = cu[b], n = cu[b + 1] - s0;
-    if (n <= 0) return;
+    if (n <= 0 || n > longest) return;
     constexpr int NT = DS_THREADS, CT = NT / L;
     const int tid = threadIdx.x;
     const int col = tid / L, l = tid % L;
@@ -1154,11 +1154,13 @@ decay_scan_kernel(const TP* __restrict__ rp, int ldr, int rc, const TP* __restri
     for (int i = 0; i < ROWS; ++i) S[(size_t)i * NT] = s[i];
 }
 
+// `longest`: requests that bring more tokens are left alone (csrc/decay_chunks.cu serves them); 0: none is.
 extern "C" int vl_decay_scan(const void* rp, int ldr, int rc, const void* kp, int ldk, int kc, const void* vp, int ldv, int vc,
                              const void* wp, int ldw, int wc, int dtype, const float* u, float* state,
                              long long state_stride, const int* cu, const int* slots, int B, float* o, int H, int D, int P,
-                             void* stream) {
+                             int longest, void* stream) {
     if (B <= 0) return VL_OK;
+    if (longest <= 0) longest = 0x7fffffff;
     if (H <= 0 || D <= 0 || P <= 0 || rc < 0 || kc < 0 || vc < 0 || wc < 0 || rc + H * D > ldr || kc + H * D > ldk ||
         vc + H * P > ldv || wc + H * D > ldw)
         return VL_ERR_ARGUMENT;
@@ -1180,7 +1182,7 @@ extern "C" int vl_decay_scan(const void* rp, int ldr, int rc, const void* kp, in
     cudaStream_t s = (cudaStream_t)stream;
 #define DS_LAUNCH1(TP, RR, LL, FF)                                                                                              \
     return vl_launch(decay_scan_kernel<TP, RR, LL, FF>, grid, dim3(DS_THREADS), smem, s, (const TP*)rp, ldr, rc, (const TP*)kp, \
-                     ldk, kc, (const TP*)vp, ldv, vc, (const TP*)wp, ldw, wc, u, state, state_stride, cu, slots, o, H, D, P, chunk, DP)
+                     ldk, kc, (const TP*)vp, ldv, vc, (const TP*)wp, ldw, wc, u, state, state_stride, cu, slots, o, H, D, P, chunk, DP, longest)
 #define DS_LAUNCH(TP, RR, LL)            \
     do {                                 \
         if (fast) DS_LAUNCH1(TP, RR, LL, true); \

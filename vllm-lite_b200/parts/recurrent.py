@@ -263,7 +263,7 @@ class TimeMix:
 
     token shifts (one kernel, five mixes) -> W_r, W_k, W_v, W_g, W_w1 each on its own mix -> tanh -> W_w2 -> the decays
     exp(-exp(z + w0)) in place (`ops.decay_from_raw`) -> the scan (`ops.decay_scan`) -> RMS norm per head,
-    weight, silu gate (`ops.gate_norm`) -> W_o.  The state of a request is one row of float32: the input row of its last
+    weight, silu gate (`ops.gate_norm`) -> W_o; long portions of bfloat16 steps: scan, norm and gate in chunks (`ops.decay_chunks`).  The state of a request is one row of float32: the input row of its last
     token, then the heads' memories in the scan's own layout.  r, k, v and the raw decay leave their products in float32
     (the products add in float32 anyway), so nothing that enters the recurrence is rounded to the model's dtype."""
     graph_safe = True
@@ -314,8 +314,17 @@ class TimeMix:
         low = self.w1(mixes[4], step, "tm.w1")
         low = ops.unary_act(low, ws.get(tag + "tm.w1t", tuple(low.shape), low.dtype), "tanh")
         w = ops.decay_from_raw(self.w2(low, step, "tm.w2", out_dtype=f32), 0, self.w0)
-        o = ws.get(tag + "tm.o", (T, H * D), f32)
-        ops.decay_scan((r, 0), (k, 0), (v, 0), (w, 0), self.u, cache.state, W, step.cu_seqlens, step.state_slots, o, H, D, D)
         gated = ws.get(tag + "tm.gated", (T, H * D), self.dtype)
-        ops.gate_norm(o, g, 0, "silu", False, self.norm, s.eps, gated, D)
+        # bfloat16 steps work long portions off in chunks (float32 as the walk, but the order of the sums follows the cut, which the
+        # float32 engine's results must not); the walk serves the others and is then told to leave the long ones alone
+        counts = [e.count for e in step.entries]
+        chunks = ops.decay_chunks_of(counts) if self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D) else 0
+        scan = (r, 0), (k, 0), (v, 0), (w, 0), self.u, cache.state, W, step.cu_seqlens, step.state_slots
+        if not chunks or min(counts) < ops.DECAY_MIN_CHUNK:
+            o = ws.get(tag + "tm.o", (T, H * D), f32)
+            ops.decay_scan(*scan, o, H, D, D, longest=ops.DECAY_MIN_CHUNK - 1 if chunks else None)
+            ops.gate_norm(o, g, 0, "silu", False, self.norm, s.eps, gated, D)
+        if chunks:                                       # (after the norm of all rows, of which the long portions' mean nothing)
+            scratch = ws.get(tag + "tm.chunks", (ops.decay_chunk_floats(chunks, H, D, D),), f32)
+            ops.decay_chunks(*scan, chunks, scratch, g, 0, self.norm, s.eps, gated, H, D, D)
         return self.o_proj(gated, step, "tm.out")
