@@ -46,8 +46,15 @@ class CacheStorage:
     def zero_slots(self, slots):
         if not slots:
             return
+        runs = []                                    # of neighbouring slots: a fill each, and no list of indices to upload (which waits)
+        for s in sorted(slots):
+            if runs and runs[-1][1] == s:
+                runs[-1][1] = s + 1
+            else:
+                runs.append([s, s + 1])
         for t in self.state:
-            t[:, slots] = 0
+            for lo, hi in runs:
+                t[:, lo:hi].zero_()
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in self.paged + self.state)

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import PagedKV
 from .base import sub_weights
 from .linear import Linear
@@ -284,7 +285,6 @@ class GqaAttention:
 
     def _call_with_options(self, h, step, cache):
         """project (q | k | v | gate) -> head work -> attention with the score options -> output gate -> output projection."""
-        from ..csrc import ops
         from . import attention_dispatch
         s, ts = self.spec, self.true_spec
         group = step.groups[cache.group]
@@ -321,7 +321,6 @@ class GqaAttention:
         return self.o_proj(out, step, "attn.o")
 
     def __call__(self, h, step, cache, sink=None):
-        from ..csrc import ops
         if self.with_options:
             return self._call_with_options(h, step, cache)
         s = self.spec

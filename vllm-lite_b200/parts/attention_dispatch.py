@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .base import QUERY_TILE
 
 
@@ -27,7 +28,6 @@ def folds_head_work(dtype, step, spec, group, num_tokens) -> bool:
     block-per-chunk kernel serves with few chunks per token (every chunk's block prepares the query heads
     again).  Measured at Qwen3-8B sizes, a step with / without: batch 8 at 4,096 keys (4 chunks) 3.77 / 3.79 ms,
     batch 16 at 1,024 keys (1 chunk) 3.99 / 4.06; batch 4 (8 chunks) 3.635 / 3.61, batch 1 (16 chunks) 3.07 / 3.065."""
-    from ..csrc import ops
     if not (ops.flash_supported(dtype, spec.head_dim) and step.max_query_len == 1):
         return False
     if ops.flash_decode_streams(dtype, num_tokens, spec.num_kv_heads, spec.head_dim, group.page_size, group.max_context):
@@ -91,7 +91,6 @@ def run(qkv, out, cache, group, step, spec, scale, fold=None, sinks=None, weight
     head h's output is multiplied by sigmoid(gate[t, h]).
     `softcap` c: score <- c tanh(score / c); `distance` (a, b), float32 [num_heads] each: a[h] ln(1 + b[h] (i - j)) is
     taken off the score of the key j that query i reads; `keep`: beside the window, the first `keep` keys stay visible."""
-    from ..csrc import ops
     if not spec.window:
         keep = None
     if softcap or distance is not None or keep:

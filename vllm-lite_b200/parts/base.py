@@ -28,6 +28,8 @@ from typing import List, Optional
 
 import torch
 
+from ..csrc import ops
+
 
 @dataclass
 class BuildContext:
@@ -42,17 +44,22 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self._buffers = {}
+        self._views = {}              # the last view handed out of every buffer: the layers of a step ask for the same ones
 
     def get(self, tag: str, shape, dtype) -> torch.Tensor:
+        key = (tag, dtype)
+        last = self._views.get(key)
+        if last is not None and last.shape == shape:
+            return last
         n = 1
         for s in shape:
             n *= int(s)
-        key = (tag, dtype)
         buf = self._buffers.get(key)
         if buf is None or buf.numel() < n:
             buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._buffers[key] = buf
-        return buf[:n].view(*shape)
+        view = self._views[key] = buf[:n].view(*shape)
+        return view
 
     def zeros(self, tag: str, n: int, dtype) -> torch.Tensor:
         """A buffer that is zero when first handed out and that its users leave zero (counters that
@@ -146,7 +153,6 @@ class Residual:
         if self.deferred is not None:
             self.deferred(None)
         if isinstance(self.pending, StreamSum):
-            from ..csrc import ops
             ops.stream_norm(self.x, self.pending)
             self.pending = None
 

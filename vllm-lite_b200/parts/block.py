@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .base import StreamSink, StreamSum, prefixed, sub_weights
 from .registry import BLOCKS, FEED_FORWARDS, MIXERS, NORMS
 from .spec import BlockSpec
@@ -130,7 +131,6 @@ class PostNormBlock:
             return residual.x, None
         buf = step.workspace.get(step.tag + "stream.cast", residual.x.shape, self.dtype)
         if residual.cast is None:
-            from ..csrc import ops
             residual.cast = ops.cast(residual.x, buf)
         return residual.cast, buf
 
@@ -322,7 +322,6 @@ class HyperConnectionBlock:
         return MIXERS.get(spec.mixer.kind).cache_need(spec.mixer)
 
     def __init__(self, spec: BlockSpec, weights: dict, ctx):
-        from ..csrc import ops
         self.spec = spec
         self.dtype = ctx.dtype
         self.streams = int(spec.streams)
@@ -346,7 +345,6 @@ class HyperConnectionBlock:
 
     def _read(self, residual, step, q, pending):
         """h for sub-layer q, after the write-back `pending` = (y, mix, out) of the sub-layer before (or None)."""
-        from ..csrc import ops
         norm = self.norm1 if q == 0 else self.norm2
         in_w = self.hc[q][0]
         T, H = residual.x.shape
@@ -368,7 +366,6 @@ class HyperConnectionBlock:
         return norm(u, None, step, tag=f"hc.norm{q}")
 
     def __call__(self, residual, step, cache):
-        from ..csrc import ops
         if residual.pending is not None or residual.normed is not None:
             raise NotImplementedError("a hyper-connection block after a block that leaves its result pending")
         pending = None
@@ -394,7 +391,6 @@ class _DeferredWriteBack:
         self.residual, self.pending = residual, pending
 
     def __call__(self, _next=None):
-        from ..csrc import ops
         r = self.residual
         y, mix, out_w = self.pending
         ops.hc_step(r.streams, y=y, mix=mix, out_w=out_w, total=r.x)

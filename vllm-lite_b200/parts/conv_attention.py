@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import FixedState, PagedKV, Several
 from .linear import Linear
 from .registry import MIXERS, POSITIONS
@@ -61,7 +62,6 @@ class ConvAttention:
         return Several((pages, FixedState((max((s.conv - 1) * (Cq + Ck), 1),))))
 
     def __init__(self, s: ConvAttentionSpec, weights: dict, ctx):
-        from ..csrc import ops
         Cq, Ck, pd = self._sizes(s)
         if s.num_heads <= 0 or s.num_kv_heads <= 0 or s.num_heads % s.num_kv_heads:
             raise ValueError(f"{s.num_kv_heads} kv heads do not divide {s.num_heads} query heads")
@@ -113,7 +113,6 @@ class ConvAttention:
         return bias
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         from . import attention_dispatch
         s, ws, tag = self.spec, step.workspace, step.tag
         pages, conv_state = cache.parts[0], cache.parts[1]

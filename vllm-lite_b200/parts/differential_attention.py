@@ -17,6 +17,7 @@ import math
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import PagedKV
 from .attention import MAX_HEAD_DIM, _pad_heads, neighbour_order, round_up
 from .linear import Linear
@@ -105,7 +106,6 @@ class DifferentialAttention:
         self.kernel_heads = _KernelHeads(nq * MAPS, nkv, self.P, s.window)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         from . import attention_dispatch
         s, ws, tag = self.spec, step.workspace, step.tag
         group = step.groups[cache.group]

@@ -11,6 +11,7 @@ An embedding part offers
 and may say `graph_safe = True` (parts/base.py)."""
 from __future__ import annotations
 
+from ..csrc import ops
 from ..cache.spec import FixedState
 from .registry import EMBEDDINGS
 from .spec import EmbeddingSpec, PairEmbeddingSpec, TensorDecl
@@ -32,7 +33,6 @@ class TokenEmbedding:
         return self.table
 
     def __call__(self, step, x):
-        from ..csrc import ops
         return ops.embed(step.tokens, self.table, x, step.err, self.spec.scale)     # an id outside the table is flagged, not read
 
 
@@ -61,7 +61,6 @@ class PairEmbedding:
         return self.table
 
     def __call__(self, step, x, cache):
-        from ..csrc import ops
         s = self.spec
         return ops.embed_pair(step.tokens, self.table, self.pairs, x, s.scale, s.buckets, s.mul_prev, s.mul_cur, cache.state,
                               step.cu_seqlens, step.state_slots, step.req_index, step.positions, step.err)

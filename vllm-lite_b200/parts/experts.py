@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .base import prefixed, sub_weights
 from .registry import FEED_FORWARDS
 from .spec import RoutedExpertsSpec, TensorDecl
@@ -62,7 +63,6 @@ class RoutedExperts:
         return d
 
     def __init__(self, spec: RoutedExpertsSpec, weights: dict, ctx):
-        from ..csrc import ops
         outputs = spec.num_experts + spec.identity           # what the router chooses from
         if spec.identity < 0 or spec.num_experts < 1 or not 0 < spec.top <= outputs:
             raise ValueError(f"routed experts: top {spec.top} of {spec.num_experts} + {spec.identity} experts")
@@ -120,7 +120,6 @@ class RoutedExperts:
         self.down = torch.stack([weights[p + down] for p in names]).contiguous()          # [E, H, I]
 
     def __call__(self, h, step):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         T, E, top, I, H = h.shape[0], s.num_experts, s.top, s.intermediate_size, s.hidden_size
         pairs = T * top

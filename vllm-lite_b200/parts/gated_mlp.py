@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .linear import Linear
 from .registry import FEED_FORWARDS
 from .spec import GatedMlpSpec, TensorDecl
@@ -37,7 +38,6 @@ class GatedMlp:
         return d
 
     def __init__(self, spec: GatedMlpSpec, weights: dict, ctx):
-        from ..csrc import ops
         known = ops.ACTIVATIONS if spec.gated else tuple(ops.UNARY_ACTIVATIONS) + ("poly_norm",)
         if spec.activation not in known or (spec.bias and not spec.gated):
             raise ValueError(f"gated_mlp: activation {spec.activation!r} ({'with' if spec.gated else 'without'} a gate); "
@@ -63,7 +63,6 @@ class GatedMlp:
         self.down = Linear(weights[down], weights[down + b].float() if spec.bias else None)
 
     def __call__(self, h, step):
-        from ..csrc import ops
         gu = self.gate_up(h, step, "mlp.gate_up")
         act = step.workspace.get(step.tag + "mlp.act", (gu.shape[0], self.spec.intermediate_size), gu.dtype)
         s = self.spec

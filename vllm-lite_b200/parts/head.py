@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .linear import Linear
 from .registry import HEADS
 from .spec import CappedHeadSpec, HeadSpec, TensorDecl
@@ -51,6 +52,5 @@ class CappedHead:
         self.proj = Linear(weights[spec.tensor])
 
     def __call__(self, h, step):
-        from ..csrc import ops
         logits = self.proj(h, step, "logits", out_dtype=torch.float32)
         return ops.scale_softcap(logits, self.spec.scale, self.spec.softcap)

@@ -37,6 +37,7 @@ from collections import namedtuple
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import PagedLatent
 from .linear import Linear, stacked
 from .registry import MIXERS
@@ -155,7 +156,6 @@ class LatentAttention:
         self.layout = HeadLayout(H, 1, self.rank, spec.window, True)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         from . import attention_dispatch
         s, ws, tag = self.spec, step.workspace, step.tag
         T = h.shape[0]

@@ -10,6 +10,8 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
+from . import matmul
 from .base import ScaledRows, StreamSink
 
 
@@ -37,13 +39,11 @@ class Linear:
     def factors_norms(self, M) -> bool:
         """Whether, for M rows, this layer's kernel can take an RMS norm's output in factored form
         (`ScaledRows`) and can add its result into the stream (`into_stream`)."""
-        from ..csrc import ops
         return (self.bias is None and self.weight.dtype == torch.bfloat16
                 and ops.gemm_bf16_small_m_ok(M, self.in_features))
 
     def into_stream(self, a, sink: StreamSink, step, tag) -> ScaledRows:
         """sink.x += a W^T; returns the next norm's output on the new stream, in factored form."""
-        from ..csrc import ops
         M = a.shape[0]
         ws = step.workspace
         rows = ws.get(step.tag + tag + ".rows", (M, self.out_features), torch.bfloat16)
@@ -55,8 +55,6 @@ class Linear:
         """silu(gate) * up of y = a W^T, W holding gate and up rows (interleaved in blocks of `group`
         rows, or gate rows then up rows when group is 0): [M, out_features / 2].  The activation runs
         inside the product kernel when that kernel can, else in a kernel of its own."""
-        from ..csrc import ops
-        from . import matmul
         if self.bias is not None and group:
             raise ValueError("the fused gate/up layout has no bias; stack gate and up as plain halves (group 0)")
         if isinstance(a, ScaledRows):
@@ -77,13 +75,10 @@ class Linear:
     def __call__(self, a, step, tag, out_dtype=None):
         y = self._product(a, step, tag, out_dtype)
         if self.bias is not None:
-            from ..csrc import ops
             ops.add_bias(y, self.bias)
         return y
 
     def _product(self, a, step, tag, out_dtype=None):
-        from ..csrc import ops
-        from . import matmul
         if isinstance(a, ScaledRows):
             M = a.rows.shape[0]
             if not self.factors_norms(M):

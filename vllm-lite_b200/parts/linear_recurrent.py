@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import FixedState
 from .linear import Linear
 from .registry import MIXERS
@@ -47,7 +48,6 @@ class MinGru:
         self.biases = tuple(_f32(weights[n + s.bias_suffix], ctx) for n in (z, x))
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         proj = self.in_proj(h, step, "mg.in")
         out = step.workspace.get(step.tag + "mg.out", (h.shape[0], self.spec.width), self.dtype)
         ops.linear_scan("min_gru", proj, self.biases, cache.state, 0, step.cu_seqlens, step.state_slots, out,
@@ -87,7 +87,6 @@ class GatedLru:
         self.decay = _f32(-float(s.rate) * torch.nn.functional.softplus(weights[lam].double()), ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         T, C = h.shape[0], s.width
         proj = self.in_proj(h, step, "lru.in")                                               # [y | x]

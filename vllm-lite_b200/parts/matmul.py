@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
+
 # The library product must add in float32 whatever the shape: with this switch left on (torch's default)
 # cuBLAS may pick kernels that cut K among blocks and add the pieces in bfloat16, and a row's result
 # could then depend on how many rows share its step.
@@ -17,14 +19,12 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 def fuses_swiglu(M, K) -> bool:
     """Whether the product for M rows runs in a kernel that can apply SwiGLU to its own tile."""
-    from ..csrc import ops
     return ops.gemm_bf16_small_m_ok(M, K) or ops.gemm_bf16_tc5_ok(M, K, fused=True)
 
 
 def gemm_bf16(a, w, out, err=None, swiglu=False):
     """swiglu (only where `fuses_swiglu`): w interleaves 8 gate rows with their 8 up rows and out is
     [M, N/2] = silu(gate) * up."""
-    from ..csrc import ops
     M, K = a.shape
     if ops.gemm_bf16_small_m_ok(M, K):
         return ops.gemm_bf16_small_m(a, w, out, err, swiglu)

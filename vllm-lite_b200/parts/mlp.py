@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .linear import Linear
 from .registry import FEED_FORWARDS
 from .spec import SwiGLUSpec, TensorDecl
@@ -40,7 +41,6 @@ class SwiGLU:
 
     def factors_norms(self, M) -> bool:
         """For M rows: the input may come as `ScaledRows` and the result may go `into_stream`."""
-        from ..csrc import ops
         return self.group == ops.SWIGLU_GROUP and self.gate_up.factors_norms(M) and self.down.factors_norms(M)
 
     def __call__(self, h, step, sink=None):

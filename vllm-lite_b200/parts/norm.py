@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from .registry import NORMS
 from .spec import NormSpec, TensorDecl
 
@@ -40,7 +41,6 @@ class RmsNorm:
     def add_normed(self, y, x, step, cast=None, mult=1.0, bias=None):
         """x += mult * norm(y + bias): what a block that norms its sub-layers' OUTPUTS calls; `cast` (a buffer in the
         activation dtype, or None) receives the new x.  y may be a `ScaledPair`.  Returns cast."""
-        from ..csrc import ops
         from .base import ScaledPair
         if isinstance(y, ScaledPair):
             if y.a_weight is not None and y.eps != self.spec.eps:
@@ -59,7 +59,6 @@ class RmsNorm:
     takes_sum = True           # `delta` may be a `StreamSum`: the kernel forms the stream's new values as it reads
 
     def __call__(self, x, delta, step, rows=None, tag="norm"):
-        from ..csrc import ops
         from .base import StreamSum
         R = x.shape[0] if rows is None else rows.shape[0]
         out = step.workspace.get(step.tag + tag, (R, self.spec.size), self.dtype)
@@ -85,14 +84,12 @@ class LayerNorm:
 
     def add_normed(self, y, x, step, cast=None, mult=1.0):
         """x += norm(y); `cast` (a buffer in the activation dtype, or None) receives the new x.  Returns cast."""
-        from ..csrc import ops
         if mult != 1.0:
             raise NotImplementedError("the layer norm's kernel adds its result as it is")
         ops.layernorm_add(y, self.weight, self.spec.eps, x, cast)
         return cast
 
     def __call__(self, x, delta, step, rows=None, tag="norm"):
-        from ..csrc import ops
         if delta is not None:
             raise NotImplementedError("the layer norm takes the stream as it is; a pending delta belongs to a pre-norm block")
         R = x.shape[0] if rows is None else rows.shape[0]
@@ -124,7 +121,6 @@ class DynTanh:
         return self.alpha, self.weight, self.bias
 
     def __call__(self, x, delta, step, rows=None, tag="norm"):
-        from ..csrc import ops
         R = x.shape[0] if rows is None else rows.shape[0]
         out = step.workspace.get(step.tag + tag, (R, self.spec.size), self.dtype)
         return ops.dyt_rows(x, delta, rows, self.alpha, self.weight, self.bias, out)

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import Several
 from .base import prefixed, sub_weights
 from .registry import MIXERS, NORMS
@@ -56,7 +57,6 @@ class ParallelMixer:
         return total
 
     def __call__(self, h, step, cache, as_pair=False):
-        from ..csrc import ops
         a = self.left(h, step, cache.parts[0])
         b = self.right(h, step, cache.parts[1])
         if as_pair:

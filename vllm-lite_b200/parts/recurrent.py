@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import FixedState
 from .linear import Linear, stacked
 from .registry import MIXERS
@@ -44,11 +45,9 @@ class StateSpace:
     @staticmethod
     def cache_need(s: StateSpaceSpec):
         inner, conv_ch, _ = StateSpace._sizes(s)
-        from ..csrc import ops
         return FixedState(((s.conv - 1) * conv_ch + ops.scan_state_floats(s.num_heads, s.state, s.vdim),))
 
     def __init__(self, s: StateSpaceSpec, weights: dict, ctx):
-        from ..csrc import ops
         if s.num_heads % s.groups or (s.num_heads * s.vdim) % s.norm_groups or s.conv < 1:
             raise ValueError(f"state space: {s.num_heads} heads in {s.groups} groups, {s.norm_groups} norm parts, {s.conv} taps")
         ops.scan_lanes(s.state)
@@ -61,7 +60,6 @@ class StateSpace:
         self.norm = _f32(weights[norm], ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         inner, conv_ch, width = self._sizes(s)
         T = h.shape[0]
@@ -91,7 +89,6 @@ class MatrixMemory:
 
     @staticmethod
     def cache_need(s: MatrixMemorySpec):
-        from ..csrc import ops
         return FixedState((ops.mlstm_state_floats(s.num_heads, s.dim, s.vdim),))
 
     def __init__(self, s: MatrixMemorySpec, weights: dict, ctx):
@@ -104,7 +101,6 @@ class MatrixMemory:
         self.norm, self.i_b, self.f_b = _f32(weights[norm], ctx), _f32(weights[i_b], ctx), _f32(weights[f_b], ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         H, D, P = s.num_heads, s.dim, s.vdim
         T = h.shape[0]
@@ -139,11 +135,9 @@ class DeltaRule:
 
     @staticmethod
     def cache_need(s: DeltaRuleSpec):
-        from ..csrc import ops
         return FixedState(((s.conv - 1) * DeltaRule._conv_channels(s) + ops.scan_state_floats(s.num_heads, s.dim, s.vdim),))
 
     def __init__(self, s: DeltaRuleSpec, weights: dict, ctx):
-        from ..csrc import ops
         if s.num_heads % s.num_kv_heads or s.conv < 1:
             raise ValueError(f"delta rule: {s.num_kv_heads} key heads do not divide {s.num_heads} heads, or no tap")
         ops.scan_lanes(s.dim)
@@ -162,7 +156,6 @@ class DeltaRule:
         self.a_log, self.dt_bias, self.norm = _f32(weights[a_log], ctx), _f32(weights[dt_bias], ctx), _f32(weights[norm], ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         H, G, D, P = s.num_heads, s.num_kv_heads, s.dim, s.vdim
         C = self._conv_channels(s)
@@ -192,7 +185,6 @@ class HeadDelta:
 
     @staticmethod
     def _state_floats(s) -> int:
-        from ..csrc import ops
         if ops.head_delta_ok(s.dim, s.vdim):
             return s.num_heads * s.dim * s.vdim
         return ops.scan_state_floats(s.num_heads, s.dim, s.vdim)
@@ -216,7 +208,6 @@ class HeadDelta:
         return FixedState(((s.conv - 1) * HeadDelta._conv_channels(s) + HeadDelta._state_floats(s),))
 
     def __init__(self, s: HeadDeltaSpec, weights: dict, ctx):
-        from ..csrc import ops
         if s.num_heads % s.num_kv_heads or s.conv < 1:
             raise ValueError(f"delta rule: {s.num_kv_heads} key heads do not divide {s.num_heads} heads, or no tap")
         ops.scan_lanes(s.dim)
@@ -228,7 +219,6 @@ class HeadDelta:
         self.a_log, self.dt_bias, self.norm = _f32(weights[a_log], ctx), _f32(weights[dt_bias], ctx), _f32(weights[norm], ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         H, G, D, P = s.num_heads, s.num_kv_heads, s.dim, s.vdim
         C = self._conv_channels(s)
@@ -282,11 +272,9 @@ class TimeMix:
 
     @staticmethod
     def cache_need(s: TimeMixSpec):
-        from ..csrc import ops
         return FixedState((s.hidden_size + ops.decay_state_floats(s.num_heads, s.dim, s.dim),))
 
     def __init__(self, s: TimeMixSpec, weights: dict, ctx):
-        from ..csrc import ops
         if s.num_heads <= 0 or s.dim <= 0 or s.decay_rank <= 0:
             raise ValueError(f"time mix: {s.num_heads} heads of {s.dim}, decay rank {s.decay_rank}")
         ops.decay_scan_shape(s.dim, s.dim)
@@ -299,7 +287,6 @@ class TimeMix:
         self.w0, self.u, self.norm = _f32(weights[w0], ctx), _f32(weights[u].reshape(-1), ctx), _f32(weights[norm], ctx)
 
     def __call__(self, h, step, cache):
-        from ..csrc import ops
         s, ws, tag = self.spec, step.workspace, step.tag
         H, D, W = s.num_heads, s.dim, s.hidden_size
         T = h.shape[0]

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc import ops
 from ..cache.spec import FixedState, Several
 from .base import CallCache, prefixed, sub_weights
 from .registry import MIXERS
@@ -52,7 +53,6 @@ class TokenShift:
 
     def __call__(self, x, step, cache):
         """x: the float32 stream [T, hidden]."""
-        from ..csrc import ops
         if self._inner_parts is None:
             own, inner = cache, None
         elif self._inner_parts == 0:
