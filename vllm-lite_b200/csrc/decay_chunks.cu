@@ -13,9 +13,8 @@
 // the middle into one factor of r_t and one of k_s, both running products of numbers below 1, as the walk's own; pairs within 8 tokens
 // multiply their few decays directly.  The products (2,016 pairs x D in a chunk, then 64 x 64 x P, 64 x D x P twice) are plain
 // multiply-adds on tiles in shared memory, which is what bounds (1) and (3).
-// One request of 2,048 tokens, 32 heads of 64 x 64: 137 us with the norm and the gate (89 + 15 + 32), against 413 for the walk and the norm's
-// kernel behind it; 128 x 128: 401 against 1,191; 512 tokens: 37 against 107; 64 tokens: 27 against 18, and of 32 requests of 64 tokens
-// 168 against 230: a lone portion wins from about 100 tokens on.
+// One request of 2,048 tokens, 32 heads of 64 x 64: 119 us with the norm and the gate, against 413 for the walk and the norm's kernel
+// behind it; 128 x 128: 395 against 1,193; 512 tokens: 37 against 107; 64 tokens: 27 against 18: a lone portion wins from about 100 tokens on.
 #include "common.cuh"
 #include "chunk_index.cuh"
 
@@ -64,10 +63,17 @@ __device__ __forceinline__ float dc_chain(const float* x, const float* w, int ld
     return f;
 }
 
+// The i-th pair of tokens (s before t) in different halves of runs of 2 `half` tokens.
+__device__ __forceinline__ void dc_pair(int i, int half, int& t, int& s) {
+    const int seg = i / (half * half), e = i - seg * half * half;
+    t = seg * 2 * half + half + e / half;
+    s = seg * 2 * half + e % half;
+}
+
 #define DCH_LDA (CT + 4)
 // Buffers of chunk and head number i = chunk * H + head: added [D][P], start [D][P] (S at the chunk's start), rdec [64][D], inner [64][P],
 // keep [D].
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const float* __restrict__ u, const int* __restrict__ cu, int B,
                   float* __restrict__ added, float* __restrict__ rdec, float* __restrict__ inner, float* __restrict__ keep, int H, int D, int P) {
     extern __shared__ __align__(16) float sm[];
@@ -81,9 +87,8 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
     const size_t ch = (size_t)blockIdx.x * H + h;
     float* R = sm;                                                // [64][LD], later the values [64][68]
     float* K = R + CT * (LD > DCH_LDA ? LD : DCH_LDA);
-    float* W = K + CT * LD;
-    float* X = W + CT * LD;                                       // r or k times one level's decays
-    float* A = X + CT * LD;                                       // [64][68]
+    float* X = K + CT * LD;                                       // r or k times one level's decays
+    float* W = X + CT * LD;                                       // the decays; when they are used up A [64][68]
     for (int i = tid; i < CT * D4; i += 256) {                    // (tokens behind the portion: nothing added, nothing decayed)
         const int t = i / D4, d = 4 * (i - t * D4);
         const size_t row = row0 + t, at = (size_t)h * D + d;
@@ -93,8 +98,9 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
         dc_st4(K + t * LD + d, in ? dc_ld4(k.p + row * k.ld + k.col + at) : z);
         dc_st4(W + t * LD + d, in ? dc_ld4(w.p + row * w.ld + w.col + at) : one);
     }
-    for (int i = tid; i < CT * DCH_LDA / 4; i += 256) dc_st4(A + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
     __syncthreads();
+    // A's elements stay in registers until the decays' place is free: three blocks fit an SM instead of two (a third of (1)'s time)
+    float far[4], mid[2], close = 0.f, near[8];
     // pairs in different halves of a run of 2 `half` tokens
 #pragma unroll
     for (int half = 32; half >= 8; half >>= 1) {
@@ -117,20 +123,18 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
                 s[1][0] += a1.x * b0.x; s[1][0] += a1.y * b0.y; s[1][0] += a1.z * b0.z; s[1][0] += a1.w * b0.w;
                 s[1][1] += a1.x * b1.x; s[1][1] += a1.y * b1.y; s[1][1] += a1.z * b1.z; s[1][1] += a1.w * b1.w;
             }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) A[(32 + ty + 16 * i) * DCH_LDA + tx + 16 * j] = s[i][j];
+            far[0] = s[0][0]; far[1] = s[0][1]; far[2] = s[1][0]; far[3] = s[1][1];
         } else {
-            const int per = half * half, lh = half == 16 ? 4 : 3;
-            for (int i = tid; i < 32 * half; i += 256) {
-                const int seg = i / per, e = i - seg * per, t = seg * 2 * half + half + (e >> lh), s = seg * 2 * half + (e & (half - 1));
+#pragma unroll
+            for (int n = 0; n < half / 8; ++n) {
+                int t, s;
+                dc_pair(tid + 256 * n, half, t, s);
                 float x = 0.f, y = 0.f;
                 for (int d = 0; d < D; d += 4) {
                     const float4 a = dc_ld4(X + t * LD + d), q = dc_ld4(X + s * LD + d);
                     x += a.x * q.x; y += a.y * q.y; x += a.z * q.z; y += a.w * q.w;
                 }
-                A[t * DCH_LDA + s] = x + y;
+                if (half == 16) mid[n] = x + y; else close = x + y;
             }
         }
         __syncthreads();
@@ -159,7 +163,7 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
 #pragma unroll
             for (int t = s; t < 8; ++t) {
                 const float v = warp_sum(sum[t]);
-                if ((tid & 31) == t) A[(t0 + t) * DCH_LDA + t0 + s] = v;
+                if ((tid & 31) == t) near[s] = v;
             }
         }
     }
@@ -169,6 +173,24 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
         const int d = i < D ? i : i - D;
         if (i < D) keep[ch * D + d] = dc_chain<true>(R + d, W + d, LD, 0, CT, [&](int t, float v) { rdec[(ch * CT + t) * D + d] = v; });
         else dc_chain<false>(K + d, W + d, LD, 0, CT, [&](int t, float v) { X[t * LD + d] = v; });
+    }
+    __syncthreads();
+    float* A = W;
+    for (int i = tid; i < CT * DCH_LDA / 4; i += 256) dc_st4(A + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) A[(32 + ty + 16 * (i >> 1)) * DCH_LDA + tx + 16 * (i & 1)] = far[i];
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+        int t, s;
+        dc_pair(n < 2 ? tid + 256 * n : tid, n < 2 ? 16 : 8, t, s);
+        A[t * DCH_LDA + s] = n < 2 ? mid[n] : close;
+    }
+    if ((tid & 31) < 8) {
+        const int t0 = 8 * (tid >> 5), t = tid & 31;
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            if (s <= t) A[(t0 + t) * DCH_LDA + t0 + s] = near[s];
     }
     for (int p0 = 0; p0 < P; p0 += 64) {                          // 64 columns of the values at a time, in the place of r
         __syncthreads();
@@ -245,7 +267,7 @@ decay_chain_kernel(const float* __restrict__ added, const float* __restrict__ ke
 }
 
 template <typename TP, int NC>                                    // NC: 64 columns of the values a step
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 decay_out_kernel(const float* __restrict__ rdec, const float* __restrict__ start, const float* __restrict__ inner,
                  const TP* __restrict__ gate, int ld, int gate_col, const float* __restrict__ norm, float eps, const int* __restrict__ cu,
                  int B, TP* __restrict__ out, int H, int D, int P) {
@@ -332,7 +354,7 @@ extern "C" int vl_decay_chunks(const float* rp, int ldr, int rc, const float* kp
     const int LD = D + 4;
     const ScanLayout lay = {lay_rows, lay_lanes, lay_cols, lay_tiles};
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t prep = sizeof(float) * CT * ((size_t)3 * LD + (LD > DCH_LDA ? LD : DCH_LDA) + DCH_LDA);
+    const size_t prep = sizeof(float) * CT * ((size_t)2 * LD + 2 * (LD > DCH_LDA ? LD : DCH_LDA));
     cudaError_t e = cudaFuncSetAttribute(decay_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
     if (e != cudaSuccess) return (int)e;
     int rcode = vl_launch(decay_prep_kernel, dim3(chunks, H), dim3(256), prep, s, DecayRows{rp, ldr, rc}, DecayRows{kp, ldk, kc}, DecayRows{vp, ldv, vc},
