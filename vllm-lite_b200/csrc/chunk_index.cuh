@@ -36,3 +36,15 @@ __device__ __forceinline__ int ci_first(const int* cu, int b, int tokens, int le
     for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
     return k;
 }
+// The request with the `rank`-th most tokens (ties: the lower index), so that a launch that walks every request from chunk to chunk begins
+// the longest walks first and the short ones fill up what they leave (more than 32 requests: in their own order).  By whole warps.
+__device__ __forceinline__ int ci_by_length(const int* cu, int B, int rank) {
+    if (B > 32) return rank;
+    const int lane = threadIdx.x & 31, n = lane < B ? cu[lane + 1] - cu[lane] : -1;
+    int ahead = 0;
+    for (int j = 0; j < B; ++j) {
+        const int o = __shfl_sync(0xffffffffu, n, j);
+        ahead += (o > n || (o == n && j < lane)) ? 1 : 0;
+    }
+    return __ffs(__ballot_sync(0xffffffffu, lane < B && ahead == rank)) - 1;
+}

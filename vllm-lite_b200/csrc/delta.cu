@@ -436,6 +436,8 @@ delta_prep_kernel(const float* __restrict__ qkv, int C, const TP* __restrict__ p
 }
 
 // ------------------------------------------------------------------------------------------ (2) from chunk to chunk
+// The longest requests' blocks come first: a block has its SM to itself, and where the launch has more blocks than SMs the short walks
+// then fill what the long ones leave (requests of 1,427, 1,045 and 809 tokens, 16 heads of 128 x 128: 179 us in the requests' order, 150 so).
 // A block owns CT value columns of one head of one request: the state's tile in registers (for its update) and in shared memory
 // (for W S).  U goes to `U` [T][H P], the state at every chunk's start to S0.
 template <int CT>
@@ -448,7 +450,7 @@ delta_walk_kernel(const float* __restrict__ qkv, int C, const float* __restrict_
     extern __shared__ __align__(16) float sm[];
     pdl_launch_dependents();
     pdl_wait();
-    const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * CT;
+    const int h = blockIdx.x, p0 = blockIdx.y * CT, b = ci_by_length(cu, gridDim.z, blockIdx.z);
     const int s0 = cu[b], n = cu[b + 1] - s0;
     if (n < DELTA_MIN_CHUNK) return;
     const int first = dl_first_chunk(cu, b), chunks = (n + DC - 1) / DC;
@@ -972,7 +974,7 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
     extern __shared__ __align__(16) float sm[];
     pdl_launch_dependents();
     pdl_wait();
-    const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * CT;
+    const int h = blockIdx.x, p0 = blockIdx.y * CT, b = ci_by_length(cu, gridDim.z, blockIdx.z);
     const int s0 = cu[b], n = cu[b + 1] - s0;
     if (n < DELTA_MIN_CHUNK) return;
     const int first = dl_first_chunk(cu, b), chunks = (n + DC - 1) / DC;
@@ -1251,7 +1253,7 @@ static int launch_walk(const float* qkv, int C, const float* Wt, const float* Ut
     const size_t smem = sizeof(float) * ((size_t)2 * (2 * D * DC + CT * DC + 2 * DC) + (size_t)D * CT + 2 * DC * CT);
     const int rc = delta_smem(delta_walk_kernel<CT>, smem);
     if (rc) return rc;
-    return vl_launch(delta_walk_kernel<CT>, dim3(H, B, (P + CT - 1) / CT), dim3(256), smem, s, qkv, C, Wt, Ut, rows, U, S0, state, state_stride,
+    return vl_launch(delta_walk_kernel<CT>, dim3(H, (P + CT - 1) / CT, B), dim3(256), smem, s, qkv, C, Wt, Ut, rows, U, S0, state, state_stride,
                      cu, slots, H, G, D, P);
 }
 template <int CT>
@@ -1262,7 +1264,7 @@ static int launch_walk_mma(const float* qkv, int C, const float* W, const float*
                                          + 4 * DC * (CT + 8) + DC * (CT + 4));
     const int rc = delta_smem(delta_walk_mma_kernel<CT>, smem);
     if (rc) return rc;
-    return vl_launch(delta_walk_mma_kernel<CT>, dim3(H, B, (P + CT - 1) / CT), dim3(512), smem, s, qkv, C, W, U0, rows, U, S0, state,
+    return vl_launch(delta_walk_mma_kernel<CT>, dim3(H, (P + CT - 1) / CT, B), dim3(512), smem, s, qkv, C, W, U0, rows, U, S0, state,
                      state_stride, cu, slots, H, G, D, P);
 }
 // MMA false: the kernels of plain float32 multiply-adds (float32 steps), else those on the tensor cores (bfloat16 steps).
