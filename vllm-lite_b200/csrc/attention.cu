@@ -521,8 +521,11 @@ decode_attention_split_kernel(const T* __restrict__ q, int q_stride,
     }
 }
 
+#define MERGE_CHUNKS 128
+#define MERGE_COLUMNS 5        // of a thread of 128: heads of up to 640 numbers
 template <typename T>
-__global__ void decode_attention_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(128)
+decode_attention_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                               const int* __restrict__ positions, T* __restrict__ out,
                                               int nq, int hd, int chunk, int S, int window,
                                               const int* __restrict__ token_index, const float* __restrict__ sinks) {
@@ -541,25 +544,54 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ part_acc
     const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     const int s0 = lo / chunk, s1 = pos / chunk;
     const size_t row0 = ((size_t)t * nq + h) * S;
+    // The chunks' weights exp(m_s - M), MERGE_CHUNKS at a time in shared memory: a number a thread, then every thread adds up its columns of the
+    // partial results in the order of the chunks, eight reads on their way together.  (Each thread used to make every weight
+    // itself, one read behind the other: 32 chunks of 16 heads of 256, 8 tokens: 15.2 us, now 5.9;
+    // 8 chunks 5.0 and 3.0.)
+    __shared__ float s_w[MERGE_CHUNKS], s_l[MERGE_CHUNKS], s_m[4];
+    const int tid = threadIdx.x;
     float M = -INFINITY;
-    for (int s = s0; s <= s1; ++s) M = fmaxf(M, part_ml[(row0 + s) * 2]);
-    float L = 0.f;
-    for (int s = s0; s <= s1; ++s) {
-        const float ms = part_ml[(row0 + s) * 2];
-        L += (ms == -INFINITY) ? 0.f : part_ml[(row0 + s) * 2 + 1] * att_exp<T>(ms - M);
+    for (int s = s0 + tid; s <= s1; s += 128) M = fmaxf(M, part_ml[(row0 + s) * 2]);
+    M = warp_max(M);
+    if ((tid & 31) == 0) s_m[tid >> 5] = M;
+    __syncthreads();
+    M = fmaxf(fmaxf(s_m[0], s_m[1]), fmaxf(s_m[2], s_m[3]));
+    for (int e0 = 0; e0 < hd; e0 += 128 * MERGE_COLUMNS) {       // (once, for every head size that the kernels take)
+    float L = 0.f, o[MERGE_COLUMNS];
+#pragma unroll
+    for (int i = 0; i < MERGE_COLUMNS; ++i) o[i] = 0.f;
+    for (int b0 = s0; b0 <= s1; b0 += MERGE_CHUNKS) {
+        const int n = min(MERGE_CHUNKS, s1 - b0 + 1);
+        __syncthreads();
+        for (int k = tid; k < n; k += 128) {
+            const float ms = part_ml[(row0 + b0 + k) * 2];
+            s_w[k] = (ms == -INFINITY) ? -1.f : att_exp<T>(ms - M);   // -1: a chunk without keys, whose parts may hold anything
+            s_l[k] = part_ml[(row0 + b0 + k) * 2 + 1];
+        }
+        __syncthreads();
+        for (int k = 0; k < n; ++k) L += s_w[k] < 0.f ? 0.f : s_l[k] * s_w[k];
+        for (int k0 = 0; k0 < n; k0 += 8) {
+            const float* p = part_acc + (row0 + b0 + k0) * hd + e0 + tid;
+#pragma unroll
+            for (int i = 0; i < MERGE_COLUMNS; ++i) {
+                if (e0 + tid + 128 * i >= hd) break;
+                float v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = k0 + k < n ? p[(size_t)k * hd + 128 * i] : 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k0 + k < n && !(s_w[k0 + k] < 0.f)) o[i] += v[k] * s_w[k0 + k];
+            }
+        }
     }
     float invL = L > 0.f ? 1.0f / L : 0.f;
     if (sinks) {                                                 // one more term exp(sink_h) in the denominator
         const float sk = sinks[h], Mx = fmaxf(M, sk), a = expf(M - Mx);
         invL = a / (L * a + expf(sk - Mx));
     }
-    for (int e = threadIdx.x; e < hd; e += blockDim.x) {
-        float o = 0.f;
-        for (int s = s0; s <= s1; ++s) {
-            const float ms = part_ml[(row0 + s) * 2];
-            if (ms != -INFINITY) o += part_acc[(row0 + s) * hd + e] * att_exp<T>(ms - M);
-        }
-        op[e] = from_f32<T>(o * invL);
+#pragma unroll
+    for (int i = 0; i < MERGE_COLUMNS; ++i)
+        if (e0 + tid + 128 * i < hd) op[e0 + tid + 128 * i] = from_f32<T>(o[i] * invL);
     }
 }
 
