@@ -102,3 +102,30 @@ def state_of(flat, H, D, P):
     rows, lanes, cols, tiles = ops().decay_scan_shape(D, P)
     x = flat.double().view(H, tiles, rows, cols, lanes)              # element (row l rows + i, column z cols + col)
     return x.permute(0, 4, 2, 1, 3).reshape(H, lanes * rows, tiles * cols)[:, :D, :P]
+
+
+# the float32 kernel of one token and head: fewer keys than groups, whole and broken pages, windows, kept keys, heads on both sides of 128
+@pytest.mark.parametrize("hd", [16, 128, 144])
+@pytest.mark.parametrize("page,window,keep", [(4, None, None), (16, 5, 3), (64, 40, 17)])
+def test_paged_attention_reads_ahead(hd, page, window, keep):
+    nq, nkv, lengths, scale = 4, 2, [1, 15, 16, 17, 33, 100, 64], hd ** -0.5
+    T, blocks = len(lengths), -(-max(lengths) // page)
+    gen = torch.Generator(device=DEV).manual_seed(hd + page)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    table = torch.randperm(T * blocks, device=DEV, generator=gen).to(torch.int32).view(T, blocks)
+    kc, vc, qkv = rnd(T * blocks, nkv, page, hd), rnd(T * blocks, nkv, page, hd), rnd(T, (nq + 2 * nkv) * hd)
+    for t, n in enumerate(lengths):                      # pages wholly behind a request's last key or between kept keys and window are gone
+        for b in range(blocks):
+            if b * page >= n or (window and (b + 1) * page <= n - window and b * page >= keep):
+                table[t, b] = -1
+    pos, req = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    out, err = torch.empty(T, nq * hd, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops().paged_attention(qkv, out, kc, vc, table, req, pos, nq, nkv, hd, scale, window, err, keep=keep)
+    assert int(err) == 0
+    for t, n in enumerate(lengths):
+        j = torch.arange(n, device=DEV)
+        seen = (j >= n - window) | (j < keep) if window else j >= 0
+        rows = lambda c: c[table[t].clamp(min=0).long()].double().transpose(0, 1).reshape(nkv, -1, hd)[:, :n].repeat_interleave(nq // nkv, 0)
+        s = torch.einsum("hd,hnd->hn", qkv[t, :nq * hd].double().view(nq, hd), rows(kc)) * scale
+        ref = torch.einsum("hn,hnd->hd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), rows(vc))
+        assert float((out[t].double().view(nq, hd) - ref).abs().max()) <= 1e-5 * float(ref.abs().max())      # float32 sums of up to 100 terms

@@ -79,29 +79,32 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
     float m = -INFINITY, lsum = 0.f;
 
     const int lo_jb = (lo / ATT_GROUPS) * ATT_GROUPS, kept = min(keep, lo);       // kept keys before the window
-    for (int jb = kept > 0 ? 0 : lo_jb; jb <= pos; jb += ATT_GROUPS) {
-        if (jb >= kept && jb < lo_jb) jb = lo_jb;                 // past the kept keys: on to the window
+    auto from = [&](int jb) { return jb >= kept && jb < lo_jb ? lo_jb : jb; };      // past the kept keys: on to the window
+    // this group's key of the sixteen from jb on: the page it lies in, -1 where it is not read
+    auto page_of = [&](int jb) -> int {
         const int j = jb + g;
-        bool valid = (j >= lo || j < kept) && (j <= pos);
-        size_t base = 0;
-        if (valid) {
-            const int blk = j / page_size;
-            const int page = blk < max_blocks ? table[blk] : -1;
-            if (page < 0 || page >= num_pages) {
-                if (l == 0) atomicOr(err, VL_DEV_BAD_PAGE);
-                valid = false;
-            } else {
-                base = (((size_t)page * nkv + kvh) * page_size + (j - blk * page_size)) * HD;
-            }
-        }
+        if (!((j >= lo || j < kept) && j <= pos)) return -1;
+        const int blk = j / page_size;
+        const int page = blk < max_blocks ? table[blk] : -1;
+        if (page >= 0 && page < num_pages) return page;
+        if (l == 0) atomicOr(err, VL_DEV_BAD_PAGE);
+        return -1;
+    };
+    auto row_of = [&](int jb, int page) -> size_t {
+        const int j = jb + g;
+        return (((size_t)page * nkv + kvh) * page_size + j % page_size) * HD;
+    };
+    auto load = [&](const T* row, float2 (&v)[R]) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = Pair<T>::load(row + 16 * r + 2 * l);
+    };
+    auto score = [&](const float2 (&kv)[R], bool valid, int j) -> float {
         float dot = 0.f;
         if (valid) {
-            const T* kp = kcache + base;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const float2 kv = Pair<T>::load(kp + 16 * r + 2 * l);
-                dot += qr[r][0] * kv.x;
-                dot += qr[r][1] * kv.y;
+                dot += qr[r][0] * kv[r].x;
+                dot += qr[r][1] * kv[r].y;
             }
         }
         dot += __shfl_xor_sync(0xffffffffu, dot, 4);
@@ -110,29 +113,59 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
         float sc = dot * scale;
         if (softcap > 0.f) sc = softcap * tanhf(sc * inv_cap);
         if (dist_a && valid) sc -= da * log1pf(db * (float)(pos - j));
-        if (valid && MODE == ATT_SIGMOID) {
+        return sc;
+    };
+    auto take = [&](const float2 (&vv)[R], float sc) {
+        if (MODE == ATT_SIGMOID) {
             const float p = 1.0f / (1.0f + expf(-(sc + hb)));
-            const T* vp = vcache + base;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const float2 vv = Pair<T>::load(vp + 16 * r + 2 * l);
-                acc[r][0] += p * vv.x;
-                acc[r][1] += p * vv.y;
+                acc[r][0] += p * vv[r].x;
+                acc[r][1] += p * vv[r].y;
             }
-        } else if (valid) {
-            const float s = sc;
-            const float mn = fmaxf(m, s);
+        } else {
+            const float mn = fmaxf(m, sc);
             const float corr = expf(m - mn);
-            const float p = expf(s - mn);
+            const float p = expf(sc - mn);
             lsum = lsum * corr + p;
-            const T* vp = vcache + base;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const float2 vv = Pair<T>::load(vp + 16 * r + 2 * l);
-                acc[r][0] = acc[r][0] * corr + p * vv.x;
-                acc[r][1] = acc[r][1] * corr + p * vv.y;
+                acc[r][0] = acc[r][0] * corr + p * vv[r].x;
+                acc[r][1] = acc[r][1] * corr + p * vv[r].y;
             }
             m = mn;
+        }
+    };
+    // A group meets few keys, so the reads' latency is what counts: while one key is worked off, the next one's key and value are on
+    // their way, and the page of the one behind it (heads of up to 128, whose rows fit the registers twice; 8 tokens x 8 heads of 32
+    // at 120 keys, float32: 8.0 us with every read waited for, 6.3 so; 4 tokens x 32 heads of 128 at 1,000 keys 66.6 and 47.7).
+    float2 kv[R], vv[R];
+    int jb = from(kept > 0 ? 0 : lo_jb);
+    if constexpr (R <= 8) {
+        float2 kn[R], vn[R];
+        int page = page_of(jb), next = from(jb + ATT_GROUPS), page1 = page_of(next);
+        if (page >= 0) { const size_t at = row_of(jb, page); load(kcache + at, kv); load(vcache + at, vv); }
+        auto one = [&](const float2 (&kc)[R], const float2 (&vc)[R], float2 (&kf)[R], float2 (&vf)[R]) {
+            const int after = from(next + ATT_GROUPS), page2 = page_of(after);
+            if (page1 >= 0) { const size_t at = row_of(next, page1); load(kcache + at, kf); load(vcache + at, vf); }
+            const float sc = score(kc, page >= 0, jb + g);
+            if (page >= 0) take(vc, sc);
+            jb = next; page = page1; next = after; page1 = page2;
+        };
+        while (jb <= pos) {                                      // (in pairs, so that no register is copied while its read is on its way)
+            one(kv, vv, kn, vn);
+            if (jb > pos) break;
+            one(kn, vn, kv, vv);
+        }
+    } else {
+        for (; jb <= pos; jb = from(jb + ATT_GROUPS)) {
+            const int page = page_of(jb);
+            const size_t at = page >= 0 ? row_of(jb, page) : 0;
+            if (page >= 0) load(kcache + at, kv);
+            const float sc = score(kv, page >= 0, jb + g);
+            if (page < 0) continue;
+            load(vcache + at, vv);
+            take(vv, sc);
         }
     }
 #pragma unroll
