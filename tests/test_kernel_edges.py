@@ -129,3 +129,43 @@ def test_paged_attention_reads_ahead(hd, page, window, keep):
         s = torch.einsum("hd,hnd->hn", qkv[t, :nq * hd].double().view(nq, hd), rows(kc)) * scale
         ref = torch.einsum("hn,hnd->hd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), rows(vc))
         assert float((out[t].double().view(nq, hd) - ref).abs().max()) <= 1e-5 * float(ref.abs().max())      # float32 sums of up to 100 terms
+
+
+# the few-row product of routed experts: items of one block and of several, more items than places, places without rows in between,
+# padding rows, K at a step's edge and not, N at a tile's edge and not
+@pytest.mark.parametrize("N,K", [(16, 512), (144, 520), (4096, 1024), (8192, 2048)])
+@pytest.mark.parametrize("groups", [[0], [2, 2, 0, 1], [1, -1, 0, -1, -1, 2, -1], [-1, -1], list(range(3)) * 7 + [-1] * 4])
+@pytest.mark.parametrize("act", [None, "silu"])
+def test_experts_product_of_few_rows(groups, N, K, act):
+    gen = torch.Generator(device=DEV).manual_seed(N + K + len(groups))
+    top, tokens, cap = 2, 24, 16 * len(groups)
+    h = torch.randn(tokens, K, device=DEV, generator=gen).to(torch.bfloat16)
+    w = (torch.randn(3, N, K, device=DEV, generator=gen) / K ** 0.5).to(torch.bfloat16)
+    rows = torch.randint(-8, tokens * top, (cap,), device=DEV, generator=gen).clamp(min=-1).to(torch.int32)      # pair or -1
+    scale = torch.rand(tokens * top, device=DEV, generator=gen)
+    tile_group = torch.tensor(groups, dtype=torch.int32, device=DEV)
+    out = torch.full((cap, N // 2 if act else N), 7.0, device=DEV, dtype=torch.bfloat16)
+    ops().gemm_grouped_fused(h, w, out, tile_group, 16, rows, top, scale, act, 1.0, 0.0, 0.0)
+    for y, e in enumerate(groups):
+        at = slice(16 * y, 16 * y + 16)
+        if e < 0:
+            assert bool((out[at] == 7.0).all())          # a place without rows is left alone
+            continue
+        r = rows[at].long()
+        a = h.double()[r.clamp(min=0) // top] * (r >= 0)[:, None]
+        s = torch.where(r >= 0, scale.double()[r.clamp(min=0)], 0.0)[:, None]
+        z, size = (a @ w[e].double().T) * s, (a.abs() @ w[e].double().abs().T) * s
+        off = K * 2.0 ** -24 * size                      # float32 sums
+        if act:
+            z, off = z.view(16, -1, 2, 8), off.view(16, -1, 2, 8)
+            g, u = z[:, :, 0].reshape(16, -1), z[:, :, 1].reshape(16, -1)
+            og, ou = off[:, :, 0].reshape(16, -1), off[:, :, 1].reshape(16, -1)
+            z, off = g / (1 + torch.exp(-g)) * u, 1.2 * og * u.abs() + g.abs() * ou
+        assert bool(((out[at].double() - z).abs() <= 2.0 ** -8 * z.abs() + off + 1e-6).all())
+    if act is None:                                      # the same rows without the index, as the second product takes them
+        sorted_rows = h[rows.clamp(min=0).long() // top].contiguous()
+        again = torch.full((cap, N), 7.0, device=DEV, dtype=torch.bfloat16)
+        ops().gemm_grouped(sorted_rows, w, again, tile_group, 16)
+        live = (tile_group >= 0).repeat_interleave(16) & (rows >= 0)
+        ref = torch.stack([sorted_rows[m].double() @ w[groups[m // 16]].double().T for m in range(cap) if live[m]]) if bool(live.any()) else again[live].double()
+        assert bool(((again[live].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
