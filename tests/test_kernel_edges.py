@@ -41,6 +41,49 @@ def test_silu_mul_layouts(T, I, group, dtype):
     assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())
 
 
+# the persistent decode attention: runs of key tiles that cut items anywhere, places without keys, a long item beside short
+# ones (few pieces allowed: runs as long as that item asks), one page and several a tile, a window, sinks
+@pytest.mark.parametrize("lengths,bound,pieces", [
+    ([1], 64, 2), ([64, 65, 63], 128, 2), ([0, 200, 0, 1, 130], 256, 3), ([4000] + [3] * 9, 4096, 2), ([4000] + [3] * 9, 4096, 6),
+    ([(37 * i * i) % 700 for i in range(70)], 2048, 6), ([300, 900, 64, 128, 1, 2047], 2048, 6), ([900, 2500, 17], 1024, 4)])
+@pytest.mark.parametrize("hd,page,window,sink", [(128, 64, None, False), (64, 16, 150, False), (128, 128, 65, True), (64, 64, None, True)])
+def test_streaming_decode_attention(lengths, bound, pieces, hd, page, window, sink):
+    nq, nkv, T, scale = 8, 2, len(lengths), hd ** -0.5
+    gen = torch.Generator(device=DEV).manual_seed(sum(lengths) + hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen).to(torch.bfloat16)
+    blocks = -(-max(max(lengths), bound) // page)
+    table = torch.randperm(T * blocks, device=DEV, generator=gen).to(torch.int32).view(T, blocks)
+    kc, vc = rnd(T * blocks, nkv, page, hd), rnd(T * blocks, nkv, page, hd)
+    qkv = rnd(T, (nq + 2 * nkv) * hd)
+    sinks = torch.randn(nq, device=DEV, generator=gen) if sink else None
+    pos = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=DEV)
+    req = torch.arange(T, dtype=torch.int32, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    acc, ml = torch.full((T * nq * pieces * hd,), float("nan"), device=DEV), torch.full((T * nq * pieces * 2,), float("nan"), device=DEV)
+    arrivals = torch.zeros(ops().flash_decode_arrivals(T, nq, nkv), dtype=torch.int32, device=DEV)
+    out = rnd(T, nq * hd)
+    for _ in range(2):                                   # twice on the same counters
+        ops().flash_decode(qkv, out, kc, vc, table, req, pos, nq, nkv, hd, scale, window, bound, acc, ml, err, chunk=-(-bound // pieces // 64) * 64,
+                           stream_kernel=True, arrivals=arrivals, sinks=sinks)
+    limit = -(-bound // (-(-bound // pieces // 64) * 64)) * (-(-bound // pieces // 64) * 64)
+    assert int(arrivals.abs().sum()) == 0
+    assert bool(int(err) & 0x10) == any(n > limit for n in lengths) and not int(err) & ~0x10
+    for t, n in enumerate(lengths):
+        got = out[t].double().view(nq, hd)
+        if n == 0 or n > limit:
+            assert not got.any()
+            continue
+        lo = max(0, n - window) if window else 0
+        rows = lambda c: c[table[t].long()].double().transpose(0, 1).reshape(nkv, -1, hd)[:, lo:n].repeat_interleave(nq // nkv, 0)
+        s = torch.einsum("hd,hnd->hn", qkv[t, :nq * hd].double().view(nq, hd), rows(kc)) * scale
+        if sinks is not None:
+            s = torch.cat([s, sinks.double()[:, None]], 1)
+        p = torch.softmax(s, -1)[:, :n - lo]
+        ref, size = torch.einsum("hn,hnd->hd", p, rows(vc)), torch.einsum("hn,hnd->hd", p, rows(vc).abs())
+        # probabilities and the result are rounded to bfloat16, the exponentials are good to about 2^-22
+        assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -8 * size + 1e-6).all()), (t, n)
+
+
 def decayed_memory(r, k, v, w, u, S):
     """float64, one request: r, k, w [T, H, D], v [T, H, P], u [H, D], S [H, D, P]; (outputs [T, H, P], the state behind them)."""
     out = torch.empty(v.shape, dtype=torch.float64, device=DEV)

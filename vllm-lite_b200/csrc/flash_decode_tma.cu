@@ -2,13 +2,18 @@
 // -DFA_HD=64 or 128.  The function and the partial-result layout are those of vl_flash_decode
 // (csrc/flash_attn.cu): a token at position p reads the keys lo..p of its request,
 //     s_j = (q . k_j) * scale;  p = softmax_j(s);  o = sum_j p_j v_j,
-// split into chunks of `chunk` key positions; each (token, KV head, chunk) yields an unnormalised
-// partial output with its maximum and sum, merged by vl_decode_attention_merge.
+// on as many blocks as there are SMs.
 //
-// A decode step is bound by one read of the keys and values, and with a block per (token, KV head,
-// chunk) each block's start-up (positions, block table, first copies) and wind-down are paid once
-// per 128 KB of stream.  Here one block per SM walks many such work items:
-//   warp 4   producer: looks up the pages of a work item and copies its K and V rows, 64 keys a
+// A decode step is bound by one read of the keys and values, so every block reads the same number of key tiles: the tiles of
+// all (token, KV head) items, one item behind the other, are cut into equal runs, whatever lengths the requests have and
+// whatever context the launch was sized for.  A block's run is a few pieces of items; an item that lies in one block's run is
+// finished there, the others leave unnormalised partial results with their maximum and sum, which the block that arrives
+// last at the item's counter adds up in the order of the pieces.  No run is shorter than an item's pieces in the scratch
+// allow (S of them).  Where the cuts lie follows from the lengths alone.
+// The blocks used to take (token, KV head, chunk of 1,024 keys) items in turn, chunk fastest, 148 apart: with 2 or 4 chunks to
+// a token a block met the same chunk of every token, and requests shorter than the context bound left half of the
+// blocks without work (64 requests of 400 to 1,500 keys, bound 2,048, 8 KV heads of 128: 78.5 us with the merge's launch, now 55.9).
+//   warp 4   producer: looks up the pages of a piece and copies its K and V rows, 64 keys a
 //        stage, by TMA boxes (cp.async.bulk.tensor.3d, 128-byte swizzle, one box per page: its blocks
 //        of 64 columns one after the other) into a ring of stages that runs on across work items; it also brings the item's
 //        query rows (bulk copies) and its description into one of two slots.  The producer runs
@@ -16,8 +21,8 @@
 //        hidden behind the stream of this one;
 //   warps 0..3   consumers: per stage each warp takes 16 of the 64 keys (mma.sync m16n8k16, the query
 //        heads of the KV head as rows), keeps its own running maximum, sum and output; at the end of
-//        an item the four are merged through shared memory in warp order and written as the item's
-//        partial result.
+//        a piece the four are merged through shared memory in warp order and written as the item's
+//        result or as a partial one.
 // Keys outside the item's range are masked by position; pages outside it, or that the block table
 // does not hold, are fetched from beyond the end of the tensor (zeros); rows of V behind the
 // request's last key are zeroed in shared memory (another request's leftovers may be anything).
@@ -47,8 +52,8 @@ constexpr int OLD = HD + 4;                            // padded row of the merg
 constexpr unsigned MERGE_BYTES = CONSUMERS * ROWS * OLD * 4;
 constexpr unsigned SMEM_BYTES = NST * STAGE_BYTES + MERGE_BYTES + 2 * Q_BYTES + 256;
 
-struct ItemInfo {                                      // what the producer tells the consumers about a work item
-    int tok, out_row, h0, nvalid, pos, c0, c1, split;  // out_row: the token's number within the launch
+struct ItemInfo {                                      // what the producer tells the consumers about a piece
+    int tok, out_row, h0, nvalid, c0, c1, piece, pieces, counter;   // out_row: the token's number within the launch; nvalid 0: the end
 };
 
 __device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], unsigned addr) {
@@ -80,16 +85,14 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsign
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 }  // namespace
 
-// Work item i = (token z, KV head and head tile y, split x), x fastest; block b takes the items
-// b, b + gridDim.x, ...
 extern "C" __global__ void __launch_bounds__(NTHREADS, 1)
 flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         const bf16* __restrict__ q, int q_stride,
                         const int* __restrict__ block_table, int max_blocks,
                         const int* __restrict__ req_index, const int* __restrict__ positions,
                         int T, int nq, int nkv, int page_size, int num_pages, float scale_log2, int window,
-                        int chunk, int S, float* __restrict__ part_acc, float* __restrict__ part_ml, unsigned* err,
-                        const int* __restrict__ token_index) {
+                        int bound, int S, float* __restrict__ part_acc, float* __restrict__ part_ml, unsigned* err,
+                        const int* __restrict__ token_index, bf16* __restrict__ out, int* arrivals, const float* __restrict__ sinks) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* ring = smem;                                            // [NST][K | V]
     float* sO = reinterpret_cast<float*>(smem + NST * STAGE_BYTES);        // [4][16][OLD]
@@ -101,18 +104,27 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     unsigned long long* q_empty = q_full + 2;                                     // [2]
     ItemInfo* info = reinterpret_cast<ItemInfo*>(q_empty + 2);                    // [2]
     __shared__ float s_m[CONSUMERS][ROWS], s_l[CONSUMERS][ROWS];
-    __shared__ int failed;
+    __shared__ int failed, s_last[2], s_scan[NTHREADS / 32], s_most, s_z, s_before;
+    __shared__ ItemInfo s_partial[2];                    // the pieces of items that other blocks share: the run's first and last
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
     if (smem_u32(smem) & 1023u) {                        // (uniform) never expected; the tiles would be misread
         if (tid == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED);
         return;
     }
+    if (tid == 32 * CONSUMERS) {                         // both maps on their way before the first copy asks for them
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    }
     if (tid == 0) {
         for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], CONSUMERS); }
         for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], CONSUMERS); }
         mbar_fence_init();
         failed = 0;
+        s_most = 0;
+        s_z = T;
+        s_before = 0;
+        s_partial[0].nvalid = s_partial[1].nvalid = 0;
     }
     for (int i = tid; i < 2 * ROWS * QLD / 2; i += NTHREADS) reinterpret_cast<unsigned*>(Qs)[i] = 0u;   // rows no head uses stay zero
     fence_proxy_async_smem();
@@ -120,63 +132,122 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const int grp = nq / nkv;
     const int htiles = (grp + ROWS - 1) / ROWS;
     const int ny = nkv * htiles;
-    const int num_items = T * ny * S;
-    pdl_wait();                                          // q and the cache are written by the kernel before
+    // the keys [lo, n) of token z (its number within the launch): none for a padded place or a position beyond the bound
+    auto keys_of = [&](int z, int* tok, int* lo) -> int {
+        const int k = token_index ? token_index[z] : z, pos = positions[k];
+        if (tok) *tok = k;
+        *lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+        return pos >= 0 && pos < bound ? pos + 1 : 0;
+    };
+    // Where this block's run lies, from the step's description alone (before the wait for the kernel before): the number of tiles, the longest
+    // item, and the token in which the run begins.  A round is a token a thread; what the first rounds found is kept.
+    constexpr int KEPT = 2;
+    int total = 0, kept = 0, own[KEPT] = {0, 0}, upto[KEPT] = {0, 0};
+    auto round = [&](int z0, int& n) -> int {            // tiles of token z0 + tid; tiles of the tokens up to it, in this round
+        int lo = 0;
+        const int z = z0 + tid, keys = z < T ? keys_of(z, nullptr, &lo) : 0, most = keys > 0 ? (keys - 1) / BN - lo / BN + 1 : 0;
+        n = ny * most;
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+        const int longest = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) atomicMax(&s_most, longest);
+        if (lane == 31) s_scan[warp] = x;
+        __syncthreads();
+        int all = 0;
+        for (int w = 0; w < NTHREADS / 32; ++w) { if (w == warp) x += all; all += s_scan[w]; }
+        total += all;
+        __syncthreads();
+        return total - all + x;
+    };
+    for (int z0 = 0, r = 0; z0 < T; z0 += NTHREADS, ++r) {
+        int n;
+        const int u = round(z0, n);
+        if (r == 0) { own[0] = n; upto[0] = u; kept = total; }
+        if (r == 1) { own[1] = n; upto[1] = u; kept = total; }
+    }
+    // (a run as long as the longest item leaves no item in more than two runs; S > 1)
+    const int grid = gridDim.x, all_tiles = total;
+    const int per = max(max((all_tiles + grid - 1) / grid, 1), (s_most + S - 2) / (S - 1));
+    const int first = (int)min((long long)blockIdx.x * per, (long long)all_tiles), last = (int)min((long long)first + per, (long long)all_tiles);
+    total = kept;                                        // the rounds that were not kept, once more
+    for (int z0 = 0, r = 0; z0 < T; z0 += NTHREADS, ++r) {
+        int n = r == 0 ? own[0] : own[1], u = r == 0 ? upto[0] : upto[1];
+        if (r >= KEPT) u = round(z0, n);
+        if (u > first && u - n <= first) { s_z = z0 + tid; s_before = u - n; }
+    }
+    __syncthreads();
 
     if (warp == CONSUMERS) {                             // ---- producer (whole warp) ----
         const int box_rows = page_size < BN ? page_size : BN, nbox = BN / box_rows;
         const int beyond = num_pages * nkv * page_size;  // a row coordinate past the tensor: zeros
-        int stage_it = 0;                                // stages issued so far, over all items
-        int n = 0;
+        int stage_it = 0;                                // stages issued so far, over all pieces
+        int z = s_z, before = s_before;
         bool ok = true;
-        for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++n) {
-            const int split = item % S, y = (item / S) % ny, z = item / (S * ny);
-            const int tok = token_index ? token_index[z] : z;
-            const int kvh = y / htiles, htile = y - kvh * htiles;
-            const int h0 = kvh * grp + htile * ROWS, nvalid = min(ROWS, grp - htile * ROWS);
-            int pos = positions[tok];
-            if ((long long)pos >= (long long)S * chunk) {  // beyond the S chunks the launch was sized for: flagged,
-                if (lane == 0 && split == 0 && err) atomicOr(err, VL_DEV_BEYOND_BOUND);   // served like an empty place
-                pos = -1;
+        struct Piece { ItemInfo ii; const int* table; int stop, kvh, row; };
+        // lane b < nbox owns box b of every key tile: the cache row of the box's first key, looked up one tile ahead of its use
+        auto lookup = [&](const Piece& p, int st) -> int {
+            if (lane >= nbox || st > (p.ii.c1 - 1) / BN) return beyond;
+            const int key = st * BN + lane * box_rows;
+            if (key >= p.ii.c1 || key + box_rows - 1 < p.ii.c0) return beyond;
+            const int blk = key / page_size;
+            const int page = blk < max_blocks ? p.table[blk] : -1;
+            if (page < 0 || page >= num_pages) {
+                atomicOr(err, VL_DEV_BAD_PAGE);
+                return beyond;
             }
-            const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-            const int c0 = max(split * chunk, lo), c1 = min((split + 1) * chunk, pos + 1);
-            const int ib = n & 1;
+            return (page * nkv + p.kvh) * page_size + (key - blk * page_size);
+        };
+        // the piece that begins with tile `at`: its item's share of this run (three reads one behind the other)
+        auto piece_at = [&](int at) -> Piece {
+            Piece p;
+            int tok = 0, lo = 0, keys = 0, tz = 0;
+            while (at < last && z < T) {
+                keys = keys_of(z, &tok, &lo);
+                tz = keys > 0 ? (keys - 1) / BN - lo / BN + 1 : 0;
+                if (at < before + ny * tz) break;
+                before += ny * tz;
+                ++z;
+            }
+            p.ii.nvalid = 0;
+            if (at >= last || z >= T) return p;          // the end of the run
+            const int y = (at - before) / tz, start = before + y * tz;                // the item's first tile
+            const int kvh = y / htiles, htile = y - kvh * htiles;
+            p.stop = min(last, start + tz);
+            p.kvh = kvh;
+            p.table = block_table + (size_t)req_index[tok] * max_blocks;
+            p.ii.tok = tok; p.ii.out_row = z;
+            p.ii.h0 = kvh * grp + htile * ROWS;
+            p.ii.nvalid = min(ROWS, grp - htile * ROWS);
+            const int tile0 = lo / BN - start;           // + a tile's number in the launch = its number in the request
+            p.ii.c0 = max((at + tile0) * BN, lo);
+            p.ii.c1 = min((p.stop + tile0) * BN, keys);
+            p.ii.piece = (int)blockIdx.x - start / per;
+            p.ii.pieces = (start + tz - 1) / per - start / per + 1;
+            p.ii.counter = z * ny + y;
+            p.row = lookup(p, p.ii.c0 / BN);
+            return p;
+        };
+        Piece cur = piece_at(first), nxt = cur;
+        pdl_wait();                                      // q and the cache are written by the kernel before
+        for (int n = 0;; ++n) {
+            const int ib = n & 1, nvalid = cur.ii.nvalid;
             if (lane == 0 && n >= 2 && !mbar_wait_bounded(&q_empty[ib], (unsigned)((n / 2 - 1) & 1))) ok = false;
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
-            const bool live = pos >= 0 && c0 < c1;
             if (lane == 0) {
-                ItemInfo ii;
-                ii.tok = tok; ii.out_row = z; ii.h0 = h0; ii.nvalid = nvalid; ii.pos = pos; ii.split = split;
-                ii.c0 = c0; ii.c1 = live ? c1 : c0;
-                info[ib] = ii;
-                mbar_arrive_expect_tx(&q_full[ib], live ? (unsigned)(nvalid * HD * 2) : 0u);
+                info[ib] = cur.ii;
+                mbar_arrive_expect_tx(&q_full[ib], (unsigned)(nvalid * HD * 2));
             }
             __syncwarp();
-            if (!live) continue;
+            if (nvalid == 0) break;
             if (lane < nvalid)
-                bulk_copy_g2s(Qs + (size_t)(ib * ROWS + lane) * QLD, q + (size_t)tok * q_stride + (size_t)(h0 + lane) * HD,
+                bulk_copy_g2s(Qs + (size_t)(ib * ROWS + lane) * QLD, q + (size_t)cur.ii.tok * q_stride + (size_t)(cur.ii.h0 + lane) * HD,
                               HD * 2, &q_full[ib]);
-            const int* table = block_table + (size_t)req_index[tok] * max_blocks;
-            const int st0 = c0 / BN, st1 = (c1 - 1) / BN;
-            // lane b < nbox owns box b of every key tile: the cache row of the box's first key, looked up
-            // one tile ahead of its use
-            auto lookup = [&](int st) -> int {
-                if (lane >= nbox || st > st1) return beyond;
-                const int first = st * BN + lane * box_rows;
-                if (first >= c1 || first + box_rows - 1 < c0) return beyond;
-                const int blk = first / page_size;
-                const int page = blk < max_blocks ? table[blk] : -1;
-                if (page < 0 || page >= num_pages) {
-                    atomicOr(err, VL_DEV_BAD_PAGE);
-                    return beyond;
-                }
-                return (page * nkv + kvh) * page_size + (first - blk * page_size);
-            };
-            int row = lookup(st0);
+            const int st0 = cur.ii.c0 / BN, st1 = (cur.ii.c1 - 1) / BN, ask = min(st0 + NST - 1, st1);
+            int row = cur.row;
             for (int st = st0; st <= st1 && ok; ++st, ++stage_it) {
-                const int row_next = lookup(st + 1);
+                const int row_next = lookup(cur, st + 1);
                 const int s = stage_it % NST;
                 if (lane == 0) {
                     if (stage_it >= NST && !mbar_wait_bounded(&empty[s], (unsigned)((stage_it / NST - 1) & 1))) ok = false;
@@ -190,11 +261,19 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     tma_load_3d(kt + KV_BYTES, &map_v, 0, row, 0, &full[s]);
                 }
                 row = row_next;
+                if (st == ask) nxt = piece_at(cur.stop);  // the next piece is found while a ring of copies is on its way
             }
+            cur = nxt;
         }
         if (!ok && lane == 0) atomicExch(&failed, 1);
     } else {                                             // ---- consumers ----
         const int g = lane >> 2, t = lane & 3;
+        // what head h's sums are multiplied by: one over L (maximum M, both in units of log2), a sink's term in it
+        auto inverse = [&](float M, float L, int h) -> float {
+            if (!sinks) return L > 0.f ? 1.0f / L : 0.f;
+            const float sk = sinks[h], m = M * 0.6931471805599453f, x = fmaxf(m, sk), a = expf(m - x);
+            return a / (L * a + expf(sk - x));
+        };
         const unsigned ring_u32 = smem_u32(ring);
         const int kr0 = warp * 16;                       // this warp's 16 keys of every stage
         // byte offsets of this lane's ldmatrix rows inside a [64 rows][128 bytes] block and its swizzle
@@ -208,20 +287,26 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         const unsigned sw = (unsigned)(lane & 7);
         int stage_it = 0, n = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++n) {
+        pdl_wait();
+        // the places without keys: rows of zeros, and the ones beyond the bound are flagged
+        for (int z = blockIdx.x; z < T; z += grid) {
+            int tok, lo;
+            if (keys_of(z, &tok, &lo) > 0) continue;
+            if (tid == 0 && err && positions[tok] >= 0) atomicOr(err, VL_DEV_BEYOND_BOUND);
+            for (int i = tid; i < nq * HD / 8; i += 32 * CONSUMERS)
+                reinterpret_cast<uint4*>(out + (size_t)tok * nq * HD)[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (;; ++n) {
             const int ib = n & 1;
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(&q_full[ib], (unsigned)((n / 2) & 1)))) { ok = false; break; }
             const ItemInfo ii = info[ib];
-            const bool live = ii.c0 < ii.c1;
+            if (ii.nvalid == 0) break;
             unsigned qf[KSTEPS][4];
-            if (live) {
 #pragma unroll
-                for (int ks = 0; ks < KSTEPS; ++ks)
-                    ldmatrix_x4(qf[ks], smem_u32(Qs + (size_t)(ib * ROWS + (lane & 7) + 8 * ((lane >> 3) & 1)) * QLD + ks * 16 + 8 * (lane >> 4)));
-            }
+            for (int ks = 0; ks < KSTEPS; ++ks)
+                ldmatrix_x4(qf[ks], smem_u32(Qs + (size_t)(ib * ROWS + (lane & 7) + 8 * ((lane >> 3) & 1)) * QLD + ks * 16 + 8 * (lane >> 4)));
             __syncwarp();
             if (lane == 0) mbar_arrive(&q_empty[ib]);    // the slot may be written again
-            if (!live) continue;
             float o[DTILES][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 #pragma unroll
             for (int d = 0; d < DTILES; ++d) { o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f; }
@@ -230,16 +315,15 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 const int s = stage_it % NST;
                 if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (unsigned)((stage_it / NST) & 1)))) { ok = false; break; }
                 const unsigned kt = ring_u32 + (unsigned)s * STAGE_BYTES, vt = kt + KV_BYTES;
-                if (st == st1 && ii.c1 - st * BN < kr0 + 16) {
-                    // Slots behind the request's last key hold whatever the page's earlier owner left
-                    // there.  Their probabilities are zero, but 0 * NaN is NaN: zero those rows of V
-                    // (this warp's 16 rows of the stage; the other warps see to theirs).
-                    unsigned char* vs = ring + (unsigned)s * STAGE_BYTES + KV_BYTES;
-                    for (int r = max(ii.c1 - st * BN, kr0); r < kr0 + 16; ++r)
-                        if (lane < CB * 8)
-                            *reinterpret_cast<uint4*>(vs + (unsigned)(lane >> 3) * blk_bytes + row_offset(r) + ((lane & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-                    fence_proxy_async_smem();            // the stage is next written by the TMA unit
-                    __syncwarp();
+                // Slots behind the request's last key hold whatever the page's earlier owner left there.  Their probabilities are zero,
+                // but 0 * NaN is NaN: those keys' values are cleared as fragments (zeroing them in shared memory and fencing it against the
+                // TMA unit's next write cost 2 to 3 us at the end of every item).
+                const int left = ii.c1 - (st * BN + kr0);        // keys of this warp's 16 that are read
+                const bool tail = left < 16;
+                unsigned keep0 = 0xffffffffu, keep1 = 0xffffffffu;
+                if (tail) {
+                    keep0 = (2 * t < left ? 0xffffu : 0u) | (2 * t + 1 < left ? 0xffff0000u : 0u);
+                    keep1 = (2 * t + 8 < left ? 0xffffu : 0u) | (2 * t + 9 < left ? 0xffff0000u : 0u);
                 }
                 float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
@@ -287,6 +371,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     unsigned vb[4];
                     const unsigned chunk16 = (unsigned)(2 * dp + (lane >> 4));            // 16-byte piece of the value row
                     ldmatrix_x4_trans(vb, vt + (chunk16 >> 3) * blk_bytes + v_row + (((chunk16 & 7) ^ sw) << 4));
+                    if (tail) { vb[0] &= keep0; vb[1] &= keep1; vb[2] &= keep0; vb[3] &= keep1; }
                     o[2 * dp][0] *= corr[0]; o[2 * dp][1] *= corr[0]; o[2 * dp][2] *= corr[1]; o[2 * dp][3] *= corr[1];
                     o[2 * dp + 1][0] *= corr[0]; o[2 * dp + 1][1] *= corr[0]; o[2 * dp + 1][2] *= corr[1]; o[2 * dp + 1][3] *= corr[1];
                     mma16816(o[2 * dp], pf, vb[0], vb[1]);
@@ -325,14 +410,45 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     acc += sO[((size_t)w * ROWS + r) * OLD + e] * wgt;
                     L += s_l[w][r] * wgt;
                 }
-                const size_t prow = ((size_t)ii.out_row * nq + (ii.h0 + r)) * S + ii.split;
-                part_acc[prow * HD + e] = acc;
-                if (e == 0) {
-                    part_ml[prow * 2] = M * 0.6931471805599453f;           // the merge kernel works in natural-log units
-                    part_ml[prow * 2 + 1] = L;
+                const int h = ii.h0 + r;
+                if (ii.pieces == 1) {
+                    out[((size_t)ii.tok * nq + h) * HD + e] = __float2bfloat16(acc * inverse(M, L, h));
+                } else {
+                    const size_t prow = ((size_t)ii.out_row * nq + h) * S + ii.piece;
+                    __stcg(part_acc + prow * HD + e, acc);
+                    if (e == 0) __stcg(reinterpret_cast<float2*>(part_ml) + prow, make_float2(M, L));
                 }
             }
-            consumer_barrier();                          // the merge buffer is free for the next item
+            if (ii.pieces > 1 && tid == 0) s_partial[n > 0] = ii;
+            consumer_barrier();                          // the merge buffer is free for the next piece
+        }
+        // The items shared with other blocks, at the end of the run so that the stream does not wait for it: count this block's
+        // pieces; whoever comes last adds up all of an item's, in their order.
+        if (ok && (s_partial[0].nvalid || s_partial[1].nvalid)) {     // (the same in all four warps: a barrier lies behind the last write)
+            __threadfence();                             // this thread's parts, before the block's arrivals are counted
+            consumer_barrier();
+            if (tid < 2) s_last[tid] = s_partial[tid].nvalid && atomicAdd(&arrivals[s_partial[tid].counter], 1) == s_partial[tid].pieces - 1;
+            consumer_barrier();
+            if (s_last[0] || s_last[1]) __threadfence();
+            for (int k = 0; k < 2; ++k) {
+                if (!s_last[k]) continue;
+                const ItemInfo ii = s_partial[k];
+                for (int idx = tid; idx < ii.nvalid * HD; idx += 32 * CONSUMERS) {
+                    const int r = idx / HD, e = idx - r * HD, h = ii.h0 + r;
+                    const size_t prow = ((size_t)ii.out_row * nq + h) * S;
+                    float M = -INFINITY, acc = 0.f, L = 0.f;
+                    for (int p = 0; p < ii.pieces; ++p) {
+                        const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml) + prow + p);
+                        const float a = __ldcg(part_acc + (prow + p) * HD + e), m = fmaxf(M, ml.x);
+                        const float old = M == -INFINITY ? 0.f : exp2_mufu(M - m), now = ml.x == -INFINITY ? 0.f : exp2_mufu(ml.x - m);
+                        acc = acc * old + a * now;
+                        L = L * old + ml.y * now;
+                        M = m;
+                    }
+                    out[((size_t)ii.tok * nq + h) * HD + e] = __float2bfloat16(acc * inverse(M, L, h));
+                }
+                if (tid == 0) arrivals[ii.counter] = 0;  // as the next launch finds it
+            }
         }
         if (!ok && lane == 0) atomicExch(&failed, 1);
     }
@@ -342,23 +458,24 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
 extern "C" int vl_flash_decode_tma_head_dim() { return HD; }
 
-// Arguments and scratch as for vl_flash_decode; page sizes that are a multiple of 8 and divide 64 or
-// are a multiple of it.  Follow with vl_decode_attention_merge.
+// Arguments and scratch (S partial results a token and head, S > 1) as for vl_flash_decode; positions from `bound` on are
+// flagged and get rows of zeros.  `arrivals`: a counter per (token, KV head, 16 query heads), zero before and after.  Page sizes
+// that are a multiple of 8 and divide 64 or are a multiple of it.
 extern "C" int vl_flash_decode_tma(const void* q, int q_stride, const void* kcache, const void* vcache,
                                    const int* block_table, int max_blocks, const int* req_index, const int* positions,
                                    int T, int nq, int nkv, int hd, int page_size, int num_pages, float scale, int window,
-                                   int chunk, int S, float* part_acc, float* part_ml, unsigned* err,
-                                   const int* token_index, void* stream) {
+                                   int bound, int S, float* part_acc, float* part_ml, unsigned* err,
+                                   const int* token_index, void* out, int* arrivals, const float* sinks, void* stream) {
     if (T <= 0) return VL_OK;
     if (hd != HD) return VL_ERR_UNSUPPORTED;
     if (nq <= 0 || nkv <= 0 || nq % nkv || page_size <= 0 || max_blocks <= 0 || num_pages <= 0 || q_stride % 8) return VL_ERR_ARGUMENT;
-    if (chunk <= 0 || chunk % BN || S <= 0) return VL_ERR_ARGUMENT;
+    if (bound <= 0 || S < 2 || !out || !arrivals || ((uintptr_t)out & 15) || ((uintptr_t)part_ml & 7)) return VL_ERR_ARGUMENT;
     if (page_size % 8 || (page_size < BN ? BN % page_size : page_size % BN)) return VL_ERR_UNSUPPORTED;
     if ((((uintptr_t)q | (uintptr_t)kcache | (uintptr_t)vcache) & 15)) return VL_ERR_UNSUPPORTED;
     const long long rows = (long long)num_pages * nkv * page_size;
     const int grp = nq / nkv, htiles = (grp + ROWS - 1) / ROWS;
-    const long long items = (long long)T * nkv * htiles * S;
-    if (rows + BN >= (1ll << 31) || items >= (1ll << 31)) return VL_ERR_UNSUPPORTED;
+    const long long most = (long long)T * nkv * htiles * ((bound + BN - 1) / BN);       // key tiles, were every place full
+    if (rows + BN >= (1ll << 31) || most >= (1ll << 31)) return VL_ERR_UNSUPPORTED;
     const int box_rows = page_size < BN ? page_size : BN;
     CUtensorMap map_k, map_v;
     int rc = tc5_make_map_blocks(&map_k, kcache, (int)rows, HD, HD, box_rows);
@@ -373,8 +490,9 @@ extern "C" int vl_flash_decode_tma(const void* q, int q_stride, const void* kcac
     }
     cudaError_t e = cudaFuncSetAttribute(flash_decode_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
-    const int grid = (int)(items < num_sms ? items : num_sms);
+    const int grid = (int)(most < num_sms ? most : num_sms);
     return vl_launch(flash_decode_tma_kernel, dim3(grid), dim3(NTHREADS), SMEM_BYTES, (cudaStream_t)stream,
                      map_k, map_v, (const bf16*)q, q_stride, block_table, max_blocks, req_index, positions, T, nq, nkv,
-                     page_size, num_pages, scale * 1.4426950408889634f, window, chunk, S, part_acc, part_ml, err, token_index);
+                     page_size, num_pages, scale * 1.4426950408889634f, window, bound, S, part_acc, part_ml, err, token_index,
+                     (bf16*)out, arrivals, sinks);
 }

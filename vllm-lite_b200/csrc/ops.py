@@ -102,7 +102,7 @@ _SIGNATURES = {
                                               c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p],
     ("flash_decode_tma", "vl_flash_decode_tma"): [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                   c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int,
-                                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+                                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     ("activation", "vl_silu_mul"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("activation", "vl_gated_act"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_void_p,
                                      c_void_p],
@@ -743,15 +743,16 @@ def flash_decode_arrivals(num_tokens, num_heads, num_kv_heads) -> int:
     return num_tokens * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
 
 
-STREAM_DECODE_MIN_KEYS = 8 * 49152      # tokens x KV heads x context bound from which the persistent TMA kernel is used
+STREAM_DECODE_MIN_KEYS = 1 << 20        # tokens x KV heads x context bound from which the persistent TMA kernel is used
 
 
 def flash_decode_streams(dtype, num_tokens, num_kv_heads, head_dim, page_size, max_context) -> bool:
     """Whether `flash_decode` left to itself serves such a step with the persistent TMA kernel (else a block per chunk).
-    Measured (Qwen3-8B heads, pages of 64): it wins from 64-position pages on (TMA boxes of 8 KB, not 2 KB) when
-    the step streams enough keys to keep every SM's block busy: 16 tokens x 4,096 keys 55.8 us against 60.0 for a
-    block per chunk, 64 x 4,096: 170 against 188, 8 x 16,384: 96 against 108; at 8 x 4,096 and below the block per
-    chunk, which merges in the same launch, is level or ahead."""
+    Its blocks read equal shares whatever the lengths, but start and end more slowly.  Measured (8 KV heads of 128, pages of 64; us, it
+    against a block per chunk): 64 requests of 400 to 1,500 keys, bound 2,048: 55.9 / 56.6, of 1,100 to 2,048: 78.0 / 85.4, of 1,500 to
+    4,096: 124 / 133, all of 4,096: 168 / 183; 16 of 3,000 to 8,192: 67.5 / 74.8; 8 of 6,000 to 16,384: 72.5 / 78.8; below that the
+    block per chunk, which also does the step's head work, is level or ahead: 32 of 400 to 1,500 keys 34.0 / 36.5, 16 of 4,096
+    52.7 / 55.0, 8 of up to 1,000 15.3 / 12.7."""
     return (flash_tc5_supported(dtype, head_dim, page_size) and page_size >= 64
             and num_tokens * num_kv_heads * int(max_context) >= STREAM_DECODE_MIN_KEYS)
 
@@ -764,9 +765,9 @@ def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, 
     keys; the chunks are merged by the block that finishes last (`arrivals`: int32 counters,
     `flash_decode_arrivals` of them, zero before the first call and left zero) or, without
     `arrivals`, by a second kernel.
-    The split pass is the persistent TMA kernel where it takes the head size, pages hold at
-    least 64 positions and the step reads STREAM_DECODE_MIN_KEYS keys or more (`stream_kernel`: None =
-    that rule, True / False to force; it always merges with the second kernel), else a block per chunk.
+    The split pass is the persistent TMA kernel where `flash_decode_streams` says so (`stream_kernel`: None =
+    that rule, True / False to force; it merges in the same launch, with as many partial results a token as the scratch
+    has room for), else a block per chunk.
     `token_index` (int32) restricts the launch to some tokens of the step (the others' rows of `out`
     are left alone); the scratch is then sized for that many tokens.
     `fold` = (q_weight, k_weight, eps, inv_freq, rotary_dim, slots) folds the step's `qk_norm_rope_write`
@@ -817,7 +818,18 @@ def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, 
             _ptr(req_index), _ptr(positions), T, num_heads, num_kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0],
             float(scale), int(window or 0), chunk, S, _ptr(part_acc), _ptr(part_ml), _ptr(err), _ptr(token_index))
     if stream_kernel:
-        _check(_fn("flash_decode_tma", "vl_flash_decode_tma", {"FA_HD": head_dim})(*args, _stream()), "vl_flash_decode_tma")
+        rows = min(part_acc.numel() // (T * num_heads * head_dim), part_ml.numel() // (2 * T * num_heads)) if T else 2
+        if rows < 2:                                 # a caller whose context is one chunk: room for an item in two runs
+            part_acc, part_ml, rows = part_acc.new_empty(2 * need_acc), part_ml.new_empty(2 * need_ml), 2
+        if arrivals is None:
+            arrivals = torch.zeros(flash_decode_arrivals(T, num_heads, num_kv_heads), dtype=torch.int32, device=qkv.device)
+        _need(arrivals, torch.int32, "arrivals", 1)
+        if arrivals.numel() < flash_decode_arrivals(T, num_heads, num_kv_heads):
+            raise KernelError("flash_decode: too few arrival counters")
+        _check(_fn("flash_decode_tma", "vl_flash_decode_tma", {"FA_HD": head_dim})(
+            *args[:16], S * chunk, rows, _ptr(part_acc), _ptr(part_ml), _ptr(err), _ptr(token_index), _ptr(out),
+            _ptr(arrivals), _ptr(sinks), _stream()), "vl_flash_decode_tma")
+        return out
     else:
         if arrivals is not None and S > _own_merge_cap(head_dim):
             arrivals = None

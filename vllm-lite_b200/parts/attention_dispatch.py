@@ -19,6 +19,7 @@ from ..csrc import ops
 from .base import QUERY_TILE
 
 
+STREAM_PIECES = 6        # runs of the persistent decode attention that may share a token's keys, at least
 FOLD_MAX_CHUNKS = 4      # most chunks per token with which the decode attention still does the head work itself
 
 
@@ -57,6 +58,11 @@ def _decode(ops, args, step, spec, group, num_tokens, max_context, token_index=N
             chunk //= 2
         own_merge = False
     S, n_acc, n_ml = ops.decode_attention_scratch(num_tokens, spec.num_heads, spec.head_dim, max_context, chunk)
+    if fold is None and variant is None and not shape and ops.flash_decode_streams(
+            args[0].dtype, num_tokens, spec.num_kv_heads, spec.head_dim, group.page_size, max_context):
+        # equal runs of key tiles, merged inside the launch: room for the pieces of an item that is long beside the others
+        pieces = max(S, STREAM_PIECES)
+        own_merge, n_acc, n_ml = True, n_acc // S * pieces, n_ml // S * pieces
     part_acc = step.workspace.get(step.tag + "attn.part_acc", (n_acc,), torch.float32)
     part_ml = step.workspace.get(step.tag + "attn.part_ml", (n_ml,), torch.float32)
     # one set of counters for all layers of a step shape: every launch leaves them zero
