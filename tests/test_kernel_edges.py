@@ -140,6 +140,40 @@ def test_decay_chunks(H, D, P, lengths, decays):
             assert torch.equal(state[:, :4], walked[:, :4])
 
 
+# one token a request, heads of every number of lanes, a request without a token and one with two (left alone)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,D,P", [(1, 4, 4), (2, 8, 128), (2, 12, 20), (3, 64, 64), (2, 100, 68), (2, 128, 128)])
+def test_decay_step(H, D, P, dtype):
+    gen = torch.Generator(device=DEV).manual_seed(D + P)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    lengths, eps = [1, 0, 1, 2, 1], 1e-5
+    T, B = sum(lengths), len(lengths)
+    cu = torch.tensor([sum(lengths[:i]) for i in range(B + 1)], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([4, 3, 0, 2, 1], dtype=torch.int32, device=DEV)
+    u, norm = rnd(H * D), 1 + 0.1 * rnd(H * P)
+    state = torch.zeros(B, ops().decay_state_floats(H, D, P) + 4, device=DEV)
+    r, k, v, w = rnd(T, H * D + 4), rnd(T, H * D), rnd(T, H * P), torch.rand(T, H * D, device=DEV, generator=gen)
+    gate = rnd(T, H * P + 8).to(dtype)
+    o = torch.empty(T, H * P, device=DEV)
+    for _ in range(2):                                   # a state that is not zero, then the step beside the walk
+        out = torch.full((T, H * P), float("nan"), device=DEV, dtype=dtype)
+        walked = state.clone()
+        scan = (r, 4), (k, 0), (v, 0), (w, 0), u
+        ops().decay_scan(*scan, walked, 4, cu, slots, o, H, D, P)
+        ops().decay_step(*scan, state, 4, cu, slots, gate, 8, norm, eps, out, H, D, P)
+        for b, n in enumerate(lengths):
+            row, st = int(cu[b]), int(slots[b])
+            if n != 1:
+                assert out[row:row + n].isnan().all()
+                continue
+            assert float((state[st] - walked[st]).abs().max()) <= 2.0 ** -22 * float(walked[st].abs().max() + 1)      # two roundings
+            y = o[row].double().view(H, P)
+            y = y / torch.sqrt((y * y).mean(-1, keepdim=True) + eps) * norm.double().view(H, P)
+            y = y * torch.nn.functional.silu(gate[row, 8:].double().view(H, P))
+            assert float((out[row].double().view(H, P) - y).norm() / y.norm()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6)
+        state = walked
+
+
 def state_of(flat, H, D, P):
     """decay_scan's state of one request as [H, D, P] in float64."""
     rows, lanes, cols, tiles = ops().decay_scan_shape(D, P)

@@ -67,6 +67,9 @@ _SIGNATURES = {
     ("recurrent", "vl_decay_scan"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                      c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                      c_int, c_int, c_int, c_void_p],
+    ("decay_chunks", "vl_decay_step"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+                                        c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                                        c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     ("decay_chunks", "vl_decay_chunks"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                           c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                                           c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
@@ -1804,18 +1807,41 @@ def decay_chunk_floats(chunks, H, D, P) -> int:
     return chunks * H * (2 * D * P + DECAY_CHUNK * (D + P) + D)
 
 
+def _decay_checks(r, k, v, w, u, gate, norm, out, H, D, P):
+    (rt, rc), (kt, kc), (vt, vc), (wt, wc) = r, k, v, w
+    for t, n in ((rt, "r"), (kt, "k"), (vt, "v"), (wt, "w")):
+        _need(t, torch.float32, n, 2)
+    _need(u, torch.float32, "u", 1); _need(norm, torch.float32, "norm", 1)
+    _need(gate, None, "gate", 2); _need(out, gate.dtype, "out", 2)
+    T = rt.shape[0]
+    if any(t.shape[0] != T for t in (kt, vt, wt, gate)) or out.shape != (T, H * P) or u.shape[0] != H * D or norm.shape[0] != H * P:
+        raise KernelError("decay_chunks, decay_step: shapes disagree")
+
+
+def decay_step(r, k, v, w, u, state, state_off, cu, slots, gate, gate_col, norm, eps, out, H, D, P):
+    """`decay_scan` and `gate_norm` in one launch, as `decay_chunks`, for the requests that bring one token; the others' rows and states
+    are left alone."""
+    _decay_checks(r, k, v, w, u, gate, norm, out, H, D, P)
+    if not decay_chunks_ok(D, P):
+        raise KernelError(f"decay_step: heads of {D} x {P} not taken")
+    (rt, rc), (kt, kc), (vt, vc), (wt, wc) = r, k, v, w
+    B = _seg_args(cu, slots)
+    rows, lanes, cols, tiles = decay_scan_shape(D, P)
+    sp, stride = _state_args(state, state_off, decay_state_floats(H, D, P))
+    _check(_fn("decay_chunks", "vl_decay_step")(
+        _ptr(rt), rt.shape[1], int(rc), _ptr(kt), kt.shape[1], int(kc), _ptr(vt), vt.shape[1], int(vc), _ptr(wt), wt.shape[1], int(wc),
+        _ptr(u), sp, stride, rows, lanes, cols, tiles, _ptr(cu), _ptr(slots), B, _ptr(gate), dtype_code(gate.dtype), gate.shape[1],
+        int(gate_col), _ptr(norm), float(eps), _ptr(out), H, D, P, _stream()), "vl_decay_step")
+    return out
+
+
 def decay_chunks(r, k, v, w, u, state, state_off, cu, slots, chunks, scratch, gate, gate_col, norm, eps, out, H, D, P):
     """What `decay_scan` and then `gate_norm` (parts of P columns, a silu gate behind the norm) do, for the requests that bring
     DECAY_MIN_CHUNK tokens or more, in chunks of 64 tokens; the others' rows and states are left alone.  r, k, v, w float32;
     `chunks`: at least `decay_chunks_of` the step; scratch float32 [decay_chunk_floats]; gate and out of one dtype."""
+    _decay_checks(r, k, v, w, u, gate, norm, out, H, D, P)
     (rt, rc), (kt, kc), (vt, vc), (wt, wc) = r, k, v, w
-    for t, n in ((rt, "r"), (kt, "k"), (vt, "v"), (wt, "w")):
-        _need(t, torch.float32, n, 2)
-    _need(u, torch.float32, "u", 1); _need(norm, torch.float32, "norm", 1); _need(scratch, torch.float32, "scratch", 1)
-    _need(gate, None, "gate", 2); _need(out, gate.dtype, "out", 2)
-    T = rt.shape[0]
-    if any(t.shape[0] != T for t in (kt, vt, wt, gate)) or out.shape != (T, H * P) or u.shape[0] != H * D or norm.shape[0] != H * P:
-        raise KernelError("decay_chunks: shapes disagree")
+    _need(scratch, torch.float32, "scratch", 1)
     if not decay_chunks_ok(D, P) or scratch.numel() < decay_chunk_floats(chunks, H, D, P):
         raise KernelError(f"decay_chunks: heads of {D} x {P} not taken, or too little scratch for {chunks} chunks")
     B = _seg_args(cu, slots)

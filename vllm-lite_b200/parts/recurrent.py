@@ -307,6 +307,9 @@ class TimeMix:
         counts = [e.count for e in step.entries]
         chunks = ops.decay_chunks_of(counts) if self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D) else 0
         scan = (r, 0), (k, 0), (v, 0), (w, 0), self.u, cache.state, W, step.cu_seqlens, step.state_slots
+        if self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D) and step.max_query_len == 1:
+            ops.decay_step(*scan, g, 0, self.norm, s.eps, gated, H, D, D)        # single tokens: the norm and the gate in the same launch
+            return self.o_proj(gated, step, "tm.out")
         if not chunks or min(counts) < ops.DECAY_MIN_CHUNK:
             o = ws.get(tag + "tm.o", (T, H * D), f32)
             ops.decay_scan(*scan, o, H, D, D, longest=ops.DECAY_MIN_CHUNK - 1 if chunks else None)
