@@ -246,3 +246,32 @@ def test_experts_product_of_few_rows(groups, N, K, act):
         live = (tile_group >= 0).repeat_interleave(16) & (rows >= 0)
         ref = torch.stack([sorted_rows[m].double() @ w[groups[m // 16]].double().T for m in range(cap) if live[m]]) if bool(live.any()) else again[live].double()
         assert bool(((again[live].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
+
+
+@pytest.mark.parametrize("H", [96, 1028, 4096, 8192])
+@pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
+def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
+    """Few rows read weights and stream ahead of the row's sum, many rows behind it: same arithmetic, so a row's bits do not depend on how many
+    rows there are (592 is the last size that reads ahead)."""
+    from vllm_lite_b200.parts.base import StreamSum
+    R = 593
+    g = torch.Generator(device=DEV).manual_seed(H)
+    x, w = torch.randn(R, H, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
+    y = torch.randn(R, H, generator=g, device=DEV).to(act)
+
+    def run(rows):
+        a, b, c = x[:rows].clone(), x[:rows].clone(), x[:rows].clone()
+        out = torch.empty(rows, H, device=DEV, dtype=act)
+        ops().add_rmsnorm(a, y[:rows].contiguous(), w, 1e-6, out)
+        ops().rmsnorm_add(y[:rows].contiguous(), w, 1e-6, 0.5, b)
+        normed = torch.empty_like(out)
+        ops().stream_norm(c, StreamSum(a=y[:rows].contiguous(), a_scale=w, mult=0.5), w, 1e-6, normed)
+        return a, out, b, c, normed
+
+    few, many = run(R - 1), run(R)
+    for f, m in zip(few, many):
+        assert torch.equal(f, m[:R - 1])
+    add = x + y.float()
+    # float32: 32 running additions a thread and 8 levels of tree leave at most 40 2^-24 on the sum, half of it on the root, and a few products
+    want = add * torch.rsqrt(add.double().pow(2).mean(-1, keepdim=True) + 1e-6).float() * w
+    assert (many[1].float() - want).abs().max() < (2 ** -8 if act == torch.bfloat16 else 2 ** -18) * want.abs().max()
