@@ -45,7 +45,8 @@ def test_silu_mul_layouts(T, I, group, dtype):
 # ones (few pieces allowed: runs as long as that item asks), one page and several a tile, a window, sinks
 @pytest.mark.parametrize("lengths,bound,pieces", [
     ([1], 64, 2), ([64, 65, 63], 128, 2), ([0, 200, 0, 1, 130], 256, 3), ([4000] + [3] * 9, 4096, 2), ([4000] + [3] * 9, 4096, 6),
-    ([(37 * i * i) % 700 for i in range(70)], 2048, 6), ([300, 900, 64, 128, 1, 2047], 2048, 6), ([900, 2500, 17], 1024, 4)])
+    ([(37 * i * i) % 700 for i in range(70)], 2048, 6), ([300, 900, 64, 128, 1, 2047], 2048, 6), ([900, 2500, 17], 1024, 4),
+    ([(13 * i) % 160 for i in range(500)], 256, 3)])     # more places than a block's threads count in one go
 @pytest.mark.parametrize("hd,page,window,sink", [(128, 64, None, False), (64, 16, 150, False), (128, 128, 65, True), (64, 64, None, True)])
 def test_streaming_decode_attention(lengths, bound, pieces, hd, page, window, sink):
     nq, nkv, T, scale = 8, 2, len(lengths), hd ** -0.5
@@ -147,9 +148,10 @@ def test_decay_step(H, D, P, dtype):
     gen = torch.Generator(device=DEV).manual_seed(D + P)
     rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
     lengths, eps = [1, 0, 1, 2, 1], 1e-5
-    T, B = sum(lengths), len(lengths)
+    lengths = lengths + [0, 0]                           # padding: its rows lie behind the last token's
+    T, B = sum(lengths) + 2, len(lengths)
     cu = torch.tensor([sum(lengths[:i]) for i in range(B + 1)], dtype=torch.int32, device=DEV)
-    slots = torch.tensor([4, 3, 0, 2, 1], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([4, 3, 0, 2, 1, 0, 0], dtype=torch.int32, device=DEV)
     u, norm = rnd(H * D), 1 + 0.1 * rnd(H * P)
     state = torch.zeros(B, ops().decay_state_floats(H, D, P) + 4, device=DEV)
     r, k, v, w = rnd(T, H * D + 4), rnd(T, H * D), rnd(T, H * P), torch.rand(T, H * D, device=DEV, generator=gen)
@@ -163,6 +165,9 @@ def test_decay_step(H, D, P, dtype):
         ops().decay_step(*scan, state, 4, cu, slots, gate, 8, norm, eps, out, H, D, P)
         for b, n in enumerate(lengths):
             row, st = int(cu[b]), int(slots[b])
+            if b >= T - 2:
+                assert not out[b].any()
+                continue
             if n != 1:
                 assert out[row:row + n].isnan().all()
                 continue

@@ -332,13 +332,17 @@ template <typename TP, int L>
 __global__ void __launch_bounds__(128)
 decay_step_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const float* __restrict__ u, float* __restrict__ state,
                   long long state_stride, const int* __restrict__ cu, const int* __restrict__ slots, const TP* __restrict__ gate, int ld,
-                  int gate_col, const float* __restrict__ norm, float eps, TP* __restrict__ out, int H, int D, int P, int Z) {
+                  int gate_col, const float* __restrict__ norm, float eps, TP* __restrict__ out, int T, int H, int D, int P, int Z) {
     constexpr int CT_ = 128 / L;                                  // columns of a tile
     __shared__ float s_o[DCH_MAX], s_part[4];
     pdl_launch_dependents();
     pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y, row = cu[b], tid = threadIdx.x, col = tid / L, l = tid % L;
-    if (cu[b + 1] - row != 1) return;
+    if (cu[b + 1] - row != 1) {
+        // the rows behind the last token (padding of a replayed step) hold zeros, not what the buffer held before
+        if (b >= cu[gridDim.y] && b < T && tid < P) out[((size_t)b * H + h) * P + tid] = from_f32<TP>(0.f);
+        return;
+    }
     float* S = state + (long long)slots[b] * state_stride + (size_t)h * Z * 4 * 128 + tid;
     const bool on = 4 * l < D;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -386,11 +390,11 @@ decay_step_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
     }
 }
 
-// One token a request (others are left alone): arguments as vl_decay_chunks'.
+// One token a request (others are left alone); T rows, of which those behind the last token become zeros; arguments as vl_decay_chunks'.
 extern "C" int vl_decay_step(const float* rp, int ldr, int rc, const float* kp, int ldk, int kc, const float* vp, int ldv, int vc,
                              const float* wp, int ldw, int wc, const float* u, float* state, long long state_stride, int lay_rows,
                              int lay_lanes, int lay_cols, int lay_tiles, const int* cu, const int* slots, int B, const void* gate, int dtype,
-                             int ldg, int gate_col, const float* norm, float eps, void* out, int H, int D, int P, void* stream) {
+                             int ldg, int gate_col, const float* norm, float eps, void* out, int T, int H, int D, int P, void* stream) {
     if (B <= 0) return VL_OK;
     if (H <= 0 || D <= 0 || P <= 0 || D > DCH_MAX || P > DCH_MAX || D % 4 || B > 65535) return VL_ERR_UNSUPPORTED;
     if (rc < 0 || kc < 0 || vc < 0 || wc < 0 || gate_col < 0 || rc + H * D > ldr || kc + H * D > ldk || vc + H * P > ldv || wc + H * D > ldw ||
@@ -402,7 +406,7 @@ extern "C" int vl_decay_step(const float* rp, int ldr, int rc, const float* kp, 
     case LL:                                                                                                                     \
         return vl_launch(decay_step_kernel<TP, LL>, dim3(H, B), dim3(128), 0, s, DecayRows{rp, ldr, rc}, DecayRows{kp, ldk, kc}, \
                          DecayRows{vp, ldv, vc}, DecayRows{wp, ldw, wc}, u, state, state_stride, cu, slots, (const TP*)gate, ldg, \
-                         gate_col, norm, eps, (TP*)out, H, D, P, lay_tiles)
+                         gate_col, norm, eps, (TP*)out, T, H, D, P, lay_tiles)
 #define DC_STEPS(TP) switch (lay_lanes) { DC_STEP(TP, 1); DC_STEP(TP, 2); DC_STEP(TP, 4); DC_STEP(TP, 8); DC_STEP(TP, 16); DC_STEP(TP, 32); }
     if (dtype == VL_BF16) DC_STEPS(bf16)
     if (dtype == VL_F32) DC_STEPS(float)

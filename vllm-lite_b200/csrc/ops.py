@@ -69,7 +69,7 @@ _SIGNATURES = {
                                      c_int, c_int, c_int, c_void_p],
     ("decay_chunks", "vl_decay_step"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                         c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
-                                        c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
+                                        c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("decay_chunks", "vl_decay_chunks"): [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                           c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                                           c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
@@ -1820,7 +1820,7 @@ def _decay_checks(r, k, v, w, u, gate, norm, out, H, D, P):
 
 def decay_step(r, k, v, w, u, state, state_off, cu, slots, gate, gate_col, norm, eps, out, H, D, P):
     """`decay_scan` and `gate_norm` in one launch, as `decay_chunks`, for the requests that bring one token; the others' rows and states
-    are left alone."""
+    are left alone, rows behind the last token become zeros."""
     _decay_checks(r, k, v, w, u, gate, norm, out, H, D, P)
     if not decay_chunks_ok(D, P):
         raise KernelError(f"decay_step: heads of {D} x {P} not taken")
@@ -1831,7 +1831,7 @@ def decay_step(r, k, v, w, u, state, state_off, cu, slots, gate, gate_col, norm,
     _check(_fn("decay_chunks", "vl_decay_step")(
         _ptr(rt), rt.shape[1], int(rc), _ptr(kt), kt.shape[1], int(kc), _ptr(vt), vt.shape[1], int(vc), _ptr(wt), wt.shape[1], int(wc),
         _ptr(u), sp, stride, rows, lanes, cols, tiles, _ptr(cu), _ptr(slots), B, _ptr(gate), dtype_code(gate.dtype), gate.shape[1],
-        int(gate_col), _ptr(norm), float(eps), _ptr(out), H, D, P, _stream()), "vl_decay_step")
+        int(gate_col), _ptr(norm), float(eps), _ptr(out), rt.shape[0], H, D, P, _stream()), "vl_decay_step")
     return out
 
 
