@@ -280,3 +280,15 @@ def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
     # float32: 32 running additions a thread and 8 levels of tree leave at most 40 2^-24 on the sum, half of it on the root, and a few products
     want = add * torch.rsqrt(add.double().pow(2).mean(-1, keepdim=True) + 1e-6).float() * w
     assert (many[1].float() - want).abs().max() < (2 ** -8 if act == torch.bfloat16 else 2 ** -18) * want.abs().max()
+
+
+def test_a_row_of_nan_is_routed_to_experts_that_exist():
+    T, K, E, top = 5, 64, 40, 4
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    h, router = torch.randn(T, K, device=DEV, generator=gen), torch.randn(E, K, device=DEV, generator=gen)
+    h[2] = float("nan")
+    ids, w = torch.full((T, top), -1, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    ops().moe_route(h, router, top, ids, w, torch.empty(ops().router_slices(K), T, E, device=DEV))
+    assert bool(((ids >= 0) & (ids < E)).all()) and bool(w[2].isnan().any())     # (and the NaN goes on)
+    good = [0, 1, 3, 4]
+    assert torch.equal(ids[good].long(), (h.double() @ router.double().T)[good].topk(top).indices)

@@ -124,6 +124,7 @@ moe_route_kernel(const float* __restrict__ z, int slices, int ntok, int E, int l
             const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
             if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
         }
+        arg = min(arg, E - 1);                           // (no value above minus infinity, as in a row of NaN: still an expert's index)
         const float zb = zl[arg];
         const float score = score_fn == MOE_SCORE_SOFTMAX ? expf(zb - zmax) / zsum : 1.0f / (1.0f + expf(-zb));
         if (lane == 0) {
