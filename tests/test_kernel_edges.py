@@ -292,3 +292,15 @@ def test_a_row_of_nan_is_routed_to_experts_that_exist():
     assert bool(((ids >= 0) & (ids < E)).all()) and bool(w[2].isnan().any())     # (and the NaN goes on)
     good = [0, 1, 3, 4]
     assert torch.equal(ids[good].long(), (h.double() @ router.double().T)[good].topk(top).indices)
+
+
+@pytest.mark.parametrize("H,offset", [(1, 0), (96, 0), (96, 1), (1024, 0), (1028, 0), (4100, 0), (4101, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_rows(H, offset, dtype):
+    V, ids = 50, torch.tensor([0, 49, 7, -1, 50, 7], dtype=torch.int32, device=DEV)
+    table = torch.randn(V * H + offset, device=DEV).to(dtype)[offset:].view(V, H)     # offset: rows off the 16-byte boundary
+    out, err = torch.full((6, H), float("nan"), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops().embed(ids, table, out, err, 3.0)
+    want = table.float()[ids.long().clamp(0, V - 1)] * 3.0
+    want[3:5] = 0
+    assert torch.equal(out, want) and int(err) != 0
