@@ -43,6 +43,13 @@ template <> struct Pair<bf16> {
 #define ATT_SOFTMAX 0
 #define ATT_SIGMOID 1
 
+// a c + p v.  Which of the two products is rounded by itself is spelled out: left to the compiler it changes with the code around it, and
+// with it the float32 logits' last bits (these are the choices it made for a plain loop over the keys).
+template <int R>
+__device__ __forceinline__ float rescaled_sum(float a, float c, float p, float v) {
+    return R == 1 ? __fmaf_rn(a, c, __fmul_rn(p, v)) : __fmaf_rn(p, v, __fmul_rn(a, c));
+}
+
 template <typename T, int R, int MODE>
 __global__ void __launch_bounds__(ATT_THREADS)
 paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
@@ -130,8 +137,8 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
             lsum = lsum * corr + p;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                acc[r][0] = acc[r][0] * corr + p * vv[r].x;
-                acc[r][1] = acc[r][1] * corr + p * vv[r].y;
+                acc[r][0] = rescaled_sum<R>(acc[r][0], corr, p, vv[r].x);
+                acc[r][1] = rescaled_sum<R>(acc[r][1], corr, p, vv[r].y);
             }
             m = mn;
         }
