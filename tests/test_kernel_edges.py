@@ -141,6 +141,36 @@ def test_decay_chunks(H, D, P, lengths, decays):
             assert torch.equal(state[:, :4], walked[:, :4])
 
 
+# a token's numbers reach its own and later outputs only, finite or not: every place in a group of four tokens, both halves of a chunk, the
+# next chunk; heads whose states have rows for all of a block's threads and heads that have not
+@pytest.mark.parametrize("D,P", [(4, 4), (20, 36), (64, 64), (128, 128)])
+@pytest.mark.parametrize("which", ["k", "v", "w"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_decay_chunks_are_causal_for_numbers_that_are_not_finite(D, P, which, bad):
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    H, T = 2, 130
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    x = dict(r=rnd(T, H * D), k=rnd(T, H * D), v=rnd(T, H * P), w=torch.exp(-torch.exp(rnd(T, H * D) - 1)))
+    gate, u, norm = rnd(T, H * P).to(torch.bfloat16), rnd(H * D), 1 + 0.1 * rnd(H * P)
+    cu, slots = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    chunks = ops().decay_chunks_of([T])
+
+    def run(x):
+        out, state = torch.empty(T, H * P, device=DEV, dtype=torch.bfloat16), torch.zeros(1, ops().decay_state_floats(H, D, P), device=DEV)
+        ops().decay_chunks((x["r"], 0), (x["k"], 0), (x["v"], 0), (x["w"], 0), u, state, 0, cu, slots, chunks,
+                           torch.empty(ops().decay_chunk_floats(chunks, H, D, P), device=DEV), gate, 0, norm, 1e-5, out, H, D, P)
+        return out
+
+    clean = run(x)
+    for s in (1, 2, 3, 30, 36, 61, 63, 67, 129):
+        spoilt = dict(x, **{which: x[which].clone()})
+        spoilt[which][s] = bad
+        got = run(spoilt)
+        first = s + 1 if which == "w" else s             # (a token's decay acts behind it)
+        assert torch.equal(got[:first], clean[:first]), s
+        assert first >= T or bool(got[first:].isnan().any()), s
+
+
 # one token a request, heads of every number of lanes, a request without a token and one with two (left alone)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("H,D,P", [(1, 4, 4), (2, 8, 128), (2, 12, 20), (3, 64, 64), (2, 100, 68), (2, 128, 128)])

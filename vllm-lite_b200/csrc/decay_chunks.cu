@@ -45,6 +45,15 @@ __device__ __forceinline__ void dc_product(float4 (&acc)[4], const float* a, int
     }
 }
 
+// The four tokens around the diagonal of A: a row takes the values up to its own token.  What lies behind is left out, not multiplied by
+// A's zero, so that an infinity or a NaN in a token's value stays out of the tokens before it.
+__device__ __forceinline__ void dc_triangle(float4 (&acc)[4], const float4 (&x)[4], const float4 (&y)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e <= i; ++e) dc_fma(acc[i], dc_at(x[i], e), y[e]);
+}
+
 // A running product of decays over `n` tokens (a multiple of 8), first to last (DOWN) or last to first, of one channel: put(t, x[t] times the decays of the tokens passed
 // before t); returns the product of all.  Eight tokens' numbers are on their way from shared memory together.
 template <bool DOWN, typename Put>
@@ -216,10 +225,14 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
                 if (d0 < 64 && k <= 4 * ty) {                     // (A is zero above the diagonal)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) x[i] = dc_ld4(A + (4 * ty + i) * DCH_LDA + k);
+                    if (k == 4 * ty) {
+                        dc_triangle(acc, x, y);
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
+                        for (int e = 0; e < 4; ++e)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) dc_fma(acc[i], dc_at(x[i], e), y[e]);
+                            for (int i = 0; i < 4; ++i) dc_fma(acc[i], dc_at(x[i], e), y[e]);
+                    }
                 }
             }
             if (cols) {
@@ -227,7 +240,14 @@ decay_prep_kernel(DecayRows r, DecayRows k, DecayRows v, DecayRows w, const floa
                 for (int i = 0; i < 4; ++i) dc_st4(added + (ch * D + d0 + i) * P + p0 + 4 * tx, sum[i]);
             }
         }
-        if (4 * ty >= D) dc_product(acc, A + 4 * ty * DCH_LDA, DCH_LDA, R + 4 * tx, DCH_LDA, 4 * ty + 4);   // (rows of the state there are none)
+        if (4 * ty >= D) {                                        // (rows of the state there are none)
+            const float* a = A + 4 * ty * DCH_LDA;
+            dc_product(acc, a, DCH_LDA, R + 4 * tx, DCH_LDA, 4 * ty);
+            float4 x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { x[i] = dc_ld4(a + i * DCH_LDA + 4 * ty); y[i] = dc_ld4(R + (4 * ty + i) * DCH_LDA + 4 * tx); }
+            dc_triangle(acc, x, y);
+        }
         if (cols) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) dc_st4(inner + (ch * CT + 4 * ty + i) * P + p0 + 4 * tx, acc[i]);
