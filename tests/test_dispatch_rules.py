@@ -1,0 +1,37 @@
+"""What the dispatchers decide and hand on, without a GPU."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from vllm_lite_b200.csrc import ops
+from vllm_lite_b200.parts import attention_dispatch
+from vllm_lite_b200.parts.base import StepBatch, Workspace
+
+
+def decode_call(monkeypatch, *, tokens, spec, bound, dtype=torch.bfloat16, **step):
+    """The arguments with which a decode step of `tokens` requests reaches `ops.flash_decode`."""
+    seen = {}
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    monkeypatch.setattr(ops, "flash_decode_max_cluster", lambda hd: 8)
+    monkeypatch.setattr(ops, "flash_decode", lambda *args, **kw: seen.update(kw, part_acc=args[13], part_ml=args[14]))
+    q = torch.empty(tokens, 8, dtype=dtype)
+    batch = SimpleNamespace(workspace=Workspace("cpu"), tag="", err=None, req_index=None, positions=None, max_query_len=1, query_tiles=None,
+                            single_tokens=None, **step)
+    group = SimpleNamespace(page_size=64, max_context=bound, block_table=None)
+    cache = SimpleNamespace(k=None, v=None)
+    attention_dispatch.run(q, None, cache, group, batch, SimpleNamespace(**spec), 1.0)
+    return seen
+
+
+QWEN = dict(num_heads=32, num_kv_heads=8, head_dim=128, window=None)
+
+
+@pytest.mark.parametrize("settled", [True, False])
+def test_a_step_says_whether_its_description_may_be_read_early(monkeypatch, settled):
+    assert decode_call(monkeypatch, tokens=64, spec=QWEN, bound=4096, settled=settled)["settled"] is settled
+
+
+def test_a_step_may_not_be_read_early_unless_it_says_so(monkeypatch):
+    assert decode_call(monkeypatch, tokens=64, spec=QWEN, bound=4096)["settled"] is False
+    assert StepBatch.__dataclass_fields__["settled"].default is False

@@ -85,6 +85,54 @@ def test_streaming_decode_attention(lengths, bound, pieces, hd, page, window, si
         assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -8 * size + 1e-6).all()), (t, n)
 
 
+# the same with dependent launches on: positions that a kernel ahead writes (itself behind a long one) are waited for, those that a copy
+# brought may be read early (`settled`); kernels that write the cache stand ahead in both
+@pytest.mark.parametrize("made_by", ["kernel", "copy"])
+def test_streaming_decode_attention_behind_dependent_launches(made_by):
+    nq, nkv, hd, page, T, bound, pieces = 8, 2, 128, 64, 24, 512, 6
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    blocks = bound // page
+    table = torch.randperm(T * blocks, device=DEV, generator=gen).to(torch.int32).view(T, blocks)
+    caches = [[rnd(T * blocks, nkv, page, hd).to(torch.bfloat16) for _ in range(2)] for _ in range(3)]
+    qkv, inv = rnd(T, (nq + 2 * nkv) * hd).to(torch.bfloat16), torch.rand(hd // 2, device=DEV, generator=gen)
+    order = torch.randperm(T, generator=torch.Generator().manual_seed(4)).to(torch.int32)
+    where = 16 * order                                   # what sorting one row an expert by expert gives, tiles of 16 rows
+    slots = torch.tensor([int(table[t, int(p) // page]) * page + int(p) % page for t, p in enumerate(where)], dtype=torch.int32, device=DEV)
+    req, ids, pinned = torch.arange(T, dtype=torch.int32, device=DEV), order.to(DEV).view(T, 1), where.pin_memory()
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    acc, ml = torch.empty(T * nq * pieces * hd, device=DEV), torch.empty(T * nq * pieces * 2, device=DEV)
+    arrivals = torch.zeros(ops().flash_decode_arrivals(T, nq, nkv), dtype=torch.int32, device=DEV)
+    cap = ops().moe_sorted_rows(T, T, 16)
+    rows, tiles = torch.empty(cap, dtype=torch.int32, device=DEV), torch.empty(cap // 16, dtype=torch.int32, device=DEV)
+    big, product = rnd(2048, 4096), torch.empty(2048, 2048, device=DEV)
+
+    def run(pdl):
+        pos = torch.zeros(T, dtype=torch.int32, device=DEV)
+        heads, outs = qkv.clone(), [torch.empty(T, nq * hd, device=DEV, dtype=torch.bfloat16) for _ in caches]
+        torch.cuda.synchronize()
+        ops().set_pdl(pdl)
+        try:
+            copied = pinned.to(DEV, non_blocking=True)
+            if made_by == "copy":
+                pos = copied
+            ops().gemm_f32(big, big[:2048], product)     # hundreds of microseconds
+            if made_by == "kernel":
+                ops().moe_align(ids, T, 16, rows, tiles, pos)
+            for (k, v), out in zip(caches, outs):
+                ops().qk_norm_rope_write(heads, copied, slots, None, None, 0.0, inv, hd, k, v, nq, nkv, hd, err)
+                ops().flash_decode(heads, out, k, v, table, req, pos, nq, nkv, hd, hd ** -0.5, None, bound, acc, ml, err, chunk=bound,
+                                   stream_kernel=True, arrivals=arrivals, settled=made_by == "copy")
+        finally:
+            ops().set_pdl(False)
+        assert torch.equal(pos.cpu(), where) and int(err) == 0 and not arrivals.any()
+        return outs
+
+    plain = run(False)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(run(True), plain))
+
+
 def decayed_memory(r, k, v, w, u, S):
     """float64, one request: r, k, w [T, H, D], v [T, H, P], u [H, D], S [H, D, P]; (outputs [T, H, P], the state behind them)."""
     out = torch.empty(v.shape, dtype=torch.float64, device=DEV)

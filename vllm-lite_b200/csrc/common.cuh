@@ -119,8 +119,11 @@ __device__ __forceinline__ bool vl_wait_gave_up(int poll, long long t0) {
 // may be brought onto the SMs as soon as every block of this one has started) and pdl_wait() before
 // it first touches memory that earlier kernels of the stream write, and before its own first write
 // to global memory: pdl_wait() returns when all earlier kernels have completed and their writes are
-// visible.  What lies before pdl_wait() may only read constants of the step (weights) and set up
-// shared memory.  Launched without the attribute, both calls do nothing.
+// visible.  What lies before pdl_wait() may only read constants of the step and set up shared memory.  Constants are
+// the weights and the step's description (positions, block tables, ...) that copies brought: a copy is never overlapped,
+// so it is complete before the kernel behind it begins and with that before every later one.  What a kernel of the
+// stream writes is none: the head work's kernels take their positions to be copied, the streaming decode attention
+// reads its description early where it is told that this is so (`settled`).  Launched without the attribute, both calls do nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

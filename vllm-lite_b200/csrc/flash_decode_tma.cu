@@ -92,7 +92,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         const int* __restrict__ req_index, const int* __restrict__ positions,
                         int T, int nq, int nkv, int page_size, int num_pages, float scale_log2, int window,
                         int bound, int S, float* __restrict__ part_acc, float* __restrict__ part_ml, unsigned* err,
-                        const int* __restrict__ token_index, bf16* __restrict__ out, int* arrivals, const float* __restrict__ sinks) {
+                        const int* __restrict__ token_index, bf16* __restrict__ out, int* arrivals, const float* __restrict__ sinks, int settled) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* ring = smem;                                            // [NST][K | V]
     float* sO = reinterpret_cast<float*>(smem + NST * STAGE_BYTES);        // [4][16][OLD]
@@ -132,6 +132,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const int grp = nq / nkv;
     const int htiles = (grp + ROWS - 1) / ROWS;
     const int ny = nkv * htiles;
+    if (!settled) pdl_wait();                            // a kernel before this one may be writing the step's description
     // the keys [lo, n) of token z (its number within the launch): none for a padded place or a position beyond the bound
     auto keys_of = [&](int z, int* tok, int* lo) -> int {
         const int k = token_index ? token_index[z] : z, pos = positions[k];
@@ -139,8 +140,8 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         *lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
         return pos >= 0 && pos < bound ? pos + 1 : 0;
     };
-    // Where this block's run lies, from the step's description alone (before the wait for the kernel before): the number of tiles, the longest
-    // item, and the token in which the run begins.  A round is a token a thread; what the first rounds found is kept.
+    // Where this block's run lies, from the step's description alone (which, `settled`, may be read before the wait for the kernel before): the
+    // number of tiles, the longest item, and the token in which the run begins.  A round is a token a thread; what the first rounds found is kept.
     constexpr int KEPT = 2;
     int total = 0, kept = 0, own[KEPT] = {0, 0}, upto[KEPT] = {0, 0};
     auto round = [&](int z0, int& n) -> int {            // tiles of token z0 + tid; tiles of the tokens up to it, in this round
@@ -183,7 +184,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         const int beyond = num_pages * nkv * page_size;  // a row coordinate past the tensor: zeros
         int stage_it = 0;                                // stages issued so far, over all pieces
         int z = s_z, before = s_before;
-        bool ok = true;
+        bool ok = true, bad_page = false;                // (flagged at the end: nothing is written before the wait)
         struct Piece { ItemInfo ii; const int* table; int stop, kvh, row; };
         // lane b < nbox owns box b of every key tile: the cache row of the box's first key, looked up one tile ahead of its use
         auto lookup = [&](const Piece& p, int st) -> int {
@@ -193,7 +194,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             const int blk = key / page_size;
             const int page = blk < max_blocks ? p.table[blk] : -1;
             if (page < 0 || page >= num_pages) {
-                atomicOr(err, VL_DEV_BAD_PAGE);
+                bad_page = true;
                 return beyond;
             }
             return (page * nkv + p.kvh) * page_size + (key - blk * page_size);
@@ -265,6 +266,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             }
             cur = nxt;
         }
+        if (bad_page && err) atomicOr(err, VL_DEV_BAD_PAGE);
         if (!ok && lane == 0) atomicExch(&failed, 1);
     } else {                                             // ---- consumers ----
         const int g = lane >> 2, t = lane & 3;
@@ -460,12 +462,13 @@ extern "C" int vl_flash_decode_tma_head_dim() { return HD; }
 
 // Arguments and scratch (S partial results a token and head, S > 1) as for vl_flash_decode; positions from `bound` on are
 // flagged and get rows of zeros.  `arrivals`: a counter per (token, KV head, 16 query heads), zero before and after.  Page sizes
-// that are a multiple of 8 and divide 64 or are a multiple of it.
+// that are a multiple of 8 and divide 64 or are a multiple of it.  `settled`: block_table, req_index, positions and token_index were
+// complete before the kernel ahead of this one in the stream began (copies brought them), so a dependent launch may read them early.
 extern "C" int vl_flash_decode_tma(const void* q, int q_stride, const void* kcache, const void* vcache,
                                    const int* block_table, int max_blocks, const int* req_index, const int* positions,
                                    int T, int nq, int nkv, int hd, int page_size, int num_pages, float scale, int window,
                                    int bound, int S, float* part_acc, float* part_ml, unsigned* err,
-                                   const int* token_index, void* out, int* arrivals, const float* sinks, void* stream) {
+                                   const int* token_index, void* out, int* arrivals, const float* sinks, int settled, void* stream) {
     if (T <= 0) return VL_OK;
     if (hd != HD) return VL_ERR_UNSUPPORTED;
     if (nq <= 0 || nkv <= 0 || nq % nkv || page_size <= 0 || max_blocks <= 0 || num_pages <= 0 || q_stride % 8) return VL_ERR_ARGUMENT;
@@ -494,5 +497,5 @@ extern "C" int vl_flash_decode_tma(const void* q, int q_stride, const void* kcac
     return vl_launch(flash_decode_tma_kernel, dim3(grid), dim3(NTHREADS), SMEM_BYTES, (cudaStream_t)stream,
                      map_k, map_v, (const bf16*)q, q_stride, block_table, max_blocks, req_index, positions, T, nq, nkv,
                      page_size, num_pages, scale * 1.4426950408889634f, window, bound, S, part_acc, part_ml, err, token_index,
-                     (bf16*)out, arrivals, sinks);
+                     (bf16*)out, arrivals, sinks, settled);
 }

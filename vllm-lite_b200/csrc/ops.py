@@ -105,7 +105,7 @@ _SIGNATURES = {
                                               c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p],
     ("flash_decode_tma", "vl_flash_decode_tma"): [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                   c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int,
-                                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+                                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     ("activation", "vl_silu_mul"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("activation", "vl_gated_act"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_void_p,
                                      c_void_p],
@@ -763,7 +763,7 @@ def flash_decode_streams(dtype, num_tokens, num_kv_heads, head_dim, page_size, m
 def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, num_heads, num_kv_heads,
                  head_dim, scale, window, max_context, part_acc, part_ml, err, chunk=DECODE_CHUNK, token_index=None,
                  stream_kernel=None, arrivals=None, fold=None, sinks=None, weighting="softmax", mask_chunk=None,
-                 head_bias=None, gate=None, softcap=None, distance=None, keep=None, numbered=False):
+                 head_bias=None, gate=None, softcap=None, distance=None, keep=None, numbered=False, settled=False):
     """Tensor-core version of `decode_attention` (bfloat16): every block takes a chunk of a token's
     keys; the chunks are merged by the block that finishes last (`arrivals`: int32 counters,
     `flash_decode_arrivals` of them, zero before the first call and left zero) or, without
@@ -781,7 +781,9 @@ def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, 
     go with the block-per-chunk kernel that merges its chunks itself (`arrivals` given, few enough chunks).
     `softcap`, `distance` (see `_check_score_shape`) go with the block-per-chunk kernel, merged either way.  `keep` (see
     `_check_keep`) goes with the block-per-chunk kernel that merges its chunks itself; `max_context` then bounds the number
-    of keys a token reads (window + keep at most), not its position.  `numbered`: the same for a window without kept keys."""
+    of keys a token reads (window + keep at most), not its position.  `numbered`: the same for a window without kept keys.
+    `settled`: copies, not kernels, brought block_table, req_index, positions and token_index, so that while dependent launches
+    are on (`set_pdl`) the TMA kernel may read them before the kernels ahead of it have ended."""
     keep = _check_keep(keep, window, mask_chunk)
     numbered = bool(keep or (numbered and window))
     _flash_checks(qkv, k_cache, v_cache, block_table, num_heads, num_kv_heads, head_dim)
@@ -831,7 +833,7 @@ def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, 
             raise KernelError("flash_decode: too few arrival counters")
         _check(_fn("flash_decode_tma", "vl_flash_decode_tma", {"FA_HD": head_dim})(
             *args[:16], S * chunk, rows, _ptr(part_acc), _ptr(part_ml), _ptr(err), _ptr(token_index), _ptr(out),
-            _ptr(arrivals), _ptr(sinks), _stream()), "vl_flash_decode_tma")
+            _ptr(arrivals), _ptr(sinks), int(settled), _stream()), "vl_flash_decode_tma")
         return out
     else:
         if arrivals is not None and S > _own_merge_cap(head_dim):

@@ -388,7 +388,7 @@ class ModelRunner:
                          num_tokens=bucket or sum(counts), num_entries=Bp, max_query_len=max(counts),
                          tag=f"g{bucket}.{longest}." if bucket else "", graph_bucket=bucket,
                          query_tiles=tiles.view(-1, 4) if tiles.numel() else None,
-                         single_tokens=single if single.numel() else None, single_context=single_context)
+                         single_tokens=single if single.numel() else None, single_context=single_context, settled=True)
 
     def _layout_python(self, entries, host_entries, bucket: int = 0) -> StepBatch:
         real_B = len(entries)
@@ -489,7 +489,7 @@ class ModelRunner:
                          tag=f"g{bucket}.{longest}." if bucket else "", graph_bucket=bucket,
                          query_tiles=dview("tiles").view(-1, 4) if tile_list else None,
                          single_tokens=dview("single") if single_list else None,
-                         single_context=max([h.start + 1 for h in host_entries if h.count == 1], default=0))
+                         single_context=max([h.start + 1 for h in host_entries if h.count == 1], default=0), settled=True)
 
     def _upload(self, meta: np.ndarray, bucket: int = 0) -> torch.Tensor:
         n = meta.shape[0]

@@ -69,7 +69,7 @@ def _decode(ops, args, step, spec, group, num_tokens, max_context, token_index=N
     arrivals = step.workspace.zeros(step.tag + "attn.arrivals", ops.flash_decode_arrivals(num_tokens, spec.num_heads, spec.num_kv_heads),
                                     torch.int32) if own_merge else None
     return ops.flash_decode(*args, max_context, part_acc, part_ml, step.err, chunk=chunk, token_index=token_index,
-                            arrivals=arrivals, fold=fold, sinks=sinks, **(variant or {}), **(shape or {}))
+                            arrivals=arrivals, fold=fold, sinks=sinks, settled=getattr(step, "settled", False), **(variant or {}), **(shape or {}))
 
 
 def _variant_decode_ok(ops, spec, num_tokens, max_context, mask_chunk) -> bool:

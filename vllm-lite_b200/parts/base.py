@@ -118,6 +118,8 @@ class StepBatch:
     query_tiles: Optional[torch.Tensor] = None   # int32 [n, 4]: (table row, first token, tokens <= QUERY_TILE, first position)
     single_tokens: Optional[torch.Tensor] = None  # int32: tokens of one-token requests, when the step also holds portions
     single_context: int = 0                      # bound on position + 1 of those tokens
+    settled: bool = False                        # copies, not kernels, brought all of the above to the device: kernels may read
+                                                 # them before the kernels ahead of them in the stream have ended
 
 
 @dataclass
