@@ -35,3 +35,17 @@ def test_a_step_says_whether_its_description_may_be_read_early(monkeypatch, sett
 def test_a_step_may_not_be_read_early_unless_it_says_so(monkeypatch):
     assert decode_call(monkeypatch, tokens=64, spec=QWEN, bound=4096)["settled"] is False
     assert StepBatch.__dataclass_fields__["settled"].default is False
+
+
+def test_counters_are_zero_again_behind_an_error_that_was_raised():
+    from vllm_lite_b200.engine.runner import ModelRunner, StepError
+    runner = ModelRunner.__new__(ModelRunner)            # no device: the error word and the workspace are all that is read
+    runner.err, runner.workspace = torch.tensor([0x2008], dtype=torch.int32), Workspace("cpu")
+    counters = runner.workspace.zeros("attn.arrivals", 5, torch.int32)
+    kept = runner.workspace.get("attn.out", (4,), torch.float32).fill_(3.0)
+    counters[2] = 4                                      # as a block leaves it whose wait ran out before its last arrival
+    with pytest.raises(StepError, match="wait"):
+        runner.check_device_errors()
+    assert not counters.any() and int(runner.err) == 0
+    assert runner.workspace.zeros("attn.arrivals", 5, torch.int32) is counters and bool((kept == 3).all())
+    runner.check_device_errors()                         # nothing left to raise

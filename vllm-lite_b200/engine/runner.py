@@ -523,9 +523,11 @@ class ModelRunner:
         self.steps += 1
 
     def check_device_errors(self):
-        """Read the device error word (synchronises); raise if a kernel refused an access."""
+        """Read the device error word (synchronises); raise if a kernel refused an access.  The runner may go on behind it: the
+        word and the kernels' counters are zero again."""
         word = int(self.err.item())
         if word:
             self.err.zero_()
+            self.workspace.rezero()                      # a wait that ran out may have left counters between their values
             what = [msg for bit, msg in _DEVICE_ERRORS.items() if word & bit]
             raise StepError("a kernel skipped an access: " + "; ".join(what))

@@ -71,6 +71,12 @@ class Workspace:
             self._buffers[key] = buf
         return buf
 
+    def rezero(self):
+        """All buffers of `zeros` zero again: a kernel that gave up leaves its counters where they stood."""
+        for key, buf in self._buffers.items():
+            if key[-1] == "zeros":
+                buf.zero_()
+
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())
 
