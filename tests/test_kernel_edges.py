@@ -85,6 +85,31 @@ def test_streaming_decode_attention(lengths, bound, pieces, hd, page, window, si
         assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -8 * size + 1e-6).all()), (t, n)
 
 
+# rows of the output, scratch and numbers of pieces that begin anywhere, among them a place without keys and one beyond the bound
+@pytest.mark.parametrize("off", [1, 3, 8])
+def test_streaming_decode_attention_off_the_boundaries(off):
+    nq, nkv, hd, page, lengths, bound, pieces = 8, 2, 128, 64, [300, 0, 1000, 17, 2000], 1024, 6
+    T, gen = len(lengths), torch.Generator(device=DEV).manual_seed(off)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen).to(torch.bfloat16)
+    blocks = 2048 // page
+    table = torch.randperm(T * blocks, device=DEV, generator=gen).to(torch.int32).view(T, blocks)
+    kc, vc, qkv = rnd(T * blocks, nkv, page, hd), rnd(T * blocks, nkv, page, hd), rnd(T, (nq + 2 * nkv) * hd)
+    pos, req = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    arrivals = torch.zeros(ops().flash_decode_arrivals(T, nq, nkv), dtype=torch.int32, device=DEV)
+
+    def run(at):
+        err, n = torch.zeros(1, dtype=torch.int32, device=DEV), T * nq * pieces
+        whole = torch.full((T * nq * hd + 16,), 7.0, device=DEV, dtype=torch.bfloat16)
+        out = whole[at:at + T * nq * hd].view(T, nq * hd)
+        acc, ml = torch.empty(n * hd + at, device=DEV)[at:], torch.empty(n * 2 + at, device=DEV)[at:]
+        ops().flash_decode(qkv, out, kc, vc, table, req, pos, nq, nkv, hd, hd ** -0.5, None, bound, acc, ml, err, chunk=bound,
+                           stream_kernel=True, arrivals=arrivals)
+        assert int(err) == 0x10 and bool((whole[:at] == 7).all()) and bool((whole[at + T * nq * hd:] == 7).all())
+        return out
+
+    assert torch.equal(run(off), run(0))
+
+
 # the same with dependent launches on: positions that a kernel ahead writes (itself behind a long one) are waited for, those that a copy
 # brought may be read early (`settled`); kernels that write the cache stand ahead in both
 @pytest.mark.parametrize("made_by", ["kernel", "copy"])

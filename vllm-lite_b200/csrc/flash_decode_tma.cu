@@ -295,8 +295,12 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             int tok, lo;
             if (keys_of(z, &tok, &lo) > 0) continue;
             if (tid == 0 && err && positions[tok] >= 0) atomicOr(err, VL_DEV_BEYOND_BOUND);
-            for (int i = tid; i < nq * HD / 8; i += 32 * CONSUMERS)
-                reinterpret_cast<uint4*>(out + (size_t)tok * nq * HD)[i] = make_uint4(0u, 0u, 0u, 0u);
+            bf16* row = out + (size_t)tok * nq * HD;
+            if ((uintptr_t)out & 15) {                   // (uniform) the caller's rows may begin anywhere
+                for (int i = tid; i < nq * HD; i += 32 * CONSUMERS) row[i] = __float2bfloat16(0.f);
+                continue;
+            }
+            for (int i = tid; i < nq * HD / 8; i += 32 * CONSUMERS) reinterpret_cast<uint4*>(row)[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         for (;; ++n) {
             const int ib = n & 1;
@@ -418,7 +422,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 } else {
                     const size_t prow = ((size_t)ii.out_row * nq + h) * S + ii.piece;
                     __stcg(part_acc + prow * HD + e, acc);
-                    if (e == 0) __stcg(reinterpret_cast<float2*>(part_ml) + prow, make_float2(M, L));
+                    if (e == 0) { __stcg(part_ml + 2 * prow, M); __stcg(part_ml + 2 * prow + 1, L); }
                 }
             }
             if (ii.pieces > 1 && tid == 0) s_partial[n > 0] = ii;
@@ -440,7 +444,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     const size_t prow = ((size_t)ii.out_row * nq + h) * S;
                     float M = -INFINITY, acc = 0.f, L = 0.f;
                     for (int p = 0; p < ii.pieces; ++p) {
-                        const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml) + prow + p);
+                        const float2 ml = make_float2(__ldcg(part_ml + 2 * (prow + p)), __ldcg(part_ml + 2 * (prow + p) + 1));
                         const float a = __ldcg(part_acc + (prow + p) * HD + e), m = fmaxf(M, ml.x);
                         const float old = M == -INFINITY ? 0.f : exp2_mufu(M - m), now = ml.x == -INFINITY ? 0.f : exp2_mufu(ml.x - m);
                         acc = acc * old + a * now;
@@ -472,7 +476,7 @@ extern "C" int vl_flash_decode_tma(const void* q, int q_stride, const void* kcac
     if (T <= 0) return VL_OK;
     if (hd != HD) return VL_ERR_UNSUPPORTED;
     if (nq <= 0 || nkv <= 0 || nq % nkv || page_size <= 0 || max_blocks <= 0 || num_pages <= 0 || q_stride % 8) return VL_ERR_ARGUMENT;
-    if (bound <= 0 || S < 2 || !out || !arrivals || ((uintptr_t)out & 15) || ((uintptr_t)part_ml & 7)) return VL_ERR_ARGUMENT;
+    if (bound <= 0 || S < 2 || !out || !arrivals) return VL_ERR_ARGUMENT;
     if (page_size % 8 || (page_size < BN ? BN % page_size : page_size % BN)) return VL_ERR_UNSUPPORTED;
     if ((((uintptr_t)q | (uintptr_t)kcache | (uintptr_t)vcache) & 15)) return VL_ERR_UNSUPPORTED;
     const long long rows = (long long)num_pages * nkv * page_size;
