@@ -83,6 +83,14 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsign
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// The same, and whether all four warps still have what they waited for: one whose wait ran out takes the others along, so that none
+// stays at a barrier that it does not reach.
+__device__ __forceinline__ bool consumers_agree(bool ok) {
+    int all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(all) : "r"((int)ok) : "memory");
+    return all != 0;
+}
 }  // namespace
 
 extern "C" __global__ void __launch_bounds__(NTHREADS, 1)
@@ -304,7 +312,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
         for (;; ++n) {
             const int ib = n & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&q_full[ib], (unsigned)((n / 2) & 1)))) { ok = false; break; }
+            if (!consumers_agree(__all_sync(0xffffffffu, mbar_wait_bounded(&q_full[ib], (unsigned)((n / 2) & 1))))) { ok = false; break; }
             const ItemInfo ii = info[ib];
             if (ii.nvalid == 0) break;
             unsigned qf[KSTEPS][4];
@@ -386,7 +394,6 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[s]);   // this warp has read the stage
             }
-            if (!ok) break;
             // the four warps' partial results, merged in warp order
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -403,7 +410,8 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 s_m[warp][g] = m_run[0]; s_l[warp][g] = l_run[0];
                 s_m[warp][g + 8] = m_run[1]; s_l[warp][g + 8] = l_run[1];
             }
-            consumer_barrier();
+            ok = consumers_agree(ok);
+            if (!ok) break;
             for (int idx = tid; idx < ii.nvalid * HD; idx += 32 * CONSUMERS) {
                 const int r = idx / HD, e = idx - r * HD;
                 float M = -INFINITY;
@@ -426,11 +434,10 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 }
             }
             if (ii.pieces > 1 && tid == 0) s_partial[n > 0] = ii;
-            consumer_barrier();                          // the merge buffer is free for the next piece
-        }
+        }                                                // (the agreement on the next piece also frees the merge buffer)
         // The items shared with other blocks, at the end of the run so that the stream does not wait for it: count this block's
         // pieces; whoever comes last adds up all of an item's, in their order.
-        if (ok && (s_partial[0].nvalid || s_partial[1].nvalid)) {     // (the same in all four warps: a barrier lies behind the last write)
+        if (ok && (s_partial[0].nvalid || s_partial[1].nvalid)) {     // (the same in all four warps, which have just agreed)
             __threadfence();                             // this thread's parts, before the block's arrivals are counted
             consumer_barrier();
             if (tid < 2) s_last[tid] = s_partial[tid].nvalid && atomicAdd(&arrivals[s_partial[tid].counter], 1) == s_partial[tid].pieces - 1;
