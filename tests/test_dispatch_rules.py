@@ -37,6 +37,18 @@ def test_a_step_may_not_be_read_early_unless_it_says_so(monkeypatch):
     assert StepBatch.__dataclass_fields__["settled"].default is False
 
 
+# where the measured times of the two decode kernels cross (requests, KV heads, head size, bound), page size 64
+@pytest.mark.parametrize("tokens,heads,size,bound,streams", [
+    (48, 8, 128, 1024, False), (64, 8, 128, 1024, False), (24, 8, 128, 2048, False), (32, 8, 128, 2048, True), (64, 8, 128, 2048, True),
+    (8, 8, 128, 4096, False), (12, 8, 128, 4096, True), (16, 8, 128, 4096, True), (16, 4, 128, 4096, False), (32, 4, 128, 4096, True),
+    (4, 8, 128, 8192, False), (8, 8, 128, 8192, True), (12, 4, 128, 8192, True), (4, 8, 128, 16384, True), (4, 4, 128, 30000, True),
+    (1, 8, 128, 32768, False), (64, 8, 128, 512, False), (64, 8, 64, 4096, False), (8, 8, 64, 16384, False)])
+def test_which_decode_kernel_serves_a_step(tokens, heads, size, bound, streams):
+    assert ops.flash_decode_streams(torch.bfloat16, tokens, heads, size, 64, bound) is streams
+    assert not ops.flash_decode_streams(torch.bfloat16, tokens, heads, size, 32, bound)      # short pages: small boxes
+    assert not ops.flash_decode_streams(torch.float32, tokens, heads, size, 64, bound)
+
+
 def test_counters_are_zero_again_behind_an_error_that_was_raised():
     from vllm_lite_b200.engine.runner import ModelRunner, StepError
     runner = ModelRunner.__new__(ModelRunner)            # no device: the error word and the workspace are all that is read

@@ -746,18 +746,29 @@ def flash_decode_arrivals(num_tokens, num_heads, num_kv_heads) -> int:
     return num_tokens * num_kv_heads * -(-(num_heads // num_kv_heads) // 16)
 
 
-STREAM_DECODE_MIN_KEYS = 1 << 20        # tokens x KV heads x context bound from which the persistent TMA kernel is used
+STREAM_DECODE_MIN_KEYS = 1 << 20        # tokens x KV heads x context bound from which the persistent TMA kernel is used, whatever the bound
 
 
 def flash_decode_streams(dtype, num_tokens, num_kv_heads, head_dim, page_size, max_context) -> bool:
     """Whether `flash_decode` left to itself serves such a step with the persistent TMA kernel (else a block per chunk).
-    Its blocks read equal shares whatever the lengths, but start and end more slowly.  Measured (8 KV heads of 128, pages of 64; us, it
-    against a block per chunk): 64 requests of 400 to 1,500 keys, bound 2,048: 55.9 / 56.6, of 1,100 to 2,048: 78.0 / 85.4, of 1,500 to
-    4,096: 124 / 133, all of 4,096: 168 / 183; 16 of 3,000 to 8,192: 67.5 / 74.8; 8 of 6,000 to 16,384: 72.5 / 78.8; below that the
-    block per chunk, which also does the step's head work, is level or ahead: 32 of 400 to 1,500 keys 34.0 / 36.5, 16 of 4,096
-    52.7 / 55.0, 8 of up to 1,000 15.3 / 12.7."""
-    return (flash_tc5_supported(dtype, head_dim, page_size) and page_size >= 64
-            and num_tokens * num_kv_heads * int(max_context) >= STREAM_DECODE_MIN_KEYS)
+    Its blocks read equal shares whatever the lengths, but start and end more slowly; short contexts leave the other kernel few
+    chunks to merge, and in steps of up to four chunks a token it also does the head work.  Measured, it against a block per chunk,
+    each with the head work in its own launch or folded in (us; 8 KV heads of 128, pages of 64, lengths from 0.3 of the bound up):
+      bound 1,024: 48 requests 42.1 / 40.0, 64: 47.9 / 44.5;  2,048: 24: 35.8 / 33.5, 32: 47.5 / 49.6, 64: 70.7 / 75.9;
+      4,096: 8: 27.4 / 25.2, 12: 39.4 / 43.7, 16: 43.3 / 49.5, 32: 70.5 / 77.1, 64: 130 / 147;
+      8,192: 8: 44.3 / 55.4, 16: 73.4 / 80.2;  16,384: 4: 46.3 / 53.2, 8: 75.8 / 82.6;  32,768: 2: 35.9 / 32.5, 4: 61.6 / 63.2
+    (4 KV heads: the same lines; 24 requests at 4,096 37.9 / 37.0; single tokens of mixed steps: within 3 us of the above, 4 at
+    16,384 45.8 / 53.9).  Heads of 64 are half as long to read, and its start is not: 64 at 4,096 93.3 / 75.2, 8 at 16,384 51.4 / 42.9."""
+    if not (flash_tc5_supported(dtype, head_dim, page_size) and page_size >= 64):
+        return False
+    bound, least = int(max_context), STREAM_DECODE_MIN_KEYS
+    if head_dim < 128:
+        least <<= 20                                     # out of reach
+    elif bound >= 4096:
+        least = least * 3 // 8
+    elif bound >= 2048:
+        least //= 2
+    return num_tokens * num_kv_heads * bound >= least
 
 
 def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, num_heads, num_kv_heads,
