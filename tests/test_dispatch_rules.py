@@ -49,6 +49,30 @@ def test_which_decode_kernel_serves_a_step(tokens, heads, size, bound, streams):
     assert not ops.flash_decode_streams(torch.float32, tokens, heads, size, 64, bound)
 
 
+def shared(heads, rank, window=None):
+    return dict(num_heads=heads, num_kv_heads=1, head_dim=rank, window=window, shared_row=True)
+
+
+# halved while all blocks still run at once (148 SMs), and with a window while the launch holds few blocks outside it
+@pytest.mark.parametrize("tokens,heads,rank,window,bound,chunk", [
+    (2, 16, 256, None, 4096, 128), (16, 16, 256, None, 1024, 128), (32, 16, 256, None, 1024, 256), (16, 16, 256, None, 2048, 256),
+    (16, 32, 256, None, 1024, 256), (32, 16, 256, None, 4096, 1024), (8, 16, 256, None, 16384, 1024), (64, 16, 256, None, 1024, 256),
+    (8, 16, 256, 1024, 16384, 128), (16, 16, 256, 1024, 16384, 256), (16, 16, 256, 1024, 4096, 128), (32, 16, 128, None, 1024, 128),
+    (32, 16, 128, 1024, 16384, 128), (64, 16, 128, 1024, 16384, 256), (64, 16, 128, None, 16384, 1024)])
+def test_chunks_of_a_shared_row(monkeypatch, tokens, heads, rank, window, bound, chunk):
+    got = decode_call(monkeypatch, tokens=tokens, spec=shared(heads, rank, window), bound=bound)
+    assert got["chunk"] == chunk and got["arrivals"] is None and got["stream_kernel"] is False
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 4, 8, 16, 32, 36, 64])
+@pytest.mark.parametrize("heads,rank,window", [(16, 256, 1024), (16, 256, 64), (32, 128, 1024), (64, 256, 2048), (16, 256, None), (16, 128, None)])
+def test_scratch_of_a_shared_row_stays_small(monkeypatch, tokens, heads, rank, window):
+    """Shorter chunks must not multiply the scratch, which nobody reserves: at most 64 MB where they are shortened."""
+    whole = 1024 if not window or window > 2048 else (256 if window <= 1024 else 512)
+    got = decode_call(monkeypatch, tokens=tokens, spec=shared(heads, rank, window), bound=131072)
+    assert got["chunk"] == whole or 4 * got["part_acc"].numel() <= 64 << 20
+
+
 def test_counters_are_zero_again_behind_an_error_that_was_raised():
     from vllm_lite_b200.engine.runner import ModelRunner, StepError
     runner = ModelRunner.__new__(ModelRunner)            # no device: the error word and the workspace are all that is read

@@ -37,28 +37,40 @@ def folds_head_work(dtype, step, spec, group, num_tokens) -> bool:
     return -(-int(group.max_context) // chunk) <= FOLD_MAX_CHUNKS
 
 
+def shared_row_chunk(num_tokens, spec, max_context, sms) -> int:
+    """Keys a block of the decode attention takes where 16 heads and more share one row (latent attention), merged by the merge kernel.
+    The step is bound by the blocks' own pace, not by bytes, and runs best with about four chunks over the keys a token reads
+    (measured, 64 tokens x 32 heads x 4,096 keys: 57 us against 71 with the chunks merged inside the launch;
+    64 x 16 heads, window 1,024 of 4,096: 19 us with chunks of 256 against 29 with chunks of 1,024).
+    Few tokens leave SMs idle that way, so chunks are halved as long as all blocks still run at once: an SM holds one block of a row of more
+    than 128 numbers, two of shorter ones (16 heads on a row of 256, lengths from 0.3 of the bound up; us, halved / not: 2 requests at 4,096
+    16.5 / 32.9, 16 at 1,024 14.6 / 17.6; with more blocks than that 32 at 1,024 24.7 / 19.0, 16 at 2,048 25.7 / 23.2, 32 at 4,096 41.9 / 35.5).
+    With a window the launch also has blocks, and scratch, for the chunks outside it: no more than 1,024 and 4,096 of them are asked
+    for (window of 1,024, bound 16,384: 8 requests 16.9 / 18.9, 16 requests 26.8 / 20.6)."""
+    tiles, short = num_tokens * -(-spec.num_heads // 16), spec.head_dim <= 128
+    reach = min(int(max_context), int(spec.window)) if spec.window else int(max_context)
+    chunk = 256 if reach <= 1024 else (512 if reach <= 2048 else 1024)
+    while (chunk > 128 and tiles * -(-reach // (chunk // 2)) <= (2 if short else 1) * sms
+           and (not spec.window or tiles * -(-int(max_context) // (chunk // 2)) <= (4096 if short else 1024))):
+        chunk //= 2
+    return chunk
+
+
 def _decode(ops, args, step, spec, group, num_tokens, max_context, token_index=None, fold=None, sinks=None, variant=None,
             shape=None):
     chunk = ops.decode_chunk_for(num_tokens, spec.num_kv_heads, max_context, head_dim=spec.head_dim)
-    own_merge = True
+    own_merge, stream = True, None
     if variant is not None:
         # the keys a token reads end at its block of the mask: chunks as short as serve that reach, merged inside the launch
         reach = min(int(max_context), int(variant["mask_chunk"] or max_context), int(spec.window or max_context))
         chunk = min(chunk, 256 if reach <= 1024 else (512 if reach <= 2048 else 1024))
     if getattr(spec, "shared_row", False) and spec.num_heads >= 16:
-        # One shared row for 16 heads and more (latent attention): the step is bound by the blocks' own pace, not by
-        # bytes, and runs best with about four chunks over the keys a token reads, merged by the merge kernel
-        # (measured, 64 tokens x 32 heads x 4,096 keys: 57 us against 71 with the chunks merged inside the launch;
-        # 64 x 16 heads, window 1,024 of 4,096: 19 us with chunks of 256 against 29 with chunks of 1,024).
-        reach = min(int(max_context), int(spec.window)) if spec.window else int(max_context)
-        chunk = 256 if reach <= 1024 else (512 if reach <= 2048 else 1024)
-        # Few tokens: such chunks leave SMs idle, and a block's own pace is what bounds the launch (8 tokens of 900 to 2,400 keys x
-        # 16 heads on a row of 256, bound 4,096: 32 us with 32 blocks of 1,024 keys, 13 with chunks of 128)
-        while chunk > 128 and num_tokens * -(-spec.num_heads // 16) * -(-reach // chunk) < 2 * ops.sm_pairs():
-            chunk //= 2
-        own_merge = False
+        # (the streaming kernel, which brings keys and values by themselves, reads the row twice: 64 tokens x 16 heads on a row of 128, bound
+        # 16,384: 99 us against 79, with a window of 1,024 45 against 27)
+        chunk = shared_row_chunk(num_tokens, spec, max_context, 2 * ops.sm_pairs())
+        own_merge, stream = False, False
     S, n_acc, n_ml = ops.decode_attention_scratch(num_tokens, spec.num_heads, spec.head_dim, max_context, chunk)
-    if fold is None and variant is None and not shape and ops.flash_decode_streams(
+    if stream is None and fold is None and variant is None and not shape and ops.flash_decode_streams(
             args[0].dtype, num_tokens, spec.num_kv_heads, spec.head_dim, group.page_size, max_context):
         # equal runs of key tiles, merged inside the launch: room for the pieces of an item that is long beside the others
         pieces = max(S, STREAM_PIECES)
@@ -69,7 +81,7 @@ def _decode(ops, args, step, spec, group, num_tokens, max_context, token_index=N
     arrivals = step.workspace.zeros(step.tag + "attn.arrivals", ops.flash_decode_arrivals(num_tokens, spec.num_heads, spec.num_kv_heads),
                                     torch.int32) if own_merge else None
     return ops.flash_decode(*args, max_context, part_acc, part_ml, step.err, chunk=chunk, token_index=token_index,
-                            arrivals=arrivals, fold=fold, sinks=sinks, settled=getattr(step, "settled", False), **(variant or {}), **(shape or {}))
+                            arrivals=arrivals, fold=fold, sinks=sinks, stream_kernel=stream, settled=getattr(step, "settled", False), **(variant or {}), **(shape or {}))
 
 
 def _variant_decode_ok(ops, spec, num_tokens, max_context, mask_chunk) -> bool:
