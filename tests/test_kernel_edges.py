@@ -356,29 +356,35 @@ def test_experts_product_of_few_rows(groups, N, K, act):
         assert bool(((again[live].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
 
 
-@pytest.mark.parametrize("H", [96, 1028, 4096, 8192])
+@pytest.mark.parametrize("H", [96, 1028, 2048, 4096, 8192])
 @pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
 def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
     """Few rows read weights and stream ahead of the row's sum, many rows behind it: same arithmetic, so a row's bits do not depend on how many
-    rows there are (592 is the last size that reads ahead)."""
+    rows there are.  593 rows never read ahead; 592 and 444 are the last that do (bfloat16, float32), 296 for rows beyond 4,096, and one
+    norm does so while a kernel before it drains."""
     from vllm_lite_b200.parts.base import StreamSum
     R = 593
     g = torch.Generator(device=DEV).manual_seed(H)
     x, w = torch.randn(R, H, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
     y = torch.randn(R, H, generator=g, device=DEV).to(act)
 
-    def run(rows):
+    def run(rows, pdl=False):
         a, b, c = x[:rows].clone(), x[:rows].clone(), x[:rows].clone()
-        out = torch.empty(rows, H, device=DEV, dtype=act)
-        ops().add_rmsnorm(a, y[:rows].contiguous(), w, 1e-6, out)
-        ops().rmsnorm_add(y[:rows].contiguous(), w, 1e-6, 0.5, b)
+        delta, out = y[:rows].contiguous(), torch.empty(rows, H, device=DEV, dtype=act)
         normed = torch.empty_like(out)
-        ops().stream_norm(c, StreamSum(a=y[:rows].contiguous(), a_scale=w, mult=0.5), w, 1e-6, normed)
+        ops().set_pdl(pdl)
+        try:
+            ops().add_rmsnorm(a, delta, w, 1e-6, out)
+            ops().rmsnorm_add(delta, w, 1e-6, 0.5, b)
+            ops().stream_norm(c, StreamSum(a=delta, a_scale=w, mult=0.5), w, 1e-6, normed)
+        finally:
+            ops().set_pdl(False)
         return a, out, b, c, normed
 
-    few, many = run(R - 1), run(R)
-    for f, m in zip(few, many):
-        assert torch.equal(f, m[:R - 1])
+    many = run(R)
+    for rows, pdl in ((592, False), (445, False), (444, False), (297, False), (296, False), (1, False), (64, True), (296, True)):
+        for f, m in zip(run(rows, pdl), many):
+            assert torch.equal(f, m[:rows]), (rows, pdl)
     add = x + y.float()
     # float32: 32 running additions a thread and 8 levels of tree leave at most 40 2^-24 on the sum, half of it on the root, and a few products
     want = add * torch.rsqrt(add.double().pow(2).mean(-1, keepdim=True) + 1e-6).float() * w

@@ -132,7 +132,8 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const TA* __restrict__
 // the sum is asked for before it (AHEAD): the weights, which no kernel of a step writes, even before the kernel before has ended
 // (64 rows of 4,096 bfloat16 behind another kernel: 3.3 us -> 2.8, rmsnorm_add 3.2 -> 2.3).  That takes registers (32 -> 48 for
 // rows of 4,096) and so blocks of an SM.  With more rows than the blocks that run at once the others' reads fill the gaps, and
-// the number of blocks is what counts (2,048 rows: 13.9 us without, 15.8 with).
+// the number of blocks is what counts: four an SM (2,048 rows: 13.9 us without, 15.8 with), of float32 rows three (592 rows of 4,096,
+// rmsnorm_add: 4.4 and 4.9), of rows beyond 4,096, a thread's eight pieces, two (400 rows of 8,192: 6.2 and 7.7, 256: 5.7 and 5.2).
 template <int VPT>
 __device__ __forceinline__ void norm_weights(const float* __restrict__ w, int H4, float4 (&g)[VPT]) {
 #pragma unroll
@@ -141,7 +142,8 @@ __device__ __forceinline__ void norm_weights(const float* __restrict__ w, int H4
         if (c < H4) g[i] = Quad<float>::load(w + 4 * c);
     }
 }
-static bool norm_reads_ahead(int rows) { return rows <= 4 * 148; }
+template <typename TA>
+static bool norm_reads_ahead(int rows, int vpt) { return rows <= (vpt > 4 ? 2 : (sizeof(TA) == 4 ? 3 : 4)) * 148; }
 
 // The same function with a row kept in registers: 16-byte loads, one pass over memory.
 // Thread i holds the float4 pieces i, i + 256, ... of the row (H a multiple of 4, at most
@@ -192,10 +194,9 @@ static bool launch_rmsnorm_vec(float* x, const TA* delta, const int* rows, const
                                float eps, cudaStream_t s) {
     if (H % 4) return false;
     const int pieces = (H / 4 + 255) / 256;
-    const bool ahead = norm_reads_ahead(R);
 #define RMS(VPT)                                                                                                                             \
-    ahead ? vl_launch(add_rmsnorm_vec_kernel<TA, VPT, true>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps)                      \
-          : vl_launch(add_rmsnorm_vec_kernel<TA, VPT, false>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps)
+    norm_reads_ahead<TA>(R, VPT) ? vl_launch(add_rmsnorm_vec_kernel<TA, VPT, true>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps) \
+                                 : vl_launch(add_rmsnorm_vec_kernel<TA, VPT, false>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps)
     if (pieces <= 1) RMS(1);
     else if (pieces <= 2) RMS(2);
     else if (pieces <= 4) RMS(4);
@@ -488,7 +489,7 @@ static int launch_rmsnorm_add(const TA* y, const float* bias, const float* w, fl
 #define RMS_ADD_(VPT, AHEAD)                                                                                                              \
     (w1 ? vl_launch(rmsnorm_add_vec_kernel<TA, VPT, true, AHEAD>, dim3(R), dim3(256), 0, s, y, bias, w, eps, mult, x, cast, H, y2, s1, s2, w1, w2) \
         : vl_launch(rmsnorm_add_vec_kernel<TA, VPT, false, AHEAD>, dim3(R), dim3(256), 0, s, y, bias, w, eps, mult, x, cast, H, y2, s1, s2, w1, w2))
-#define RMS_ADD(VPT) return norm_reads_ahead(R) ? RMS_ADD_(VPT, true) : RMS_ADD_(VPT, false)
+#define RMS_ADD(VPT) return norm_reads_ahead<TA>(R, VPT) ? RMS_ADD_(VPT, true) : RMS_ADD_(VPT, false)
     if (H % 4 == 0 && pieces <= 1) RMS_ADD(1);
     if (H % 4 == 0 && pieces <= 2) RMS_ADD(2);
     if (H % 4 == 0 && pieces <= 4) RMS_ADD(4);
@@ -625,18 +626,20 @@ static int launch_stream_norm(float* x, const StreamSumArgs<TA>& p, const int* r
     const bool vec = H % 4 == 0 && (((uintptr_t)x | (uintptr_t)p.base | (uintptr_t)p.sa | (uintptr_t)p.sb | (uintptr_t)p.add |
                                      (uintptr_t)p.vec | (uintptr_t)p.a | (uintptr_t)p.b | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
 #define STREAM_NORM(KERNEL) return vl_launch(KERNEL, dim3(R), dim3(256), 0, s, x, p, rows, w, eps, out, H)
-#define STREAM_NORM_VEC(VPT)                                                            \
-    do {                                                                               \
-        if (norm_reads_ahead(R)) STREAM_NORM((stream_norm_vec_kernel<TA, VPT, true>)); \
-        STREAM_NORM((stream_norm_vec_kernel<TA, VPT, false>));                         \
+// This kernel has more to read before the sum, and reads ahead only where that is worth it: rows of up to 2,048 (32 rows: 2.9 us -> 2.6), and
+// of up to 4,096 while a kernel before it drains (3.4 -> 3.1; else 3.1 and 3.4); rows of one piece a thread 1.8 and 2.1, of eight 4.7 and 4.9.
+#define STREAM_NORM_AHEAD(VPT)                                                                                                  \
+    do {                                                                                                                        \
+        if (norm_reads_ahead<TA>(R, VPT) && (VPT < 4 || vl_pdl_enabled())) STREAM_NORM((stream_norm_vec_kernel<TA, VPT, true>)); \
+        STREAM_NORM((stream_norm_vec_kernel<TA, VPT, false>));                                                                  \
     } while (0)
-    if (vec && pieces <= 1) STREAM_NORM_VEC(1);
-    if (vec && pieces <= 2) STREAM_NORM_VEC(2);
-    if (vec && pieces <= 4) STREAM_NORM_VEC(4);
-    if (vec && pieces <= 8) STREAM_NORM_VEC(8);
+    if (vec && pieces <= 1) STREAM_NORM((stream_norm_vec_kernel<TA, 1, false>));
+    if (vec && pieces <= 2) STREAM_NORM_AHEAD(2);
+    if (vec && pieces <= 4) STREAM_NORM_AHEAD(4);
+    if (vec && pieces <= 8) STREAM_NORM((stream_norm_vec_kernel<TA, 8, false>));
     STREAM_NORM(stream_norm_kernel<TA>);
 #undef STREAM_NORM
-#undef STREAM_NORM_VEC
+#undef STREAM_NORM_AHEAD
 }
 
 extern "C" int vl_stream_norm(float* x, const float* base, const void* a, const float* sa, const void* b, const float* sb, float mult,
