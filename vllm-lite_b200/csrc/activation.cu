@@ -18,8 +18,18 @@
 #define VL_ACT_RELU 1
 #define VL_ACT_CAPPED_SWISH 2
 
-template <typename T>
-__global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total, int group, int act,
+template <int ACT>
+__device__ __forceinline__ float gated_value(float g, float u, float alpha, float limit, float shift) {
+    if (ACT == VL_ACT_RELU) return fmaxf(g, 0.f) * u;
+    if (ACT == VL_ACT_CAPPED_SWISH) {
+        if (limit > 0.f) { g = fminf(g, limit); u = fminf(fmaxf(u, -limit), limit); }
+        return g / (1.0f + expf(-alpha * g)) * (u + shift);
+    }
+    return g / (1.0f + expf(-g)) * u;
+}
+
+template <typename T, int ACT>
+__global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total, int group,
                                  float alpha, float limit, float shift, const float* __restrict__ bias) {
     pdl_launch_dependents();
     pdl_wait();
@@ -34,22 +44,13 @@ __global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, 
         g += bias[gi];
         u += bias[gi + (group > 0 ? group : I)];
     }
-    float r;
-    if (act == VL_ACT_RELU) {
-        r = fmaxf(g, 0.f) * u;
-    } else if (act == VL_ACT_CAPPED_SWISH) {
-        if (limit > 0.f) { g = fminf(g, limit); u = fminf(fmaxf(u, -limit), limit); }
-        r = g / (1.0f + expf(-alpha * g)) * (u + shift);
-    } else {
-        r = g / (1.0f + expf(-g)) * u;
-    }
-    out[idx] = from_f32<T>(r);
+    out[idx] = from_f32<T>(gated_value<ACT>(g, u, alpha, limit, shift));
 }
 
 // I a multiple of 8, and so is the group if there is one: eight outputs a thread, 16-byte accesses.  A pass over memory
 // (or over what L2 still holds of the product): 536 x 12,288 bfloat16 outputs 8.9 us, 27.4 us one by one.
-template <typename T>
-__global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total8, int group, int act,
+template <typename T, int ACT>
+__global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t total8, int group,
                                      float alpha, float limit, float shift, const float* __restrict__ bias) {
     pdl_launch_dependents();
     pdl_wait();
@@ -67,43 +68,37 @@ __global__ void gated_act_vec_kernel(const T* __restrict__ gu, T* __restrict__ o
         for (int e = 0; e < 8; ++e) { g[e] += bias[gi + e]; u[e] += bias[ui + e]; }
     }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        float gg = g[e], uu = u[e];
-        if (act == VL_ACT_RELU) {
-            r[e] = fmaxf(gg, 0.f) * uu;
-        } else if (act == VL_ACT_CAPPED_SWISH) {
-            if (limit > 0.f) { gg = fminf(gg, limit); uu = fminf(fmaxf(uu, -limit), limit); }
-            r[e] = gg / (1.0f + expf(-alpha * gg)) * (uu + shift);
-        } else {
-            r[e] = gg / (1.0f + expf(-gg)) * uu;
-        }
-    }
+    for (int e = 0; e < 8; ++e) r[e] = gated_value<ACT>(g[e], u[e], alpha, limit, shift);
     store8(out + t * (size_t)I + i, r);
+}
+
+// Eight exponentials and divisions one behind the other take a thread longer than one, which is all that a small launch consists of: 8 x 160
+// bfloat16 outputs of silu 1.45 us one by one and 1.86 by eights, 64 x 1,024: 1.66 and 2.08, 16 x 12,288: 2.17 both, 384 x 1,024: 2.68 and 2.28;
+// float32 256 x 1,024: 2.18 and 2.37, 384 x 1,024: 2.69 and 2.56.  Without an exponential eight are never slower (relu, 21 x 12,288: 2.08 and 1.66).
+template <typename T, int ACT>
+static constexpr size_t gated_vec_min() { return ACT == VL_ACT_RELU ? 0 : (sizeof(T) == 2 ? 3 << 16 : 5 << 16); }
+template <typename T, int ACT>
+static int launch_gated_act(const T* gu, T* out, int T_, int I, int group, float alpha, float limit, float shift, const float* bias, cudaStream_t s) {
+    const size_t total = (size_t)T_ * I;
+    if (total >= gated_vec_min<T, ACT>() && group % 8 == 0 && I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0)
+        return vl_launch(gated_act_vec_kernel<T, ACT>, dim3((unsigned)((total / 8 + 255) / 256)), dim3(256), 0, s, gu, out, I, total / 8, group,
+                         alpha, limit, shift, bias);
+    return vl_launch(gated_act_kernel<T, ACT>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, gu, out, I, total, group, alpha, limit,
+                     shift, bias);
 }
 
 extern "C" int vl_gated_act(const void* gu, void* out, int dtype, int T, int I, int group, int act, float alpha,
                             float limit, float shift, const float* bias, void* stream) {
     if (T <= 0 || I <= 0) return VL_OK;
     if (group < 0 || (group > 0 && I % group) || act < 0 || act > 2) return VL_ERR_ARGUMENT;
-    const size_t total = (size_t)T * I;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (group % 8 == 0 && I % 8 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
-        const size_t total8 = total / 8;
-        const unsigned b8 = (unsigned)((total8 + 255) / 256);
-        if (dtype == VL_F32)
-            return vl_launch(gated_act_vec_kernel<float>, dim3(b8), dim3(256), 0, s, (const float*)gu, (float*)out, I, total8, group, act,
-                             alpha, limit, shift, bias);
-        if (dtype == VL_BF16)
-            return vl_launch(gated_act_vec_kernel<bf16>, dim3(b8), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total8, group, act,
-                             alpha, limit, shift, bias);
-    }
-    if (dtype == VL_F32)
-        return vl_launch(gated_act_kernel<float>, dim3(blocks), dim3(256), 0, s, (const float*)gu, (float*)out, I, total, group,
-                         act, alpha, limit, shift, bias);
-    if (dtype == VL_BF16)
-        return vl_launch(gated_act_kernel<bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)gu, (bf16*)out, I, total, group,
-                         act, alpha, limit, shift, bias);
+#define GATED(TA)                                                                                                                              \
+    act == VL_ACT_SILU ? launch_gated_act<TA, VL_ACT_SILU>((const TA*)gu, (TA*)out, T, I, group, alpha, limit, shift, bias, s)                  \
+    : act == VL_ACT_RELU ? launch_gated_act<TA, VL_ACT_RELU>((const TA*)gu, (TA*)out, T, I, group, alpha, limit, shift, bias, s)                \
+                         : launch_gated_act<TA, VL_ACT_CAPPED_SWISH>((const TA*)gu, (TA*)out, T, I, group, alpha, limit, shift, bias, s)
+    if (dtype == VL_F32) return GATED(float);
+    if (dtype == VL_BF16) return GATED(bf16);
+#undef GATED
     return VL_ERR_UNSUPPORTED;
 }
 
