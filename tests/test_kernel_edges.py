@@ -338,6 +338,33 @@ def test_paged_attention_reads_ahead(hd, page, window, keep):
         assert float((out[t].double().view(nq, hd) - ref).abs().max()) <= 1e-5 * float(ref.abs().max())      # float32 sums of up to 100 terms
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd", [16, 64, 96, 128, 144])
+@pytest.mark.parametrize("weighting,window", [("softmax", None), ("softmax", 40), ("sigmoid", None)])
+def test_paged_attention_holds_the_same_bits_for_few_and_for_many_tokens(hd, dtype, weighting, window):
+    """Few blocks read a key ahead, many do not: the arithmetic is the same, and a token's bits depend on its positions alone."""
+    nq, nkv, lengths, page = 4, 2, [1, 15, 16, 17, 33, 100, 64], 16
+    n, blocks = len(lengths), -(-max(lengths) // page)
+    gen = torch.Generator(device=DEV).manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen).to(dtype)
+    table = torch.randperm(n * blocks, device=DEV, generator=gen).to(torch.int32).view(n, blocks)
+    kc, vc, qkv = rnd(n * blocks, nkv, page, hd), rnd(n * blocks, nkv, page, hd), rnd(n, (nq + 2 * nkv) * hd)
+    bias = torch.randn(nq, device=DEV, generator=gen) if weighting == "sigmoid" else None
+
+    def run(times):
+        pos = torch.tensor([m - 1 for m in lengths] * times, dtype=torch.int32, device=DEV)
+        req = torch.arange(n, dtype=torch.int32, device=DEV).repeat(times)
+        out, err = torch.empty(n * times, nq * hd, device=DEV, dtype=dtype), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops().paged_attention(qkv.repeat(times, 1), out, kc, vc, table, req, pos, nq, nkv, hd, hd ** -0.5, window, err,
+                              weighting=weighting, head_bias=bias)
+        assert int(err) == 0
+        return out.view(times, n, nq * hd)
+
+    few = run(1)
+    for times in (21, 22, 37, 38):                       # 588 and 616 blocks, 1,036 and 1,064
+        assert bool((run(times) == few).all()), times
+
+
 # the few-row product of routed experts: items of one block and of several, more items than places, places without rows in between,
 # padding rows, K at a step's edge and not, N at a tile's edge and not
 @pytest.mark.parametrize("N,K", [(16, 512), (144, 520), (4096, 1024), (8192, 2048)])

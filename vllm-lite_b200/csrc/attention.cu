@@ -50,7 +50,7 @@ __device__ __forceinline__ float rescaled_sum(float a, float c, float p, float v
     return R == 1 ? __fmaf_rn(a, c, __fmul_rn(p, v)) : __fmaf_rn(p, v, __fmul_rn(a, c));
 }
 
-template <typename T, int R, int MODE>
+template <typename T, int R, int MODE, bool AHEAD>
 __global__ void __launch_bounds__(ATT_THREADS)
 paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
                        const T* __restrict__ kcache, const T* __restrict__ vcache,
@@ -105,13 +105,14 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = Pair<T>::load(row + 16 * r + 2 * l);
     };
-    auto score = [&](const float2 (&kv)[R], bool valid, int j) -> float {
+    auto score = [&](auto key, bool valid, int j) -> float {      // key(r): the row's r-th pair of this lane
         float dot = 0.f;
         if (valid) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                dot += qr[r][0] * kv[r].x;
-                dot += qr[r][1] * kv[r].y;
+                const float2 kv = key(r);
+                dot += qr[r][0] * kv.x;
+                dot += qr[r][1] * kv.y;
             }
         }
         dot += __shfl_xor_sync(0xffffffffu, dot, 4);
@@ -122,13 +123,14 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
         if (dist_a && valid) sc -= da * log1pf(db * (float)(pos - j));
         return sc;
     };
-    auto take = [&](const float2 (&vv)[R], float sc) {
+    auto take = [&](auto value, float sc) {
         if (MODE == ATT_SIGMOID) {
             const float p = 1.0f / (1.0f + expf(-(sc + hb)));
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                acc[r][0] += p * vv[r].x;
-                acc[r][1] += p * vv[r].y;
+                const float2 vv = value(r);
+                acc[r][0] += p * vv.x;
+                acc[r][1] += p * vv.y;
             }
         } else {
             const float mn = fmaxf(m, sc);
@@ -137,26 +139,25 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
             lsum = lsum * corr + p;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                acc[r][0] = rescaled_sum<R>(acc[r][0], corr, p, vv[r].x);
-                acc[r][1] = rescaled_sum<R>(acc[r][1], corr, p, vv[r].y);
+                const float2 vv = value(r);
+                acc[r][0] = rescaled_sum<R>(acc[r][0], corr, p, vv.x);
+                acc[r][1] = rescaled_sum<R>(acc[r][1], corr, p, vv.y);
             }
             m = mn;
         }
     };
-    // A group meets few keys, so the reads' latency is what counts: while one key is worked off, the next one's key and value are on
-    // their way, and the page of the one behind it (heads of up to 128, whose rows fit the registers twice; 8 tokens x 8 heads of 32
-    // at 120 keys, float32: 8.0 us with every read waited for, 6.3 so; 4 tokens x 32 heads of 128 at 1,000 keys 66.6 and 47.7).
-    float2 kv[R], vv[R];
+    // AHEAD: a group meets few keys, so the reads' latency is what counts: while one key is worked off, the next one's key and value are on
+    // their way, and the page of the one behind it.  Rows have to fit the registers twice (`reads_ahead`).
     int jb = from(kept > 0 ? 0 : lo_jb);
-    if constexpr (R <= 8) {
-        float2 kn[R], vn[R];
+    if constexpr (AHEAD) {
+        float2 kv[R], vv[R], kn[R], vn[R];
         int page = page_of(jb), next = from(jb + ATT_GROUPS), page1 = page_of(next);
         if (page >= 0) { const size_t at = row_of(jb, page); load(kcache + at, kv); load(vcache + at, vv); }
         auto one = [&](const float2 (&kc)[R], const float2 (&vc)[R], float2 (&kf)[R], float2 (&vf)[R]) {
             const int after = from(next + ATT_GROUPS), page2 = page_of(after);
             if (page1 >= 0) { const size_t at = row_of(next, page1); load(kcache + at, kf); load(vcache + at, vf); }
-            const float sc = score(kc, page >= 0, jb + g);
-            if (page >= 0) take(vc, sc);
+            const float sc = score([&](int r) { return kc[r]; }, page >= 0, jb + g);
+            if (page >= 0) take([&](int r) { return vc[r]; }, sc);
             jb = next; page = page1; next = after; page1 = page2;
         };
         while (jb <= pos) {                                      // (in pairs, so that no register is copied while its read is on its way)
@@ -166,13 +167,21 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
         }
     } else {
         for (; jb <= pos; jb = from(jb + ATT_GROUPS)) {
-            const int page = page_of(jb);
-            const size_t at = page >= 0 ? row_of(jb, page) : 0;
-            if (page >= 0) load(kcache + at, kv);
-            const float sc = score(kv, page >= 0, jb + g);
-            if (page < 0) continue;
-            load(vcache + at, vv);
-            take(vv, sc);
+            const int j = jb + g;
+            bool valid = (j >= lo || j < kept) && (j <= pos);
+            size_t at = 0;
+            if (valid) {
+                const int blk = j / page_size;
+                const int page = blk < max_blocks ? table[blk] : -1;
+                if (page < 0 || page >= num_pages) {
+                    if (l == 0) atomicOr(err, VL_DEV_BAD_PAGE);
+                    valid = false;
+                } else {
+                    at = (((size_t)page * nkv + kvh) * page_size + (j - blk * page_size)) * HD;
+                }
+            }
+            const float sc = score([&](int r) { return Pair<T>::load(kcache + at + 16 * r + 2 * l); }, valid, j);
+            if (valid) take([&](int r) { return Pair<T>::load(vcache + at + 16 * r + 2 * l); }, sc);
         }
     }
 #pragma unroll
@@ -214,6 +223,15 @@ paged_attention_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ ou
     }
 }
 
+// Reading ahead takes registers (heads of 128: 64 -> 124), and with them half of an SM's blocks.  It pays while all blocks run at once, four
+// an SM for heads of more than 64 numbers and seven below; with more of them the others fill the gaps (float32, us, ahead / not: 8
+// tokens x 32 heads of 128 at 1,000 keys 48 / 64, 64 tokens at 500 keys, window 64, 25 / 20, 200 at 200 keys 141 / 123; 8 heads of 32: 64 tokens
+// 20.6 / 23.8, 200 tokens 20.4 / 18.0).  bfloat16 rows of up to 64 numbers arrive in one read a lane and more, and lose (16 heads of 64, 8 tokens 7.0 / 6.7).
+template <int R>
+static bool reads_ahead(dim3 grid) {
+    return (size_t)grid.x * grid.y <= 148 * (R > 4 ? 4 : 7);
+}
+
 template <typename T>
 static int launch_paged_attention(int R, dim3 grid, cudaStream_t s, const T* q, int q_stride, T* out,
                                   const T* kc, const T* vc, const int* bt, int max_blocks,
@@ -221,16 +239,21 @@ static int launch_paged_attention(int R, dim3 grid, cudaStream_t s, const T* q, 
                                   int num_pages, float scale, int window, const float* sinks, int mode, int chunk,
                                   const float* head_bias, const T* gate, int gate_stride, float softcap,
                                   const float* dist_a, const float* dist_b, int keep, unsigned* err) {
+#define ATT_LAUNCH(RR, MODE, AHEAD)                                                               \
+    paged_attention_kernel<T, RR, MODE, AHEAD><<<grid, ATT_THREADS, 0, s>>>(                      \
+        q, q_stride, out, kc, vc, bt, max_blocks, req, pos, nq, nkv, page_size, num_pages,        \
+        scale, window, sinks, chunk, head_bias, gate, gate_stride, softcap, dist_a, dist_b, keep, err)
 #define ATT_CASE(RR)                                                                              \
     case RR:                                                                                      \
-        if (mode == ATT_SIGMOID)                                                                  \
-            paged_attention_kernel<T, RR, ATT_SIGMOID><<<grid, ATT_THREADS, 0, s>>>(              \
-                q, q_stride, out, kc, vc, bt, max_blocks, req, pos, nq, nkv, page_size, num_pages,\
-                scale, window, sinks, chunk, head_bias, gate, gate_stride, softcap, dist_a, dist_b, keep, err);          \
-        else                                                                                      \
-            paged_attention_kernel<T, RR, ATT_SOFTMAX><<<grid, ATT_THREADS, 0, s>>>(              \
-                q, q_stride, out, kc, vc, bt, max_blocks, req, pos, nq, nkv, page_size, num_pages,\
-                scale, window, sinks, chunk, head_bias, gate, gate_stride, softcap, dist_a, dist_b, keep, err);          \
+        if constexpr (RR <= 8 && (sizeof(T) == 4 || RR > 4)) {                                    \
+            if (reads_ahead<RR>(grid)) {                                                          \
+                if (mode == ATT_SIGMOID) ATT_LAUNCH(RR, ATT_SIGMOID, true);                       \
+                else ATT_LAUNCH(RR, ATT_SOFTMAX, true);                                           \
+                break;                                                                            \
+            }                                                                                     \
+        }                                                                                         \
+        if (mode == ATT_SIGMOID) ATT_LAUNCH(RR, ATT_SIGMOID, false);                              \
+        else ATT_LAUNCH(RR, ATT_SOFTMAX, false);                                                  \
         break;
     switch (R) {
         ATT_CASE(1) ATT_CASE(2) ATT_CASE(3) ATT_CASE(4) ATT_CASE(5) ATT_CASE(6) ATT_CASE(7) ATT_CASE(8)
@@ -239,6 +262,7 @@ static int launch_paged_attention(int R, dim3 grid, cudaStream_t s, const T* q, 
         default: return VL_ERR_UNSUPPORTED;
     }
 #undef ATT_CASE
+#undef ATT_LAUNCH
     return vl_launch_status();
 }
 
