@@ -440,6 +440,36 @@ def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
     assert (many[1].float() - want).abs().max() < (2 ** -8 if act == torch.bfloat16 else 2 ** -18) * want.abs().max()
 
 
+# the router's product on tiles of 16 and of 64 rows: a row's bits do not depend on how many rows there are (the taller tiles begin at 1,536 rows of
+# eight parts of K, 3,009 of four, 12,225 of one, with up to 64 columns), remainders in rows and columns
+@pytest.mark.parametrize("K,N,sizes", [(2048, 32, (1535, 1536, 1537)), (1024, 40, (3008, 3009, 3073)), (264, 8, (12224, 12225)), (1024, 130, (1535, 1536, 1600))])
+def test_router_product_holds_the_same_bits_on_both_tiles(K, N, sizes):
+    gen = torch.Generator(device=DEV).manual_seed(K)
+    h = torch.randn(sizes[-1], K, device=DEV, generator=gen).to(torch.bfloat16)
+    router, parts = torch.randn(N, K, device=DEV, generator=gen).to(torch.bfloat16), ops().router_slices(K)
+
+    def run(rows):
+        sums = torch.full((parts, rows, N), float("nan"), device=DEV)
+        ids, w = torch.empty(rows, 1, dtype=torch.int32, device=DEV), torch.empty(rows, 1, device=DEV)
+        ops().moe_route(h[:rows], router, 1, ids, w, sums)
+        return sums
+
+    few = run(16)
+    for rows in sizes:
+        sums = run(rows)
+        assert torch.equal(sums[:, :16], few)
+        # (another tile's remainder: the last rows by themselves)
+        assert torch.equal(sums[:, rows - 1], run_rows(h[rows - 1:rows], router, parts))
+        ref, size = h[:rows].double() @ router.double().T, h[:rows].double().abs() @ router.double().abs().T
+        assert bool(((sums.double().sum(0) - ref).abs() <= K * 2.0 ** -24 * size).all())      # K roundings of sums that stay below it
+
+
+def run_rows(h, router, parts):
+    sums = torch.empty(parts, h.shape[0], router.shape[0], device=DEV)
+    ops().moe_route(h.contiguous(), router, 1, torch.empty(h.shape[0], 1, dtype=torch.int32, device=DEV), torch.empty(h.shape[0], 1, device=DEV), sums)
+    return sums[:, 0]
+
+
 def test_a_row_of_nan_is_routed_to_experts_that_exist():
     T, K, E, top = 5, 64, 40, 4
     gen = torch.Generator(device=DEV).manual_seed(5)

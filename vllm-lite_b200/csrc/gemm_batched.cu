@@ -639,9 +639,10 @@ extern "C" int vl_gemm_rows_f32w(const void* A, int a_dtype, const void* W, int 
     cudaStream_t s = (cudaStream_t)stream;
     if (a_dtype == VL_BF16 && w_dtype == VL_BF16 && gm_aligned(A, W, Kc, K, K, Kc, Kc, 0) && !vl_batched_simt_only()) {
         // both operands bfloat16: their products are exact in float32, the tensor cores add them in float32
-        // many rows: taller tiles, which all run at once, each of a few steps of K (3,281 x 32 x 2,048: 13.9 us with 16 rows, 8.2 with
-        // 64; 1,024 rows 5.6 and 6.7, 2,048 rows 9.8 and 7.3; an element's sum runs over K in the same steps)
-        if (M >= 1536) {
+        // many rows: taller tiles, each of a few steps of K (3,281 x 32 x 2,048: 13.9 us with 16 rows, 8.2 with 64; 2,048 rows 9.8 and 7.3;
+        // an element's sum runs over K in the same steps).  There have to be enough of them: 128 blocks, 2,048 x 32 x 1,024 in four parts, take
+        // 10.8 us, tiles of 16 rows 9.8, and 1,024 rows in eight 6.7 and 5.6
+        if (M >= 1536 && (long long)((M + 63) / 64) * grid.x * slices >= 192) {
             grid.y = (M + 63) / 64;
             return launch_mma_kernel<64, float>(grid, s, Kc, (const bf16*)A, (const bf16*)W, C, M, N, Kc, K, K, N, (long long)Kc,
                                                 (long long)Kc, cs, (const int*)nullptr, 0ll, (const int*)nullptr, 1,
