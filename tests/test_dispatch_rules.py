@@ -85,3 +85,26 @@ def test_counters_are_zero_again_behind_an_error_that_was_raised():
     assert not counters.any() and int(runner.err) == 0
     assert runner.workspace.zeros("attn.arrivals", 5, torch.int32) is counters and bool((kept == 3).all())
     runner.check_device_errors()                         # nothing left to raise
+
+
+# single slots, one run, a few runs, scattered ones (the last of the pool and the first among them), a list in no order
+@pytest.mark.parametrize("slots", [[], [5], [3, 4, 5, 6], [9, 1, 0], [0, 2, 4, 6], list(range(63, -1, -2)), list(range(64)), [63, 0, 31, 7, 8, 12]])
+def test_fresh_slots_are_zeroed_in_few_launches(slots):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from vllm_lite_b200.cache.storage import CacheStorage
+    writes = []
+
+    class Count(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if any(name in str(func) for name in ("zero_", "fill_", "index_put_", "copy_")):
+                writes.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    state = [torch.full((2, 64, 3), 7.0), torch.full((1, 64, 2, 2), 7, dtype=torch.int32), torch.full((3, 64), 7.0, dtype=torch.bfloat16)]
+    with Count():
+        CacheStorage.zero_slots(SimpleNamespace(state=state), slots)
+    for t in state:
+        for s in range(64):
+            assert bool((t[:, s] == (0 if s in slots else 7)).all()), s
+    assert len(writes) <= 3 * len(state)

@@ -15,6 +15,7 @@ import torch
 from ..parts.base import CallCache
 from .manager import CacheLayout
 
+FILL_RUNS = 3        # most runs of neighbouring slots that are filled one by one
 _STATE_DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
 
 
@@ -46,15 +47,23 @@ class CacheStorage:
     def zero_slots(self, slots):
         if not slots:
             return
-        runs = []                                    # of neighbouring slots: a fill each, and no list of indices to upload (which waits)
+        runs = []                                    # of neighbouring slots: a fill each, and no list of indices to upload
         for s in sorted(slots):
             if runs and runs[-1][1] == s:
                 runs[-1][1] = s + 1
             else:
                 runs.append([s, s + 1])
-        for t in self.state:
-            for lo, hi in runs:
-                t[:, lo:hi].zero_()
+        if len(runs) <= FILL_RUNS:
+            for t in self.state:
+                for lo, hi in runs:
+                    t[:, lo:hi].zero_()
+        elif self.state:
+            # scattered slots: one launch a tensor, the list uploaded once and, from pinned memory, without waiting for the steps before
+            index, device = torch.tensor(sorted(slots)), self.state[0].device
+            if device.type == "cuda":
+                index = index.pin_memory().to(device, non_blocking=True)
+            for t in self.state:
+                t.index_fill_(1, index, 0)
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in self.paged + self.state)
