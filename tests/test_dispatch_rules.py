@@ -108,3 +108,19 @@ def test_fresh_slots_are_zeroed_in_few_launches(slots):
         for s in range(64):
             assert bool((t[:, s] == (0 if s in slots else 7)).all()), s
     assert len(writes) <= 3 * len(state)
+
+
+@pytest.mark.parametrize("counts,heads,dim,pays", [
+    ([95, 40], 32, 64, False), ([96], 32, 64, False), ([96, 96], 32, 64, True), ([127], 32, 64, False), ([128], 8, 64, True),
+    ([96] * 4, 8, 64, False), ([96] * 8, 8, 64, True), ([96, 1, 1, 1, 1, 1, 1, 1], 8, 64, False), ([128, 96], 4, 64, True),
+    ([96], 16, 128, False), ([159], 16, 128, False), ([160], 16, 128, True), ([96], 24, 128, True), ([96, 96], 16, 128, True),
+    ([223], 8, 128, False), ([224], 4, 96, True), ([127], 32, 32, False), ([128], 128, 32, True), ([191, 128], 128, 32, False),
+    ([192, 128], 128, 32, True), ([], 32, 64, False)])
+def test_which_portions_of_a_time_mixing_are_cut_into_chunks(counts, heads, dim, pays):
+    assert ops.decay_chunks_pay(counts, heads, dim) is pays
+
+
+@pytest.mark.parametrize("tokens,heads,dim,pays", [(1, 4, 64, True), (1, 32, 32, True), (1, 16, 128, False), (2, 16, 128, False),
+                                                   (3, 16, 128, True), (1, 32, 128, False), (2, 32, 128, True), (4, 8, 96, False), (5, 8, 96, True)])
+def test_which_single_tokens_of_a_time_mixing_take_a_block_a_head(tokens, heads, dim, pays):
+    assert ops.decay_step_pays(tokens, heads, dim) is pays

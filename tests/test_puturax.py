@@ -511,6 +511,62 @@ def test_time_mixing_in_portions_and_slots(dtype, H_, D_, rank, W):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("H_,D_,rank,W", [(4, 32, 16, 128), (2, 64, 8, 96), (1, 128, 4, 64)])
+def test_time_mixing_of_long_portions_beside_short_ones(H_, D_, rank, W):
+    """bfloat16 steps that hold portions on both sides of a chunk's least length, in every order, then single tokens: long ones go through
+    the chunked kernels, the others through the walk, whose norm also passes over the long ones' rows first.  Every buffer begins as NaN.
+    The outputs against the float64 mixer; the states against a run of the same steps that only walks."""
+    from vllm_lite_b200.csrc import ops
+    from vllm_lite_b200.parts import spec as S
+    from vllm_lite_b200.parts.base import CallCache, Entry, Workspace
+
+    class Fresh(Workspace):
+        def get(self, tag, shape, dtype):
+            known = (tag, dtype) in self._buffers
+            t = super().get(tag, shape, dtype)
+            return t if known or not t.is_floating_point() else t.fill_(float("nan"))
+
+    spec = S.TimeMixSpec(W, H_, D_, rank, 1e-5)
+
+    def edit(t):
+        t["w0"] = (t["w0"].float() * 2 - 2.0).to(torch.bfloat16)
+        for m in "rkvgw":
+            t["mu." + m] = (t["mu." + m].float().abs().clamp(max=1.0)).to(torch.bfloat16)
+
+    part, tensors = build_part(spec, torch.bfloat16, 81, edit=edit)
+    need, slots = type(part).cache_need(spec), [3, 0, 2]
+    steps = [[1, 130, 95], [96, 230, 1], [224, 1, 0], [96, 0, 0], [0, 127, 240], [1, 1, 1], [1, 1, 1]]
+    h = [rand((sum(s[b] for s in steps), W), 82 + b, torch.bfloat16) for b in range(3)]
+    cut = []
+
+    def run(with_entries):
+        state, at, got = torch.zeros((4,) + need.shape, dtype=torch.float32, device=DEV), [0] * 3, [[], [], []]
+        for lens in steps:
+            live = [b for b in range(3) if lens[b]]
+            n = [lens[b] for b in live]
+            step = mini_step(n, [slots[b] for b in live], [at[b] for b in live])
+            step.workspace = Fresh(torch.device(DEV))
+            if with_entries:
+                step.entries = [Entry(b, at[b], lens[b], slots[b]) for b in live]
+                cut.append(ops.decay_chunks_of(n) > 0 and ops.decay_chunks_pay(n, H_, D_))
+            rows = torch.cat([h[b][at[b]:at[b] + lens[b]] for b in live]).contiguous()
+            out = part(rows, step, CallCache(state=state)).clone()
+            for b, rows in zip(live, out.split(n)):
+                got[b].append(rows)
+                at[b] += lens[b]
+        return [torch.cat(g) for g in got], state
+
+    got, state = run(True)
+    _, walked = run(False)
+    assert cut == [D_ <= 64, True, True, False, True, False, False]
+    for b in range(3):
+        close(got[b], P.time_mixing(h[b].double().cpu(), tensors, dict(heads=H_, dim=D_), 1e-5), torch.bfloat16, f"request {b}", tol=3e-2)
+        # float32 sums in another order: hundreds of terms, each rounded to 2^-24 of sums of their size
+        assert float((state[slots[b]] - walked[slots[b]]).norm()) <= 2.0 ** -17 * float(walked[slots[b]].norm())
+    assert not state[1].any()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H_,G_,D_,V_,every", [(4, 2, 16, 24, 4), (3, 3, 20, 6, 1), (8, 2, 64, 48, 7), (2, 1, 128, 128, 100), (1, 1, 6, 20, 3)])
 def test_head_norms_query_factor_and_value_norm(dtype, H_, G_, D_, V_, every):

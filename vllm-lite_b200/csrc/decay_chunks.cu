@@ -14,7 +14,8 @@
 // multiply their few decays directly.  The products (2,016 pairs x D in a chunk, then 64 x 64 x P, 64 x D x P twice) are plain
 // multiply-adds on tiles in shared memory, which is what bounds (1) and (3).
 // One request of 2,048 tokens, 32 heads of 64 x 64: 119 us with the norm and the gate, against 413 for the walk and the norm's kernel
-// behind it; 128 x 128: 395 against 1,193; 512 tokens: 37 against 107; 64 tokens: 27 against 18: a lone portion wins from about 100 tokens on.
+// behind it; 128 x 128: 395 against 1,193; 512 tokens: 37 against 107; 64 tokens: 27 against 18.  A lone portion wins from 100 to 220 tokens on, by the
+// heads' number and size (the caller decides; ops.decay_chunks_pay has the measurements).
 #include "common.cuh"
 #include "chunk_index.cuh"
 

@@ -1815,6 +1815,32 @@ def decay_chunks_of(counts) -> int:
     return sum(-(-n // DECAY_CHUNK) for n in counts if n >= DECAY_MIN_CHUNK)
 
 
+def decay_chunks_pay(counts, H, D) -> bool:
+    """Whether a step's long portions are worth cutting into chunks: whether the longest has the tokens at which the walk falls behind.
+    A launch of few heads takes 26 us in chunks (50 with heads of more than 64); the walk is slowed down by many heads, large ones first,
+    and the chunks by a portion's short last one.  Measured, walk and norm / chunks, us, `heads` those of all long portions:
+      heads of 128: 8 heads, 192 tokens 46.9 / 50.0, 16: 129 43.4 / 50.8, 160 53 / 51, 24: 96 60.2 / 52.3, 32: 96 62.9 / 54.4;
+      heads of 96: 8 heads, 192 tokens 45.9 / 43.6, 16: 160 43.8 / 43.9, 32: 96 56.8 / 44.9;
+      heads of 64: 8 heads, 96 tokens 21.6 / 25.9, 128 26.9 / 26.3, 32: 96 23.4 / 25.7, 128 30.0 / 26.4, 64: 96 29.8 / 27.7;
+      heads of 32: 32 heads, 96 tokens 20.0 / 21.8, 128 25.7 / 22.6, 128: 128 32.8 / 28.2, 256: 144 51.0 / 62.7, 192 66.3 / 63.2."""
+    long = [n for n in counts if n >= DECAY_MIN_CHUNK]
+    heads = len(long) * H
+    if D > 64:
+        least = DECAY_MIN_CHUNK if heads >= 24 else (160 if heads >= 16 else 224)
+    elif D > 32:
+        least = DECAY_MIN_CHUNK if heads >= 64 else 128
+    else:
+        least = 128 if heads <= 128 else 192
+    return max(long, default=0) >= least
+
+
+def decay_step_pays(tokens, H, D) -> bool:
+    """Whether `decay_step` serves a step of single tokens better than the walk and the norm behind it: a block owns a whole head, and
+    few large heads leave most SMs idle (walk and norm / step, us: 16 heads of 128, 1 token 5.7 / 7.9, 2: 7.5 / 8.5, 3: 9.6 / 8.6; 8 heads
+    of 96, 3 tokens 5.7 / 7.0, 4: 7.0 / 7.0; 16 of 64, 1 token 4.7 / 3.4)."""
+    return D <= 64 or tokens * H > 32
+
+
 def decay_chunk_floats(chunks, H, D, P) -> int:
     """Floats of `decay_chunks`' scratch."""
     return chunks * H * (2 * D * P + DECAY_CHUNK * (D + P) + D)

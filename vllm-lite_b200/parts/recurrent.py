@@ -305,9 +305,10 @@ class TimeMix:
         # bfloat16 steps work long portions off in chunks (float32 as the walk, but the order of the sums follows the cut, which the
         # float32 engine's results must not); the walk serves the others and is then told to leave the long ones alone
         counts = [e.count for e in step.entries]
-        chunks = ops.decay_chunks_of(counts) if self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D) else 0
+        fast = self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D)
+        chunks = ops.decay_chunks_of(counts) if fast and ops.decay_chunks_pay(counts, H, D) else 0
         scan = (r, 0), (k, 0), (v, 0), (w, 0), self.u, cache.state, W, step.cu_seqlens, step.state_slots
-        if self.dtype == torch.bfloat16 and ops.decay_chunks_ok(D, D) and step.max_query_len == 1:
+        if fast and step.max_query_len == 1 and ops.decay_step_pays(T, H, D):
             ops.decay_step(*scan, g, 0, self.norm, s.eps, gated, H, D, D)        # single tokens: the norm and the gate in the same launch
             return self.o_proj(gated, step, "tm.out")
         if not chunks or min(counts) < ops.DECAY_MIN_CHUNK:
