@@ -124,3 +124,15 @@ def test_which_portions_of_a_time_mixing_are_cut_into_chunks(counts, heads, dim,
                                                    (3, 16, 128, True), (1, 32, 128, False), (2, 32, 128, True), (4, 8, 96, False), (5, 8, 96, True)])
 def test_which_single_tokens_of_a_time_mixing_take_a_block_a_head(tokens, heads, dim, pays):
     assert ops.decay_step_pays(tokens, heads, dim) is pays
+
+
+@pytest.mark.parametrize("heads,dim", [(32, 64), (16, 128), (2, 16), (7, 100)])
+def test_only_bfloat16_steps_reserve_room_for_chunks_of_a_time_mixing(heads, dim):
+    from vllm_lite_b200.cache.sizing import _mixer_width
+    from vllm_lite_b200.parts.spec import TimeMixSpec
+    spec, tokens = TimeMixSpec(heads * dim, heads, dim, 16, 1e-5), 4096
+    walk = _mixer_width(spec, 4)
+    assert walk == 5 * spec.hidden_size + 12 * heads * dim - heads * dim + 32        # the products, mixes, gate and rows alone
+    for n in (96, 129, 200, 1000, 4096):                 # portions whose last chunks are as short as they come, and one long one
+        chunks = ops.decay_chunks_of([n] * (tokens // n))
+        assert 4 * ops.decay_chunk_floats(chunks, heads, dim, dim) <= 2 * (_mixer_width(spec, 2) - walk) * tokens

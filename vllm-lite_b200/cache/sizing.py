@@ -33,18 +33,18 @@ def state_bytes(layout: CacheLayout, max_requests: int) -> int:
     return total
 
 
-def _mixer_width(mixer) -> int:
-    """Elements per token of a mixer's intermediates (float32 buffers count twice), a bound for the reserve."""
+def _mixer_width(mixer, itemsize: int = 2) -> int:
+    """Elements (of `itemsize` bytes) per token of a mixer's intermediates (float32 buffers count twice), a bound for the reserve."""
     if mixer is None:
         return 0
     if hasattr(mixer, "inner"):                                         # a mixer behind a token shift: the mixed rows
-        return _mixer_width(mixer.inner) + getattr(mixer, "hidden_size", 0)
+        return _mixer_width(mixer.inner, itemsize) + getattr(mixer, "hidden_size", 0)
     if hasattr(mixer, "conv") and hasattr(mixer, "num_kv_heads") and hasattr(mixer, "head_dim"):
         # attention behind convolutions: the stacked projection, its convolved float32 copy, queries and context
         hd = -(-mixer.head_dim // 16) * 16
         return (mixer.num_heads + mixer.num_kv_heads) * mixer.head_dim * 3 + mixer.num_heads * (2 * hd + 1)
     if hasattr(mixer, "left") and hasattr(mixer, "right"):              # two mixers side by side, plus their sum
-        return _mixer_width(mixer.left) + _mixer_width(mixer.right) + 2 * getattr(mixer.left, "hidden_size", 0)
+        return _mixer_width(mixer.left, itemsize) + _mixer_width(mixer.right, itemsize) + 2 * getattr(mixer.left, "hidden_size", 0)
     if hasattr(mixer, "num_kv_heads") and hasattr(mixer, "head_dim"):
         hd = max(mixer.head_dim, getattr(mixer, "v_head_dim", None) or 0)
         gate = mixer.num_heads if getattr(mixer, "gate", None) else 0  # an output gate as wide as the heads
@@ -77,9 +77,9 @@ def _mixer_width(mixer) -> int:
         return (2 * hd + 2 * hp + 2 * mixer.num_heads) + 2 * hp + hp
     if hasattr(mixer, "decay_rank") and not hasattr(mixer, "gate_rank"):
         # time mixing: five mixes of the input, r, k, v and the raw decay in float32, the gate, the scan's result, the gated rows
-        # ... and, in chunks of 64 tokens (a portion's last one may be short), per head two states, two rows a token and one
+        # ... and in bfloat16, in chunks of 64 tokens (a portion's last one may be short), per head two states, two rows a token and one
         hd = mixer.num_heads * mixer.dim
-        chunks = 2 * 2 * mixer.num_heads * (2 * mixer.dim * mixer.dim // 64 + 2 * mixer.dim + mixer.dim // 64 + 1)
+        chunks = 2 * 2 * mixer.num_heads * (2 * mixer.dim * mixer.dim // 64 + 2 * mixer.dim + mixer.dim // 64 + 1) if itemsize == 2 else 0
         return 5 * mixer.hidden_size + 8 * hd + hd + 2 * mixer.decay_rank + 2 * hd + hd + chunks
     if hasattr(mixer, "unit_eps") and not hasattr(mixer, "decay_rank"):
         # delta rule with one decay per head: one product (with the gate, two numbers a head and up to 7 rows of padding), its
@@ -105,7 +105,7 @@ def activation_reserve(plan, max_step_tokens: int, max_requests: int, max_contex
     for block in plan.layers:
         mixer, ffn = getattr(block, "mixer", None), getattr(block, "ffn", None)
         streams = max(streams, int(getattr(block, "streams", 1) or 1))
-        w = _mixer_width(mixer)
+        w = _mixer_width(mixer, itemsize)
         if hasattr(ffn, "top"):
             # routed experts: every token's row `top` times (sorted copy, gate and up, activation, result), tiles padded
             w += 2 * ffn.top * (3 * ffn.intermediate_size + 2 * H)
