@@ -132,7 +132,7 @@ def test_only_bfloat16_steps_reserve_room_for_chunks_of_a_time_mixing(heads, dim
     from vllm_lite_b200.parts.spec import TimeMixSpec
     spec, tokens = TimeMixSpec(heads * dim, heads, dim, 16, 1e-5), 4096
     walk = _mixer_width(spec, 4)
-    assert walk == 5 * spec.hidden_size + 12 * heads * dim - heads * dim + 32        # the products, mixes, gate and rows alone
+    assert walk == 5 * spec.hidden_size + 12 * heads * dim + 2 * 16        # the products, mixes, gate and rows alone
     for n in (96, 129, 200, 1000, 4096):                 # portions whose last chunks are as short as they come, and one long one
         chunks = ops.decay_chunks_of([n] * (tokens // n))
         assert 4 * ops.decay_chunk_floats(chunks, heads, dim, dim) <= 2 * (_mixer_width(spec, 2) - walk) * tokens
