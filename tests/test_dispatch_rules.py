@@ -136,3 +136,14 @@ def test_only_bfloat16_steps_reserve_room_for_chunks_of_a_time_mixing(heads, dim
     for n in (96, 129, 200, 1000, 4096):                 # portions whose last chunks are as short as they come, and one long one
         chunks = ops.decay_chunks_of([n] * (tokens // n))
         assert 4 * ops.decay_chunk_floats(chunks, heads, dim, dim) <= 2 * (_mixer_width(spec, 2) - walk) * tokens
+
+
+def test_constants_that_the_chunked_time_mixing_and_its_caller_share():
+    import ctypes
+
+    from vllm_lite_b200.csrc import build
+    lib = build.load("decay_chunks")
+    lib.vl_decay_chunk_floats.restype = ctypes.c_longlong
+    assert lib.vl_decay_min_chunk() == ops.DECAY_MIN_CHUNK
+    for sizes in ((1, 1, 4, 4), (7, 32, 64, 64), (3, 5, 100, 68), (4096, 16, 128, 128)):
+        assert lib.vl_decay_chunk_floats(*sizes) == ops.decay_chunk_floats(*sizes)

@@ -365,6 +365,49 @@ def test_paged_attention_holds_the_same_bits_for_few_and_for_many_tokens(hd, dty
         assert bool((run(times) == few).all()), times
 
 
+# the merge of a token's chunks: one, a batch of 128, more than one batch; chunks without keys in between, whose parts may hold anything; a window
+# that begins behind some chunks; padding; sinks; columns of one thread's five and the rest
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("S", [1, 8, 127, 128, 129, 256, 300])
+@pytest.mark.parametrize("hd,window,sink", [(16, None, False), (128, 2100, True), (576, None, True), (640, 500, False)])
+def test_merge_of_chunks(S, hd, window, sink, dtype):
+    nq, chunk, gen = 3, 16, torch.Generator(device=DEV).manual_seed(S + hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    last = [S * chunk - 1, 0, -1, S * chunk // 2, max(S * chunk - 17, 0)]
+    T = len(last)
+    acc, ml = rnd(T, nq, S, hd), torch.stack([3 * rnd(T, nq, S), rnd(T, nq, S).abs() + 0.1], -1)
+    empty = rnd(T, nq, S) < -1
+    for t, p in enumerate(last):                         # chunks behind the last key or before the window are never read
+        lo = max(0, p - window + 1) if window else 0
+        empty[t, :, p // chunk if p >= 0 else 0] = False
+        out_of_reach = torch.ones(S, dtype=torch.bool, device=DEV)
+        out_of_reach[lo // chunk:p // chunk + 1] = p < 0
+        acc[t][:, out_of_reach], ml[t][:, out_of_reach] = float("nan"), float("nan")
+    inside = ~ml[..., 0].isnan() & empty
+    ml[..., 0][inside] = float("-inf")
+    ml[..., 1][inside], acc[inside] = float("nan"), float("nan")
+    pos = torch.tensor(last, dtype=torch.int32, device=DEV)
+    sinks = rnd(nq) if sink else None
+    out = torch.full((T, nq * hd), 7.0, device=DEV, dtype=dtype)
+    o = ops()
+    o._check(o._fn("attention", "vl_decode_attention_merge")(acc.data_ptr(), ml.data_ptr(), pos.data_ptr(), out.data_ptr(), o.dtype_code(dtype), T, nq, hd,
+                                                             chunk, S, window or 0, None, sinks.data_ptr() if sink else None, o._stream()), "merge")
+    m = torch.where(ml[..., 0].isnan(), float("-inf"), ml[..., 0].double())
+    top = m.max(-1, keepdim=True).values.clamp(min=-1e30)
+    w = torch.exp(m - top)
+    parts = torch.where((w > 0)[..., None], acc.double(), 0.0)
+    total = (w * torch.where(w > 0, ml[..., 1].double(), 0.0)).sum(-1)
+    if sink:
+        total = total + torch.exp(sinks.double() - top[..., 0])
+    live = torch.tensor([p >= 0 for p in last], device=DEV)[:, None, None]
+    ref = torch.where(live, (w[..., None] * parts).sum(2) / total[..., None], 0.0)
+    size = torch.where(live, (w[..., None] * parts.abs()).sum(2) / total[..., None], 0.0)
+    # S roundings of float32 sums, weights good to 2^-20 (bfloat16: the fast exponential), the output's rounding
+    rel = (S + 8) * 2.0 ** -24 + 2.0 ** -20
+    got = out.double().view(T, nq, hd)
+    assert bool(((got - ref).abs() <= rel * size + (2.0 ** -8 if dtype == torch.bfloat16 else 0) * ref.abs()).all())
+
+
 # the few-row product of routed experts: items of one block and of several, more items than places, places without rows in between,
 # padding rows, K at a step's edge and not, N at a tile's edge and not
 @pytest.mark.parametrize("N,K", [(16, 512), (144, 520), (4096, 1024), (8192, 2048)])
