@@ -609,9 +609,8 @@ decode_attention_merge_kernel(const float* __restrict__ part_acc, const float* _
     const int s0 = lo / chunk, s1 = pos / chunk;
     const size_t row0 = ((size_t)t * nq + h) * S;
     // The chunks' weights exp(m_s - M), MERGE_CHUNKS at a time in shared memory: a number a thread, then every thread adds up its columns of the
-    // partial results in the order of the chunks, eight reads on their way together.  (Each thread used to make every weight
-    // itself, one read behind the other: 32 chunks of 16 heads of 256, 8 tokens: 15.2 us, now 5.9;
-    // 8 chunks 5.0 and 3.0.)
+    // partial results in the order of the chunks, eight reads on their way together (32 chunks of 16 heads of 256, 8 tokens: 5.9 us, 15.2
+    // where each thread makes every weight itself, one read behind the other; 8 chunks 3.0 and 5.0).
     __shared__ float s_w[MERGE_CHUNKS], s_l[MERGE_CHUNKS], s_m[4];
     const int tid = threadIdx.x;
     float M = -INFINITY;

@@ -9,10 +9,10 @@
 // whatever context the launch was sized for.  A block's run is a few pieces of items; an item that lies in one block's run is
 // finished there, the others leave unnormalised partial results with their maximum and sum, which the block that arrives
 // last at the item's counter adds up in the order of the pieces.  No run is shorter than an item's pieces in the scratch
-// allow (S of them).  Where the cuts lie follows from the lengths alone.
-// The blocks used to take (token, KV head, chunk of 1,024 keys) items in turn, chunk fastest, 148 apart: with 2 or 4 chunks to
-// a token a block met the same chunk of every token, and requests shorter than the context bound left half of the
-// blocks without work (64 requests of 400 to 1,500 keys, bound 2,048, 8 KV heads of 128: 78.5 us with the merge's launch, now 55.9).
+// allow (S of them).  Where the cuts lie, and with them the last bits of a result, follows from the lengths of all requests, the number of
+// blocks and S: the same request beside others, or in a step sized for another bound, may differ by rounding.
+// (Dealing out (token, KV head, chunk of 1,024 keys) items in turn leaves half of the blocks without work where requests are shorter
+// than the bound: 64 requests of 400 to 1,500 keys, bound 2,048, 8 KV heads of 128: 78.5 us with the merge's launch, 55.9 in equal runs.)
 //   warp 4   producer: looks up the pages of a piece and copies its K and V rows, 64 keys a
 //        stage, by TMA boxes (cp.async.bulk.tensor.3d, 128-byte swizzle, one box per page: its blocks
 //        of 64 columns one after the other) into a ring of stages that runs on across work items; it also brings the item's
@@ -24,10 +24,10 @@
 //        a piece the four are merged through shared memory in warp order and written as the item's
 //        result or as a partial one.
 // Keys outside the item's range are masked by position; pages outside it, or that the block table
-// does not hold, are fetched from beyond the end of the tensor (zeros); rows of V behind the
-// request's last key are zeroed in shared memory (another request's leftovers may be anything).
-// Every wait on an mbarrier is bounded; when one expires the block records VL_DEV_WAIT_EXPIRED and
-// stops.
+// does not hold, are fetched from beyond the end of the tensor (zeros); the values of keys
+// behind the request's last one are cleared as fragments (another request's leftovers may be anything).
+// Every wait on an mbarrier is bounded; when one expires the block's consumers give up together, the block records
+// VL_DEV_WAIT_EXPIRED and stops.  It has then not counted its pieces: whoever clears the error zeroes the counters too.
 #include "tc5.cuh"
 
 #ifndef FA_HD

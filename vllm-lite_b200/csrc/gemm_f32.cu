@@ -10,9 +10,9 @@
 // What bounds it: for few rows the latency of the weights' way in, for many the multiply-adds.  Tiles of A and W come
 // in by cp.async, a ring of STAGES steps of BK columns, so that a small product asks for everything at once and a large
 // one never waits for memory between its steps; both stay k-fastest in shared memory, rows BK + 4 floats apart (a
-// quarter warp's 16-byte reads then meet no bank twice), and a thread takes four values of k per read.  The product
-// it replaces waited for one step of 16 columns after another: 8 x 320 x 96 8.0 us, now 2.9; 8 x 96 x 256 19.2 and 4.7; 1 x 4,096
-// x 4,096 292 and 60; 64 x 6,144 x 4,096 453 and 178; 1,024 x 4,096 x 4,096 1,508 and 902 (38 TFLOP/s).
+// quarter warp's 16-byte reads then meet no bank twice), and a thread takes four values of k per read.  Measured, and beside it
+// tiles of 64 x 64 without the ring, one step of 16 columns after another: 8 x 320 x 96 2.9 us and 8.0; 8 x 96 x 256 4.7 and 19.2; 1 x 4,096
+// x 4,096 60 and 292; 64 x 6,144 x 4,096 178 and 453; 1,024 x 4,096 x 4,096 902 (38 TFLOP/s) and 1,508.
 #include "common.cuh"
 
 __device__ __forceinline__ void gf_copy(float* smem, const float* gmem, int bytes, bool wide) {   // the rest of 16 (4) bytes: zeros

@@ -1,8 +1,10 @@
 """Chooses the attention kernel for a step.
 
 Every kernel computes the same function of (query token, its request's pages);
-which one runs depends on the dtype and on the shape of the step only.  The
-float32 path always takes the one kernel whose order of additions depends on
+which one runs depends on the dtype and on the shape of the step only.  In bfloat16
+the order of a sum may depend on more: the streaming decode kernel cuts the keys of
+all requests into equal runs, so a request's last bits follow the lengths of its neighbours
+(within rounding).  The float32 path always takes the one kernel whose order of additions depends on
 positions alone, so its results are bit-for-bit independent of the batch.  In
 bfloat16 the tensor-core kernels run: requests that bring one token (decoding)
 go to the kernel that splits each token's key range over many blocks, requests
