@@ -777,8 +777,8 @@ def flash_decode(qkv, out, k_cache, v_cache, block_table, req_index, positions, 
                  head_bias=None, gate=None, softcap=None, distance=None, keep=None, numbered=False, settled=False):
     """Tensor-core version of `decode_attention` (bfloat16): every block takes a chunk of a token's
     keys; the chunks are merged by the block that finishes last (`arrivals`: int32 counters,
-    `flash_decode_arrivals` of them, zero before the first call and left zero) or, without
-    `arrivals`, by a second kernel.
+    `flash_decode_arrivals` of them, zero before the first call and left zero; a launch that reports an expired
+    wait in `err` may leave others, and they have to be zeroed with it) or, without `arrivals`, by a second kernel.
     The split pass is the persistent TMA kernel where `flash_decode_streams` says so (`stream_kernel`: None =
     that rule, True / False to force; it merges in the same launch, with as many partial results a token as the scratch
     has room for), else a block per chunk.
