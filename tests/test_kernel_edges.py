@@ -47,7 +47,7 @@ def test_silu_mul_layouts(T, I, group, dtype):
 @pytest.mark.parametrize("T,I,group", [(3, 64, 0), (3, 64, 8), (5, 36, 4), (409, 480, 24), (410, 480, 24), (410, 792, 0), (415, 792, 8), (300, 1100, 0)])
 @pytest.mark.parametrize("act", ["silu", "relu", "capped"])
 def test_gated_activations_by_ones_and_by_eights(T, I, group, act, dtype):
-    o, alpha = ops(), 1.7 if act == "capped" else 1.0
+    o, alpha = ops(), float(torch.tensor(1.7)) if act == "capped" else 1.0       # 1.7 as the kernel gets it, in float32
     gu, out = (torch.randn(T, 2 * I, device=DEV) * 4).to(dtype), torch.empty(T, I, device=DEV, dtype=dtype)
     bias = torch.randn(2 * I, device=DEV) if act == "capped" else None
     o._check(o._fn("activation", "vl_gated_act")(gu.data_ptr(), out.data_ptr(), o.dtype_code(dtype), T, I, group, ("silu", "relu", "capped").index(act),
@@ -57,8 +57,8 @@ def test_gated_activations_by_ones_and_by_eights(T, I, group, act, dtype):
     if act == "capped":
         g, u = g.clamp(max=5), u.clamp(-5, 5) + 1
     ref = g.clamp(min=0) * u if act == "relu" else g / (1 + torch.exp(-alpha * g)) * u
-    # the exponential's argument is rounded, an error of alpha |g| 2^-24 in its result; a handful of roundings more, and the output's own (eight
-    # bits: at most 2^-8 of the number)
+    # the exponential's argument is rounded, an error of alpha |g| 2^-24 in its result; a handful of roundings more (at most 8 x 2^-24: the
+    # exponential 2^-22, the sum, the quotient, u + 1, the product), and the output's own (eight bits: at most 2^-8 of the number)
     rel = (alpha * float(g.abs().max()) + 8) * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)
     assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())
 
