@@ -40,6 +40,15 @@ def test_the_paired_product_has_no_path_to_dependent_launch():
         assert 0 < body.index("pdl_wait();") < body.index("alloc"), name
 
 
+def test_the_grouped_product_of_paired_blocks_has_no_path_to_dependent_launch():
+    import re
+    code = re.sub(r"//[^\n]*", "", (build.CSRC / "gemm_tc5_grouped.cu").read_text())
+    assert "ProgrammaticStreamSerialization" not in code and "vl_launch(" not in code and "vl_pdl_enabled" not in code
+    assert re.search(r"cfg\.numAttrs\s*=\s*1\s*;", code) and code.count("numAttrs") == 1 and code.count("cudaLaunchKernelEx") == 1
+    body = code[code.index("__global__"):]
+    assert 0 < body.index("pdl_wait();") < body.index("alloc_pair")
+
+
 def test_dependent_launch_is_off_until_switched_on():
     assert ops._pdl is False or ops._pdl_libs            # the module's default; a test before may have stepped
     for name, defines in kernel_libraries():

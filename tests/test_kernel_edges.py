@@ -535,3 +535,52 @@ def test_embedding_rows(H, offset, dtype):
     want = table.float()[ids.long().clamp(0, V - 1)] * 3.0
     want[3:5] = 0
     assert torch.equal(out, want) and int(err) != 0
+
+
+# the many-row product of routed experts: groups without rows, of less than a tile, at its edges and of several; fewer tiles than
+# pairs of SMs and more; N below, at and beside a tile's edge, K with a short last block
+@pytest.mark.parametrize("sizes", [[0, 16, 0, 256, 272, 0], [32, 240, 256, 16, 48], [700, 0, 1333, 5], [3] * 40, [0, 0, 2048]])
+@pytest.mark.parametrize("N,K", [(16, 72), (192, 1096), (512, 2048), (2064, 520)])
+@pytest.mark.parametrize("act", [None, "silu", "relu", "capped_swish", "relu2"])
+def test_experts_product_of_many_rows(sizes, N, K, act):
+    G = len(sizes)
+    gen = torch.Generator(device=DEV).manual_seed(N + K + sum(sizes))
+    starts = [0]
+    for n in sizes:
+        starts.append(starts[-1] + -(-n // 16) * 16)
+    cap = starts[-1] + 32                                # rows behind the last group, which nobody writes
+    rows = torch.randn(cap, K, device=DEV, generator=gen).to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device=DEV, generator=gen) / K ** 0.5).to(torch.bfloat16)
+    scale = torch.rand(cap, device=DEV, generator=gen) if act == "silu" else None
+    index = torch.randperm(cap, device=DEV, generator=gen).to(torch.int32) if act == "silu" else None
+    gated = act in ("silu", "relu", "capped_swish")
+    e = torch.zeros(1, dtype=torch.int32, device=DEV)
+    start_rows = torch.tensor(starts, dtype=torch.int32, device=DEV)
+    outs = []
+    for _ in range(2):
+        out = torch.full((cap, N // 2 if gated else N), 7.0, device=DEV, dtype=torch.bfloat16)
+        ops().gemm_grouped_tc5(rows, w, out, start_rows, e, index, scale, act, 1.5, 0.8, 0.25)
+        outs.append(out)
+    assert int(e.item()) == 0 and torch.equal(outs[0], outs[1])
+    assert bool((outs[0][starts[-1]:] == 7.0).all())
+    for g in (g for g in range(G) if sizes[g]):
+        at = slice(starts[g], starts[g + 1])
+        s = scale.double()[index[at].long()][:, None] if scale is not None else 1.0
+        z = (rows[at].double() @ w[g].double().T) * s
+        off = K * 2.0 ** -24 * (rows[at].double().abs() @ w[g].double().abs().T) * s        # float32 sums
+        if gated:
+            z, off = z.view(z.shape[0], -1, 2, 8), off.view(z.shape[0], -1, 2, 8)
+            p, u = z[:, :, 0].reshape(z.shape[0], -1), z[:, :, 1].reshape(z.shape[0], -1)
+            op, ou = off[:, :, 0].reshape(z.shape[0], -1), off[:, :, 1].reshape(z.shape[0], -1)
+            if act == "relu":
+                z, off = p.clamp(min=0) * u, op * u.abs() + p.abs() * ou + op * ou
+            else:
+                a, shift = 1.0, 0.0
+                if act == "capped_swish":
+                    a, shift, p, u = 1.5, 0.25, p.clamp(max=0.8), u.clamp(-0.8, 0.8)
+                # |d/dp p sigmoid(a p)| <= 1.1; sigmoid by the fast exponential and a division: a few roundings
+                z, off = p / (1 + torch.exp(-a * p)) * (u + shift), 1.2 * op * (u + shift).abs() + p.abs() * ou + 2.0 ** -20 * (p * (u + shift)).abs()
+        elif act == "relu2":
+            off = 2 * z.abs() * off + off * off
+            z = z.clamp(min=0) ** 2
+        assert bool(((outs[0][at].double() - z).abs() <= 2.0 ** -8 * z.abs() + off + 1e-6).all()), g

@@ -141,7 +141,8 @@ moe_route_kernel(const float* __restrict__ z, int slices, int ntok, int E, int l
 
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ ids, int npairs, int E, int bm, int cap, int max_tiles,
-                 int* __restrict__ sorted_rows, int* __restrict__ tile_group, int* __restrict__ place) {
+                 int* __restrict__ sorted_rows, int* __restrict__ tile_group, int* __restrict__ place,
+                 int* __restrict__ starts) {
     __shared__ int s_count[MOE_MAX_EXPERTS];
     __shared__ int s_start[MOE_MAX_EXPERTS];
     pdl_launch_dependents();
@@ -167,11 +168,13 @@ moe_align_kernel(const int* __restrict__ ids, int npairs, int E, int bm, int cap
             for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (tid >= o) x += y; }
             if (e < E) {
                 s_start[e] = (at + x - tiles) * bm;
+                if (starts) starts[e] = (at + x - tiles) * bm;
                 for (int y = 0; y < tiles; ++y) tile_group[at + x - tiles + y] = e;
                 s_count[e] = 0;                          // now the cursor of the expert's rows
             }
             at += __shfl_sync(0xffffffffu, x, 31);
         }
+        if (starts && tid == 0) starts[E] = at * bm;
     }
     __syncthreads();
     for (int p = tid; p < npairs; p += 1024) {
@@ -274,14 +277,14 @@ extern "C" int vl_moe_route(const float* z, int slices, int T, int E, int ldz, i
 }
 
 // cap = rows of the sorted buffer (a multiple of bm, at least npairs rounded up per expert: npairs + E * (bm - 1)
-// rounded up to bm is always enough); max_tiles = cap / bm.
+// rounded up to bm is always enough); max_tiles = cap / bm.  starts (optional, [E + 1]): the first row of every expert.
 extern "C" int vl_moe_align(const int* ids, int npairs, int E, int bm, int cap, int* sorted_rows, int* tile_group,
-                            int* place, void* stream) {
+                            int* place, int* starts, void* stream) {
     if (npairs <= 0) return VL_OK;
     if (E <= 0 || E > MOE_MAX_EXPERTS || bm <= 0 || cap % bm || cap < npairs) return VL_ERR_ARGUMENT;
     if ((long long)cap < (long long)npairs + (long long)min(E, npairs) * (bm - 1)) return VL_ERR_ARGUMENT;
     return vl_launch(moe_align_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, ids, npairs, E, bm, cap, cap / bm,
-                     sorted_rows, tile_group, place);
+                     sorted_rows, tile_group, place, starts);
 }
 
 extern "C" int vl_moe_gather(const void* h, int dtype, const int* sorted_rows, const float* weights, int cap, int top,

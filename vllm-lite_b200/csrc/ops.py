@@ -127,7 +127,7 @@ _SIGNATURES = {
     ("gemm_batched", "vl_gemm_rows_f32w"): [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("gemm_tc5_grouped", "vl_gemm_bf16_tc5_grouped"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                                        c_void_p, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
-    ("moe", "vl_moe_align"): [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+    ("moe", "vl_moe_align"): [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     ("moe", "vl_moe_gather"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ("moe", "vl_moe_combine"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_void_p, c_void_p],
@@ -1259,41 +1259,52 @@ def moe_route(h, router, top, ids, weights, logits, score="sigmoid", renormalize
            "vl_moe_route")
 
 
-TC5_GROUPED_TILE = 128    # rows per tile of the grouped tcgen05 product
+TC5_GROUPED_TILE = 16     # the groups' rows of the grouped tcgen05 product begin on multiples of this
 
 
 def gemm_grouped_tc5_ok(dtype, pairs, num_experts, K) -> bool:
     """Whether a routed feed-forward of `pairs` (token, choice) rows runs its products on the tcgen05 tensor cores:
-    bfloat16, rows on 16-byte boundaries, and enough rows that the experts' tiles of 128 rows are mostly full."""
+    bfloat16, rows on 16-byte boundaries, and enough rows that an expert's share is worth a tile."""
     return dtype == torch.bfloat16 and K % 8 == 0 and pairs >= max(1024, 96 * num_experts)
 
 
-def gemm_grouped_tc5(rows, w, out, tile_group, err, row_index=None, row_scale=None, act=None, alpha=1.0, limit=0.0, shift=0.0):
-    """The grouped product on the tcgen05 tensor cores: rows [cap, K] sorted in tiles of 128, w [G, N, K], out [cap, N]
-    or, with `act` (w then interleaves 8 gate rows with their 8 up rows), [cap, N / 2] = act(gate, up).
+def gemm_grouped_tc5(rows, w, out, starts, err, row_index=None, row_scale=None, act=None, alpha=1.0, limit=0.0, shift=0.0):
+    """The grouped product on the tcgen05 tensor cores: rows [cap, K] sorted by group, group g's rows are
+    starts[g] .. starts[g + 1] (int32 [G + 1], `moe_align`), w [G, N, K], out [cap, N] or, with `act` (w then interleaves 8 gate rows
+    with their 8 up rows), [cap, N / 2] = act(gate, up).
     row_scale: the float32 sums of row m are multiplied by row_scale[row_index[m]] first."""
     _need(rows, torch.bfloat16, "rows", 2); _need(w, torch.bfloat16, "w", 3); _need(out, torch.bfloat16, "out", 2)
-    _need(tile_group, torch.int32, "tile_group", 1)
+    _need(starts, torch.int32, "starts", 1)
     G, N, K = w.shape
     cap = rows.shape[0]
-    if rows.shape[1] != K or out.shape != (cap, N // 2 if act in ACTIVATIONS else N) or cap % TC5_GROUPED_TILE \
-            or tile_group.shape[0] < cap // TC5_GROUPED_TILE:
+    if rows.shape[1] != K or out.shape != (cap, N // 2 if act in ACTIVATIONS else N) or starts.shape[0] < G + 1:
         raise KernelError("gemm_grouped_tc5: shapes disagree")
+    if row_index is not None:
+        _need(row_index, torch.int32, "row_index", 1)
+        if row_index.shape[0] < cap:
+            raise KernelError("gemm_grouped_tc5: an index for every row")
+    if row_scale is not None:
+        _need(row_scale, torch.float32, "row_scale")
     _check(_fn("gemm_tc5_grouped", "vl_gemm_bf16_tc5_grouped")(
-        _ptr(rows), _ptr(w), _ptr(out), cap, N, K, G, _ptr(tile_group), _ptr(row_index), _ptr(row_scale),
+        _ptr(rows), _ptr(w), _ptr(out), cap, N, K, G, _ptr(starts), _ptr(row_index), _ptr(row_scale),
         _act_code(act), float(alpha), float(limit), float(shift), _ptr(err), _stream()),
         "vl_gemm_bf16_tc5_grouped")
     return out
 
 
-def moe_align(ids, num_experts, bm, sorted_rows, tile_group, place):
+def moe_align(ids, num_experts, bm, sorted_rows, tile_group, place, starts=None):
+    """starts (int32 [num_experts + 1]): the first sorted row of every expert, and the end of the last one's."""
     _need(ids, torch.int32, "ids"); _need(sorted_rows, torch.int32, "sorted_rows", 1)
     _need(tile_group, torch.int32, "tile_group", 1); _need(place, torch.int32, "place", 1)
     n, cap = ids.numel(), sorted_rows.shape[0]
     if cap != moe_sorted_rows(n, num_experts, bm) or tile_group.shape[0] < cap // bm or place.shape[0] < n:
         raise KernelError("moe_align: buffer sizes do not match the number of pairs")
+    if starts is not None:
+        _need(starts, torch.int32, "starts", 1)
+        if starts.shape[0] < num_experts + 1:
+            raise KernelError("moe_align: a start for every expert and the end of the last")
     _check(_fn("moe", "vl_moe_align")(_ptr(ids), n, int(num_experts), int(bm), cap, _ptr(sorted_rows), _ptr(tile_group),
-                                      _ptr(place), _stream()), "vl_moe_align")
+                                      _ptr(place), _ptr(starts), _stream()), "vl_moe_align")
 
 
 def moe_gather(h, sorted_rows, weights, top, rows, scale_input):

@@ -140,14 +140,15 @@ class RoutedExperts:
         last = dict(add_weight=share)
         if s.identity:
             last.update(ids=ids, identity_from=E, h=h)
-        ops.moe_align(ids, E, bm, sorted_rows, tile_group, place)
+        starts = ws.get(tag + "moe.starts", (E + 1,), torch.int32) if big else None
+        ops.moe_align(ids, E, bm, sorted_rows, tile_group, place, starts)
         act = ws.get(tag + "moe.act", (cap, I), self.dtype)
         if big:
             # many rows: both products on the tcgen05 tensor cores, from a sorted copy of the tokens' rows
             rows = ops.moe_gather(h, sorted_rows, weights, top, ws.get(tag + "moe.rows", (cap, H), self.dtype), False)
-            ops.gemm_grouped_tc5(rows, self.gate_up, act, tile_group, step.err, sorted_rows,
+            ops.gemm_grouped_tc5(rows, self.gate_up, act, starts, step.err, sorted_rows,
                                  weights if s.scale_input else None, s.activation, s.alpha, s.limit, s.up_shift)
-            res = ops.gemm_grouped_tc5(act, self.down, ws.get(tag + "moe.down", (cap, H), self.dtype), tile_group, step.err)
+            res = ops.gemm_grouped_tc5(act, self.down, ws.get(tag + "moe.down", (cap, H), self.dtype), starts, step.err)
             return ops.moe_combine(res, place, weights, top, ws.get(tag + "moe.out", (T, H), self.dtype), not s.scale_input,
                                    add=self._shared(h, step), **last)
         if self.fused:
