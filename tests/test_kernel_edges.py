@@ -584,3 +584,28 @@ def test_experts_product_of_many_rows(sizes, N, K, act):
             off = 2 * z.abs() * off + off * off
             z = z.clamp(min=0) ** 2
         assert bool(((outs[0][at].double() - z).abs() <= 2.0 ** -8 * z.abs() + off + 1e-6).all()), g
+
+
+# functions of one argument: eight, four and single values a thread, and buffers that begin anywhere
+@pytest.mark.parametrize("act", ["gelu", "tanh", "relu2"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,off", [(1, 0), (7, 0), (12, 0), (148 * 2048 - 8, 0), (148 * 2048, 0), (148 * 2048 + 4, 0), (4096, 1)])
+def test_unary_activation(act, dtype, n, off):
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    x = (3 * torch.randn(n + off, device=DEV, generator=gen)).to(dtype)[off:]
+    x[: min(n, 5)] = torch.tensor([0.0, -12.9, 13.1, -0.0, 1e-30], device=DEV, dtype=dtype)[: min(n, 5)]
+    out = torch.full((n + off,), 7.0, device=DEV, dtype=dtype)[off:]
+    ops().unary_act(x, out, act)
+    v = x.double()
+    ref = v * 0.5 * torch.special.erfc(-v / 2 ** 0.5) if act == "gelu" else torch.tanh(v) if act == "tanh" else v.clamp(min=0) ** 2
+    # gelu in float32: the exponent z^2 (up to 85 here) carries a rounding of 2^-23, the polynomial 2^-22, the rest a few roundings
+    rel = (85 + 8) * 2.0 ** -23 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)
+    assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-37).all())
+
+
+def test_gelu_beyond_numbers():
+    x = torch.tensor([float("inf"), float("nan"), 3e38, -3e38], device=DEV)
+    out = torch.empty_like(x)
+    ops().unary_act(x, out, "gelu")
+    got = out.tolist()
+    assert got[0] == float("inf") and got[1] != got[1] and got[2] == x[2].item() and got[3] == 0.0

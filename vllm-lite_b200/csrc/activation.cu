@@ -108,40 +108,76 @@ extern "C" int vl_silu_mul(const void* gu, void* out, int dtype, int T, int I, i
 
 // A function of one argument, element by element in float32: act 16 = the square of max(v, 0), 17 = tanh(v), 18 = gelu(v) =
 // v times the normal distribution function at v (the codes continue those of the gated activations, which take two).
-__device__ __forceinline__ float unary_value(float v, int act) {
-    if (act == 16) { v = fmaxf(v, 0.f); return v * v; }
-    if (act == 18) return 0.5f * v * (1.0f + erff(v * 0.70710678f));     // erf(v / sqrt(2))
-    return act == 17 ? tanhf(v) : v;
+#define VL_ACT_RELU2 16
+#define VL_ACT_TANH 17
+#define VL_ACT_GELU 18
+// The normal distribution function at v is erfc(-v / sqrt(2)) / 2, and for z >= 0 erfc(z) = e^(-z^2) f(t), t = 1 / (1 + 0.44 z), with f(t) =
+// erfc(z) e^(z^2) smooth on (0, 1]: a polynomial of degree 8 without a constant, fitted to scipy's erfcx over z = 0 .. 10 by least
+// squares of the relative error with weights drawn to its largest places (1.8e-7).  It bounds the kernel by memory where 1 + erff(z) bound
+// it by its instructions (3,281 x 8,192 bfloat16: 39 us, 45 % more instructions), and keeps the small values for v < 0 that the sum cancels:
+// against 64 bits over -9 .. 9 1.6e-8 of the 2-norm (1 + erff: 1.7e-8), relative error at -5 .. -3 2.5e-6 (0.05).
+__device__ __forceinline__ float gelu_value(float v) {
+    const float z = fminf(fabsf(v) * 0.70710678f, 14.0f), t = __fdividef(1.0f, fmaf(0.44f, z, 1.0f));
+    float f = 0.07122346758842468f;
+    f = fmaf(f, t, -0.2779480218887329f);
+    f = fmaf(f, t, 0.2966874837875366f);
+    f = fmaf(f, t, -0.020180651918053627f);
+    f = fmaf(f, t, 0.21581222116947174f);
+    f = fmaf(f, t, 0.21731355786323547f);
+    f = fmaf(f, t, 0.24887117743492126f);
+    f = fmaf(f, t, 0.24822095036506653f);
+    const float half = 0.5f * t * f * __expf(-z * z);
+    return v * (v > 0.f ? 1.0f - half : half);
 }
-// VEC = 4: a thread takes four neighbouring values (one 16- or 8-byte access each way), when the buffers allow it.
-template <typename T, int VEC>
-__global__ void unary_act_kernel(const T* __restrict__ in, T* __restrict__ out, size_t n, int act) {
+template <int ACT> __device__ __forceinline__ float unary_value(float v) {
+    if (ACT == VL_ACT_RELU2) { v = fmaxf(v, 0.f); return v * v; }
+    if (ACT == VL_ACT_GELU) return gelu_value(v);
+    return tanhf(v);
+}
+// VEC = 8, 4: a thread takes eight or four neighbouring values, when the buffers allow it; eight where that still gives every SM
+// a block.
+template <typename T, int ACT, int VEC>
+__global__ void __launch_bounds__(256)
+unary_act_kernel(const T* __restrict__ in, T* __restrict__ out, size_t n) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * VEC;
     if (i >= n) return;
-    if (VEC == 4) {
+    if constexpr (VEC == 8) {
+        float v[8];
+        load8(in + i, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = unary_value<ACT>(v[j]);
+        store8(out + i, v);
+    } else if constexpr (VEC == 4) {
         const float4 v = Quad<T>::load(in + i);
-        Quad<T>::store(out + i, make_float4(unary_value(v.x, act), unary_value(v.y, act), unary_value(v.z, act), unary_value(v.w, act)));
+        Quad<T>::store(out + i, make_float4(unary_value<ACT>(v.x), unary_value<ACT>(v.y), unary_value<ACT>(v.z), unary_value<ACT>(v.w)));
     } else {
-        out[i] = from_f32<T>(unary_value(to_f32(in[i]), act));
+        out[i] = from_f32<T>(unary_value<ACT>(to_f32(in[i])));
     }
+}
+
+template <typename T, int ACT>
+static int launch_unary(const T* in, T* out, long long n, cudaStream_t s) {
+    const bool aligned = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+    const int vec = !aligned || n % 4 ? 1 : n % 8 == 0 && n >= 148 * 256 * 8 ? 8 : 4;
+    const dim3 blocks((unsigned)((n / vec + 255) / 256));
+    if (vec == 8) return vl_launch(unary_act_kernel<T, ACT, 8>, blocks, dim3(256), 0, s, in, out, (size_t)n);
+    if (vec == 4) return vl_launch(unary_act_kernel<T, ACT, 4>, blocks, dim3(256), 0, s, in, out, (size_t)n);
+    return vl_launch(unary_act_kernel<T, ACT, 1>, blocks, dim3(256), 0, s, in, out, (size_t)n);
 }
 
 extern "C" int vl_unary_act(const void* in, void* out, int dtype, long long n, int act, void* stream) {
     if (n <= 0) return VL_OK;
-    if (act < 16 || act > 18) return VL_ERR_ARGUMENT;
+    if (act < VL_ACT_RELU2 || act > VL_ACT_GELU) return VL_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    const bool vec = n % 4 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
-    const unsigned blocks = (unsigned)((n / (vec ? 4 : 1) + 255) / 256);
-    if (dtype == VL_F32) {
-        if (vec) return vl_launch(unary_act_kernel<float, 4>, dim3(blocks), dim3(256), 0, s, (const float*)in, (float*)out, (size_t)n, act);
-        return vl_launch(unary_act_kernel<float, 1>, dim3(blocks), dim3(256), 0, s, (const float*)in, (float*)out, (size_t)n, act);
-    }
-    if (dtype == VL_BF16) {
-        if (vec) return vl_launch(unary_act_kernel<bf16, 4>, dim3(blocks), dim3(256), 0, s, (const bf16*)in, (bf16*)out, (size_t)n, act);
-        return vl_launch(unary_act_kernel<bf16, 1>, dim3(blocks), dim3(256), 0, s, (const bf16*)in, (bf16*)out, (size_t)n, act);
-    }
+#define UNARY(T)                                                                                             \
+    act == VL_ACT_RELU2  ? launch_unary<T, VL_ACT_RELU2>((const T*)in, (T*)out, n, s)                        \
+    : act == VL_ACT_TANH ? launch_unary<T, VL_ACT_TANH>((const T*)in, (T*)out, n, s)                         \
+                         : launch_unary<T, VL_ACT_GELU>((const T*)in, (T*)out, n, s)
+    if (dtype == VL_F32) return UNARY(float);
+    if (dtype == VL_BF16) return UNARY(bf16);
+#undef UNARY
     return VL_ERR_UNSUPPORTED;
 }
 

@@ -1262,10 +1262,13 @@ def moe_route(h, router, top, ids, weights, logits, score="sigmoid", renormalize
 TC5_GROUPED_TILE = 16     # the groups' rows of the grouped tcgen05 product begin on multiples of this
 
 
-def gemm_grouped_tc5_ok(dtype, pairs, num_experts, K) -> bool:
+def gemm_grouped_tc5_ok(dtype, tokens, pairs, num_experts, K) -> bool:
     """Whether a routed feed-forward of `pairs` (token, choice) rows runs its products on the tcgen05 tensor cores:
-    bfloat16, rows on 16-byte boundaries, and enough rows that an expert's share is worth a tile."""
-    return dtype == torch.bfloat16 and K % 8 == 0 and pairs >= max(1024, 96 * num_experts)
+    bfloat16, rows on 16-byte boundaries, and enough rows.  Both products with the rows' copy against `gemm_grouped_fused` (32 experts,
+    2,048 x 1,024, top 4): 100 tokens 92 us against 95, 173: 93 against 211, 400: 95 against 212, 1,024: 105 against 440; 8 experts top 2, 100
+    tokens 34 against 68; 128 experts top 8, 100 tokens 280 against 303, 512: 290 against 706.  Steps of up to 64 tokens, whose kernels
+    start while the one before them ends, stay with the other (64 tokens of 32 experts 91 against 88)."""
+    return dtype == torch.bfloat16 and K % 8 == 0 and tokens > 64 and pairs >= 6 * num_experts
 
 
 def gemm_grouped_tc5(rows, w, out, starts, err, row_index=None, row_scale=None, act=None, alpha=1.0, limit=0.0, shift=0.0):

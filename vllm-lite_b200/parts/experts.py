@@ -123,7 +123,7 @@ class RoutedExperts:
         s, ws, tag = self.spec, step.workspace, step.tag
         T, E, top, I, H = h.shape[0], s.num_experts, s.top, s.intermediate_size, s.hidden_size
         pairs = T * top
-        big = self.fused and ops.gemm_grouped_tc5_ok(self.dtype, pairs, E, H) and I % 8 == 0
+        big = self.fused and ops.gemm_grouped_tc5_ok(self.dtype, T, pairs, E, H) and I % 8 == 0
         # tiles of 16 rows while an expert gets 16 rows or fewer on average (decoding: the products are then bound
         # by the experts' weights, and taller tiles would spend their time on rows of padding)
         bm = ops.TC5_GROUPED_TILE if big else (16 if pairs <= max(SMALL_STEP_PAIRS, 16 * E) else 64)
