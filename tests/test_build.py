@@ -140,3 +140,40 @@ def test_host_core_bindings_match_the_c_declarations():
         assert want == ("void" if fn.restype is None else py_kind(fn.restype)), name
         found += 1
     assert found >= 19
+
+
+def test_entry_points_are_called_as_ctypes_calls_them(tmp_path):
+    """The extension module hands whole numbers and floats to a C function by the calling convention's own rules; ctypes is the
+    reference, for argument lists longer than the registers and with floats anywhere between."""
+    import random
+    import subprocess
+    import pytest
+    bind = build.load_ext("bind")
+    kinds = {"p": ("const void*", ctypes.c_void_p), "i": ("int", ctypes.c_int), "l": ("long long", ctypes.c_longlong), "f": ("float", ctypes.c_float)}
+    rng = random.Random(5)
+    sigs = ["p", "f", "ffffffff", "i" * 30, "pifl" * 8] + ["".join(rng.choice("ppiilf" if k < 8 else "ppiil") for k in range(rng.randint(1, 38)))
+                                                           for _ in range(12)]
+    sigs = [s for s in sigs if s.count("f") <= 8]
+    body = ""
+    for n, s in enumerate(sigs):
+        args = ", ".join(f"{kinds[k][0]} a{i}" for i, k in enumerate(s))
+        terms = " ".join(f"s = s * 31 + (long long)({'a%d * 8' % i if k == 'f' else '(long long)a%d' % i});" for i, k in enumerate(s))
+        body += f'extern "C" int f{n}({args}) {{ unsigned long long s = 7; {terms} return (int)(s % 1000003); }}\n'
+    (tmp_path / "f.cpp").write_text(body)
+    subprocess.run([build.find_cxx(), "-O1", "-shared", "-fPIC", "-o", str(tmp_path / "f.so"), str(tmp_path / "f.cpp")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "f.so"))
+    for n, s in enumerate(sigs):
+        fn = getattr(lib, f"f{n}")
+        fn.argtypes, fn.restype = [kinds[k][1] for k in s], ctypes.c_int
+        entry = bind.Entry(ctypes.cast(fn, ctypes.c_void_p).value, s)
+        for _ in range(3):
+            args = [{"p": rng.choice([None, rng.randrange(1 << 47)]), "i": rng.randint(-(1 << 31), (1 << 31) - 1),
+                     "l": rng.randint(-(1 << 62), 1 << 62), "f": rng.randint(-4000, 4000) / 8}[k] for k in s]
+            assert entry(*args) == fn(*args), s
+        with pytest.raises(TypeError):
+            entry(*args, 0)
+    with pytest.raises(TypeError):
+        bind.Entry(ctypes.cast(lib.f0, ctypes.c_void_p).value, "i")("text")
+    for bad in ("x", "f" * 9, "i" * 41):
+        with pytest.raises(ValueError):
+            bind.Entry(1, bad)

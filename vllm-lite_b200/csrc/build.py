@@ -176,6 +176,78 @@ def host_library_path(name: str) -> Path:
     raise BuildError(f"could not build host/{name}.cpp: {last}")
 
 
+# ---- extension modules of Python (C++ beside torch's headers): csrc/host/<name>.cpp -------------------
+EXT_SOURCES = ("bind",)
+
+
+def _ext_flags():
+    import sysconfig
+    import torch
+    root = Path(torch.__file__).resolve().parent / "include"
+    cuda = Path(find_nvcc()).resolve().parent.parent / "include"
+    return ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-isystem", str(root), "-isystem", str(root / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda),
+            "-I", sysconfig.get_paths()["include"]]
+
+
+def _ext_libs():
+    import torch
+    lib = Path(torch.__file__).resolve().parent / "lib"
+    return [f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def ext_library_path(name: str) -> Path:
+    """Path of the up-to-date extension module `name`; its file name carries the versions it was compiled against."""
+    import torch
+    src = CSRC / "host" / f"{name}.cpp"
+    if not src.is_file():
+        raise BuildError(f"no C++ source {src}")
+    h = hashlib.sha256(src.read_bytes())
+    h.update(f"{torch.__version__} {torch._C._GLIBCXX_USE_CXX11_ABI} {sys.version} {EXT_SOURCES}".encode())
+    fname = f"ext_{name}.{h.hexdigest()[:12]}.so"
+    for d in _build_dirs():
+        if (d / fname).is_file():
+            return d / fname
+    last = None
+    for d in _build_dirs():
+        try:
+            d.mkdir(parents=True, exist_ok=True)
+            out = d / fname
+            tmp = out.with_suffix(f".tmp{os.getpid()}.so")
+            _say(f"compiling host/{name}.cpp beside torch {torch.__version__} ...")
+            proc = subprocess.run([find_cxx()] + _ext_flags() + ["-o", str(tmp), str(src)] + _ext_libs(), capture_output=True, text=True)
+            if proc.returncode != 0:
+                tmp.unlink(missing_ok=True)
+                raise BuildError(f"C++ compiler failed on host/{name}.cpp:\n{proc.stdout}{proc.stderr}")
+            os.replace(tmp, out)
+            for stale in d.glob(f"ext_{name}.*.so"):
+                if stale != out and ".tmp" not in stale.name:
+                    try:
+                        stale.unlink()
+                    except OSError:
+                        pass
+            return out
+        except (OSError, BuildError) as e:
+            last = e
+    raise BuildError(f"could not build host/{name}.cpp: {last}")
+
+
+def load_ext(name: str):
+    """The extension module `name`, built first if it is absent."""
+    key = ("ext", name)
+    with _lock:
+        mod = _loaded.get(key)
+        if mod is None:
+            import importlib.machinery
+            import importlib.util
+            loader = importlib.machinery.ExtensionFileLoader(name, str(ext_library_path(name)))
+            spec = importlib.util.spec_from_file_location(name, loader.path, loader=loader)
+            mod = importlib.util.module_from_spec(spec)
+            loader.exec_module(mod)
+            _loaded[key] = mod
+        return mod
+
+
 def load_host(name: str) -> ctypes.CDLL:
     key = ("host", name)
     with _lock:
@@ -204,4 +276,6 @@ def build_all(names=SOURCES) -> dict:
             out[f"{n}.{_variant(d)}"] = library_path(n, d)
     for n in HOST_SOURCES:
         out[f"host/{n}"] = host_library_path(n)
+    for n in EXT_SOURCES:
+        out[f"host/{n}"] = ext_library_path(n)
     return out

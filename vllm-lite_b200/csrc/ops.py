@@ -199,21 +199,15 @@ def _fn(lib: str, name: str, defines=None):
             setter.argtypes, setter.restype = [c_int], None
             setter(int(_pdl))
             _pdl_libs[holder] = setter
-        f = getattr(handle, name)
-        f.argtypes = _SIGNATURES[(lib, name)]
-        f.restype = c_int
-        _functions[key] = f
+        address = ctypes.cast(getattr(handle, name), c_void_p).value
+        f = _functions[key] = _bind.Entry(address, "".join(_KINDS[t] for t in _SIGNATURES[(lib, name)]))
     return f
 
 
-def _ptr(t):
-    return None if t is None else t.data_ptr()
-
-
-def _stream():
-    """The current stream of the current device, as `torch.cuda.current_stream().cuda_stream` gives it, without the stream object
-    (0.4 us instead of 4: a step of a prompt asks once a launch)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+_bind = build.load_ext("bind")        # what is done for every launch, in C++ (csrc/host/bind.cpp)
+_KINDS = {c_void_p: "p", c_int: "i", c_longlong: "l", c_float: "f"}
+_ptr = _bind.pointer                  # a tensor, an address or None: an entry point takes any of them where it wants a pointer
+_stream = _bind.stream                # the current stream of the current device, as `torch.cuda.current_stream().cuda_stream` gives it
 
 
 def _check(code: int, name: str):
@@ -226,7 +220,7 @@ def _check(code: int, name: str):
     raise KernelError(f"{name}: CUDA error {code} at launch")
 
 
-def _need(t, dtype, name, ndim=None):
+def _say_what_is_wrong(t, dtype, name, ndim=None):
     if not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor; the engine has no CPU path")
     if dtype is not None and t.dtype != dtype:
@@ -235,6 +229,10 @@ def _need(t, dtype, name, ndim=None):
         raise KernelError(f"{name} must be contiguous")
     if ndim is not None and t.dim() != ndim:
         raise KernelError(f"{name} must have {ndim} dimensions, got {tuple(t.shape)}")
+
+
+_bind.setup(_say_what_is_wrong)
+_need = _bind.need                    # raises as the function above does
 
 
 # ---------------------------------------------------------------- embed / norm
@@ -1433,6 +1431,11 @@ def gemm_bf16_tc5(a, w, out, err=None, swiglu=False):
     _check(_fn("gemm_tc5", "vl_gemm_bf16_tc5")(_ptr(a), _ptr(w), _ptr(out), dtype_code(out.dtype), M, N, K,
                                                K, K, width, _ptr(err), int(swiglu), _stream()), "vl_gemm_bf16_tc5")
     return out
+
+
+def mm(a, w, out):
+    """out = a @ w^T by the library (cuBLAS through torch), out in a's dtype or float32: `torch.mm` without what Python adds to it."""
+    return _bind.mm(a, w, out)
 
 
 _sm_pairs = None

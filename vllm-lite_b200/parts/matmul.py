@@ -37,6 +37,4 @@ def gemm_bf16(a, w, out, err=None, swiglu=False):
         return ops.gemm_bf16_tc5(a, w, out, err, swiglu)
     if swiglu:
         raise ValueError("the library product has no fused activation; ask fuses_swiglu() first")
-    if out.dtype == torch.bfloat16:
-        return torch.mm(a, w.t(), out=out)
-    return torch.mm(a, w.t(), out_dtype=torch.float32, out=out)      # float32 logits from bfloat16 operands
+    return ops.mm(a, w, out)                                         # (out float32: logits from bfloat16 operands)
