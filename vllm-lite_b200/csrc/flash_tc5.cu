@@ -198,7 +198,9 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     fence_proxy_async_smem();
     __syncthreads();
 
-    if (warp == 4) {                                             // ---- TMA producer (whole warp) ----
+    // (the roles by the warp's own number, for the issuers' sake; the softmax rows keep theirs by the thread's: seven registers less)
+    const int role = warp_number();
+    if (role == 4) {                                             // ---- TMA producer (whole warp) ----
         const int* table = block_table + (size_t)req * max_blocks;
         const int box_rows = page_size < BN ? page_size : BN, nbox = BN / box_rows;
         const int beyond = num_pages * nkv * page_size;          // a row coordinate past the tensor: zeros
@@ -269,8 +271,9 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             if (ok) mbar_arrive(&v_fixed);
             else atomicExch(&failed, 1);
         }
-    } else if (warp == 5) {
-        if (lane == 0) {                                         // ---- issuer of the scores S = Q K^T ----
+    } else if (role == 5) {
+        {                                                        // ---- issuer of the scores S = Q K^T ----
+            const bool lead = elect_one();
             constexpr unsigned idesc_qk = make_idesc(BM, BN);
             // descriptors: upper words once, lower words (the address field, in 16-byte units) by addition
             const unsigned long long dq = make_smem_desc(Qs), dk = make_smem_desc(Ks);
@@ -279,25 +282,28 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it & 1;
                 // the score buffer is free once every row of the tile two before has been read
-                if ((it >= 2 && !mbar_wait_bounded(&s_free[s], (unsigned)((it / 2 - 1) & 1))) ||
-                    !mbar_wait_bounded(&k_full[s], (unsigned)((it / 2) & 1))) { ok = false; break; }
+                if ((it >= 2 && !warp_wait(&s_free[s], (unsigned)((it / 2 - 1) & 1))) ||
+                    !warp_wait(&k_full[s], (unsigned)((it / 2) & 1))) { ok = false; break; }
                 tc5_fence_after();
                 const unsigned kb = k_lo + (unsigned)s * (KV_STAGE >> 4), tc = tmem_base + (unsigned)(s * BN);
+                if (lead) {
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks) {
-                    // 16 columns further on: 32 bytes inside the swizzled row; 64 columns: the next block of rows
-                    const unsigned qo = (unsigned)(ks >> 2) * (BM * ROW_BYTES >> 4) + (unsigned)(ks & 3) * 2;
-                    const unsigned ko = (unsigned)(ks >> 2) * (BN * ROW_BYTES >> 4) + (unsigned)(ks & 3) * 2;
-                    if (ks == 0) mma_lo<false>(tc, q_lo + qo, kb + ko, kmaj_hi, kmaj_hi, idesc_qk);
-                    else mma_lo<true>(tc, q_lo + qo, kb + ko, kmaj_hi, kmaj_hi, idesc_qk);
+                    for (int ks = 0; ks < HD / 16; ++ks) {
+                        // 16 columns further on: 32 bytes inside the swizzled row; 64 columns: the next block of rows
+                        const unsigned qo = (unsigned)(ks >> 2) * (BM * ROW_BYTES >> 4) + (unsigned)(ks & 3) * 2;
+                        const unsigned ko = (unsigned)(ks >> 2) * (BN * ROW_BYTES >> 4) + (unsigned)(ks & 3) * 2;
+                        if (ks == 0) mma_lo<false>(tc, q_lo + qo, kb + ko, kmaj_hi, kmaj_hi, idesc_qk);
+                        else mma_lo<true>(tc, q_lo + qo, kb + ko, kmaj_hi, kmaj_hi, idesc_qk);
+                    }
+                    tc5_commit(&k_empty[s]);
+                    tc5_commit(&s_full[s]);
                 }
-                tc5_commit(&k_empty[s]);
-                tc5_commit(&s_full[s]);
             }
-            if (!ok) atomicExch(&failed, 1);
+            if (!ok && lead) atomicExch(&failed, 1);
         }
-    } else if (warp == 6) {
-        if (lane == 0) {                                         // ---- issuer of the output O += P V ----
+    } else if (role == 6) {
+        {                                                        // ---- issuer of the output O += P V ----
+            const bool lead = elect_one();
             constexpr unsigned idesc_pv = make_idesc(BM, HD) | IDESC_B_MN_MAJOR;
             const unsigned long long dp = make_smem_desc(Ps);
             const unsigned long long dv = make_smem_desc_lbo_sbo(Vs, BN * ROW_BYTES, 8 * ROW_BYTES);
@@ -306,21 +312,23 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             bool ok = true;
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it & 1;
-                if (!mbar_wait_bounded(&p_full, (unsigned)(it & 1)) ||
-                    !mbar_wait_bounded(&v_full[s], (unsigned)((it / 2) & 1)) ||
-                    (it == n_tiles - 1 && !mbar_wait_bounded(&v_fixed, 0u))) { ok = false; break; }
+                if (!warp_wait(&p_full, (unsigned)(it & 1)) ||
+                    !warp_wait(&v_full[s], (unsigned)((it / 2) & 1)) ||
+                    (it == n_tiles - 1 && !warp_wait(&v_fixed, 0u))) { ok = false; break; }
                 tc5_fence_after();
                 const unsigned vb = v_lo + (unsigned)s * (KV_STAGE >> 4);
+                if (lead) {
 #pragma unroll
-                for (int k = 0; k < BN / 16; ++k) {
-                    // 16 keys further on: 32 bytes inside a row of P, 16 rows of 128 bytes of V
-                    if (k == 0 && it == 0) mma_lo<false>(tmem_base + O_COL, p_lo, vb, kmaj_hi, v_hi, idesc_pv);
-                    else mma_lo<true>(tmem_base + O_COL, p_lo + (unsigned)k * 2, vb + (unsigned)k * (16 * ROW_BYTES >> 4), kmaj_hi, v_hi, idesc_pv);
+                    for (int k = 0; k < BN / 16; ++k) {
+                        // 16 keys further on: 32 bytes inside a row of P, 16 rows of 128 bytes of V
+                        if (k == 0 && it == 0) mma_lo<false>(tmem_base + O_COL, p_lo, vb, kmaj_hi, v_hi, idesc_pv);
+                        else mma_lo<true>(tmem_base + O_COL, p_lo + (unsigned)k * 2, vb + (unsigned)k * (16 * ROW_BYTES >> 4), kmaj_hi, v_hi, idesc_pv);
+                    }
+                    tc5_commit(&v_empty[s]);
+                    tc5_commit(&pv_done);
                 }
-                tc5_commit(&v_empty[s]);
-                tc5_commit(&pv_done);
             }
-            if (!ok) atomicExch(&failed, 1);
+            if (!ok && lead) atomicExch(&failed, 1);
         }
     } else {                                                     // ---- softmax: a thread per query row ----
         const int row = warp * 32 + lane;
@@ -353,9 +361,30 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             mbar_arrive(&s_free[s]);                             // the scores are in registers: the buffer may be written again
             const int j0 = tile_of(it) * BN;
             if constexpr (SHAPED) {
+                // shape_score, two scores an instruction where there is one for two
+                if (cap_l2 > 0.f) {
+                    const unsigned long long k2 = pair(scale_log2 * toc, scale_log2 * toc), zero2 = pair(0.f, 0.f);
+                    const unsigned long long m2 = pair(-2.f * cap_l2, -2.f * cap_l2), c2 = pair(cap_l2, cap_l2), one2 = pair(1.f, 1.f);
 #pragma unroll
-                for (int c = 0; c < BN; ++c)
-                    sv[c] = __float_as_uint(shape_score(__uint_as_float(sv[c]) * scale_log2, cap_l2, toc, da, db, qpos - (j0 + c)));
+                    for (int c = 0; c < BN; c += 2) {
+                        float e0, e1, r0, r1;
+                        unpair(fma2(pair(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), k2, zero2), e0, e1);
+                        unpair(add2(pair(ss_exp2(e0), ss_exp2(e1)), one2), e0, e1);
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(e0));
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(e1));
+                        unpair(fma2(pair(r0, r1), m2, c2), e0, e1);
+                        sv[c] = __float_as_uint(e0);
+                        sv[c + 1] = __float_as_uint(e1);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < BN; ++c) sv[c] = __float_as_uint(__uint_as_float(sv[c]) * scale_log2);
+                }
+                if (da != 0.f) {
+#pragma unroll
+                    for (int c = 0; c < BN; ++c)
+                        sv[c] = __float_as_uint(shape_score(__uint_as_float(sv[c]), 0.f, 0.f, da, db, qpos - (j0 + c)));
+                }
             }
             // (warp-uniform) does any row of this warp see a key of the tile that it must not read?
             const bool edge = (j0 + BN - 1 > pos0 + warp * 32) || j0 < warp_first;

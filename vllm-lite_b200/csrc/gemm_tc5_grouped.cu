@@ -35,9 +35,8 @@ constexpr unsigned W_BYTES = ROWS * BK * 2, A_BYTES = COLS / 2 * BK * 2, STAGE_B
 constexpr int STAGES = 6, ACCS = 2;
 constexpr int GROUPS = 2, NUM_THREADS = 64 + GROUPS * 128;
 constexpr int MAX_EXPERTS = 1024;
-constexpr int ISSUE = 2;                     // K blocks of W asked for together: 256 bytes of every row
 constexpr int TOKEN_BOXES = 8;               // boxes of 16, 32 .. 128 rows of A
-constexpr unsigned TURN_BYTES = 32 * 272;    // a group's chunk on its way: 32 rows of C x 128 bfloat16, 16 bytes of padding a row
+constexpr unsigned CHUNK_BYTES = 32 * 272;    // a group's chunk on its way: 32 rows of C x 128 bfloat16, 16 bytes of padding a row
 
 enum { PLAIN = 0, SILU = 1, OTHER = 2 };     // the epilogue: C as it is; silu(gate) * up; what Args::act says
 
@@ -155,11 +154,11 @@ gemm_tc5_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     extern __shared__ unsigned char grouped_smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)grouped_smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full_bar[ACCS], acc_empty_bar[ACCS];
-    __shared__ __align__(16) unsigned char turn_all[GROUPS][TURN_BYTES];
+    __shared__ __align__(16) unsigned char turn_all[GROUPS][CHUNK_BYTES];
     __shared__ unsigned tmem_base_slot;
     __shared__ int failed;
     __shared__ Tables tb;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
     if (threadIdx.x == 0) {
@@ -196,67 +195,66 @@ gemm_tc5_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     const unsigned tmem_base = tmem_base_slot;
     const int tiles = tb.tile[f.groups];
 
-    if (warp == 0) {
-        if (lane == 0) {                                     // ---- TMA producer ----
-            int it = 0, s = 0, e = 0;                        // s = it % STAGES
-            unsigned phase = 1;                              // of the stage's next "free"
-            bool ok = true;
-            for (int tile = pair; tile < tiles && ok; tile += pairs) {
-                const Tile t = tile_at(f, tb, tile, e);
-                const int own = t.T / 2;                     // rows of A that this block brings
-                const CUtensorMap* map_a = &maps_a.m[own / 16 - 1];
-                const unsigned bytes = W_BYTES + (unsigned)(own * BK * 2);
-                for (int kb = 0; kb < f.kb && ok; kb += ISSUE) {
-                    const int n = min(ISSUE, f.kb - kb), s_first = s;
-                    for (int j = 0; j < n; ++j, ++it) {
-                        if (it >= STAGES && !mbar_wait_bounded(&empty_bar[s], phase)) {
-                            atomicOr(&failed, 1);
-                            ok = false;
-                            break;
-                        }
-                        if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * bytes);       // the bytes of both blocks
-                        tma_load_2d_pair(smem + (size_t)s * STAGE_BYTES, &map_w, (kb + j) * BK, t.wrow + rank * ROWS,
-                                         map_to_rank(smem_u32(&full_bar[s]), 0));
-                        if (++s == STAGES) { s = 0; phase ^= 1u; }
-                    }
-                    if (!ok) break;
-                    for (int j = 0, sa = s_first; j < n; ++j, sa = sa + 1 == STAGES ? 0 : sa + 1)
-                        tma_load_2d_pair(smem + (size_t)sa * STAGE_BYTES + W_BYTES, map_a, (kb + j) * BK, t.t0 + rank * own,
-                                         map_to_rank(smem_u32(&full_bar[sa]), 0));
+    if (warp == 0) {                                         // ---- TMA producer ----
+        const bool lead = elect_one();
+        int s = 0, e = 0;
+        unsigned phase = 1;                                  // of the stage's next "free": the first round finds all free
+        bool ok = true;
+        for (int tile = pair; tile < tiles && ok; tile += pairs) {
+            const Tile t = tile_at(f, tb, tile, e);
+            const int own = t.T / 2;                         // rows of A that this block brings
+            const CUtensorMap* map_a = &maps_a.m[own / 16 - 1];
+            const unsigned bytes = W_BYTES + (unsigned)(own * BK * 2);
+            for (int kb = 0; kb < f.kb; ++kb) {
+                if (!warp_wait(&empty_bar[s], phase)) {
+                    if (lead) atomicOr(&failed, 1);
+                    ok = false;
+                    break;
                 }
+                if (lead) {
+                    if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * bytes);       // the bytes of both blocks
+                    const unsigned bar = map_to_rank(smem_u32(&full_bar[s]), 0);
+                    unsigned char* st = smem + (size_t)s * STAGE_BYTES;
+                    tma_load_2d_pair(st, &map_w, kb * BK, t.wrow + rank * ROWS, bar);
+                    tma_load_2d_pair(st + W_BYTES, map_a, kb * BK, t.t0 + rank * own, bar);
+                }
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {                        // ---- MMA issuer of the pair ----
+        if (rank == 0) {                                     // ---- MMA issuer of the pair ----
+            const bool lead = elect_one();
             int s = 0, e = 0, i = 0;
             unsigned phase = 0;
             bool ok = true;
             for (int tile = pair; tile < tiles && ok; tile += pairs, ++i) {
                 const unsigned idesc = make_idesc(2 * ROWS, tile_at(f, tb, tile, e).T);
                 const int acc = i % ACCS;
-                if (i >= ACCS && !mbar_wait_bounded(&acc_empty_bar[acc], (unsigned)((i / ACCS - 1) & 1))) {
-                    atomicOr(&failed, 2);
+                if (i >= ACCS && !warp_wait(&acc_empty_bar[acc], (unsigned)((i / ACCS - 1) & 1))) {
+                    if (lead) atomicOr(&failed, 2);
                     break;
                 }
                 tc5_fence_after();
                 const unsigned tmem_c = tmem_base + (unsigned)(acc * COLS);
                 for (int kb = 0; kb < f.kb; ++kb) {
-                    if (!mbar_wait_bounded(&full_bar[s], phase)) {
-                        atomicOr(&failed, 4);
+                    if (!warp_wait(&full_bar[s], phase)) {
+                        if (lead) atomicOr(&failed, 4);
                         ok = false;
                         break;
                     }
                     tc5_fence_after();
                     const unsigned char* st = smem + (size_t)s * STAGE_BYTES;
                     const unsigned long long wdesc = make_smem_desc(st), adesc = make_smem_desc(st + W_BYTES);
+                    if (lead) {
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        mma_pair(tmem_c, wdesc + (unsigned long long)(k * 2), adesc + (unsigned long long)(k * 2), idesc,
-                                 (kb > 0 || k > 0) ? 1u : 0u);
-                    commit_pair(&empty_bar[s]);              // both blocks' stages are free once these have read them
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            mma_pair(tmem_c, wdesc + (unsigned long long)(k * 2), adesc + (unsigned long long)(k * 2), idesc,
+                                     (kb > 0 || k > 0) ? 1u : 0u);
+                        commit_pair(&empty_bar[s]);          // both blocks' stages are free once these have read them
+                        if (kb + 1 == f.kb) commit_pair(&acc_full_bar[acc]);
+                    }
                     if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                if (ok) commit_pair(&acc_full_bar[acc]);
             }
         }
     } else {                                                 // ---- epilogue: warps 2..9 ----

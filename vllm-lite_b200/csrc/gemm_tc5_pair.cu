@@ -18,8 +18,8 @@
 //                        tells both epilogues; the warp of either block allocates and frees TMEM
 //                        (512 columns: two accumulators, so that a tile's products run during the
 //                        epilogue of the tile before);
-//   warps 2..5           epilogue of the block's 128 rows, as in csrc/gemm_tc5.cu; when done they
-//                        arrive on the first block's mbarrier (256 arrivals free an accumulator).
+//   warps 2..9           epilogue of the block's 128 rows, as in csrc/gemm_tc5.cu; when done they
+//                        arrive on the first block's mbarrier (512 arrivals free an accumulator).
 // Any M and N (the TMA unit fills what lies outside with zeros), K a multiple of 8.  Every wait on
 // an mbarrier is bounded: when one expires the block records VL_DEV_WAIT_EXPIRED, stops, and
 // still joins the pair's last barrier and frees its TMEM.
@@ -30,7 +30,7 @@ using namespace tc5;
 namespace {
 constexpr int BM_CTA = 128, BM = 256, BK = 64, UMMA_K = 16;
 constexpr int BN_MMA = 256, BN_CTA = 128;    // one product: 256 columns of the tile, 128 rows of W from each block
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 64 + 256;        // copies, products, eight warps of epilogue
 constexpr unsigned A_BYTES = BM_CTA * BK * 2, W_BYTES = BN_CTA * BK * 2;
 constexpr unsigned TMEM_COLS = 512;
 
@@ -57,7 +57,7 @@ __device__ __forceinline__ void tile_corner(int tile, int tiles_m, int tiles_n, 
 }  // namespace
 
 template <typename TO, int BN>
-__global__ void __launch_bounds__(NUM_THREADS)
+__global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                      TO* __restrict__ C, int M, int N, int K, int ldc, unsigned* err, int tiles_m, int tiles_n, int swiglu) {
     constexpr int STAGES = Shape<BN>::STAGES, ACCS = Shape<BN>::ACCS, HALVES = Shape<BN>::HALVES;
@@ -65,9 +65,10 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     extern __shared__ unsigned char pair_smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)pair_smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full_bar[2], acc_empty_bar[2];
+    __shared__ __align__(16) unsigned char turn[8][TURN_BYTES];
     __shared__ unsigned tmem_base_slot;
     __shared__ int failed;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number();
     const unsigned rank = cluster_rank();                    // 0: the block that issues the pair's products
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int k_blocks = (K + BK - 1) / BK;
@@ -75,7 +76,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
-        for (int i = 0; i < ACCS; ++i) { mbar_init(&acc_full_bar[i], 1); mbar_init(&acc_empty_bar[i], 2 * 128); }
+        for (int i = 0; i < ACCS; ++i) { mbar_init(&acc_full_bar[i], 1); mbar_init(&acc_empty_bar[i], 2 * 256); }
         mbar_fence_init();
         failed = 0;
     }
@@ -92,20 +93,21 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tc5_fence_after();
     const unsigned tmem_base = tmem_base_slot;
 
-    if (warp == 0) {
-        if (lane == 0) {                                     // ---- TMA producer ----
-            int it = 0;
-            bool ok = true;
-            for (int tile = pair; tile < total_tiles && ok; tile += num_pairs) {
-                int m0, n0;
-                tile_corner<BN>(tile, tiles_m, tiles_n, m0, n0);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES && !mbar_wait_bounded(&empty_bar[s], (unsigned)((it / STAGES - 1) & 1))) {
-                        atomicOr(&failed, 1);
-                        ok = false;
-                        break;
-                    }
+    if (warp == 0) {                                         // ---- TMA producer ----
+        const bool lead = elect_one();
+        int s = 0;
+        unsigned phase = 1;                                  // of the stage's next "free": the first round finds all free
+        bool ok = true;
+        for (int tile = pair; tile < total_tiles && ok; tile += num_pairs) {
+            int m0, n0;
+            tile_corner<BN>(tile, tiles_m, tiles_n, m0, n0);
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_wait(&empty_bar[s], phase)) {
+                    if (lead) atomicOr(&failed, 1);
+                    ok = false;
+                    break;
+                }
+                if (lead) {
                     if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * STAGE_BYTES);       // the bytes of both blocks
                     const unsigned bar = map_to_rank(smem_u32(&full_bar[s]), 0);
                     unsigned char* st = smem + (size_t)s * STAGE_BYTES;
@@ -114,46 +116,52 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     for (int h = 0; h < HALVES; ++h)     // this block's 128 rows of W for each product of 256 columns
                         tma_load_2d_pair(st + A_BYTES + h * W_BYTES, &map_w, kb * BK, n0 + h * BN_MMA + (int)rank * BN_CTA, bar);
                 }
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {                        // ---- MMA issuer of the pair ----
+        if (rank == 0) {                                     // ---- MMA issuer of the pair ----
+            const bool lead = elect_one();
             constexpr unsigned idesc = make_idesc(BM, BN_MMA);
-            int it = 0, local = 0;
+            int s = 0, local = 0;
+            unsigned phase = 0;
             bool ok = true;
             for (int tile = pair; tile < total_tiles && ok; tile += num_pairs, ++local) {
                 const int acc = local % ACCS;
-                if (local >= ACCS && !mbar_wait_bounded(&acc_empty_bar[acc], (unsigned)((local / ACCS - 1) & 1))) {
-                    atomicOr(&failed, 2);
+                if (local >= ACCS && !warp_wait(&acc_empty_bar[acc], (unsigned)((local / ACCS - 1) & 1))) {
+                    if (lead) atomicOr(&failed, 2);
                     break;
                 }
                 tc5_fence_after();
                 const unsigned tmem_c = tmem_base + (unsigned)(acc * BN);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait_bounded(&full_bar[s], (unsigned)((it / STAGES) & 1))) {
-                        atomicOr(&failed, 4);
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!warp_wait(&full_bar[s], phase)) {
+                        if (lead) atomicOr(&failed, 4);
                         ok = false;
                         break;
                     }
                     tc5_fence_after();
                     const unsigned char* st = smem + (size_t)s * STAGE_BYTES;
                     const unsigned long long adesc = make_smem_desc(st);
+                    if (lead) {
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h) {
-                        const unsigned long long bdesc = make_smem_desc(st + A_BYTES + h * W_BYTES);
+                        for (int h = 0; h < HALVES; ++h) {
+                            const unsigned long long bdesc = make_smem_desc(st + A_BYTES + h * W_BYTES);
 #pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k)
-                            mma_pair(tmem_c + (unsigned)(h * BN_MMA), adesc + (unsigned long long)(k * 2),
-                                     bdesc + (unsigned long long)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                            for (int k = 0; k < BK / UMMA_K; ++k)
+                                mma_pair(tmem_c + (unsigned)(h * BN_MMA), adesc + (unsigned long long)(k * 2),
+                                         bdesc + (unsigned long long)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        }
+                        commit_pair(&empty_bar[s]);          // both blocks' stages are free once these MMAs have read them
+                        if (kb + 1 == k_blocks) commit_pair(&acc_full_bar[acc]);     // both halves of this accumulator are complete
                     }
-                    commit_pair(&empty_bar[s]);              // both blocks' stages are free once these MMAs have read them
+                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                if (ok) commit_pair(&acc_full_bar[acc]);     // both halves of this accumulator are complete
             }
         }
-    } else {                                                 // ---- epilogue: warps 2..5 ----
+    } else {                                                 // ---- epilogue: warps 2..9 ----
         const int quarter = warp & 3;                        // the TMEM lanes this warp may read
+        const bool wide = ((uintptr_t)C & 15) == 0 && (size_t)ldc * sizeof(TO) % 16 == 0;
         const unsigned freed = map_to_rank(smem_u32(&acc_empty_bar[0]), 0);
         int local = 0;
         for (int tile = pair; tile < total_tiles; tile += num_pairs, ++local) {
@@ -165,12 +173,8 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             tc5_fence_after();
             int m0, n0;
             tile_corner<BN>(tile, tiles_m, tiles_n, m0, n0);
-            const int row = m0 + (int)rank * BM_CTA + quarter * 32 + lane;
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                unsigned v[32];
-                tc5_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN + c0), v);
-                if (row < M) store_chunk32<TO>(v, C + (size_t)row * ldc, n0 + c0, N, swiglu);
-            }
+            store_rows<TO, BN>(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN), turn[warp - 2], C,
+                               m0 + (int)rank * BM_CTA + quarter * 32, n0, M, N, ldc, (warp - 2) >> 2, swiglu, wide);
             tc5_fence_before();
             mbar_arrive_remote(freed + (unsigned)(acc * sizeof(unsigned long long)));
         }
@@ -231,12 +235,10 @@ extern "C" int vl_gemm_bf16_tc5_pair(const void* A, const void* W, void* C, int 
     if (lda < K || ldw < K) return VL_ERR_ARGUMENT;
     if (((uintptr_t)A | (uintptr_t)W) & 15) return VL_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    // Which width.  A tile of 512 columns costs about 1.8 tiles of 256 (measured: neither keeps the tensor pipe
-    // busier than about 80 %, what the shared memory of an SM moves bounds both) plus an epilogue that nothing
-    // hides, and loses more when a pair walks many tiles (4,096 x 24,576 x 4,096: 560 us against 624).  It wins
-    // where it saves a round of the pairs of SMs and the rounds are few: at 2,048 rows of Qwen3-8B o 53.9 ->
-    // 50.1 us and down 155.5 -> 142.0 (one round of 64 tiles instead of two of 128), at 4,096 rows down 341 ->
-    // 320; q/k/v and gate/up stay at 256 (80.2 against 100.5, 295.8 against 312.7).
+    // Which width.  A K block of a tile of 512 columns costs 1.93 of one of 256, and its epilogue, which nothing hides, 6.5 more: it wins
+    // where it saves a round of the pairs of SMs and K is long (us, 256 / 512): 2,048 rows x 12,288 -> 4,096 147.8 / 150.5 with the
+    // clocks down, 3,000 x 8,192 -> 2,048 83.9 / 81.3, 4,096 x 12,288 -> 4,096 281.6 / 271.4; 2,048 x 2,048 -> 8,192 49.5 / 51.5, 2,048 x 4,096 -> 4,096
+    // 49.0 / 48.7, 2,048 x 4,096 -> 6,144 70.1 / 88.2.
     static int pairs = 0;
     if (!pairs) {
         int dev = 0, sms = 0;
@@ -246,7 +248,7 @@ extern "C" int vl_gemm_bf16_tc5_pair(const void* A, const void* W, void* C, int 
     }
     const long long kb = (K + BK - 1) / BK, tm = (M + BM - 1) / BM;
     const long long r256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, r512 = (tm * ((N + 511) / 512) + pairs - 1) / pairs;
-    int wide = N > 256 && r512 <= 2 && r512 * (18 * kb + 60) < r256 * 10 * kb;
+    int wide = N > 256 && r512 <= 2 && r512 * (193 * kb + 650) < r256 * 100 * kb;
     if (const char* v = getenv("VLLM_LITE_B200_PAIR_WIDTH")) {      // 256 or 512: for tests and measurements
         const int w = atoi(v);
         if (w == 256 || w == 512) wide = w == 512;

@@ -1411,16 +1411,27 @@ def gemm_bf16_small_m(a, w, out, err=None, swiglu=False, scaled=None, sink=None)
     return out
 
 
-# From this many rows on the tcgen05 kernels are used: 1,024 where the activation is fused into the product
-# (the library would need a kernel of its own for it: level at 1,024 rows, ahead beyond), 2,048 for a plain
-# product (measured at 1,024 rows, q/k/v and down of Qwen3-8B: 58 and 82 us against the library's 41 and 73;
-# at 2,048 rows 81 and 156 against 72 and 137; at 4,096 rows 158 and 358 against 165 and 314).
+# From this many rows on the tcgen05 kernels are used.  2,048 for a plain product (us, the better kernel here against the library's: 1,024
+# rows, q/k/v and down of Qwen3-8B 45 / 36 and 72 / 68, 1,536 rows 51 / 50 and 122 / 100, 2,048 rows 70 / 69 and 135 / 131).  1,024 where
+# the activation is fused into the product, which the library needs a kernel of its own for, and from 512 rows on where the last
+# round of tiles is not left to few pairs of SMs (gate/up of Qwen3-8B against the library and that kernel: 512 rows 75 / 81, 536
+# 104 / 87, 640 105 / 107, 768 104 / 111, 900 144 / 142, 1,024 142 / 152, 1,280 169 / 200, 1,536 197 / 216).
 TC5_MIN_M = 1024
+TC5_MIN_M_FULL = 512
 TC5_MIN_M_PLAIN = 2048
 
 
-def gemm_bf16_tc5_ok(M, K, fused=False) -> bool:
-    return M >= (TC5_MIN_M if fused else TC5_MIN_M_PLAIN) and K % 8 == 0
+def gemm_bf16_tc5_ok(M, K, fused=False, N=None) -> bool:
+    """N (of a fused product): rows of w, by which a product of less than 1,024 rows is judged."""
+    if K % 8:
+        return False
+    if not fused:
+        return M >= TC5_MIN_M_PLAIN
+    if M >= TC5_MIN_M or M < TC5_MIN_M_FULL or not N:
+        return M >= TC5_MIN_M
+    tiles = -(-M // 256) * -(-N // 256)
+    places = -(-tiles // sm_pairs()) * sm_pairs()
+    return 4 * places * 256 * 256 <= 5 * M * N           # at most a quarter more tile than product
 
 
 def gemm_bf16_tc5(a, w, out, err=None, swiglu=False):

@@ -35,6 +35,19 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
     }
     return false;
 }
+// The warps that issue copies and products run their loops with all 32 lanes, and one of them, elected once, issues.  A loop under "if
+// (lane == 0)" is divergent code to the compiler, which then moves every operand of a copy or a product (descriptors, addresses, coordinates) to
+// the uniform registers that the instruction reads one by one: 550 cycles a K block of 64, whatever the tile's size, where
+// the tensor cores want 256 to 512.  So the number of the warp, the outcome of a wait and everything derived from them are the warp's own.
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    unsigned lead;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(lead));
+    return lead != 0;
+}
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
 // x = element index along K (a multiple of 8: the copy starts on a 16-byte boundary), y = row
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
     asm volatile(
@@ -194,64 +207,77 @@ __device__ __forceinline__ void commit_pair(unsigned long long* bar) {
                  ::"r"(smem_u32(bar)), "h"(mask) : "memory");
 }
 
-// Stores 32 neighbouring columns (from column `col` of the product) of one row of the accumulator.
-// swiglu: the 32 columns are two blocks of 8 gate and 8 up columns and become 16 columns of C at col / 2:
-// C[8b + i] = silu(y[16b + i]) * y[16b + 8 + i].  `crow` points at the row of C.
+// The epilogue of the products that lay the rows of A along tensor memory's lanes: every second 32 columns (64 with swiglu), from
+// number `half` on, of a warp's 32 rows (row0 ..) of an accumulator of BN columns (columns n0 .. of the product) to C.
+// A thread holds a row, and 32 rows of C are 32 lines of memory: stored from there, 16 bytes a thread, the accesses bound the epilogue
+// (540 cycles for four warps' 32 columns).  So 64 bytes a row are laid down in shared memory first (`turn`, TURN_BYTES a warp; rows 80 bytes
+// apart: eight neighbouring threads meet in no bank) and leave four threads a row.
+// swiglu: blocks of 8 gate and 8 up columns become 8 columns of C: C[8b + i] = silu(y[16b + i]) * y[16b + 8 + i].
+// `wide`: rows of C begin on 16-byte boundaries.
+constexpr int TURN_STRIDE = 80, TURN_BYTES = 32 * TURN_STRIDE;
+
 template <typename TO>
-__device__ __forceinline__ void store_chunk32(const unsigned (&v)[32], TO* crow, int col, int N, int swiglu) {
+__device__ __forceinline__ void store_turned(const unsigned char* turn, TO* __restrict__ C, int row0, int col0, int M, int out_n, int ldc, bool wide) {
+    constexpr int EACH = 16 / sizeof(TO);
+    const int lane = threadIdx.x & 31, col = col0 + (lane & 3) * EACH;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = i * 8 + (lane >> 2);
+        const unsigned char* src = turn + r * TURN_STRIDE + (lane & 3) * 16;
+        if (row0 + r >= M) continue;
+        TO* dst = C + (size_t)(row0 + r) * ldc + col;
+        if (wide && col + EACH <= out_n) {
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+        } else {
+            for (int j = 0; j < EACH; ++j)
+                if (col + j < out_n) dst[j] = reinterpret_cast<const TO*>(src)[j];
+        }
+    }
+    __syncwarp();                                                                // the next line may be laid down
+}
+
+template <typename TO, int BN>
+__device__ __forceinline__ void store_rows(unsigned tmem, unsigned char* turn, TO* __restrict__ C, int row0, int n0, int M, int N, int ldc,
+                                           int half, int swiglu, bool wide) {
+    TO* line = reinterpret_cast<TO*>(turn + (threadIdx.x & 31) * TURN_STRIDE);
     if (swiglu) {
-        TO* dst = crow + col / 2;
+        constexpr int OUT = 64 / sizeof(TO);                                     // columns of C of a line
+        for (int c0 = half * 2 * OUT; c0 < BN && n0 + c0 < N; c0 += 4 * OUT) {
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-            if (col + 16 * blk + 16 <= N) {
-                float o[8];
+            for (int c = 0; c < 2 * OUT; c += 32) {
+                unsigned v[32];
+                tc5_ld32(tmem + (unsigned)(c0 + c), v);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float gt = __uint_as_float(v[16 * blk + i]), up = __uint_as_float(v[16 * blk + 8 + i]);
-                    o[i] = gt / (1.0f + __expf(-gt)) * up;
-                }
-                if constexpr (sizeof(TO) == 2) {
-                    uint4 q;
-                    unsigned* w = reinterpret_cast<unsigned*>(&q);
+                for (int b = 0; b < 2; ++b) {
+                    float o[8];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        __nv_bfloat162 p = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-                        w[i] = *reinterpret_cast<unsigned*>(&p);
+                    for (int i = 0; i < 8; ++i) {
+                        const float gt = __uint_as_float(v[16 * b + i]), up = __uint_as_float(v[16 * b + 8 + i]);
+                        o[i] = gt / (1.0f + __expf(-gt)) * up;
                     }
-                    if ((((uintptr_t)(dst + 8 * blk)) & 15) == 0) {
-                        *reinterpret_cast<uint4*>(dst + 8 * blk) = q;
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) dst[8 * blk + i] = from_f32<TO>(o[i]);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) dst[8 * blk + i] = from_f32<TO>(o[i]);
+                    store8(line + c / 2 + 8 * b, o);
                 }
             }
+            store_turned(turn, C, row0, (n0 + c0) / 2, M, N / 2, ldc, wide);
         }
         return;
     }
-    TO* dst = crow + col;
-    if (col + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
-        if constexpr (sizeof(TO) == 2) {
-            uint4 q[4];
-            unsigned* w = reinterpret_cast<unsigned*>(q);
+    for (int c0 = half * 32; c0 < BN && n0 + c0 < N; c0 += 64) {
+        unsigned v[32];
+        tc5_ld32(tmem + (unsigned)c0, v);
+        constexpr int OUT = 64 / sizeof(TO);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-                w[i] = *reinterpret_cast<unsigned*>(&p);
+        for (int c = 0; c < 32; c += OUT) {
+#pragma unroll
+            for (int b = 0; b < OUT; b += 8) {
+                float o[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[c + b + i]);
+                store8(line + b, o);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst)[i] = q[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                reinterpret_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            store_turned(turn, C, row0, n0 + c0 + c, M, N, ldc, wide);
         }
-    } else {
-        for (int i = 0; i < 32; ++i)
-            if (col + i < N) dst[i] = from_f32<TO>(__uint_as_float(v[i]));
     }
 }
 }  // namespace tc5

@@ -68,7 +68,7 @@ class Linear:
         ws = step.workspace
         out = ws.get(step.tag + tag + ".act", (M, self.out_features // 2), a.dtype)
         if (group == ops.SWIGLU_GROUP and self.bias is None and self.weight.dtype == torch.bfloat16
-                and a.dtype == torch.bfloat16 and matmul.fuses_swiglu(M, self.in_features)):
+                and a.dtype == torch.bfloat16 and matmul.fuses_swiglu(M, self.in_features, self.out_features)):
             return matmul.gemm_bf16(a, self.weight, out, step.err, swiglu=True)
         return ops.silu_mul(self(a, step, tag), out, group)
 

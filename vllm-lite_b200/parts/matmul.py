@@ -17,9 +17,9 @@ from ..csrc import ops
 torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 
-def fuses_swiglu(M, K) -> bool:
+def fuses_swiglu(M, K, N=None) -> bool:
     """Whether the product for M rows runs in a kernel that can apply SwiGLU to its own tile."""
-    return ops.gemm_bf16_small_m_ok(M, K) or ops.gemm_bf16_tc5_ok(M, K, fused=True)
+    return ops.gemm_bf16_small_m_ok(M, K) or ops.gemm_bf16_tc5_ok(M, K, fused=True, N=N)
 
 
 def gemm_bf16(a, w, out, err=None, swiglu=False):
@@ -28,11 +28,12 @@ def gemm_bf16(a, w, out, err=None, swiglu=False):
     M, K = a.shape
     if ops.gemm_bf16_small_m_ok(M, K):
         return ops.gemm_bf16_small_m(a, w, out, err, swiglu)
-    if ops.gemm_bf16_tc5_ok(M, K, fused=swiglu):
-        # Two SMs on a 256 x 256 tile halve the rows of w each SM copies; measured faster (3 to 7 %) when
-        # there are tiles for every pair of SMs or K is long, slower (2 to 6 %) for the short, narrow products.
-        N = w.shape[0]
-        if -(-M // 256) * -(-N // 256) >= ops.sm_pairs() or K >= 8192:
+    N = w.shape[0]
+    if ops.gemm_bf16_tc5_ok(M, K, fused=swiglu, N=N):
+        # Two SMs on a 256 x 256 tile halve the rows of w each SM copies; faster where there are tiles for every pair of SMs, or K is long
+        # and the other kernel's tiles are wide (us, one SM / two: 2,048 x 4,096 -> 4,096 56 / 49, 2,048 x 8,192 -> 2,048 52 / 49, 4,096 x 4,096 ->
+        # 640 27.6 / 25.5; 2,048 x 2,048 -> 2,048 16.9 / 16.8, 2,048 x 4,096 -> 640 20.2 / 24.7, 4,096 x 2,048 -> 832 16.4 / 16.5)
+        if -(-M // 256) * -(-N // 256) >= ops.sm_pairs() or (K >= 4096 and -(-M // 128) * -(-N // 128) > 2 * ops.sm_pairs()):
             return ops.gemm_bf16_tc5_pair(a, w, out, err, swiglu)
         return ops.gemm_bf16_tc5(a, w, out, err, swiglu)
     if swiglu:
