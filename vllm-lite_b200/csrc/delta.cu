@@ -706,7 +706,8 @@ delta_out_kernel(const float* __restrict__ qkv, int C, const TP* __restrict__ pr
 // bfloat16 numbers are exact in float32, and of the nine products of parts the six down to 2^-16 of the largest are added, in
 // float32, the small ones first; what is left out lies below 2^-24 of a product (Henry, Tang, Heinecke, "Leveraging the
 // bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations").  Operands stay float32 in memory and are split in
-// registers as fragments of mma.sync m16n8k16.  Same three launches, the same buffers (W and U0 row by row, [64][D], [64][P]).
+// registers as fragments of mma.sync m16n8k16, but for what the walk (2) multiplies by, which (1) and the walk itself leave in parts.
+// Same three launches; W, U0 and the k rows row by row.
 struct FragA { unsigned h[4], m[4], l[4]; };
 struct FragB { unsigned h[2], m[2], l[2]; };
 __device__ __forceinline__ void split2(float x, float y, unsigned& h, unsigned& m, unsigned& l) {
@@ -720,19 +721,12 @@ __device__ __forceinline__ void split2(float x, float y, unsigned& h, unsigned& 
     m = pack(x, y);
     l = pack(x - __uint_as_float(m << 16), y - __uint_as_float(m & 0xffff0000u));
 }
-// rows r, r + 8 and columns k, k + 1, k + 8, k + 9 (r, k: this lane's own) of a matrix stored row by row / column by column
+// rows r, r + 8 and columns k, k + 1, k + 8, k + 9 (r, k: this lane's own) of a matrix stored row by row
 __device__ __forceinline__ void frag_a_rows(FragA& f, const float* p, int ld, int r, int k) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 v = *reinterpret_cast<const float2*>(p + (r + 8 * (e & 1)) * ld + k + 8 * (e >> 1));
         split2(v.x, v.y, f.h[e], f.m[e], f.l[e]);
-    }
-}
-__device__ __forceinline__ void frag_a_cols(FragA& f, const float* p, int ld, int r, int k) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const float* q = p + (k + 8 * (e >> 1)) * ld + r + 8 * (e & 1);
-        split2(q[0], q[ld], f.h[e], f.m[e], f.l[e]);
     }
 }
 // column n, rows k, k + 1, k + 8, k + 9 of B: stored with k along a row ([n][k]) / with n along a row ([k][n])
@@ -749,6 +743,63 @@ __device__ __forceinline__ void frag_b_kn(FragB& f, const float* p, int ld, int 
         const float* q = p + (k + 8 * e) * ld + n;
         split2(q[0], q[ld], f.h[e], f.m[e], f.l[e]);
     }
+}
+// The same operands from matrices that lie in shared memory as their three parts already (`step` bytes from one to the next, rows of `ld`
+// bytes, an odd number of 16): an instruction a fragment and part, where splitting float32 takes fifty.
+__device__ __forceinline__ void dl_ldsm4(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void dl_ldsm4_turned(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void dl_ldsm2_turned(unsigned (&r)[2], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+// rows r0 .. r0 + 15, columns k0 .. k0 + 15 of A, stored row by row ([m][k]) / column by column ([k][m])
+__device__ __forceinline__ void parts_a_rows(FragA& f, unsigned p, int step, int ld, int r0, int k0) {
+    const int lane = threadIdx.x & 31;
+    const unsigned at = p + (r0 + (lane & 15)) * ld + (k0 + (lane >> 4) * 8) * 2;
+    dl_ldsm4(f.h, at); dl_ldsm4(f.m, at + step); dl_ldsm4(f.l, at + 2 * step);
+}
+__device__ __forceinline__ void parts_a_cols(FragA& f, unsigned p, int step, int ld, int r0, int k0) {
+    const int lane = threadIdx.x & 31, i = lane >> 3;
+    const unsigned at = p + (k0 + (i >> 1) * 8 + (lane & 7)) * ld + (r0 + (i & 1) * 8) * 2;
+    dl_ldsm4_turned(f.h, at); dl_ldsm4_turned(f.m, at + step); dl_ldsm4_turned(f.l, at + 2 * step);
+}
+// N tiles of 8 columns from n0 on, rows k0 .. k0 + 15 of B, stored with n along a row ([k][n])
+template <int N>
+__device__ __forceinline__ void parts_b(FragB* f, unsigned p, int step, int ld, int n0, int k0) {
+    const int lane = threadIdx.x & 31, i = lane >> 3;
+    if constexpr (N == 1) {
+        const unsigned at = p + (k0 + (lane & 15)) * ld + n0 * 2;
+        dl_ldsm2_turned(f[0].h, at); dl_ldsm2_turned(f[0].m, at + step); dl_ldsm2_turned(f[0].l, at + 2 * step);
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; j += 2) {
+            const unsigned at = p + (k0 + (i & 1) * 8 + (lane & 7)) * ld + (n0 + 8 * j + (i >> 1) * 8) * 2;
+            unsigned r[4];
+            dl_ldsm4_turned(r, at);
+            f[j].h[0] = r[0]; f[j].h[1] = r[1]; f[j + 1].h[0] = r[2]; f[j + 1].h[1] = r[3];
+            dl_ldsm4_turned(r, at + step);
+            f[j].m[0] = r[0]; f[j].m[1] = r[1]; f[j + 1].m[0] = r[2]; f[j + 1].m[1] = r[3];
+            dl_ldsm4_turned(r, at + 2 * step);
+            f[j].l[0] = r[0]; f[j].l[1] = r[1]; f[j + 1].l[0] = r[2]; f[j + 1].l[1] = r[3];
+        }
+    }
+}
+// A matrix of 64 rows of D numbers (Dp: up to the next 16) in parts lies in global memory as the walk wants it in shared memory, a copy
+// of one piece: rows of an odd number of 16 bytes, part after part.
+__host__ __device__ __forceinline__ int parts_ld(int Dp) { return Dp * 2 + 16; }
+__host__ __device__ __forceinline__ int parts_matrix(int Dp) { return DC * parts_ld(Dp); }
+// two neighbouring numbers of a matrix of parts
+template <typename P>
+__device__ __forceinline__ void store_parts(P* p, int step, float x, float y) {
+    unsigned h, m, l;
+    split2(x, y, h, m, l);
+    unsigned char* b = reinterpret_cast<unsigned char*>(p);
+    *reinterpret_cast<unsigned*>(b) = h;
+    *reinterpret_cast<unsigned*>(b + step) = m;
+    *reinterpret_cast<unsigned*>(b + 2 * step) = l;
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -771,9 +822,8 @@ __device__ __forceinline__ void mma_f32(float (*d)[4], const FragA& a, const Fra
 #pragma unroll
     for (int j = 0; j < N; ++j) mma_bf16(d[j], a.h, b[j].h);
 }
-// row strides on which the fragments' accesses meet no shared-memory bank twice: pairs along a row / single numbers down a column
+// the row stride on which the fragments' accesses, pairs along a row, meet no shared-memory bank twice
 __host__ __device__ __forceinline__ int ld_pairs(int n) { return n + ((8 - n) & 31); }
-__host__ __device__ __forceinline__ int ld_singles(int n) { return n + ((4 - n) & 15); }
 __host__ __device__ __forceinline__ int up16(int n) { return (n + 15) & ~15; }
 
 // (1) A warp's share of the lower triangle's twenty 16 x 8 tiles: up to two runs (row of tiles, first, last)
@@ -789,8 +839,8 @@ template <typename TP>
 __global__ void __launch_bounds__(256, 2)
 delta_prep_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict__ proj, int ld, int a_col, int b_col,
                       const float* __restrict__ dt_bias, const float* __restrict__ A_log, float q_scale, float unit_eps,
-                      const int* __restrict__ cu, int B, float* __restrict__ Wo, float* __restrict__ Uo, float* __restrict__ M,
-                      float* __restrict__ rows, int H, int G, int D, int P) {
+                      const int* __restrict__ cu, int B, unsigned char* __restrict__ Wo, unsigned char* __restrict__ Ko, float* __restrict__ Uo,
+                      float* __restrict__ M, float* __restrict__ rows, int H, int G, int D, int P) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float s_beta[DC], s_hi[DC], s_lo[DC], s_kn[DC], s_qn[DC];
     pdl_launch_dependents();
@@ -828,6 +878,19 @@ delta_prep_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict
             st4(K + t * LD + 4 * lane, make_float4(k[i].x * kn, k[i].y * kn, k[i].z * kn, k[i].w * kn));
         }
         if (lane == 0) { s_kn[t] = kn; s_qn[t] = qn; }
+    }
+    if (h % (H / G) == 0) {                                       // the k rows as they are, in parts, once a group of heads
+        unsigned char* ko = Ko + ((size_t)blockIdx.x * G + g) * 3 * parts_matrix(Dp);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (4 * lane < Dp) {
+                unsigned p[3][2];
+                split2(k[i].x, k[i].y, p[0][0], p[1][0], p[2][0]);
+                split2(k[i].z, k[i].w, p[0][1], p[1][1], p[2][1]);
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+                    *reinterpret_cast<uint2*>(ko + e * parts_matrix(Dp) + (warp + 8 * i) * parts_ld(Dp) + 8 * lane) = make_uint2(p[e][0], p[e][1]);
+            }
     }
     __syncthreads();
     const size_t ch = (size_t)blockIdx.x * H + h;
@@ -922,11 +985,12 @@ delta_prep_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict
                     x[i][j][2 * half + 1] = f * v.y;
                 }
             }
-        float* dst = values ? Uo + ch * DC * P : Wo + ch * DC * D;
+        float* dst = Uo + ch * DC * P;
+        unsigned char* wdst = Wo + ch * 3 * parts_matrix(Dp);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             FragB f[4];
-            auto turn = [&]() {                                   // this block row as the second operand
+            auto lay = [&]() {                                    // this block row, row by row
                 __syncwarp();
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -934,21 +998,42 @@ delta_prep_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict
                     *reinterpret_cast<float2*>(X + (gl + 8) * PREP_LDX + 8 * j + 2 * tl) = make_float2(x[i][j][2], x[i][j][3]);
                 }
                 __syncwarp();
+            };
+            auto turn = [&]() {                                   // ... as the second operand
 #pragma unroll
                 for (int j = 0; j < 4; ++j) frag_b_kn(f[j], X, PREP_LDX, 8 * j + gl, 2 * tl);
             };
+            lay();
             turn();
             FragA a;
             frag_a_rows(a, Ti + 16 * i * PREP_LDT, PREP_LDT, gl, 2 * tl);
 #pragma unroll
             for (int j = 0; j < 4; ++j) x[i][j][0] = x[i][j][1] = x[i][j][2] = x[i][j][3] = 0.f;
             mma_f32<4>(x[i], a, f);
+            lay();
+            if (values) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int col = c0 + 8 * j + 2 * tl;
-                if (col < width) {
-                    *reinterpret_cast<float2*>(dst + (size_t)(16 * i + gl) * width + col) = make_float2(x[i][j][0], x[i][j][1]);
-                    *reinterpret_cast<float2*>(dst + (size_t)(16 * i + gl + 8) * width + col) = make_float2(x[i][j][2], x[i][j][3]);
+                for (int j = 0; j < 4; ++j) {
+                    const int col = c0 + 8 * j + 2 * tl;
+                    if (col < width) {
+                        *reinterpret_cast<float2*>(dst + (size_t)(16 * i + gl) * width + col) = make_float2(x[i][j][0], x[i][j][1]);
+                        *reinterpret_cast<float2*>(dst + (size_t)(16 * i + gl + 8) * width + col) = make_float2(x[i][j][2], x[i][j][3]);
+                    }
+                }
+            } else if (c0 + 16 * (lane & 1) < Dp) {               // in parts, as the walk multiplies by it: 16 columns of a row a lane (D .. Dp: zeros)
+                const float* at = X + (lane >> 1) * PREP_LDX + 16 * (lane & 1);
+                unsigned char* to = wdst + (16 * i + (lane >> 1)) * parts_ld(Dp) + 2 * (c0 + 16 * (lane & 1));
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float4 v = ld4(at + 8 * e), w = ld4(at + 8 * e + 4);
+                    uint4 h, m, l;
+                    split2(v.x, v.y, h.x, m.x, l.x);
+                    split2(v.z, v.w, h.y, m.y, l.y);
+                    split2(w.x, w.y, h.z, m.z, l.z);
+                    split2(w.z, w.w, h.w, m.w, l.w);
+                    *reinterpret_cast<uint4*>(to + 16 * e) = h;
+                    *reinterpret_cast<uint4*>(to + 16 * e + parts_matrix(Dp)) = m;
+                    *reinterpret_cast<uint4*>(to + 16 * e + 2 * parts_matrix(Dp)) = l;
                 }
             }
             if (i < 3) {
@@ -964,14 +1049,26 @@ delta_prep_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict
 }
 
 // (2) CT value columns of one head and request: the state's tile as accumulators of the second product and, for the first, in
-// shared memory.
+// shared memory, in parts.  The requests' chunks follow one another, so this is bound by the way through one chunk: what a warp issues
+// between two barriers.  W and the k rows come from (1) in parts, each by one bulk copy: splitting them here, every tile of columns
+// anew, and 16 copies a thread and chunk were a third of that.  Requests of 809, 1,427 and 1,045 tokens, 16 heads of 128 x 128: 115 us
+// (150 before, and 106 instead of 94 for (1); parts fetched by copies of 16 bytes: 160).  A buffer of each: W's is free from the end of
+// the first product on, the k rows' from the end of the second, and each is filled beside the other product.
+template <int CT> struct WalkShape {
+    static constexpr int LDS = CT * 2 + 16, LDR = CT + 8;         // bytes of a row of parts; floats of a row of partial sums
+    static size_t bytes(int Dp) {
+        return (size_t)6 * parts_matrix(Dp) + 3 * (size_t)Dp * LDS + 3 * DC * LDS + sizeof(float) * (2 * (DC * CT + 2 * DC) + 4 * DC * LDR);
+    }
+};
 template <int CT>
 __global__ void __launch_bounds__(512)
-delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restrict__ W, const float* __restrict__ U0,
+delta_walk_mma_kernel(const unsigned char* __restrict__ W, const unsigned char* __restrict__ Kp, const float* __restrict__ U0,
                       const float* __restrict__ rows, float* __restrict__ U, float* __restrict__ S0, float* __restrict__ state,
-                      long long state_stride, const int* __restrict__ cu, const int* __restrict__ slots, int H, int G, int D, int P) {
-    constexpr int NT = CT / 8, LDS = CT + 4, LDR = CT + 8, NH = NT / 2;
-    extern __shared__ __align__(16) float sm[];
+                      long long state_stride, const int* __restrict__ cu, const int* __restrict__ slots, int H, int G, int D, int P,
+                      unsigned* err) {
+    constexpr int NT = CT / 8, NH = NT / 2, LDS = WalkShape<CT>::LDS, LDR = WalkShape<CT>::LDR;
+    extern __shared__ __align__(16) unsigned char walk_sm[];
+    __shared__ __align__(8) unsigned long long w_bar, k_bar;
     pdl_launch_dependents();
     pdl_wait();
     const int h = blockIdx.x, p0 = blockIdx.y * CT, b = ci_by_length(cu, gridDim.z, blockIdx.z);
@@ -979,73 +1076,81 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
     if (n < DELTA_MIN_CHUNK) return;
     const int first = dl_first_chunk(cu, b), chunks = (n + DC - 1) / DC;
     const int g = h / (H / G), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gl = lane >> 2, tl = lane & 3;
-    const int Dp = up16(D), LDW = ld_pairs(Dp), LDK = ld_singles(Dp);
-    const int stage = DC * LDW + DC * LDK + DC * CT + 2 * DC;
-    float* Ss = sm + 2 * stage;                                   // [Dp][LDS]
-    float* red = Ss + Dp * LDS;                                   // [4][64][LDR]
-    float* Us = red + 4 * DC * LDR;                               // [64][LDS]: U times the k rows' factors
-    if (Dp > D)                                                   // columns D .. Dp of both stages, once: no copy writes them
-        for (int i = tid; i < 2 * DC * (Dp - D); i += 512) {
-            const int t = i / (Dp - D), col = D + i - t * (Dp - D);
-            float* w = sm + (t >= DC ? stage : 0);
-            w[(t & (DC - 1)) * LDW + col] = 0.f;
-            w[DC * LDW + (t & (DC - 1)) * LDK + col] = 0.f;
-        }
-    auto fetch = [&](int c, int buf) {
-        float* w = sm + buf * stage;
-        float* k = w + DC * LDW;
-        float* u = k + DC * LDK;
-        float* f = u + DC * CT;
+    const int Dp = up16(D), LD = parts_ld(Dp), MAT = parts_matrix(Dp), SP = Dp * LDS, UP = DC * LDS;
+    unsigned char* Ws = walk_sm;                                  // [3][64][LD bytes]
+    unsigned char* Ks = Ws + 3 * MAT;                             // the same
+    unsigned char* Sp = Ks + 3 * MAT;                             // the state [3][Dp][LDS]
+    unsigned char* Up = Sp + 3 * SP;                              // U times the k rows' factors [3][64][LDS]
+    float* u0 = reinterpret_cast<float*>(Up + 3 * UP);            // two of [64][CT] and 128 factors
+    float* red = u0 + 2 * (DC * CT + 2 * DC);                     // [4][64][LDR]
+    if (tid == 0) {
+        tc5::mbar_init(&w_bar, 1);
+        tc5::mbar_init(&k_bar, 1);
+        tc5::mbar_fence_init();
+    }
+    __syncthreads();
+    auto fetch_parts = [&](unsigned char* dst, const unsigned char* src, unsigned long long* bar) {        // one thread
+        tc5::mbar_arrive_expect_tx(bar, 3u * MAT);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(tc5::smem_u32(dst)), "l"(src), "r"(3u * MAT), "r"(tc5::smem_u32(bar)) : "memory");
+    };
+    auto fetch_w = [&](int c) {
         const size_t ch = (size_t)(first + c) * H + h;
-        const int m = min(DC, n - c * DC);
-        if (4 * lane < D) {
-            const float* wg = W + ch * DC * D + 4 * lane;
-            const float* kg = qkv + (size_t)(s0 + c * DC) * C + (size_t)(G + g) * D + 4 * lane;
-#pragma unroll
-            for (int i = 0; i < DC / 16; ++i) {
-                const int t = warp + 16 * i;
-                dl_copy16(w + t * LDW + 4 * lane, wg + t * D, true);
-                dl_copy16(k + t * LDK + 4 * lane, t < m ? kg + (size_t)t * C : kg, t < m);
-            }
-        }
+        float* u = u0 + (c & 1) * (DC * CT + 2 * DC);
+        if (tid == 0) fetch_parts(Ws, W + ch * 3 * MAT, &w_bar);
         if (tid < DC * CT / 4) {
             const int t = tid / (CT / 4), col = 4 * (tid % (CT / 4));
             const bool ok = p0 + col < P;
             dl_copy16(u + t * CT + col, ok ? U0 + (ch * DC + t) * P + p0 + col : U0, ok);
         }
-        if (tid < 2 * DC / 4) dl_copy16(f + 4 * tid, rows + ch * DL_ROWS * DC + DC + 4 * tid, true);
+        if (tid < 2 * DC / 4) dl_copy16(u + DC * CT + 4 * tid, rows + ch * DL_ROWS * DC + DC + 4 * tid, true);
+        dl_commit();
     };
+    auto fetch_k = [&](int c) {
+        if (tid == 0) fetch_parts(Ks, Kp + ((size_t)(first + c) * G + g) * 3 * MAT, &k_bar);
+    };
+    auto drain = [&](int c) {                                     // copies in flight when a wait ran out: waited for once more
+        tc5::mbar_wait_bounded(&w_bar, (unsigned)(c & 1));
+        tc5::mbar_wait_bounded(&k_bar, (unsigned)(c & 1));
+        if (c + 1 < chunks) tc5::mbar_wait_bounded(&w_bar, (unsigned)((c + 1) & 1));
+        dl_wait<0>();
+    };
+    fetch_w(0);
+    fetch_k(0);
     // second product: rows 16 mt2 .. of the state, half of its columns' tiles from nlo on
     const int mt2 = warp & 7, nlo = (warp >> 3) * NH;
     const bool owner = 16 * mt2 < Dp;
     float* gs = state + (long long)slots[b] * state_stride + (size_t)h * D * P + p0;
     const int da = 16 * mt2 + gl, db = da + 8;
-    float sr[NH][4];
+    float sr[NH][4] = {};
+    auto keep_parts = [&](int j) {
+        unsigned char* at = Sp + da * LDS + (8 * (nlo + j) + 2 * tl) * 2;
+        store_parts(at, SP, sr[j][0], sr[j][1]);
+        store_parts(at + 8 * LDS, SP, sr[j][2], sr[j][3]);
+    };
 #pragma unroll
     for (int j = 0; j < NH; ++j) {
         const int col = 8 * (nlo + j) + 2 * tl;
         float2 x = make_float2(0.f, 0.f), y = x;
-        if (owner) {
-            if (p0 + col < P) {
-                if (da < D) x = *reinterpret_cast<const float2*>(gs + (size_t)da * P + col);
-                if (db < D) y = *reinterpret_cast<const float2*>(gs + (size_t)db * P + col);
-            }
-            *reinterpret_cast<float2*>(Ss + da * LDS + col) = x;
-            *reinterpret_cast<float2*>(Ss + db * LDS + col) = y;
+        if (owner && p0 + col < P) {
+            if (da < D) x = *reinterpret_cast<const float2*>(gs + (size_t)da * P + col);
+            if (db < D) y = *reinterpret_cast<const float2*>(gs + (size_t)db * P + col);
         }
         sr[j][0] = x.x; sr[j][1] = x.y; sr[j][2] = y.x; sr[j][3] = y.y;
+        if (owner) keep_parts(j);
     }
     // first product: tokens 16 mt1 .., every fourth step of 16 rows of the state
     const int mt1 = warp & 3, kh = warp >> 2;
-    fetch(0, 0);
-    dl_commit();
+    const unsigned ws = tc5::smem_u32(Ws), ks = tc5::smem_u32(Ks), sp = tc5::smem_u32(Sp), up = tc5::smem_u32(Up);
 #pragma unroll 1
     for (int c = 0; c < chunks; ++c) {
         dl_wait<0>();
-        __syncthreads();
-        const float* w = sm + (c & 1) * stage;
-        const float* k = w + DC * LDW;
-        const float* u = k + DC * LDK;
+        if (__syncthreads_or(!tc5::mbar_wait_bounded(&w_bar, (unsigned)(c & 1)))) {        // (everyone waits; a wait that ran out ends the block)
+            if (tid == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_DELTA);
+            drain(c);
+            return;
+        }
+        const float* u = u0 + (c & 1) * (DC * CT + 2 * DC);
         const float* f = u + DC * CT;
         if (owner) {
             float* so = S0 + (((size_t)(first + c) * H + h) * D) * P + p0;
@@ -1064,10 +1169,9 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
 #pragma unroll 2
         for (int d = 16 * kh; d < Dp; d += 64) {
             FragA a;
-            frag_a_rows(a, w, LDW, 16 * mt1 + gl, d + 2 * tl);
+            parts_a_rows(a, ws, MAT, LD, 16 * mt1, d);
             FragB q[NT];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) frag_b_kn(q[j], Ss, LDS, 8 * j + gl, d + 2 * tl);
+            parts_b<NT>(q, sp, SP, LDS, 0, d);
             mma_f32<NT>(acc, a, q);
         }
 #pragma unroll
@@ -1075,8 +1179,8 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
 #pragma unroll
             for (int half = 0; half < 2; ++half)
                 *reinterpret_cast<float2*>(red + (kh * DC + 16 * mt1 + gl + 8 * half) * LDR + 8 * j + 2 * tl) = make_float2(acc[j][2 * half], acc[j][2 * half + 1]);
-        if (c + 1 < chunks) { fetch(c + 1, (c + 1) & 1); dl_commit(); }       // (that stage was last read before this chunk began)
         __syncthreads();
+        if (c + 1 < chunks) fetch_w(c + 1);
         const int m = min(DC, n - c * DC);
 #pragma unroll
         for (int i = 0; i < DC * CT / 2 / 512; ++i) {             // two columns of a token a thread: the four parts, in order
@@ -1088,10 +1192,14 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
                 r.x += q.x; r.y += q.y;
             }
             const float2 v0 = *reinterpret_cast<const float2*>(u + t * CT + col), v = make_float2(v0.x - r.x, v0.y - r.y);
-            *reinterpret_cast<float2*>(Us + t * LDS + col) = make_float2(v.x * f[t], v.y * f[t]);
+            store_parts(Up + t * LDS + col * 2, UP, v.x * f[t], v.y * f[t]);
             if (t < m && p0 + col < P) *reinterpret_cast<float2*>(U + (size_t)(s0 + c * DC + t) * H * P + (size_t)h * P + p0 + col) = v;
         }
-        __syncthreads();
+        if (__syncthreads_or(!tc5::mbar_wait_bounded(&k_bar, (unsigned)(c & 1)))) {
+            if (tid == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_DELTA);
+            drain(c);
+            return;
+        }
         if (owner) {
             const float keep = f[DC];
 #pragma unroll
@@ -1099,19 +1207,16 @@ delta_walk_mma_kernel(const float* __restrict__ qkv, int C, const float* __restr
 #pragma unroll
             for (int t = 0; t < DC; t += 16) {
                 FragA a;
-                frag_a_cols(a, k, LDK, 16 * mt2 + gl, t + 2 * tl);
+                parts_a_cols(a, ks, MAT, LD, 16 * mt2, t);
                 FragB q[NH];
-#pragma unroll
-                for (int j = 0; j < NH; ++j) frag_b_kn(q[j], Us, LDS, 8 * (nlo + j) + gl, t + 2 * tl);
+                parts_b<NH>(q, up, UP, LDS, 8 * nlo, t);
                 mma_f32<NH>(sr, a, q);
             }
 #pragma unroll
-            for (int j = 0; j < NH; ++j) {
-                const int col = 8 * (nlo + j) + 2 * tl;
-                *reinterpret_cast<float2*>(Ss + da * LDS + col) = make_float2(sr[j][0], sr[j][1]);
-                *reinterpret_cast<float2*>(Ss + db * LDS + col) = make_float2(sr[j][2], sr[j][3]);
-            }
+            for (int j = 0; j < NH; ++j) keep_parts(j);
         }
+        __syncthreads();                                          // K's buffer has been read
+        if (c + 1 < chunks) fetch_k(c + 1);
     }
     if (owner) {
 #pragma unroll
@@ -1238,9 +1343,10 @@ delta_out_mma_kernel(const float* __restrict__ qkv, int C, const TP* __restrict_
 }
 
 extern "C" int vl_delta_min_chunk() { return DELTA_MIN_CHUNK; }
-// Floats of the scratch for a launch of up to `chunks` chunks: W^T, U0^T, M, row factors, chunk states (U has its own [T, H P]).
+// Floats of the scratch for a launch of up to `chunks` chunks: W and the k rows in three bfloat16 parts each (float32 steps: W^T alone, in
+// their place), U0, M, row factors, chunk states (U has its own [T, H P]).
 extern "C" long long vl_delta_chunk_floats(int chunks, int H, int D, int P) {
-    return (long long)chunks * H * ((long long)D * DC + (long long)P * DC + DC * DC + DL_ROWS * DC + (long long)D * P);
+    return (long long)chunks * H * (6ll * (parts_matrix(up16(D)) / 4) + (long long)P * DC + DC * DC + DL_ROWS * DC + (long long)D * P);
 }
 
 template <typename K>
@@ -1257,44 +1363,52 @@ static int launch_walk(const float* qkv, int C, const float* Wt, const float* Ut
                      cu, slots, H, G, D, P);
 }
 template <int CT>
-static int launch_walk_mma(const float* qkv, int C, const float* W, const float* U0, const float* rows, float* U, float* S0, float* state,
-                           long long state_stride, const int* cu, const int* slots, int B, int H, int G, int D, int P, cudaStream_t s) {
-    const int Dp = up16(D);
-    const size_t smem = sizeof(float) * ((size_t)2 * (DC * (ld_pairs(Dp) + ld_singles(Dp)) + DC * CT + 2 * DC) + (size_t)Dp * (CT + 4)
-                                         + 4 * DC * (CT + 8) + DC * (CT + 4));
+static int launch_walk_mma(const unsigned char* W, const unsigned char* Kp, const float* U0, const float* rows, float* U, float* S0, float* state,
+                           long long state_stride, const int* cu, const int* slots, int B, int H, int G, int D, int P, unsigned* err, cudaStream_t s) {
+    const size_t smem = WalkShape<CT>::bytes(up16(D));
     const int rc = delta_smem(delta_walk_mma_kernel<CT>, smem);
     if (rc) return rc;
-    return vl_launch(delta_walk_mma_kernel<CT>, dim3(H, (P + CT - 1) / CT, B), dim3(512), smem, s, qkv, C, W, U0, rows, U, S0, state,
-                     state_stride, cu, slots, H, G, D, P);
+    return vl_launch(delta_walk_mma_kernel<CT>, dim3(H, (P + CT - 1) / CT, B), dim3(512), smem, s, W, Kp, U0, rows, U, S0, state,
+                     state_stride, cu, slots, H, G, D, P, err);
 }
 // MMA false: the kernels of plain float32 multiply-adds (float32 steps), else those on the tensor cores (bfloat16 steps).
 template <typename TP, bool MMA>
 static int launch_chunks(const float* qkv, int C, const TP* proj, int ld, int a_col, int b_col, int gate_col, const float* dt_bias,
                          const float* A_log, float q_scale, float unit_eps, const float* norm, float eps, float* state,
                          long long state_stride, const int* cu, const int* slots, int B, int chunks, float* scratch, float* U, TP* out,
-                         int H, int G, int D, int P, int sms, cudaStream_t s) {
+                         int H, int G, int D, int P, int sms, unsigned* err, cudaStream_t s) {
     const size_t n = (size_t)chunks * H;
+    const int Dp = up16(D);
     float* W = scratch;
-    float* U0 = W + n * D * DC;
+    unsigned char* Wp = reinterpret_cast<unsigned char*>(scratch);
+    unsigned char* Kp = Wp + n * 3 * parts_matrix(Dp);
+    float* U0 = W + n * 6 * (parts_matrix(Dp) / 4);
     float* M = U0 + n * P * DC;
     float* rows = M + n * DC * DC;
     float* S0 = rows + n * DL_ROWS * DC;
-    const int Dp = up16(D);
     int rc;
     {
         auto kernel = [] { if constexpr (MMA) return delta_prep_mma_kernel<TP>; else return delta_prep_kernel<TP>; }();
         const size_t smem = sizeof(float) * (MMA ? (size_t)DC * ld_pairs(Dp) + prep_second(D, P) + DC * PREP_LDN + 4 * 16 * PREP_LDT + 8 * 16 * PREP_LDX
                                                  : (size_t)2 * DC * (D + 4) + DC * PREP_LDA);
         if ((rc = delta_smem(kernel, smem))) return rc;
-        rc = vl_launch(kernel, dim3(chunks, H), dim3(256), smem, s, qkv, C, proj, ld, a_col, b_col, dt_bias, A_log, q_scale, unit_eps, cu, B,
-                       W, U0, M, rows, H, G, D, P);
+        if constexpr (MMA)
+            rc = vl_launch(kernel, dim3(chunks, H), dim3(256), smem, s, qkv, C, proj, ld, a_col, b_col, dt_bias, A_log, q_scale, unit_eps, cu, B,
+                           Wp, Kp, U0, M, rows, H, G, D, P);
+        else
+            rc = vl_launch(kernel, dim3(chunks, H), dim3(256), smem, s, qkv, C, proj, ld, a_col, b_col, dt_bias, A_log, q_scale, unit_eps, cu, B,
+                           W, U0, M, rows, H, G, D, P);
         if (rc) return rc;
     }
     // narrow tiles of columns while they leave an SM to every block
     const bool narrow = (long long)H * B * ((P + 15) / 16) <= sms;
-#define DELTA_WALK(FN) FN(qkv, C, W, U0, rows, U, S0, state, state_stride, cu, slots, B, H, G, D, P, s)
-    if constexpr (MMA) rc = narrow ? DELTA_WALK(launch_walk_mma<16>) : DELTA_WALK(launch_walk_mma<32>);
-    else rc = narrow ? DELTA_WALK(launch_walk<16>) : DELTA_WALK(launch_walk<32>);
+#define DELTA_WALK(FN, A, B_) FN(A, B_, U0, rows, U, S0, state, state_stride, cu, slots, B, H, G, D, P, err, s)
+    if constexpr (MMA) {
+        rc = narrow ? DELTA_WALK(launch_walk_mma<16>, Wp, Kp) : DELTA_WALK(launch_walk_mma<32>, Wp, Kp);
+    } else {
+        rc = narrow ? launch_walk<16>(qkv, C, W, U0, rows, U, S0, state, state_stride, cu, slots, B, H, G, D, P, s)
+                    : launch_walk<32>(qkv, C, W, U0, rows, U, S0, state, state_stride, cu, slots, B, H, G, D, P, s);
+    }
 #undef DELTA_WALK
     if (rc) return rc;
     auto outputs = [&](auto kernel, size_t smem) {
@@ -1318,7 +1432,7 @@ static int launch_chunks(const float* qkv, int C, const TP* proj, int ld, int a_
 extern "C" int vl_delta_chunks(const float* qkv, int C, const void* proj, int dtype, int ld, int a_col, int b_col, int gate_col,
                                const float* dt_bias, const float* A_log, float q_scale, float unit_eps, const float* norm, float eps,
                                float* state, long long state_stride, const int* cu, const int* slots, int B, int chunks, float* scratch,
-                               float* U, void* out, int H, int G, int D, int P, int sms, void* stream) {
+                               float* U, void* out, int H, int G, int D, int P, int sms, unsigned* err, void* stream) {
     if (B <= 0 || chunks <= 0) return VL_OK;
     if (!delta_sizes_ok(H, G, D, P, C) || B > 65535 || H > 65535) return VL_ERR_UNSUPPORTED;
     if (ld % 4 || gate_col % 4 || state_stride % 4 ||
@@ -1327,9 +1441,9 @@ extern "C" int vl_delta_chunks(const float* qkv, int C, const void* proj, int dt
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == VL_F32)
         return launch_chunks<float, false>(qkv, C, (const float*)proj, ld, a_col, b_col, gate_col, dt_bias, A_log, q_scale, unit_eps, norm, eps,
-                                    state, state_stride, cu, slots, B, chunks, scratch, U, (float*)out, H, G, D, P, sms, s);
+                                    state, state_stride, cu, slots, B, chunks, scratch, U, (float*)out, H, G, D, P, sms, err, s);
     if (dtype == VL_BF16)
         return launch_chunks<bf16, true>(qkv, C, (const bf16*)proj, ld, a_col, b_col, gate_col, dt_bias, A_log, q_scale, unit_eps, norm, eps,
-                                   state, state_stride, cu, slots, B, chunks, scratch, U, (bf16*)out, H, G, D, P, sms, s);
+                                   state, state_stride, cu, slots, B, chunks, scratch, U, (bf16*)out, H, G, D, P, sms, err, s);
     return VL_ERR_UNSUPPORTED;
 }

@@ -164,7 +164,7 @@ _SIGNATURES = {
                                  c_int, c_int, c_int, c_void_p, c_void_p],
     ("delta", "vl_delta_chunks"): [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float,
                                    c_void_p, c_float, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ("recurrent", "vl_gate_norm"): [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p,
                                     c_int, c_int, c_int, c_void_p],
 }
@@ -1739,12 +1739,12 @@ def delta_step(qkv, proj, a_col, b_col, gate_col, dt_bias, A_log, q_scale, unit_
 
 def delta_chunk_floats(chunks, H, D, P) -> int:
     """Floats of the scratch that `delta_chunks` needs for so many chunks (csrc/delta.cu)."""
-    c = DELTA_CHUNK
-    return chunks * H * (D * c + P * c + c * c + 3 * c + D * P)
+    c, rows = DELTA_CHUNK, -(-D // 16) * 16              # two matrices in three bfloat16 parts: 2 x 3 / 2 floats a number
+    return chunks * H * (3 * (rows + 8) * c + P * c + c * c + 3 * c + D * P)
 
 
 def delta_chunks(qkv, proj, a_col, b_col, gate_col, dt_bias, A_log, q_scale, unit_eps, norm, eps, state, state_off, cu, slots, chunks, scratch,
-                 u, out, H, G, D, P):
+                 u, out, H, G, D, P, err=None):
     """The same for the requests that bring DELTA_MIN_CHUNK tokens or more, in chunks of 64 tokens.  `chunks`: a bound on the
     chunks of the step; scratch float32 of `delta_chunk_floats`; u float32 [T, H P]."""
     global launch_count
@@ -1755,7 +1755,7 @@ def delta_chunks(qkv, proj, a_col, b_col, gate_col, dt_bias, A_log, q_scale, uni
     _check(_fn("delta", "vl_delta_chunks")(
         _ptr(qkv), qkv.shape[1], _ptr(proj), dtype_code(proj.dtype), proj.shape[1], int(a_col), int(b_col), int(gate_col), _ptr(dt_bias),
         _ptr(A_log), float(q_scale), float(unit_eps), _ptr(norm), float(eps), sp, stride, _ptr(cu), _ptr(slots), B, int(chunks), _ptr(scratch),
-        _ptr(u), _ptr(out), H, G, D, P, 2 * sm_pairs(), _stream()), "vl_delta_chunks")
+        _ptr(u), _ptr(out), H, G, D, P, 2 * sm_pairs(), _ptr(err), _stream()), "vl_delta_chunks")
     launch_count += 2             # three launches
     return out
 

@@ -236,7 +236,8 @@ class HeadDelta:
             if step.max_query_len >= ops.DELTA_MIN_CHUNK:
                 chunks = T // ops.DELTA_CHUNK + B
                 scratch = ws.get(tag + "hd.chunks", (ops.delta_chunk_floats(chunks, H, D, P),), torch.float32)
-                ops.delta_chunks(*args, chunks, scratch, ws.get(tag + "hd.u", (T, H * P), torch.float32), gated, H, G, D, P)
+                ops.delta_chunks(*args, chunks, scratch, ws.get(tag + "hd.u", (T, H * P), torch.float32), gated, H, G, D, P,
+                                 err=step.err)
             if step.max_query_len < ops.DELTA_MIN_CHUNK or B > 1:
                 ops.delta_step(*args, gated, H, G, D, P, err=step.err)
             return self.o_proj(gated, step, "hd.out")
