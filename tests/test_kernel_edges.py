@@ -28,6 +28,19 @@ def test_gemm_f32_tiles(M, N, K):
     assert torch.equal(one[0], out[M - 1])               # whichever tile made the row
 
 
+# the activation in the product's epilogue: the bits of the product and the activation by themselves, in every tile
+@pytest.mark.parametrize("I,K,group", [(1, 1, 0), (7, 63, 0), (160, 96, 8), (161, 97, 0), (24, 64, 4), (352, 260, 16), (4104, 68, 8)])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 64, 65, 130])
+def test_gemm_f32_with_its_activation(M, I, K, group):
+    gen = torch.Generator(device=DEV).manual_seed(M * 131 + I + K)
+    a, w = torch.randn(M, K, device=DEV, generator=gen), torch.randn(2 * I, K, device=DEV, generator=gen)
+    product, want = torch.empty(M, 2 * I, device=DEV), torch.empty(M, I, device=DEV)
+    out = torch.full((M, I), float("nan"), device=DEV)
+    ops().silu_mul(ops().gemm_f32(a, w, product), want, group)
+    ops().gemm_f32(a, w, out, swiglu=True, group=group)
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,I,group", [(1, 8, 0), (3, 4096, 0), (5, 12, 0), (2, 7, 0), (3, 64, 8), (3, 64, 16), (5, 36, 4), (7, 48, 24)])
 def test_silu_mul_layouts(T, I, group, dtype):

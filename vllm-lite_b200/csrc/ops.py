@@ -131,7 +131,7 @@ _SIGNATURES = {
     ("moe", "vl_moe_gather"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ("moe", "vl_moe_combine"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_void_p, c_void_p],
-    ("gemm_f32", "vl_gemm_f32_nt"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    ("gemm_f32", "vl_gemm_f32_nt"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     ("gemm_bf16", "vl_gemm_bf16_small_m"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                             c_void_p, c_int, c_void_p],
     ("gemm_bf16", "vl_gemm_bf16_small_m_fused"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -1344,14 +1344,17 @@ def moe_combine(result, place, weights, top, out, scale_output, add=None, add_we
 
 
 # ---------------------------------------------------------------- matrix products
-def gemm_f32(a, w, out):
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K)."""
+def gemm_f32(a, w, out, swiglu=False, group=0):
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K).  swiglu: out[M, N / 2] = silu(gate) * up, the rows of w
+    being gates and ups in `silu_mul`'s layout of columns (group 0 or a power of two)."""
     _need(a, torch.float32, "a", 2); _need(w, torch.float32, "w", 2); _need(out, torch.float32, "out", 2)
     M, K = a.shape
     N = w.shape[0]
-    if w.shape[1] != K or out.shape != (M, N):
-        raise KernelError(f"gemm_f32: shapes disagree a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
-    _check(_fn("gemm_f32", "vl_gemm_f32_nt")(_ptr(a), _ptr(w), _ptr(out), M, N, K, K, K, N, _stream()), "vl_gemm_f32_nt")
+    cols = N // 2 if swiglu else N
+    if w.shape[1] != K or out.shape != (M, cols) or (swiglu and (N % 2 or group < 0 or group & (group - 1) or (group and cols % group))):
+        raise KernelError(f"gemm_f32: shapes disagree a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}, group {group}")
+    _check(_fn("gemm_f32", "vl_gemm_f32_nt")(_ptr(a), _ptr(w), _ptr(out), M, N, K, K, K, cols, int(swiglu), int(group), _stream()),
+           "vl_gemm_f32_nt")
     return out
 
 

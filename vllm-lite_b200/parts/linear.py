@@ -70,6 +70,8 @@ class Linear:
         if (group == ops.SWIGLU_GROUP and self.bias is None and self.weight.dtype == torch.bfloat16
                 and a.dtype == torch.bfloat16 and matmul.fuses_swiglu(M, self.in_features, self.out_features)):
             return matmul.gemm_bf16(a, self.weight, out, step.err, swiglu=True)
+        if self.bias is None and self.weight.dtype == a.dtype == torch.float32 and group & (group - 1) == 0:
+            return ops.gemm_f32(a, self.weight, out, swiglu=True, group=group)
         return ops.silu_mul(self(a, step, tag), out, group)
 
     def __call__(self, a, step, tag, out_dtype=None):
