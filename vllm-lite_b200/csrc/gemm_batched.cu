@@ -11,7 +11,7 @@
 // place or on its neighbours.  In float32 this is the true 32-bit product; in bfloat16 it is the
 // fallback for the sizes that the tensor-core version does not take.
 // Tiles of BM x 64 x 16 (BM = 64 or 16), 256 threads; any M, N, K.
-#include "common.cuh"
+#include "tc5.cuh"
 
 // VLLM_LITE_B200_BATCHED_SIMT=1 keeps bfloat16 products on the FFMA kernel (tests compare the two).
 static inline bool vl_batched_simt_only() {
@@ -291,151 +291,235 @@ static int launch_mma_kernel(dim3 grid, cudaStream_t s, int K, Args... args) {
 }
 
 // The same for the few rows an expert gets in a decode step (tiles of 16 rows), where the launch is one read of the reached experts'
-// weights: blocks that stay.  The (tile, 64 columns) items up to the last tile that holds rows are dealt out evenly, every G-th to a block
-// (those of places without rows in between, which a sort leaves none of, are passed over), and the ring of copies runs on from one
-// item into the next, so that neither places without rows nor the start of an item interrupt the stream.  An element's sum runs over
-// K in the same steps as above.  Against a block per place and 64 columns, weights from memory, 32 experts of 2,048 x 2,048 gate/up,
-// top 4: 32 tokens 61.8 -> 52.0 us (the read alone takes 40), 8 tokens 51.8 -> 37.1 (24); 64 experts of 2,816 x 4,096, top 6, 64 tokens 279 ->
-// 269 (219).  Rings of 3 and 6 stages instead of 4, with the old grid: 72 and 81 us at 32 tokens.
-#define GE_MIN_STEPS 8                                           // steps of 64 columns of K (the next item is found during the first of them)
-template <typename TC>
-__global__ void __launch_bounds__(128)
-gemm_experts_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, TC* __restrict__ C, int N, int K, int lda, int ldc,
-                    const int* __restrict__ tile_group, int tiles, long long w_gs, const int* __restrict__ row_index, int index_div,
-                    const float* __restrict__ row_scale, int act, float alpha, float limit, float shift) {
-    constexpr int BM = 16, CH = GM_BK / 8;
-    extern __shared__ __align__(16) unsigned char gm_smem[];
-    bf16 (*As)[BM][GM_LDS] = reinterpret_cast<bf16 (*)[BM][GM_LDS]>(gm_smem);
-    bf16 (*Ws)[GM_BN][GM_LDS] = reinterpret_cast<bf16 (*)[GM_BN][GM_LDS]>(gm_smem + (size_t)GM_NST * BM * GM_LDS * sizeof(bf16));
-    __shared__ int s_src[2][BM];                                 // source rows of an item's tile (-1: zeros), this item's and the next one's
-    __shared__ int s_tiles;
+// weights: blocks that stay, each with a ring of NST stages (64 rows of W by TMA and the tile's 16 rows of A, 128 columns of K) that its
+// fifth warp fills as far ahead as there is room and the other four, 16 columns of the product each, work off: 14 MB of weights under way.
+// The (tile, 64 columns) items up to the last tile that holds rows are dealt out in rounds, an item a block; a last round that would leave
+// more than half of the blocks idle is cut into items of 32 or 16 columns, as far as there are blocks for them.  (Tiles of places without rows
+// in between, which a sort leaves none of, are passed over.)  An element's sum runs over K in the same steps as above.
+// Gate/up and down, weights from memory, against four blocks an SM whose threads all copied, multiplied and met at a barrier every 64 columns
+// of K (in brackets the read alone): 32 experts of 2,048 x 1,024, top 4: 1 token 13.4 + 7.8 -> 11.1 + 7.0 us (5.1 + 2.6), 8 tokens 43.5 + 25.4 ->
+// 37.7 + 21.8 (29.5 + 14.8), 32: 53.9 + 32.1 -> 48.8 + 27.7 (39.8 + 19.9); 64 of 4,096 x 1,408, top 6: 8 tokens 164 + 85 -> 140 + 70 (131 + 65),
+// 64: 281 + 144 -> 227 + 115 (226 + 113).  Nine stages of 64 columns of K, two blocks an SM: 232 + 120, and 52.4 + 29.7 at the 53.9 + 32.1; five stages
+// of 128: 232 + 119; three, three blocks an SM: 235 + 121.  The last are the better ones where two blocks an SM would need a second
+// round and three do not (32 experts, 3 tokens: 20.3 + 10.1 against 24.1 + 11.9, and 22.5 + 12.5 before).
+#define GE_MIN_STEPS 8                                           // steps of 64 columns of K (fewer: the kernel above)
+#define GE_BK 128
+#define GE_NST 4                                                 // two blocks an SM
+#define GE_NST_FEW 3                                             // three
+#define GE_W (GM_BN * 128)                                       // bytes of 64 columns of W's rows, and of A's, in TMA's 128-byte swizzle
+#define GE_A (16 * 128)
+#define GE_STAGE (2 * GE_W + 2 * GE_A)
+struct GeMaps { CUtensorMap w[3]; };                             // boxes of 64, 32 and 16 rows
+struct GeItem { int i, m0, n0, width, group; };                  // group < 0: nothing to do
+template <typename TC, int NST>
+__global__ void __launch_bounds__(160)
+gemm_experts_kernel(const bf16* __restrict__ A, const __grid_constant__ GeMaps maps, TC* __restrict__ C, int N, int K, int lda, int ldc,
+                    const int* __restrict__ tile_group, int tiles, const int* __restrict__ row_index, int index_div,
+                    const float* __restrict__ row_scale, int act, float alpha, float limit, float shift, unsigned* err) {
+    extern __shared__ unsigned char ge_smem[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ge_smem) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) unsigned long long full[NST], empty[NST];
+    __shared__ int s_tiles, s_issued, s_expired;
     pdl_launch_dependents();
+    const int tid = threadIdx.x, warp = tc5::warp_number(), lane = tid & 31;
+    if (tid == 0) {
+        s_tiles = s_issued = s_expired = 0;
+        for (int i = 0; i < NST; ++i) {
+            tc5::mbar_init(&full[i], 33);                        // every lane's copies of A, and W
+            tc5::mbar_init(&empty[i], 4);
+        }
+        tc5::mbar_fence_init();
+    }
     pdl_wait();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) s_tiles = 0;
     __syncthreads();
     int live = 0;                                                // tiles up to the last one that holds rows
-    for (int y = tid; y < tiles; y += 128) if (tile_group[y] >= 0) live = y + 1;
+    for (int y = tid; y < tiles; y += 160) if (tile_group[y] >= 0) live = y + 1;
     live = __reduce_max_sync(0xffffffffu, live);
     if (lane == 0) atomicMax(&s_tiles, live);
     __syncthreads();
     live = s_tiles;
-    const int across = (N + GM_BN - 1) / GM_BN, items = live * across;
-    if (items == 0) return;
-    const int each = (items + (int)gridDim.x - 1) / (int)gridDim.x, G = (items + each - 1) / each, KT = (K + GM_BK - 1) / GM_BK;
-    if ((int)blockIdx.x >= G) return;
-    struct Item { const bf16* w; int m0, n0, i; };
-    auto find = [&](int i, int which) -> Item {                  // this block's first item from i on; s_src[which] is there behind the next barrier
-        Item t = {W, 0, 0, i};
-        int group = -1;
-        for (; t.i < items; t.i += G)
-            if ((group = tile_group[t.i / across]) >= 0) break;
-        if (t.i < items) {
-            const int y = t.i / across;
-            t.m0 = y * BM;
-            t.n0 = (t.i - y * across) * GM_BN;
-            t.w = W + (size_t)group * w_gs;
-            if (tid < BM) {
-                const int p = row_index ? row_index[t.m0 + tid] : t.m0 + tid;
-                s_src[which][tid] = p < 0 ? -1 : (row_index ? p / index_div : p);
-            }
+    const int across = (N + GM_BN - 1) / GM_BN, items = live * across, P = (int)gridDim.x, KT = (K + GE_BK - 1) / GE_BK;
+    const int whole = items / P * P, rest = items - whole, cut = rest * 4 <= P ? 2 : (rest * 2 <= P ? 1 : 0), total = whole + (rest << cut);
+    auto item = [&](int i) -> GeItem {
+        GeItem t = {i, 0, 0, 0, -1};
+        if (i < total) {
+            const int at = i < whole ? i : whole + ((i - whole) >> cut), y = at / across;
+            t.width = i < whole ? GM_BN : GM_BN >> cut;
+            t.m0 = 16 * y;
+            t.n0 = (at - y * across) * GM_BN + (i < whole ? 0 : ((i - whole) & ((1 << cut) - 1)) * t.width);
+            t.group = t.n0 < N ? __shfl_sync(0xffffffffu, tile_group[y], 0) : -1;
         }
         return t;
     };
-    auto load_stage = [&](int st, int kt, const Item& t, int which) {
-        const int k0 = kt * GM_BK;
-        {
-            const int r = tid / CH, c = tid % CH, k = k0 + c * 8, src = s_src[which][r];      // 16 rows x 8 pieces: one a thread
-            const bool ok = src >= 0 && k < K;
-            gm_cp_async16(&As[st][r][c * 8], ok ? A + (size_t)src * lda + k : A, ok);
-        }
+    if (warp == 4) {
+        int st = 0, round = 0, issued = 0;
+        bool ok = true;
+        auto source = [&](const GeItem& t) {                     // lane r < 16: the tile's row r in A (-1: zeros)
+            if (lane >= 16 || t.group < 0) return -1;
+            const int p = row_index ? row_index[t.m0 + lane] : t.m0 + lane;
+            return p < 0 ? -1 : (row_index ? p / index_div : p);
+        };
+        const bool lead = tc5::elect_one();
+        GeItem cur = item(blockIdx.x);
+        int src = source(cur);
+        while (cur.i < total && ok) {
+            const GeItem nxt = item(cur.i + P);                  // (its loads are on their way while this item's copies are issued)
+            const int nsrc = source(nxt);
+            if (cur.group >= 0) {
+                const int c = lane & 15, r0 = lane >> 4, to = 2 * GE_W + (c >> 3) * GE_A;
+                const bf16* from[8];                             // this lane's pieces of A: 16 bytes of the rows r0 + 2 i
 #pragma unroll
-        for (int i = 0; i < GM_BN * CH / 128; ++i) {
-            const int idx = tid + 128 * i, r = idx / CH, c = idx % CH, k = k0 + c * 8;
-            const bool ok = t.n0 + r < N && k < K;
-            gm_cp_async16(&Ws[st][r][c * 8], ok ? t.w + (size_t)(t.n0 + r) * K + k : W, ok);
-        }
-    };
-    int which = 0, st = 0;
-    Item cur = find(blockIdx.x, 0), nxt = cur;
-    if (cur.i >= items) return;
-    __syncthreads();
-    for (int s = 0; s < GM_NST - 1; ++s) { load_stage(s, s, cur, 0); gm_commit(); }
-    const int g = lane >> 2, t2 = (lane & 3) * 2;
-    const bool pair_ok = (ldc & 1) == 0 && (((uintptr_t)C) & 3) == 0;
-    for (; cur.i < items; cur = nxt, which ^= 1) {
-        float acc[2][4];
+                for (int i = 0; i < 8; ++i) {
+                    const int r = __shfl_sync(0xffffffffu, src, r0 + 2 * i);
+                    from[i] = r >= 0 ? A + (size_t)r * lda + c * 8 : nullptr;
+                }
+                const CUtensorMap* map = &maps.w[cur.width == 64 ? 0 : (cur.width == 32 ? 1 : 2)];
+                const int wrow = cur.group * N + cur.n0;
+#pragma unroll 1
+                for (int kt = 0; kt < KT; ++kt) {
+                    if (round && !tc5::warp_wait(&empty[st], (round - 1) & 1)) { ok = false; break; }
+                    unsigned char* stage = ring + st * GE_STAGE;
+                    if (lead) {
+                        tc5::mbar_arrive_expect_tx(&full[st], 2 * cur.width * 128);
+                        tc5::tma_load_2d(stage, map, kt * GE_BK, wrow, &full[st]);
+                        tc5::tma_load_2d(stage + GE_W, map, kt * GE_BK + GM_BK, wrow, &full[st]);
+                    }
+                    const bool inside = kt * GE_BK + c * 8 < K;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        for (int kt = 0; kt < KT; ++kt) {
-            gm_wait<GM_NST - 2>();
-            __syncthreads();
-            const int nk = kt + GM_NST - 1, into = (st + GM_NST - 1) % GM_NST;
-            if (nk < KT) load_stage(into, nk, cur, which);
-            else if (nxt.i < items) load_stage(into, nk - KT, nxt, which ^ 1);
-            gm_commit();
-            if (kt == 0) nxt = find(cur.i + G, which ^ 1);
-#pragma unroll
-            for (int kk = 0; kk < GM_BK / 16; ++kk) {
-                unsigned a[4], b[4];
-                gm_ldmatrix_x4(a, &As[st][lane & 15][kk * 16 + (lane >> 4) * 8]);
-                gm_ldmatrix_x4(b, &Ws[st][warp * 16 + (lane & 7) + ((lane >> 4) << 3)][kk * 16 + ((lane >> 3) & 1) * 8]);
-                gm_mma16816(acc[0], a, b[0], b[1]);
-                gm_mma16816(acc[1], a, b[2], b[3]);
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = r0 + 2 * i;
+                        const bool in = inside && from[i];
+                        gm_cp_async16(stage + to + r * 128 + (((c & 7) ^ (r & 7)) << 4), in ? from[i] + kt * GE_BK : A, in);
+                    }
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc5::smem_u32(&full[st])) : "memory");
+                    ++issued;
+                    if (++st == NST) { st = 0; ++round; }
+                }
             }
-            st = (st + 1) % GM_NST;
+            cur = nxt;
+            src = nsrc;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (lead) s_issued = issued;
+        if (!ok && lead) s_expired = 1;
+    } else {
+        int st = 0, round = 0;
+        bool ok = true;
+        const int g = lane >> 2, t2 = (lane & 3) * 2;
+        const bool pair_ok = (ldc & 1) == 0 && (((uintptr_t)C) & 3) == 0;
+        const int ar = lane & 15, ac = lane >> 4, br = warp * 16 + (lane & 7) + ((lane >> 4) << 3), bc = (lane >> 3) & 1;
+        GeItem cur = item(blockIdx.x);
+        while (cur.i < total && ok) {
+            const GeItem nxt = item(cur.i + P);
+            if (cur.group >= 0) {
+                const bool mine = 16 * warp < cur.width;
+                float scale[2] = {1.0f, 1.0f};
+                if (row_scale) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int m = cur.m0 + g + half * 8;
-            float scale = 1.0f;
-            if (row_scale) {
-                const int p = row_index ? row_index[m] : m;
-                scale = p >= 0 ? row_scale[p] : 0.f;
-            }
-            TC* crow = C + (size_t)m * ldc;
-            if (act == GM_ACT_NONE || act >= GM_ACT_UNARY) {
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int n = cur.n0 + warp * 16 + j * 8 + t2;
-                    const float v0 = gm_unary(acc[j][2 * half] * scale, act), v1 = gm_unary(acc[j][2 * half + 1] * scale, act);
-                    if (sizeof(TC) == 2 && pair_ok && n + 1 < N) {
-                        __nv_bfloat162 pr = __floats2bfloat162_rn(v0, v1);
-                        *reinterpret_cast<unsigned*>(crow + n) = *reinterpret_cast<unsigned*>(&pr);
-                    } else {
-                        if (n < N) crow[n] = from_f32<TC>(v0);
-                        if (n + 1 < N) crow[n + 1] = from_f32<TC>(v1);
+                    for (int half = 0; half < 2; ++half) {
+                        const int m = cur.m0 + g + half * 8, p = row_index ? row_index[m] : m;
+                        scale[half] = p >= 0 ? row_scale[p] : 0.f;
                     }
                 }
-            } else {                                             // 8 gate columns, then their 8 up columns
-                const int n = (cur.n0 + warp * 16) / 2 + t2;
+                float acc[2][4];
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    if (n + e < N / 2)
-                        crow[n + e] = from_f32<TC>(gm_gated(acc[0][2 * half + e] * scale, acc[1][2 * half + e] * scale, act, alpha, limit, shift));
+                for (int j = 0; j < 2; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+#pragma unroll 1
+                for (int kt = 0; kt < KT; ++kt) {
+                    if (!tc5::warp_wait(&full[st], round & 1)) { ok = false; break; }
+                    if (mine) {
+                        const unsigned char* w = ring + st * GE_STAGE;
+                        const unsigned char* x = w + 2 * GE_W;
+                        unsigned a[8][4], b[8][4];
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk) {
+                            gm_ldmatrix_x4(a[kk], x + (kk >> 2) * GE_A + ar * 128 + (((2 * (kk & 3) + ac) ^ (ar & 7)) << 4));
+                            gm_ldmatrix_x4(b[kk], w + (kk >> 2) * GE_W + br * 128 + (((2 * (kk & 3) + bc) ^ (br & 7)) << 4));
+                        }
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk) {
+                            gm_mma16816(acc[0], a[kk], b[kk][0], b[kk][1]);
+                            gm_mma16816(acc[1], a[kk], b[kk][2], b[kk][3]);
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) tc5::mbar_arrive(&empty[st]);
+                    if (++st == NST) { st = 0; ++round; }
+                }
+                if (!ok) break;
+                if (mine) {
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        TC* crow = C + (size_t)(cur.m0 + g + half * 8) * ldc;
+                        if (act == GM_ACT_NONE || act >= GM_ACT_UNARY) {
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                const int n = cur.n0 + warp * 16 + j * 8 + t2;
+                                const float v0 = gm_unary(acc[j][2 * half] * scale[half], act), v1 = gm_unary(acc[j][2 * half + 1] * scale[half], act);
+                                if (sizeof(TC) == 2 && pair_ok && n + 1 < N) {
+                                    __nv_bfloat162 pr = __floats2bfloat162_rn(v0, v1);
+                                    *reinterpret_cast<unsigned*>(crow + n) = *reinterpret_cast<unsigned*>(&pr);
+                                } else {
+                                    if (n < N) crow[n] = from_f32<TC>(v0);
+                                    if (n + 1 < N) crow[n + 1] = from_f32<TC>(v1);
+                                }
+                            }
+                        } else {                                 // 8 gate columns, then their 8 up columns
+                            const int n = (cur.n0 + warp * 16) / 2 + t2;
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                if (n + e < N / 2)
+                                    crow[n + e] = from_f32<TC>(gm_gated(acc[0][2 * half + e] * scale[half], acc[1][2 * half + e] * scale[half],
+                                                                        act, alpha, limit, shift));
+                        }
+                    }
+                }
             }
+            cur = nxt;
         }
+        if (!ok && lane == 0) s_expired = 1;
     }
-    gm_wait<0>();
+    __syncthreads();
+    if (s_expired && tid == 0) {                                 // copies that nobody waited for: waited for once more
+        for (int n = s_issued > NST ? s_issued - NST : 0; n < s_issued; ++n) tc5::mbar_wait_bounded(&full[n % NST], (n / NST) & 1);
+        if (err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_EXPERTS);
+    }
 }
 
-static int launch_experts(const bf16* A, const bf16* W, bf16* C, int M, int N, int K, int lda, int ldc, const int* tile_group, long long w_gs,
-                          const int* row_index, int index_div, const float* row_scale, int act, float alpha, float limit, float shift, cudaStream_t s) {
-    const size_t smem = (size_t)GM_NST * (16 + GM_BN) * GM_LDS * sizeof(bf16);
-    static int places = 0;                                       // blocks that fit the device at once
+// Blocks of the kernel that fit the device at once (0: the error in `rc`).
+template <int NST>
+static int experts_places(int& rc) {
+    static int places = 0;
     if (!places) {
+        const size_t smem = (size_t)NST * GE_STAGE + 1024;
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
-        cudaError_t e = cudaFuncSetAttribute(gemm_experts_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
+        rc = (int)cudaFuncSetAttribute(gemm_experts_kernel<bf16, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (rc) return 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_experts_kernel<bf16>, 128, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_experts_kernel<bf16, NST>, 160, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
         places = sms * per_sm;
     }
-    const long long most = (long long)(M / 16) * ((N + GM_BN - 1) / GM_BN);
-    if (most >= (1ll << 30)) return VL_ERR_UNSUPPORTED;
-    return vl_launch(gemm_experts_kernel<bf16>, dim3((unsigned)(most < places ? most : places)), dim3(128), smem, s, A, W, C, N, K, lda, ldc,
-                     tile_group, M / 16, w_gs, row_index, index_div, row_scale, act, alpha, limit, shift);
+    return places;
+}
+
+static int launch_experts(const bf16* A, const bf16* W, bf16* C, int M, int N, int K, int lda, int ldc, const int* tile_group, int groups,
+                          const int* row_index, int index_div, const float* row_scale, int act, float alpha, float limit, float shift,
+                          unsigned* err, cudaStream_t s) {
+    const long long items = (long long)(M / 16) * ((N + GM_BN - 1) / GM_BN);
+    if (items >= (1ll << 28) || (long long)groups * N >= (1ll << 31)) return VL_ERR_UNSUPPORTED;
+    int rc = 0;
+    const int places = experts_places<GE_NST>(rc), more = rc ? 0 : experts_places<GE_NST_FEW>(rc);
+    if (rc) return rc;
+    GeMaps maps;
+    for (int i = 0; i < 3 && !rc; ++i) rc = tc5_make_map(&maps.w[i], W, groups * N, K, K, GM_BN >> i);
+    if (rc) return rc;
+    auto launch = [&](auto kernel, int nst, int blocks) {
+        return vl_launch(kernel, dim3((unsigned)(4 * items < blocks ? 4 * items : blocks)), dim3(160), (size_t)nst * GE_STAGE + 1024, s, A, maps, C, N, K,
+                         lda, ldc, tile_group, M / 16, row_index, index_div, row_scale, act, alpha, limit, shift, err);
+    };
+    if (items > places && items <= more) return launch(gemm_experts_kernel<bf16, GE_NST_FEW>, GE_NST_FEW, more);
+    return launch(gemm_experts_kernel<bf16, GE_NST>, GE_NST, places);
 }
 
 // The plain batched product for many rows (one matrix per batch on column slices of wide activations, e.g. the gates of a
@@ -577,10 +661,10 @@ template <typename TC>
 static int launch_batched_mma(const bf16* A, const bf16* W, TC* C, int M, int N, int K, int lda, int ldw, int ldc,
                               long long a_bs, long long w_bs, long long c_bs, int batch, const int* tile_group,
                               long long w_gs, int bm, const int* row_index, int index_div, const float* row_scale,
-                              int act, float alpha, float limit, float shift, const bf16* gate, int gate_ld, cudaStream_t s) {
+                              int act, float alpha, float limit, float shift, const bf16* gate, int gate_ld, int groups, unsigned* err, cudaStream_t s) {
     if constexpr (sizeof(TC) == 2) {
-        if (bm == 16 && tile_group && batch == 1 && ldw == K && !gate && (K + GM_BK - 1) / GM_BK >= GE_MIN_STEPS)
-            return launch_experts(A, W, C, M, N, K, lda, ldc, tile_group, w_gs, row_index, index_div, row_scale, act, alpha, limit, shift, s);
+        if (bm == 16 && tile_group && batch == 1 && ldw == K && w_gs == (long long)N * K && groups > 0 && !gate && (K + GM_BK - 1) / GM_BK >= GE_MIN_STEPS)
+            return launch_experts(A, W, C, M, N, K, lda, ldc, tile_group, groups, row_index, index_div, row_scale, act, alpha, limit, shift, err, s);
     }
     dim3 grid((N + GM_BN - 1) / GM_BN, (M + bm - 1) / bm, batch);
     if (grid.y > 65535 || grid.z > 65535) return VL_ERR_UNSUPPORTED;
@@ -608,7 +692,8 @@ static int launch_batched(const T* A, const T* W, TC* C, int M, int N, int K, in
 // c_dtype: the operands' dtype, or float32 (the sums as they are).
 extern "C" int vl_gemm_batched_nt(const void* A, const void* W, void* C, int dtype, int c_dtype, int M, int N, int K,
                                   int lda, int ldw, int ldc, long long a_bs, long long w_bs, long long c_bs,
-                                  int batch, const int* tile_group, long long w_gs, int bm, const void* gate, int gate_ld, void* stream) {
+                                  int batch, const int* tile_group, long long w_gs, int bm, const void* gate, int gate_ld, int groups, unsigned* err,
+                                  void* stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return VL_OK;
     if (K <= 0 || lda < K || ldw < K || ldc < N || (bm != 64 && bm != 16)) return VL_ERR_ARGUMENT;
     if (tile_group && M % bm) return VL_ERR_ARGUMENT;
@@ -624,7 +709,7 @@ extern "C" int vl_gemm_batched_nt(const void* A, const void* W, void* C, int dty
             return launch_batched_wide((const bf16*)A, (const bf16*)W, (float*)C, M, N, K, lda, ldw, ldc, a_bs, w_bs, c_bs, batch, nullptr, 0, s);
         if (gm_aligned(A, W, K, lda, ldw, a_bs, w_bs, w_gs) && !vl_batched_simt_only())
             return launch_batched_mma((const bf16*)A, (const bf16*)W, (float*)C, M, N, K, lda, ldw, ldc, a_bs, w_bs, c_bs,
-                                      batch, tile_group, w_gs, bm, nullptr, 1, nullptr, GM_ACT_NONE, 0.f, 0.f, 0.f, nullptr, 0, s);
+                                      batch, tile_group, w_gs, bm, nullptr, 1, nullptr, GM_ACT_NONE, 0.f, 0.f, 0.f, nullptr, 0, 0, nullptr, s);
         return launch_batched<bf16, float>((const bf16*)A, (const bf16*)W, (float*)C, M, N, K, lda, ldw, ldc,
                                            a_bs, w_bs, c_bs, batch, tile_group, w_gs, bm, nullptr, 0, s);
     }
@@ -635,7 +720,7 @@ extern "C" int vl_gemm_batched_nt(const void* A, const void* W, void* C, int dty
                                        (const bf16*)gate, gate_ld, s);
         if (gm_aligned(A, W, K, lda, ldw, a_bs, w_bs, w_gs) && !vl_batched_simt_only())
             return launch_batched_mma((const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc, a_bs, w_bs, c_bs,
-                                      batch, tile_group, w_gs, bm, nullptr, 1, nullptr, GM_ACT_NONE, 0.f, 0.f, 0.f, (const bf16*)gate, gate_ld, s);
+                                      batch, tile_group, w_gs, bm, nullptr, 1, nullptr, GM_ACT_NONE, 0.f, 0.f, 0.f, (const bf16*)gate, gate_ld, groups, err, s);
         return launch_batched<bf16, bf16>((const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc,
                                     a_bs, w_bs, c_bs, batch, tile_group, w_gs, bm, (const bf16*)gate, gate_ld, s);
     }
@@ -692,12 +777,12 @@ extern "C" int vl_gemm_grouped_fused_ok(int K, int N, int act) {
 // [cap, N] sums (W: blocks of 8 gate rows and their 8 up rows) into C [cap, N / 2].  M = cap, a multiple of bm.
 extern "C" int vl_gemm_grouped_fused(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldc,
                                      const int* tile_group, long long w_gs, int bm, const int* row_index, int index_div,
-                                     const float* row_scale, int act, float alpha, float limit, float shift, void* stream) {
+                                     const float* row_scale, int act, float alpha, float limit, float shift, int groups, unsigned* err, void* stream) {
     if (M <= 0 || N <= 0) return VL_OK;
     if (K <= 0 || lda < K || (bm != 64 && bm != 16) || M % bm || !tile_group || index_div <= 0) return VL_ERR_ARGUMENT;
     const bool gated = act >= 0 && act < GM_ACT_UNARY;
     if (act < GM_ACT_NONE || (act > 2 && act != GM_ACT_UNARY) || ldc < (gated ? N / 2 : N)) return VL_ERR_ARGUMENT;
     if (!vl_gemm_grouped_fused_ok(K, N, act) || !gm_aligned(A, W, K, lda, K, 0, 0, w_gs)) return VL_ERR_UNSUPPORTED;
     return launch_batched_mma((const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, K, ldc, 0, 0, 0, 1, tile_group, w_gs, bm,
-                              row_index, index_div, row_scale, act, alpha, limit, shift, nullptr, 0, (cudaStream_t)stream);
+                              row_index, index_div, row_scale, act, alpha, limit, shift, nullptr, 0, groups, err, (cudaStream_t)stream);
 }

@@ -118,10 +118,10 @@ _SIGNATURES = {
                                          c_void_p, c_void_p, c_void_p],
     ("gemm_batched", "vl_gemm_batched_nt"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                              c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_int,
-                                             c_void_p],
+                                             c_int, c_void_p, c_void_p],
     ("gemm_batched", "vl_gemm_grouped_fused"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                                 c_longlong, c_int, c_void_p, c_int, c_void_p, c_int, c_float, c_float, c_float,
-                                                c_void_p],
+                                                c_int, c_void_p, c_void_p],
     ("moe", "vl_moe_route"): [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float,
                               c_void_p, c_void_p, c_void_p, c_void_p],
     ("gemm_batched", "vl_gemm_rows_f32w"): [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
@@ -1141,13 +1141,13 @@ def gemm_heads(a, w, out, gate=None, gate_col=0):
         gp, gld = gate.data_ptr() + gate_col * gate.element_size(), gate.shape[1]
     _check(_fn("gemm_batched", "vl_gemm_batched_nt")(
         _ptr(a), _ptr(w), _ptr(out), dtype_code(a.dtype), dtype_code(out.dtype), T, N, K, a.shape[1], K, H * N, K, N * K, N, H, None, 0,
-        16 if T <= 16 else 64, gp, gld, _stream()), "vl_gemm_batched_nt")
+        16 if T <= 16 else 64, gp, gld, 0, None, _stream()), "vl_gemm_batched_nt")
     return out
 
 
-def gemm_grouped(rows, w, out, tile_group, bm):
+def gemm_grouped(rows, w, out, tile_group, bm, err=None):
     """rows [cap, K] sorted by group in tiles of `bm` rows (`moe_align`), w [G, N, K], out [cap, N]:
-    tile y is multiplied by w[tile_group[y]]; tiles with a negative group are skipped."""
+    tile y is multiplied by w[tile_group[y]]; tiles with a negative group are skipped.  `err`: the step's device error word."""
     _need(rows, None, "rows", 2); _need(w, rows.dtype, "w", 3); _need(out, rows.dtype, "out", 2)
     _need(tile_group, torch.int32, "tile_group", 1)
     G, N, K = w.shape
@@ -1156,7 +1156,7 @@ def gemm_grouped(rows, w, out, tile_group, bm):
         raise KernelError("gemm_grouped: shapes disagree")
     _check(_fn("gemm_batched", "vl_gemm_batched_nt")(
         _ptr(rows), _ptr(w), _ptr(out), dtype_code(rows.dtype), dtype_code(rows.dtype), cap, N, K, K, K, N, 0, 0, 0, 1, _ptr(tile_group), N * K,
-        int(bm), None, 0, _stream()), "vl_gemm_batched_nt")
+        int(bm), None, 0, G, _ptr(err), _stream()), "vl_gemm_batched_nt")
     return out
 
 
@@ -1171,7 +1171,7 @@ def gemm_grouped_fused_ok(dtype, K, N, act=None) -> bool:
 
 
 def gemm_grouped_fused(a, w, out, tile_group, bm, row_index, index_div, row_scale=None, act=None, alpha=1.0, limit=0.0,
-                       shift=0.0):
+                       shift=0.0, err=None):
     """The grouped product with a routed feed-forward's neighbours folded in (bfloat16, tensor cores):
     sorted row m is row row_index[m] // index_div of a [rows, K] (negative: zeros), times w[tile_group[y]]
     ([G, N, K]); the float32 sums are multiplied by row_scale[row_index[m]] when given; with `act`, w holds
@@ -1188,7 +1188,7 @@ def gemm_grouped_fused(a, w, out, tile_group, bm, row_index, index_div, row_scal
         _need(row_scale, torch.float32, "row_scale")
     _check(_fn("gemm_batched", "vl_gemm_grouped_fused")(
         _ptr(a), _ptr(w), _ptr(out), cap, N, K, K, width, _ptr(tile_group), N * K, int(bm), _ptr(row_index), int(index_div),
-        _ptr(row_scale), _act_code(act), float(alpha), float(limit), float(shift), _stream()),
+        _ptr(row_scale), _act_code(act), float(alpha), float(limit), float(shift), G, _ptr(err), _stream()),
         "vl_gemm_grouped_fused")
     return out
 

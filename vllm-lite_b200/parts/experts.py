@@ -153,15 +153,15 @@ class RoutedExperts:
                                    add=self._shared(h, step), **last)
         if self.fused:
             ops.gemm_grouped_fused(h, self.gate_up, act, tile_group, bm, sorted_rows, top,
-                                   weights if s.scale_input else None, s.activation, s.alpha, s.limit, s.up_shift)
+                                   weights if s.scale_input else None, s.activation, s.alpha, s.limit, s.up_shift, step.err)
         else:
             rows = ops.moe_gather(h, sorted_rows, weights, top, ws.get(tag + "moe.rows", (cap, H), self.dtype), s.scale_input)
-            gu = ops.gemm_grouped(rows, self.gate_up, ws.get(tag + "moe.gate_up", (cap, self.first_n), self.dtype), tile_group, bm)
+            gu = ops.gemm_grouped(rows, self.gate_up, ws.get(tag + "moe.gate_up", (cap, self.first_n), self.dtype), tile_group, bm, step.err)
             if s.gated:
                 ops.gated_act(gu, act, s.activation, 0, s.alpha, s.limit, s.up_shift)
             else:
                 ops.unary_act(gu, act, s.activation)
-        res = ops.gemm_grouped(act, self.down, ws.get(tag + "moe.down", (cap, H), self.dtype), tile_group, bm)
+        res = ops.gemm_grouped(act, self.down, ws.get(tag + "moe.down", (cap, H), self.dtype), tile_group, bm, step.err)
         out = ws.get(tag + "moe.out", (T, H), self.dtype)
         return ops.moe_combine(res, place, weights, top, out, not s.scale_input, add=self._shared(h, step), **last)
 
