@@ -147,3 +147,20 @@ def test_constants_that_the_chunked_time_mixing_and_its_caller_share():
     assert lib.vl_decay_min_chunk() == ops.DECAY_MIN_CHUNK
     for sizes in ((1, 1, 4, 4), (7, 32, 64, 64), (3, 5, 100, 68), (4096, 16, 128, 128)):
         assert lib.vl_decay_chunk_floats(*sizes) == ops.decay_chunk_floats(*sizes)
+
+
+# where the measured times cross (148 SMs): the weight-streaming product up to 8 rows, a tile of W an SM, the library
+@pytest.mark.parametrize("M,N,K,few", [
+    (8, 2048, 2048, False), (9, 2048, 2048, True), (16, 7104, 2048, True), (16, 7120, 2048, False), (17, 4736, 2048, True), (24, 4752, 8192, False),
+    (25, 6144, 4096, True), (32, 6144, 2048, False), (32, 7120, 4096, False), (33, 2368, 512, True), (48, 2384, 512, False), (49, 64, 512, False),
+    (12, 2048, 2052, False)])
+def test_which_products_of_few_rows_take_a_tile_an_sm(monkeypatch, M, N, K, few):
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    assert ops.gemm_bf16_few_ok(M, N, K) is few
+
+
+@pytest.mark.parametrize("tokens,pairs,experts,K,big", [(64, 4096, 32, 2048, False), (65, 192, 32, 2048, True), (65, 191, 32, 2048, False),
+                                                        (100, 800, 128, 2048, True), (100, 764, 128, 2048, False), (512, 4096, 64, 2044, False)])
+def test_which_experts_products_run_on_tcgen05(tokens, pairs, experts, K, big):
+    assert ops.gemm_grouped_tc5_ok(torch.bfloat16, tokens, pairs, experts, K) is big
+    assert not ops.gemm_grouped_tc5_ok(torch.float32, tokens, pairs, experts, K)

@@ -41,6 +41,43 @@ def test_gemm_f32_with_its_activation(M, I, K, group):
     assert torch.equal(out, want)
 
 
+# tiles of 16, 32 and 48 rows of W, one to three of 16 rows of A, their edges, warps without a block of K and K's last block cut
+@pytest.mark.parametrize("N,K", [(1, 8), (24, 72), (64, 2048), (2368, 520), (2370, 136), (4752, 1032), (7104, 64)])
+@pytest.mark.parametrize("M", [1, 9, 16, 17, 32, 33, 48])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_product_of_few_rows(M, N, K, out_dtype):
+    gen = torch.Generator(device=DEV).manual_seed(M * 131 + N + K)
+    a = torch.randn(M, K, device=DEV, generator=gen).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=gen) / K ** 0.5).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = torch.full((M + 1, N), 7.0, device=DEV, dtype=out_dtype)
+    ops().gemm_bf16_few(a, w, out[:M], err)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # float32 sums of K exact products, then one rounding to the result's type
+    bound = (K + 8) * 2.0 ** -24 * size + (2.0 ** -8 * ref.abs() if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:M].double() - ref).abs() <= bound).all()) and bool((out[M:] == 7.0).all()) and not int(err)
+    if N % 16 == 0:
+        act = torch.empty(M, N // 2, device=DEV, dtype=out_dtype)
+        ops().gemm_bf16_few(a, w, act, err, swiglu=True)
+        g, u = (ref.view(M, -1, 2, 8)[:, :, i].reshape(M, -1) for i in (0, 1))
+        og, ou = ((K + 8) * 2.0 ** -24 * size.view(M, -1, 2, 8)[:, :, i].reshape(M, -1) for i in (0, 1))
+        ref = g / (1 + torch.exp(-g)) * u
+        # |silu'| < 1.1, |silu(g)| <= |g|, and a float32 exponential, quotient and product
+        bound = 1.2 * og * u.abs() + g.abs() * ou + 2.0 ** -20 * ref.abs() + (2.0 ** -8 * ref.abs() if out_dtype == torch.bfloat16 else 0) + 1e-30
+        assert bool(((act.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 256, 128), (128, 640, 2048), (300, 384, 136)])      # few tiles: 128 columns wide
+def test_tcgen05_product_with_few_tiles(M, N, K):
+    gen = torch.Generator(device=DEV).manual_seed(M + N + K)
+    a = torch.randn(M, K, device=DEV, generator=gen).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=gen) / K ** 0.5).bfloat16()
+    err, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.full((M, N), float("nan"), device=DEV)
+    ops().gemm_bf16_tc5(a, w, out, err)
+    bound = (K + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all()) and not int(err)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,I,group", [(1, 8, 0), (3, 4096, 0), (5, 12, 0), (2, 7, 0), (3, 64, 8), (3, 64, 16), (5, 36, 4), (7, 48, 24)])
 def test_silu_mul_layouts(T, I, group, dtype):

@@ -137,6 +137,8 @@ _SIGNATURES = {
     ("gemm_bf16", "vl_gemm_bf16_small_m_fused"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                   c_void_p, c_int, c_void_p, c_int, c_float, c_int, c_void_p, c_int,
                                                   c_void_p, c_void_p, c_void_p, c_void_p],
+    ("gemm_few", "vl_gemm_bf16_few"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                       c_void_p],
     ("gemm_tc5", "vl_gemm_bf16_tc5"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                        c_void_p, c_int, c_void_p],
     ("gemm_tc5_pair", "vl_gemm_bf16_tc5_pair"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -1360,7 +1362,8 @@ def gemm_f32(a, w, out, swiglu=False, group=0):
 
 SMALL_M = 16              # most rows of the weight-streaming product, which is also what its kernel takes; measured at
                           # Qwen3-8B sizes, context 4,096: batch 12 decodes in 5.00 ms against 5.18 ms with the library
-                          # product from 9 rows on, batch 16 in 5.42 against 5.60 (the norms and SwiGLU run inside it)
+                          # product from 9 rows on, batch 16 in 5.42 against 5.60 (the norms and SwiGLU run inside it);
+                          # `gemm_bf16_few` serves 9 rows and more where its tiles fit
 
 
 def gemm_bf16_small_m_ok(M, K) -> bool:
@@ -1411,6 +1414,32 @@ def gemm_bf16_small_m(a, w, out, err=None, swiglu=False, scaled=None, sink=None)
         if not 0 < grid.value <= NORM_PARTIALS:
             raise KernelError(f"gemm_bf16_small_m: {grid.value} blocks do not fit the partial sums")
         return grid.value
+    return out
+
+
+FEW_M = 48                # most rows that its kernel takes
+
+
+def gemm_bf16_few_ok(M, N, K) -> bool:
+    """Whether `gemm_bf16_few` is the fastest product for these sizes: a tile of 16, 32 or 48 rows of w an SM, beside `gemm_bf16_small_m` up to
+    16 rows and the library's product beyond (both sides' times stand in csrc/gemm_few.cu; where the line lies, us here / there: 8
+    rows 2,048 x 2,048 3.7 / 3.2; 32 rows 6,144 x 2,048 7.2 / 7.3, x 4,096 11.7 / 12.6, 24 rows 7.2 / 6.6 and 11.6 / 11.4; 48 rows 2,048 x 2,048
+    4.3 / 5.0, 3,072 x 2,048 6.0 / 5.5; 7,168 x 5,120, a second round of tiles, 22 / 15)."""
+    if not 8 < M <= FEW_M or K % 8:
+        return False
+    sms = 2 * sm_pairs()
+    if M <= 16:
+        return N <= 48 * sms
+    if M <= 32:
+        return N <= 32 * sms or (M > 24 and K >= 4096 and N <= 48 * sms)
+    return N <= 16 * sms
+
+
+def gemm_bf16_few(a, w, out, err=None, swiglu=False):
+    """out[M, N] = a[M, K] @ w[N, K]^T for M <= FEW_M, operands, sums and swiglu as in `gemm_bf16_small_m`."""
+    M, N, K, width = _gemm_shapes(a, w, out, swiglu)
+    _check(_fn("gemm_few", "vl_gemm_bf16_few")(_ptr(a), _ptr(w), _ptr(out), dtype_code(out.dtype), M, N, K, K, K, width, int(swiglu),
+                                               2 * sm_pairs(), _ptr(err), _stream()), "vl_gemm_bf16_few")
     return out
 
 
