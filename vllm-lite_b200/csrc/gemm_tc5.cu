@@ -5,10 +5,10 @@
 // stream instead.
 //
 // A block computes 128 x BN tiles of C, one after the other (one block per SM).  Roles:
-//   warp 0, one thread   TMA producer: tiled bulk tensor copies (cp.async.bulk.tensor.2d, 128-byte
+//   warp 0               TMA producer: tiled bulk tensor copies (cp.async.bulk.tensor.2d, 128-byte
 //                        swizzle) of a 128 x 64 tile of A and a BN x 64 tile of W per stage into a
 //                        ring of shared-memory stages, completion on an mbarrier per stage;
-//   warp 1, one thread   issues tcgen05.mma (cta_group::1, kind::f16, M 128, N BN, K 16) on shared
+//   warp 1               issues tcgen05.mma (cta_group::1, kind::f16, M 128, N BN, K 16) on shared
 //                        memory descriptors, 4 per stage; tcgen05.commit hands the stage back to
 //                        the producer and, after the last one, signals the epilogue;
 //                        the warp also allocates and frees 2 x BN columns of TMEM: two accumulators,

@@ -4,22 +4,23 @@
 // the rows of W along its columns.  A group brings a few hundred rows or fewer, so half a tile would be padding
 // and W would be read once for every 128 rows.  Here the operands change places: 256 rows of W are the rows of a
 // tile, which a pair of SMs computes (tcgen05 cta_group::2, as in csrc/gemm_tc5_pair.cu), and up to 256 rows of A its
-// columns, as many as the group has (in steps of 32).  A K block of a tile costs an SM 16 KB of W and up to 16 KB of A, which is
-// what bounds the kernel (an SM takes in about 60 bytes a cycle): 256 columns want them in 512 cycles.
+// columns, as many as the group has (in steps of 32).  A K block of a tile costs an SM 16 KB of W and up to 16 KB of A, which 256
+// columns want in 512 cycles (half of what an SM takes in); with fewer columns, and while an expert's rows are few, W's way out of
+// memory bounds the kernel.
 //
 // Tiles are taken in turn by all pairs (pair p the tiles p, p + pairs, ..), those of a group's rows of A innermost, then its
 // rows of W, so that what runs at the same time shares its rows of W and of A in L2.  (Equal shares of neighbouring tiles, cut
 // anywhere along K, were built and measured: every pair is then in a group of its own, nothing is shared, and 148 SMs
 // that leave float32 pieces take 10 us for it: 104 us where this order takes 71.)
-// 32 groups of 256 rows, 2,048 x 2,048 a gate/up: 98 us with 128 rows of A as the tile's rows -> 71 (964 TFLOP/s, W at 3.8 TB/s),
-// 2,048 x 1,024: 50 -> 43; groups of 384 rows 163 (of unequal sizes, in a model) -> 103 and 78 -> 56.
+// 32 groups of 256 rows, 2,048 x 2,048 a gate/up: 98 us with 128 rows of A as the tile's rows -> 68 (1,011 TFLOP/s),
+// 2,048 x 1,024: 50 -> 40; groups of 384 rows 163 (of unequal sizes, in a model) -> 88 and 78 -> 50.
 //
 // The epilogue can do what a routed feed-forward needs around its first product: multiply the float32
 // sums of row m by row_scale[row_index[m]] (the expert weight on the input: W (s a) = s (W a)), and
 // apply the gated activation to blocks of 8 gate and 8 up columns (act 0..2: C is [M, N / 2]) or, act 16, the
 // square of max(v, 0) to every column of a plain W.
 //
-// Roles: warp 0 one thread copies (TMA, 128-byte swizzle), warp 1 one thread of the pair's first block issues the products,
+// Roles: warp 0 copies (TMA, 128-byte swizzle; an elected lane), warp 1 of the pair's first block issues the products,
 // warps 2..9 are the epilogue: two groups of four warps, each takes every second chunk of 32 columns of the accumulator,
 // turns it round through shared memory (a thread holds one row of W there, a row of C wants them side by side) and
 // stores 16 bytes a thread.  Two accumulators in tensor memory: a tile's epilogue runs beside the next tile's products.

@@ -34,11 +34,10 @@ constexpr int NUM_THREADS = 64 + 256;        // copies, products, eight warps of
 constexpr unsigned A_BYTES = BM_CTA * BK * 2, W_BYTES = BN_CTA * BK * 2;
 constexpr unsigned TMEM_COLS = 512;
 
-// The tile's width.  256: two accumulators in TMEM, 6 stages of 32 KB; a stage feeds 512 cycles of the tensor
-// core with 32 KB, more than an SM takes in (about 52 bytes a cycle), so the tensor pipe is busy 74 to 83 % of
-// a tile's time.  512: one accumulator of all 512 columns, 4 stages of 48 KB (A once for two products per 16
-// columns of K): 48 KB per 1,024 cycles, the tensor pipe no longer waits, but the epilogue of a tile no
-// longer runs beside the products of the next.  The launcher picks by the rounds of tiles either needs.
+// The tile's width.  256: two accumulators in TMEM, 6 stages of 32 KB; a stage is 512 cycles of the tensor core and takes 523 (705
+// while the copies and the products were issued by single threads).  512: one accumulator of all 512 columns, 4 stages of 48 KB (A once for
+// two products per 16 columns of K), 1,032 cycles for 1,024, but the epilogue of a tile no longer runs beside the products of the
+// next.  The launcher picks by the rounds of tiles either needs.
 template <int BN> struct Shape {
     static constexpr int HALVES = BN / BN_MMA;                                 // products per 16 columns of K
     static constexpr int STAGES = BN == 256 ? 6 : 4;
