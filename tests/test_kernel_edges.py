@@ -67,6 +67,28 @@ def test_product_of_few_rows(M, N, K, out_dtype):
         assert bool(((act.double() - ref).abs() <= bound).all())
 
 
+# a block a row and a warp a row (4,000 and more), columns beyond a round of accesses, sums over one to five choices: the arithmetic in order
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,K,top,scale", [(5, 96, 2, True), (1999, 264, 2, True), (1400, 2056, 3, False), (900, 4104, 5, True), (1400, 100, 3, True)])
+def test_sorted_rows_and_their_sums(T, K, top, scale, dtype):
+    E, bm = 8, 16
+    gen = torch.Generator(device=DEV).manual_seed(T + K)
+    ids = torch.rand(T, E, device=DEV, generator=gen).topk(top).indices.to(torch.int32).contiguous()
+    weights, h = torch.rand(T, top, device=DEV, generator=gen), torch.randn(T, K, device=DEV, generator=gen).to(dtype)
+    cap = ops().moe_sorted_rows(T * top, E, bm)
+    order, place = (torch.empty(n, dtype=torch.int32, device=DEV) for n in (cap, T * top))
+    ops().moe_align(ids, E, bm, order, torch.empty(cap // bm, dtype=torch.int32, device=DEV), place)
+    rows = ops().moe_gather(h, order, weights, top, torch.full((cap, K), 7.0, device=DEV, dtype=dtype), scale)
+    pair = order.long().clamp(min=0)
+    want = h[pair // top].float() * (weights.view(-1)[pair][:, None] if scale else 1.0)
+    assert torch.equal(rows, torch.where(order[:, None] >= 0, want, 0.0).to(dtype))
+    out = ops().moe_combine(rows, place, weights, top, torch.empty(T, K, device=DEV, dtype=dtype), True)
+    ref = (rows[place.long()].double().view(T, top, K) * weights.double()[:, :, None])
+    # float32 products and sums, then one rounding to the result's type
+    bound = 2 * top * 2.0 ** -24 * ref.abs().sum(1) + (2.0 ** -8 if dtype == torch.bfloat16 else 0) * ref.sum(1).abs() * 1.01 + 1e-30
+    assert bool(((out.double() - ref.sum(1)).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(129, 256, 128), (128, 640, 2048), (300, 384, 136)])      # few tiles: 128 columns wide
 def test_tcgen05_product_with_few_tiles(M, N, K):
     gen = torch.Generator(device=DEV).manual_seed(M + N + K)

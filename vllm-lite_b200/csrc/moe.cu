@@ -216,6 +216,44 @@ __global__ void moe_gather_kernel(const T* __restrict__ h, const int* __restrict
     for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = scale_input ? from_f32<T>(w * to_f32(src[k])) : src[k];
 }
 
+// The same for many rows of whole 16-byte pieces, where what bounds the launch is how much is under way: a warp a row, eight accesses each.
+// 8,704 rows of 2,048 bfloat16 numbers 10.1 -> 7.9 us, 20,600 rows 23.3 -> 18.0, 4,032 5.3 -> 5.0; of few rows a block a row is done sooner (880
+// rows 2.6 us, 2.9 so).
+#define GATHER_MANY 4000
+#define GATHER_WARPS 8
+template <typename T>
+__global__ void __launch_bounds__(32 * GATHER_WARPS)
+moe_gather_many_kernel(const T* __restrict__ h, const int* __restrict__ sorted_rows, const float* __restrict__ weights, int cap, int top, int K,
+                       int scale_input, T* __restrict__ rows) {
+    constexpr int V = 16 / sizeof(T), U = 8;                 // values an access, accesses at a time
+    pdl_launch_dependents();
+    pdl_wait();
+    const int r = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= cap) return;
+    const int p = sorted_rows[r];
+    T* dst = rows + (size_t)r * K;
+    const T* src = h + (size_t)(p < 0 ? 0 : p / top) * K;
+    const float w = p >= 0 && scale_input ? weights[p] : 1.0f;
+    for (int k0 = lane * V; k0 < K; k0 += 32 * V * U) {
+        uint4 v[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            const int k = k0 + 32 * V * i;
+            v[i] = p >= 0 && k < K ? *reinterpret_cast<const uint4*>(src + k) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            const int k = k0 + 32 * V * i;
+            if (p >= 0 && scale_input) {
+                T* e = reinterpret_cast<T*>(&v[i]);
+#pragma unroll
+                for (int c = 0; c < V; ++c) e[c] = from_f32<T>(w * to_f32(e[c]));
+            }
+            if (k < K) *reinterpret_cast<uint4*>(dst + k) = v[i];
+        }
+    }
+}
+
 template <typename T>
 __global__ void moe_combine_kernel(const T* __restrict__ result, const int* __restrict__ place,
                                    const float* __restrict__ weights, int top, int N, int scale_output,
@@ -292,12 +330,14 @@ extern "C" int vl_moe_gather(const void* h, int dtype, const int* sorted_rows, c
     if (cap <= 0) return VL_OK;
     if (top <= 0 || K <= 0) return VL_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == VL_F32)
-        return vl_launch(moe_gather_kernel<float>, dim3(cap), dim3(128), 0, s, (const float*)h, sorted_rows, weights, top, K,
-                         scale_input, (float*)rows);
-    if (dtype == VL_BF16)
-        return vl_launch(moe_gather_kernel<bf16>, dim3(cap), dim3(128), 0, s, (const bf16*)h, sorted_rows, weights, top, K,
-                         scale_input, (bf16*)rows);
+    const bool many = cap >= GATHER_MANY && K % 8 == 0;
+#define GATHER(T)                                                                                                                    \
+    if (many) return vl_launch(moe_gather_many_kernel<T>, dim3((cap + GATHER_WARPS - 1) / GATHER_WARPS), dim3(32 * GATHER_WARPS), 0, s,      \
+                               (const T*)h, sorted_rows, weights, cap, top, K, scale_input, (T*)rows);                               \
+    return vl_launch(moe_gather_kernel<T>, dim3(cap), dim3(128), 0, s, (const T*)h, sorted_rows, weights, top, K, scale_input, (T*)rows)
+    if (dtype == VL_F32) { GATHER(float); }
+    if (dtype == VL_BF16) { GATHER(bf16); }
+#undef GATHER
     return VL_ERR_UNSUPPORTED;
 }
 
@@ -307,11 +347,13 @@ extern "C" int vl_moe_combine(const void* result, int dtype, const int* place, c
     if (T <= 0) return VL_OK;
     if (top <= 0 || N <= 0 || (h && !ids)) return VL_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
+    // blocks that have columns of a row (the others: 2,048 rows of 2,048, top 4, 10.3 us, 8.1 without)
+    const int across = N % 8 == 0 ? (N + 1023) / 1024 : (N + 511) / 512;
     if (dtype == VL_F32)
-        return vl_launch(moe_combine_kernel<float>, dim3(T, (N + 511) / 512), dim3(128), 0, s, (const float*)result, place, weights, top, N,
+        return vl_launch(moe_combine_kernel<float>, dim3(T, across), dim3(128), 0, s, (const float*)result, place, weights, top, N,
                          scale_output, (float*)out, (const float*)add, add_weight, ids, identity_from, (const float*)h);
     if (dtype == VL_BF16)
-        return vl_launch(moe_combine_kernel<bf16>, dim3(T, (N + 511) / 512), dim3(128), 0, s, (const bf16*)result, place, weights, top, N,
+        return vl_launch(moe_combine_kernel<bf16>, dim3(T, across), dim3(128), 0, s, (const bf16*)result, place, weights, top, N,
                          scale_output, (bf16*)out, (const bf16*)add, add_weight, ids, identity_from, (const bf16*)h);
     return VL_ERR_UNSUPPORTED;
 }
