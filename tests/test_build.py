@@ -1,6 +1,9 @@
 """The CUDA libraries as files: they build for sm_100a without a GPU and export what the engine
 switches at run time (no GPU needed: nothing is launched)."""
 import ctypes
+import re
+
+import pytest
 
 from vllm_lite_b200.csrc import build, ops
 
@@ -47,6 +50,15 @@ def test_the_grouped_product_of_paired_blocks_has_no_path_to_dependent_launch():
     assert re.search(r"cfg\.numAttrs\s*=\s*1\s*;", code) and code.count("numAttrs") == 1 and code.count("cudaLaunchKernelEx") == 1
     body = code[code.index("__global__"):]
     assert 0 < body.index("pdl_wait();") < body.index("alloc_pair")
+
+
+# A wait is given up by each lane at its own time.  Where the lanes then meet again (a warp's barrier, a load of tensor memory), one that left
+# by itself would let the others wait for good: whoever breaks off a loop over a wait does so by the vote of the warp.
+@pytest.mark.parametrize("name", ["gemm_tc5", "gemm_tc5_pair", "gemm_tc5_grouped", "gemm_few", "gemm_batched", "flash_tc5"])
+def test_no_lane_leaves_a_loop_by_itself_when_a_wait_runs_out(name):
+    code = re.sub(r"//[^\n]*", "", (build.CSRC / f"{name}.cu").read_text())
+    assert "wait" in code and not re.search(r"if\s*\(\s*!\s*(tc5::)?mbar_wait_bounded", code)
+    assert "__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))" in (build.CSRC / "tc5.cuh").read_text()
 
 
 def test_dependent_launch_is_off_until_switched_on():

@@ -143,7 +143,7 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         int local = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local) {
             const int acc = local & 1;
-            if (!mbar_wait_bounded(&acc_full_bar[acc], (unsigned)((local / 2) & 1))) {
+            if (!warp_wait(&acc_full_bar[acc], (unsigned)((local / 2) & 1))) {       // the whole warp stays or leaves
                 atomicOr(&failed, 8);
                 break;
             }

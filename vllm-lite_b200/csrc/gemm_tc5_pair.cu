@@ -165,7 +165,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         int local = 0;
         for (int tile = pair; tile < total_tiles; tile += num_pairs, ++local) {
             const int acc = local % ACCS;
-            if (!mbar_wait_bounded(&acc_full_bar[acc], (unsigned)((local / ACCS) & 1))) {
+            if (!warp_wait(&acc_full_bar[acc], (unsigned)((local / ACCS) & 1))) {    // the whole warp stays or leaves
                 atomicOr(&failed, 8);
                 break;
             }
