@@ -164,3 +164,55 @@ def test_which_products_of_few_rows_take_a_tile_an_sm(monkeypatch, M, N, K, few)
 def test_which_experts_products_run_on_tcgen05(tokens, pairs, experts, K, big):
     assert ops.gemm_grouped_tc5_ok(torch.bfloat16, tokens, pairs, experts, K) is big
     assert not ops.gemm_grouped_tc5_ok(torch.float32, tokens, pairs, experts, K)
+
+
+# Products of paired blocks never run among programmatic launches: up to 64 tokens none is chosen, beyond them a recorded step asks the model.
+def test_no_product_of_paired_blocks_among_programmatic_launches(monkeypatch):
+    from vllm_lite_b200.engine.runner import PDL_MAX_TOKENS, launches_dependent
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    for T in (1, 2, PDL_MAX_TOKENS - 1, PDL_MAX_TOKENS):
+        assert not any(ops.gemm_grouped_tc5_ok(torch.bfloat16, T, T * top, E, 2048) for top in (1, 2, 8, 64) for E in (1, 2, 8, 128))
+    for M in range(1, ops.TC5_MIN_M_FULL):
+        assert not any(ops.gemm_bf16_tc5_ok(M, 4096, fused, N) for fused in (False, True) for N in (None, 256, 24576))
+    yes, no = (lambda tokens: True), (lambda tokens: False)
+    assert launches_dependent(PDL_MAX_TOKENS, True, yes) and launches_dependent(PDL_MAX_TOKENS, False, yes)
+    assert not launches_dependent(PDL_MAX_TOKENS + 1, True, yes) and launches_dependent(PDL_MAX_TOKENS + 1, True, no)
+    assert not launches_dependent(PDL_MAX_TOKENS + 1, False, no)
+
+
+def test_a_recorded_step_asks_the_model_for_paired_products(monkeypatch):
+    from types import SimpleNamespace
+    from vllm_lite_b200.engine.runner import ModelRunner
+    from vllm_lite_b200.parts.base import BuildContext
+    from vllm_lite_b200.parts.experts import RoutedExperts
+    from vllm_lite_b200.parts.model import CausalLM
+
+    class Launched(Exception):
+        pass
+
+    def forward(batch, caches):
+        raise Launched
+
+    E, top, H, I = 8, 2, 64, 16
+    ctx = BuildContext(torch.device("cpu"), torch.bfloat16)
+    from vllm_lite_b200.parts.spec import RoutedExpertsSpec
+    spec = RoutedExpertsSpec(hidden_size=H, intermediate_size=I, num_experts=E, top=top)
+    weights = {n: torch.zeros(d.shape, dtype=torch.bfloat16) for n, d in RoutedExperts.declare(spec).items()}
+    part = RoutedExperts(spec, weights, ctx)
+    assert ctx.paired == [part.may_pair]
+    model = CausalLM.__new__(CausalLM)
+    model.ctx, model.forward = ctx, forward
+    runner = ModelRunner.__new__(ModelRunner)
+    runner.model, runner.storage, runner._graphs = model, SimpleNamespace(call_caches=[]), {}
+    states = []
+    monkeypatch.setattr(ops, "set_pdl", states.append)
+    for tokens, paired in ((64, False), (128, True), (256, True), (512, True)):
+        assert part.may_pair(tokens) is paired and model.may_pair(tokens) is paired
+        with pytest.raises(Launched):
+            runner._forward_graph(SimpleNamespace(graph_bucket=tokens, num_tokens=tokens, groups=[]))
+        assert states.pop() is not paired
+    ctx.paired.clear()                                   # a dense model: only where its own products may be paired ones
+    for tokens, on in ((256, True), (512, False), (4096, False)):
+        with pytest.raises(Launched):
+            runner._forward_graph(SimpleNamespace(graph_bucket=tokens, num_tokens=tokens, groups=[]))
+        assert states.pop() is on

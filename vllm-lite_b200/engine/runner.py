@@ -54,6 +54,13 @@ _DEVICE_ERRORS = {1: "a token id outside the vocabulary", 2: "a cache slot outsi
 PDL_MAX_TOKENS = 64
 
 
+def launches_dependent(tokens: int, recorded: bool, may_pair) -> bool:
+    """Whether a step's kernels are launched that way.  A recorded step of more tokens (one a request) is too, since its kernels are a decode
+    step's whatever their number, unless `may_pair(tokens)`: a product of paired blocks never runs among such launches, where one once
+    stood still (csrc/gemm_tc5_pair.cu), and none is ever chosen for PDL_MAX_TOKENS tokens or fewer."""
+    return tokens <= PDL_MAX_TOKENS or (recorded and not may_pair(tokens))
+
+
 def _align4(n: int) -> int:
     return (n + 3) & ~3
 
@@ -161,7 +168,7 @@ class ModelRunner:
             logits = self._forward_graph(batch)[:sum(len(e.want) for e in entries)]
         else:
             from ..csrc import ops
-            ops.set_pdl(batch.num_tokens <= PDL_MAX_TOKENS)
+            ops.set_pdl(launches_dependent(batch.num_tokens, False, self.model.may_pair))
             logits = self.model.forward(batch, self.storage.call_caches)
         self.finish(batch)
         return logits
@@ -253,7 +260,7 @@ class ModelRunner:
         if entry is None:
             # first sight of this bucket: run it as it is (also sizes the workspace), then record
             from ..csrc import ops
-            ops.set_pdl(True)                          # a decode step: one token a request
+            ops.set_pdl(launches_dependent(batch.num_tokens, True, self.model.may_pair))
             logits = self.model.forward(batch, self.storage.call_caches)
             torch.cuda.current_stream().synchronize()
             before = ops.launch_count

@@ -23,7 +23,7 @@ tensors, the step's batch and the cache of its own call.
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import List, Optional
 
 import torch
@@ -35,6 +35,8 @@ from ..csrc import ops
 class BuildContext:
     device: torch.device
     dtype: torch.dtype            # activation / model dtype: torch.bfloat16 or torch.float32
+    # what the parts add that may launch a product of paired blocks: tokens of a step -> whether it can be among its kernels
+    paired: list = field(default_factory=list, compare=False)
 
 
 class Workspace:

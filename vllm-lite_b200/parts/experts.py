@@ -118,12 +118,18 @@ class RoutedExperts:
             # per expert [gate rows; up rows], stacked over experts: [E, 2I, H]
             self.gate_up = torch.stack([torch.cat([weights[p + gate], weights[p + up]], dim=0) for p in names]).contiguous()
         self.down = torch.stack([weights[p + down] for p in names]).contiguous()          # [E, H, I]
+        ctx.paired.append(self.may_pair)
+
+    def may_pair(self, T) -> bool:
+        """Whether T tokens run their products on the tcgen05 tensor cores, in paired blocks."""
+        s = self.spec
+        return self.fused and ops.gemm_grouped_tc5_ok(self.dtype, T, T * s.top, s.num_experts, s.hidden_size)
 
     def __call__(self, h, step):
         s, ws, tag = self.spec, step.workspace, step.tag
         T, E, top, I, H = h.shape[0], s.num_experts, s.top, s.intermediate_size, s.hidden_size
         pairs = T * top
-        big = self.fused and ops.gemm_grouped_tc5_ok(self.dtype, T, pairs, E, H) and I % 8 == 0
+        big = self.may_pair(T)
         # tiles of 16 rows while an expert gets 16 rows or fewer on average (decoding: the products are then bound
         # by the experts' weights, and taller tiles would spend their time on rows of padding)
         bm = ops.TC5_GROUPED_TILE if big else (16 if pairs <= max(SMALL_STEP_PAIRS, 16 * E) else 64)

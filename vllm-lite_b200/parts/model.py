@@ -67,6 +67,11 @@ class CausalLM:
         self.keeps_embedding = any(call.add_embedding for call in plan.order)
         self.graph_safe = all(getattr(part, "graph_safe", False) for part in [self.embedding, self.head] + self.layers)
 
+    def may_pair(self, tokens: int) -> bool:
+        """Whether a step of so many tokens can hold a product of paired blocks (csrc/gemm_tc5_pair.cu, csrc/gemm_tc5_grouped.cu)."""
+        from ..csrc import ops
+        return tokens >= ops.TC5_MIN_M_FULL or any(asks(tokens) for asks in self.ctx.paired)
+
     def forward(self, step, caches, watch=None) -> torch.Tensor:
         """Logits float32 [len(step.logit_rows), vocab].  `watch(i, x)`, when given, is called after every entry of
         the running order with the stream brought up to date (a reader for tests and comparisons)."""
