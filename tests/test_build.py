@@ -61,6 +61,32 @@ def test_no_lane_leaves_a_loop_by_itself_when_a_wait_runs_out(name):
     assert "__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))" in (build.CSRC / "tc5.cuh").read_text()
 
 
+def test_the_engine_is_imported_without_a_compiler(tmp_path):
+    """An import builds nothing: without a compiler on the path and without built files the package, its engine and the checks of `ops`
+    are there; only a launch needs more."""
+    import os
+    import shutil
+    import subprocess
+    import sys
+    root = build.CSRC.parent.parent
+    for package in ("vllm_lite_b200", "vllm-lite_b200"):
+        shutil.copytree(root / package, tmp_path / package, ignore=shutil.ignore_patterns("_build", "__pycache__"))
+    code = """
+import torch
+import vllm_lite_b200.engine
+from vllm_lite_b200.csrc import ops
+try:
+    ops.cast(torch.zeros(4), torch.zeros(4))
+except ops.KernelError as e:
+    print("refused:", e)
+"""
+    hidden = {k: v for k, v in os.environ.items() if k not in ("CXX", "NVCC", "CUDA_HOME", "PYTHONPATH")}
+    hidden.update(PATH=str(tmp_path), TMPDIR=str(tmp_path))
+    run = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=tmp_path, env=hidden)
+    assert run.returncode == 0 and "CUDA tensor" in run.stdout, run.stderr
+    assert not list(tmp_path.rglob("*.so"))
+
+
 def test_dependent_launch_is_off_until_switched_on():
     assert ops._pdl is False or ops._pdl_libs            # the module's default; a test before may have stepped
     for name, defines in kernel_libraries():

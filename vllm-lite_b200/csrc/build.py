@@ -180,11 +180,28 @@ def host_library_path(name: str) -> Path:
 EXT_SOURCES = ("bind",)
 
 
+def _cuda_headers() -> Path:
+    """The folder of cuda_runtime_api.h: beside nvcc, or in the package of CUDA's runtime that torch installs."""
+    import importlib.util
+    cands = []
+    try:
+        cands.append(Path(find_nvcc()).resolve().parent.parent / "include")
+    except BuildError:
+        pass
+    spec = importlib.util.find_spec("nvidia")
+    for root in (spec.submodule_search_locations or ()) if spec else ():
+        cands.append(Path(root) / "cuda_runtime" / "include")
+    for cand in cands:
+        if (cand / "cuda_runtime_api.h").is_file():
+            return cand
+    raise BuildError("cuda_runtime_api.h not found (looked beside nvcc and in the nvidia.cuda_runtime package)")
+
+
 def _ext_flags():
     import sysconfig
     import torch
     root = Path(torch.__file__).resolve().parent / "include"
-    cuda = Path(find_nvcc()).resolve().parent.parent / "include"
+    cuda = _cuda_headers()
     return ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
             "-isystem", str(root), "-isystem", str(root / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda),
             "-I", sysconfig.get_paths()["include"]]

@@ -11,6 +11,7 @@
 //   mm(a, w, out)                     out = a w^T by the library; out in a's dtype or float32
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+#include <structmember.h>
 #include <cstring>
 #include <string>
 #include <ATen/core/Tensor.h>
@@ -167,7 +168,7 @@ PyObject* entry_new(PyTypeObject* type, PyObject* args, PyObject*) {
     return reinterpret_cast<PyObject*>(e);
 }
 
-PyMemberDef entry_members[] = {{"__vectorcalloffset__", Py_T_PYSSIZET, offsetof(Entry, call), Py_READONLY, nullptr}, {nullptr, 0, 0, 0, nullptr}};
+PyMemberDef entry_members[] = {{"__vectorcalloffset__", T_PYSSIZET, offsetof(Entry, call), READONLY, nullptr}, {nullptr, 0, 0, 0, nullptr}};
 PyType_Slot entry_slots[] = {{Py_tp_new, (void*)entry_new}, {Py_tp_call, (void*)PyVectorcall_Call}, {Py_tp_members, entry_members}, {0, nullptr}};
 PyType_Spec entry_spec = {"bind.Entry", sizeof(Entry), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL | Py_TPFLAGS_IMMUTABLETYPE, entry_slots};
 

@@ -202,14 +202,34 @@ def _fn(lib: str, name: str, defines=None):
             setter(int(_pdl))
             _pdl_libs[holder] = setter
         address = ctypes.cast(getattr(handle, name), c_void_p).value
-        f = _functions[key] = _bind.Entry(address, "".join(_KINDS[t] for t in _SIGNATURES[(lib, name)]))
+        f = _functions[key] = _load_bind().Entry(address, "".join(_KINDS[t] for t in _SIGNATURES[(lib, name)]))
     return f
 
 
-_bind = build.load_ext("bind")        # what is done for every launch, in C++ (csrc/host/bind.cpp)
+# What is done for every launch, in C++ (csrc/host/bind.cpp): the three functions below, until the first entry point is asked for.  Importing this
+# module needs no compiler, and no tensor on the CPU ever does.
+_bind = None
 _KINDS = {c_void_p: "p", c_int: "i", c_longlong: "l", c_float: "f"}
-_ptr = _bind.pointer                  # a tensor, an address or None: an entry point takes any of them where it wants a pointer
-_stream = _bind.stream                # the current stream of the current device, as `torch.cuda.current_stream().cuda_stream` gives it
+
+
+def _load_bind():
+    global _bind, _need, _ptr, _stream
+    if _bind is None:
+        bind = build.load_ext("bind")
+        bind.setup(_say_what_is_wrong)
+        _need, _ptr, _stream = bind.need, bind.pointer, bind.stream
+        _bind = bind
+    return _bind
+
+
+def _ptr(t):
+    """A tensor, an address or None: an entry point takes any of them where it wants a pointer."""
+    return t
+
+
+def _stream():
+    """The current stream of the current device, as `torch.cuda.current_stream().cuda_stream` gives it."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check(code: int, name: str):
@@ -233,8 +253,7 @@ def _say_what_is_wrong(t, dtype, name, ndim=None):
         raise KernelError(f"{name} must have {ndim} dimensions, got {tuple(t.shape)}")
 
 
-_bind.setup(_say_what_is_wrong)
-_need = _bind.need                    # raises as the function above does
+_need = _say_what_is_wrong
 
 
 # ---------------------------------------------------------------- embed / norm
@@ -1478,7 +1497,7 @@ def gemm_bf16_tc5(a, w, out, err=None, swiglu=False):
 
 def mm(a, w, out):
     """out = a @ w^T by the library (cuBLAS through torch), out in a's dtype or float32: `torch.mm` without what Python adds to it."""
-    return _bind.mm(a, w, out)
+    return _load_bind().mm(a, w, out)
 
 
 _sm_pairs = None
