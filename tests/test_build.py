@@ -215,3 +215,51 @@ def test_entry_points_are_called_as_ctypes_calls_them(tmp_path):
     for bad in ("x", "f" * 9, "i" * 41):
         with pytest.raises(ValueError):
             bind.Entry(1, bad)
+
+
+def test_the_library_product_is_torchs_own_in_all_its_forms():
+    """`ops.mm` goes through the dispatcher with all of its keys: a gradient is refused, modes and tensor types of somebody's own are
+    asked, warnings and errors are torch's (the product itself runs on the CPU here)."""
+    import torch
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Functions(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func.__name__)
+            return func(*args, **(kwargs or {}))
+
+    class Calls(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func.__name__)
+            return func(*args, **(kwargs or {}))
+
+    class Own(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(func.__name__)
+            return super().__torch_function__(func, types, args, kwargs or {})
+
+    seen = []
+    a, w = torch.randn(5, 8), torch.randn(3, 8)
+    out, want = torch.empty(5, 3), a @ w.t()
+    assert ops.mm(a, w, out) is out and torch.equal(out, torch.mm(a, w.t()))
+    for bad in ((a.clone().requires_grad_(), w, out), (a, torch.nn.Parameter(w), out)):
+        for product in (ops.mm, ops._torch_mm):
+            with pytest.raises(RuntimeError, match="automatic differentiation"):
+                product(*bad)
+        with torch.no_grad():
+            assert torch.equal(ops.mm(*bad), want)
+    for mode in (Functions, Calls):
+        with mode():
+            ops.mm(a, w, out)
+        assert any(name.startswith("mm") for name in seen), mode
+        seen.clear()
+    ops.mm(a.as_subclass(Own), w, out)
+    assert "mm" in seen
+    with pytest.raises(RuntimeError, match="shapes cannot be multiplied"):
+        ops.mm(a, torch.randn(3, 7), out)
+    with pytest.warns(UserWarning, match="resized"):
+        ops.mm(a, w, torch.empty(1, 3))
+    with pytest.raises(TypeError):
+        ops.mm(a, w, None)

@@ -4,29 +4,33 @@
 // requests 3.8 ms for 2 ms on the GPU).
 //
 //   need(t, dtype, name, ndim=None)   a CUDA tensor of that dtype (None: any), contiguous, of ndim dimensions (None: any); otherwise the
-//                                     function given to `setup` is called with the same arguments and says what is wrong
+//                                     first function given to `setup` is called with the same arguments and says what is wrong
 //   pointer(t)                        t itself: an entry point takes tensors, addresses and None where it wants a pointer
 //   Entry(address, signature)         an `extern "C" int` function: one letter an argument: p pointer, i int, l long long, f float
 //   stream()                          the current stream of the current device
-//   mm(a, w, out)                     out = a w^T by the library; out in a's dtype or float32
+//   mm(a, w, out)                     out = a w^T by the library, as torch.mm(a, w.t(), out=out) does it; out in a's dtype or float32
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <structmember.h>
 #include <cstring>
-#include <string>
 #include <ATen/core/Tensor.h>
-#include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/ops/mm.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 
 namespace {
-PyObject* g_slow_need = nullptr;
+PyObject *g_slow_need = nullptr, *g_slow_mm = nullptr;
 
-PyObject* setup(PyObject*, PyObject* fn) {
-    Py_INCREF(fn);
-    Py_XSETREF(g_slow_need, fn);
+PyObject* setup(PyObject*, PyObject* args) {
+    PyObject *need, *mm;
+    if (!PyArg_ParseTuple(args, "OO", &need, &mm)) return nullptr;
+    Py_INCREF(need);
+    Py_XSETREF(g_slow_need, need);
+    Py_INCREF(mm);
+    Py_XSETREF(g_slow_mm, mm);
     Py_RETURN_NONE;
 }
 
@@ -65,25 +69,22 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         PyErr_SetString(PyExc_TypeError, "mm(a, w, out) takes three tensors");
         return nullptr;
     }
-    const at::Tensor a = THPVariable_Unpack(args[0]), w = THPVariable_Unpack(args[1]);
-    at::Tensor out = THPVariable_Unpack(args[2]);
-    std::string what;
-    Py_BEGIN_ALLOW_THREADS
-    try {
-        at::AutoDispatchBelowADInplaceOrView guard;              // buffers and weights without gradients: nothing to record
+    // Whoever watches torch's functions or brings a tensor type of their own is asked as `torch.mm` asks them.  What the dispatcher decides by
+    // (gradients, modes, transforms) it decides here too: the call passes all of its keys.
+    bool watched = at::impl::torch_function_mode_enabled();
+    for (int i = 0; i < 3 && !watched; ++i) watched = !THPVariable_CheckTypeExact(Py_TYPE(args[i]));
+    if (watched) return PyObject_Vectorcall(g_slow_mm, args, n, nullptr);
+    HANDLE_TH_ERRORS
+    {
+        const at::Tensor a = THPVariable_Unpack(args[0]), w = THPVariable_Unpack(args[1]);
+        at::Tensor out = THPVariable_Unpack(args[2]);
+        pybind11::gil_scoped_release others_run;
         if (out.scalar_type() == a.scalar_type()) at::mm_out(out, a, w.t());
         else at::mm_out(out, a, w.t(), out.scalar_type());
-    } catch (const std::exception& e) {
-        what = e.what();
-        if (what.empty()) what = "mm failed";
-    }
-    Py_END_ALLOW_THREADS
-    if (!what.empty()) {
-        PyErr_SetString(PyExc_RuntimeError, what.c_str());
-        return nullptr;
     }
     Py_INCREF(args[2]);
     return args[2];
+    END_HANDLE_TH_ERRORS
 }
 
 // ---- entry points --------------------------------------------------------------------------------------------------------
@@ -172,7 +173,7 @@ PyMemberDef entry_members[] = {{"__vectorcalloffset__", T_PYSSIZET, offsetof(Ent
 PyType_Slot entry_slots[] = {{Py_tp_new, (void*)entry_new}, {Py_tp_call, (void*)PyVectorcall_Call}, {Py_tp_members, entry_members}, {0, nullptr}};
 PyType_Spec entry_spec = {"bind.Entry", sizeof(Entry), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL | Py_TPFLAGS_IMMUTABLETYPE, entry_slots};
 
-PyMethodDef methods[] = {{"setup", setup, METH_O, nullptr},
+PyMethodDef methods[] = {{"setup", setup, METH_VARARGS, nullptr},
                          {"need", (PyCFunction)(void (*)(void))need, METH_FASTCALL | METH_KEYWORDS, nullptr},
                          {"pointer", pointer, METH_O, nullptr},
                          {"stream", stream, METH_NOARGS, nullptr},

@@ -216,7 +216,7 @@ def _load_bind():
     global _bind, _need, _ptr, _stream
     if _bind is None:
         bind = build.load_ext("bind")
-        bind.setup(_say_what_is_wrong)
+        bind.setup(_say_what_is_wrong, _torch_mm)
         _need, _ptr, _stream = bind.need, bind.pointer, bind.stream
         _bind = bind
     return _bind
@@ -1493,6 +1493,10 @@ def gemm_bf16_tc5(a, w, out, err=None, swiglu=False):
     _check(_fn("gemm_tc5", "vl_gemm_bf16_tc5")(_ptr(a), _ptr(w), _ptr(out), dtype_code(out.dtype), M, N, K,
                                                K, K, width, _ptr(err), int(swiglu), _stream()), "vl_gemm_bf16_tc5")
     return out
+
+
+def _torch_mm(a, w, out):
+    return torch.mm(a, w.t(), out=out) if out.dtype == a.dtype else torch.mm(a, w.t(), out_dtype=out.dtype, out=out)
 
 
 def mm(a, w, out):
