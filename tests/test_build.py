@@ -217,6 +217,19 @@ def test_entry_points_are_called_as_ctypes_calls_them(tmp_path):
             bind.Entry(1, bad)
 
 
+def test_every_kernel_reports_a_wait_that_ran_out_under_its_own_name():
+    from vllm_lite_b200.engine.runner import _DEVICE_ERRORS
+    bits = {m.group(1): int(m.group(2), 16) for m in re.finditer(r"#define (VL_DEV_IN_\w+) (0x[0-9a-f]+)u", (build.CSRC / "common.cuh").read_text())}
+    roles = [1 << (16 + i) for i in range(4)]
+    assert len(set(bits.values())) == len(bits) and all(b & (b - 1) == 0 and b not in roles and b in _DEVICE_ERRORS for b in bits.values())
+    assert len(set(_DEVICE_ERRORS.values())) == len(_DEVICE_ERRORS)
+    users = {}
+    for path in build.CSRC.glob("*.cu"):
+        for name in set(re.findall(r"VL_DEV_IN_\w+", path.read_text())):
+            users.setdefault(name, []).append(path.stem)
+    assert set(users) == set(bits) and all(len(files) == 1 for files in users.values()), users
+
+
 def test_the_library_product_is_torchs_own_in_all_its_forms():
     """`ops.mm` goes through the dispatcher with all of its keys: a gradient is refused, modes and tensor types of somebody's own are
     asked, warnings and errors are torch's (the product itself runs on the CPU here)."""

@@ -29,7 +29,9 @@
 #define VL_DEV_IN_FLASH_DECODE_TMA 0x2000u
 #define VL_DEV_IN_DELTA 0x4000u
 #define VL_DEV_IN_GEMM_EXPERTS 0x8000u
-// ... and, in the two tcgen05 products, which waits gave up in the block (shifted left by 16):
+#define VL_DEV_IN_GEMM_GROUPED 0x100000u
+#define VL_DEV_IN_GEMM_FEW 0x200000u
+// ... and, in the three tcgen05 products, which waits gave up in the block (shifted left by 16):
 // 1 a free stage (copying thread), 2 a free accumulator, 4 a filled stage (both: issuing thread),
 // 8 a complete accumulator (epilogue)
 #define VL_DEV_ROLE_SHIFT 16

@@ -127,7 +127,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int i = done; i < iw; ++i) { tc5::warp_wait(&wf[w], wp); if (++w == S::WS) { w = 0; wp ^= 1; } }
         for (int i = done; i < ia; ++i) { tc5::warp_wait(&af[a], ap); if (++a == S::AS) { a = 0; ap ^= 1; } }
         if (lane == 0) s_expired = 1;
-        if (lane == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_SMALL_M);
+        if (lane == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_FEW);
     }
     __syncthreads();                                              // every warp's places are done with
     if (s_expired) return;

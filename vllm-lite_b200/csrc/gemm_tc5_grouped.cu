@@ -297,7 +297,7 @@ gemm_tc5_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     tc5_fence_after();
     if (warp == 1) dealloc_pair(tmem_base, ACCS * COLS);
     if (threadIdx.x == 0 && failed && f.err)
-        atomicOr(f.err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_TC5_PAIR | ((unsigned)failed << VL_DEV_ROLE_SHIFT));
+        atomicOr(f.err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_GROUPED | ((unsigned)failed << VL_DEV_ROLE_SHIFT));
 }
 
 // ---- host side -------------------------------------------------------------------------------

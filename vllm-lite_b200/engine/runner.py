@@ -43,7 +43,8 @@ _DEVICE_ERRORS = {1: "a token id outside the vocabulary", 2: "a cache slot outsi
                   0x400: "in the tcgen05 product", 0x800: "in the paired tcgen05 product",
                   0x1000: "in the tcgen05 attention", 0x2000: "in the streaming decode attention",
                   0x4000: "in the delta rule", 0x8000: "in the experts' product of few rows",
-                  # ... and, in the tcgen05 products, for what
+                  0x100000: "in the experts' product of many rows", 0x200000: "in the product of 9 to 48 rows",
+                  # ... and, in the three tcgen05 products, for what
                   0x10000: "for a free stage", 0x20000: "for a free accumulator", 0x40000: "for a filled stage",
                   0x80000: "for a complete accumulator"}
 
