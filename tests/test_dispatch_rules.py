@@ -216,3 +216,49 @@ def test_a_recorded_step_asks_the_model_for_paired_products(monkeypatch):
         with pytest.raises(Launched):
             runner._forward_graph(SimpleNamespace(graph_bucket=tokens, num_tokens=tokens, groups=[]))
         assert states.pop() is on
+
+
+# What a pre-norm block asks of its parts: the sum into the stream, where both neighbours should factor the norm between them; the float32 sums, where
+# they could but take a faster product; else a result in the activation dtype.
+@pytest.mark.parametrize("can,should", [((1, 1), (1, 1)), ((1, 1), (0, 1)), ((1, 1), (1, 0)), ((1, 1), (0, 0)), ((1, 0), (1, 0)), ((0, 0), (0, 0))])
+@pytest.mark.parametrize("nxt", [None, True, False])
+def test_a_pre_norm_block_never_rounds_what_it_could_add_in_float32(can, should, nxt):
+    from vllm_lite_b200.parts.base import Residual
+    from vllm_lite_b200.parts.block import PreNormBlock
+
+    class Part:
+        def __init__(self, i):
+            self.i, self.asked = i, None
+
+        def can_factor_norms(self, M):
+            return bool(can[self.i])
+
+        def factors_norms(self, M):
+            return bool(should[self.i])
+
+        def __call__(self, h, *rest, sink=None, sums=False):
+            self.asked = "sink" if sink is not None else "sums" if sums else "rounded"
+            return self.asked
+
+    class Norm(SimpleNamespace):
+        def __call__(self, x, delta, step, tag):
+            return tag
+
+    block = PreNormBlock.__new__(PreNormBlock)
+    block.mixer, block.ffn = Part(0), Part(1)
+    block.norm1, block.norm2 = (Norm(factorable=True, weight=None, spec=SimpleNamespace(eps=0.0, size=0)) for _ in range(2))
+    residual, after = Residual(None), Norm(weight=None, spec=SimpleNamespace(eps=0.0, size=0))
+    block(residual, SimpleNamespace(num_tokens=12), None, next_norm=None if nxt is None else (after, nxt))
+    assert block.mixer.asked == ("rounded" if not all(can) else "sink" if all(should) else "sums")
+    assert block.ffn.asked == ("rounded" if nxt is None or not can[1] else "sink" if nxt and should[1] else "sums")
+    assert (residual.normed_for is after) == (block.ffn.asked == "sink") == (residual.pending is None)
+
+
+def test_layers_of_4096_columns_leave_their_sums(monkeypatch):
+    """Nine to sixteen rows: the product that takes a tile an SM, and no less of the residual than the weight-streaming product adds."""
+    from vllm_lite_b200.parts.linear import Linear
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    wide, narrow = (Linear(torch.empty(64, K, dtype=torch.bfloat16)) for K in (4096, 2048))
+    for M in (1, 8, 9, 16, 17):
+        assert wide.can_factor_norms(M) is narrow.can_factor_norms(M) is (M <= 16)
+        assert narrow.factors_norms(M) is (M <= 16) and wide.factors_norms(M) is (M <= 8)

@@ -555,6 +555,24 @@ def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
     assert (many[1].float() - want).abs().max() < (2 ** -8 if act == torch.bfloat16 else 2 ** -18) * want.abs().max()
 
 
+# a residual of float32 sums beside bfloat16 rows: x + delta is one float32 addition, vectorised, by eights and one by one
+@pytest.mark.parametrize("H", [96, 1030, 4096, 16384])
+@pytest.mark.parametrize("rows", [1, 12, 700])
+def test_norm_adds_float32_sums(H, rows):
+    g = torch.Generator(device=DEV).manual_seed(H + rows)
+    x, d, w = (torch.randn(n, generator=g, device=DEV) for n in ((rows, H), (rows, H), (H,)))
+    a, out = x.clone(), torch.empty(rows, H, device=DEV, dtype=torch.bfloat16)
+    ops().add_rmsnorm(a, d, w, 1e-6, out)
+    assert torch.equal(a, x + d)
+    b, same = a.clone(), torch.empty_like(out)
+    ops().add_rmsnorm(b, None, w, 1e-6, same)                                 # the norm of the stream that the addition left
+    assert torch.equal(same, out) and torch.equal(a, b)
+    pick = torch.tensor([rows - 1, 0], dtype=torch.int32, device=DEV)
+    few, c = torch.empty(2, H, device=DEV, dtype=torch.bfloat16), x.clone()
+    ops().add_rmsnorm(c, d, w, 1e-6, few, rows=pick)
+    assert torch.equal(few, out[pick.long()]) and torch.equal(c, x)
+
+
 # the router's product on tiles of 16 and of 64 rows: a row's bits do not depend on how many rows there are (the taller tiles begin at 1,536 rows of
 # eight parts of K, 3,009 of four, 12,225 of one, with up to 64 columns), remainders in rows and columns
 @pytest.mark.parametrize("K,N,sizes", [(2048, 32, (1535, 1536, 1537)), (1024, 40, (3008, 3009, 3073)), (264, 8, (12224, 12225)), (1024, 130, (1535, 1536, 1600))])

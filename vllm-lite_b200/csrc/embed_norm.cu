@@ -100,15 +100,15 @@ __global__ void embed_pair_kernel(const int* __restrict__ ids, const TW* __restr
 // rows == nullptr: row r of the output is row r of x (and x is updated in place
 // when delta is given).  rows != nullptr: output row r is made from x[rows[r]]
 // (+ delta[rows[r]]) and x is left untouched.
-template <typename TA>
-__global__ void add_rmsnorm_kernel(float* __restrict__ x, const TA* __restrict__ delta,
+template <typename TA, typename TD>
+__global__ void add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta,
                                    const int* __restrict__ rows, const float* __restrict__ w,
                                    TA* __restrict__ out, int H, float eps) {
     __shared__ float scratch[32];
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
     float* xr = x + (size_t)src * H;
-    const TA* dr = delta ? delta + (size_t)src * H : nullptr;
+    const TD* dr = delta ? delta + (size_t)src * H : nullptr;
     float ss = 0.f;
     for (int i = threadIdx.x; i < H; i += 256) {
         float v = xr[i];
@@ -148,9 +148,9 @@ static bool norm_reads_ahead(int rows, int vpt) { return rows <= (vpt > 4 ? 2 : 
 // The same function with a row kept in registers: 16-byte loads, one pass over memory.
 // Thread i holds the float4 pieces i, i + 256, ... of the row (H a multiple of 4, at most
 // 256 * 4 * VPT values).  The sum of squares is taken piece by piece in that fixed order.
-template <typename TA, int VPT, bool AHEAD>
+template <typename TA, typename TD, int VPT, bool AHEAD>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_vec_kernel(float* __restrict__ x, const TA* __restrict__ delta, const int* __restrict__ rows,
+add_rmsnorm_vec_kernel(float* __restrict__ x, const TD* __restrict__ delta, const int* __restrict__ rows,
                        const float* __restrict__ w, TA* __restrict__ out, int H, float eps) {
     __shared__ float scratch[32];
     pdl_launch_dependents();
@@ -161,7 +161,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const TA* __restrict__ delta, cons
     pdl_wait();
     const int src = rows ? rows[r] : r;
     float* xr = x + (size_t)src * H;
-    const TA* dr = delta ? delta + (size_t)src * H : nullptr;
+    const TD* dr = delta ? delta + (size_t)src * H : nullptr;
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -169,7 +169,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const TA* __restrict__ delta, cons
         if (c < H4) {
             v[i] = Quad<float>::load(xr + 4 * c);
             if (dr) {
-                const float4 d = Quad<TA>::load(dr + 4 * c);
+                const float4 d = Quad<TD>::load(dr + 4 * c);
                 v[i].x += d.x; v[i].y += d.y; v[i].z += d.z; v[i].w += d.w;
                 if (!rows) Quad<float>::store(xr + 4 * c, v[i]);
             }
@@ -189,14 +189,14 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const TA* __restrict__ delta, cons
     }
 }
 
-template <typename TA>
-static bool launch_rmsnorm_vec(float* x, const TA* delta, const int* rows, const float* w, TA* out, int R, int H,
+template <typename TA, typename TD>
+static bool launch_rmsnorm_vec(float* x, const TD* delta, const int* rows, const float* w, TA* out, int R, int H,
                                float eps, cudaStream_t s) {
     if (H % 4) return false;
     const int pieces = (H / 4 + 255) / 256;
 #define RMS(VPT)                                                                                                                             \
-    norm_reads_ahead<TA>(R, VPT) ? vl_launch(add_rmsnorm_vec_kernel<TA, VPT, true>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps) \
-                                 : vl_launch(add_rmsnorm_vec_kernel<TA, VPT, false>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps)
+    norm_reads_ahead<TA>(R, VPT) ? vl_launch(add_rmsnorm_vec_kernel<TA, TD, VPT, true>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps) \
+                                 : vl_launch(add_rmsnorm_vec_kernel<TA, TD, VPT, false>, dim3(R), dim3(256), 0, s, x, delta, rows, w, out, H, eps)
     if (pieces <= 1) RMS(1);
     else if (pieces <= 2) RMS(2);
     else if (pieces <= 4) RMS(4);
@@ -693,19 +693,20 @@ extern "C" int vl_embed_pair(const int* ids, const void* table, const void* pair
     return VL_ERR_UNSUPPORTED;
 }
 
-extern "C" int vl_add_rmsnorm(float* x, const void* delta, const int* rows, const float* w, void* out,
+// delta in the output's dtype, or in float32 (a product's sums as they are: the residual of a step whose products add to the stream in float32)
+template <typename TA, typename TD>
+static void launch_rmsnorm(float* x, const void* delta, const int* rows, const float* w, void* out, int R, int H, float eps, cudaStream_t s) {
+    if (!launch_rmsnorm_vec<TA, TD>(x, (const TD*)delta, rows, w, (TA*)out, R, H, eps, s))
+        add_rmsnorm_kernel<TA, TD><<<R, 256, 0, s>>>(x, (const TD*)delta, rows, w, (TA*)out, H, eps);
+}
+extern "C" int vl_add_rmsnorm(float* x, const void* delta, int delta_dtype, const int* rows, const float* w, void* out,
                               int act_dtype, int R, int H, float eps, void* stream) {
     if (R <= 0) return VL_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (act_dtype == VL_F32) {
-        if (!launch_rmsnorm_vec<float>(x, (const float*)delta, rows, w, (float*)out, R, H, eps, s))
-            add_rmsnorm_kernel<float><<<R, 256, 0, s>>>(x, (const float*)delta, rows, w, (float*)out, H, eps);
-    } else if (act_dtype == VL_BF16) {
-        if (!launch_rmsnorm_vec<bf16>(x, (const bf16*)delta, rows, w, (bf16*)out, R, H, eps, s))
-            add_rmsnorm_kernel<bf16><<<R, 256, 0, s>>>(x, (const bf16*)delta, rows, w, (bf16*)out, H, eps);
-    } else {
-        return VL_ERR_UNSUPPORTED;
-    }
+    if (act_dtype == VL_F32 && delta_dtype == VL_F32) launch_rmsnorm<float, float>(x, delta, rows, w, out, R, H, eps, s);
+    else if (act_dtype == VL_BF16 && delta_dtype == VL_BF16) launch_rmsnorm<bf16, bf16>(x, delta, rows, w, out, R, H, eps, s);
+    else if (act_dtype == VL_BF16 && delta_dtype == VL_F32) launch_rmsnorm<bf16, float>(x, delta, rows, w, out, R, H, eps, s);
+    else return VL_ERR_UNSUPPORTED;
     return vl_launch_status();
 }
 

@@ -47,7 +47,7 @@ _SIGNATURES = {
                                         c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int,
                                         c_void_p],
     ("activation", "vl_poly_norm"): [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p],
-    ("embed_norm", "vl_add_rmsnorm"): [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
+    ("embed_norm", "vl_add_rmsnorm"): [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     ("embed_norm", "vl_add_bias"): [c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p],
     ("embed_norm", "vl_cast"): [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p],
     ("rope_cache", "vl_qk_norm_rope_write"): [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
@@ -285,20 +285,21 @@ def embed_pair(ids, table, pairs, out, scale, buckets, mul_prev, mul_cur, state,
 
 
 def add_rmsnorm(x, delta, weight, eps, out, rows=None):
-    """x float32 [T, H] (+= delta when given and rows is None); out[r] = rmsnorm(x[row r] (+ delta)) * weight."""
+    """x float32 [T, H] (+= delta when given and rows is None); out[r] = rmsnorm(x[row r] (+ delta)) * weight.  delta in out's
+    dtype or float32."""
     _need(x, torch.float32, "x", 2); _need(weight, torch.float32, "weight", 1); _need(out, None, "out", 2)
     H = x.shape[1]
     R = x.shape[0] if rows is None else rows.shape[0]
     if weight.shape[0] != H or out.shape != (R, H):
         raise KernelError(f"norm shapes disagree: x {tuple(x.shape)}, weight {tuple(weight.shape)}, out {tuple(out.shape)}")
     if delta is not None:
-        _need(delta, out.dtype, "delta", 2)
+        _need(delta, torch.float32 if delta.dtype == torch.float32 else out.dtype, "delta", 2)
         if delta.shape != x.shape:
             raise KernelError(f"delta {tuple(delta.shape)} must match x {tuple(x.shape)}")
     if rows is not None:
         _need(rows, torch.int32, "rows", 1)
-    _check(_fn("embed_norm", "vl_add_rmsnorm")(_ptr(x), _ptr(delta), _ptr(rows), _ptr(weight), _ptr(out),
-                                               dtype_code(out.dtype), R, H, float(eps), _stream()), "vl_add_rmsnorm")
+    _check(_fn("embed_norm", "vl_add_rmsnorm")(_ptr(x), _ptr(delta), dtype_code((out if delta is None else delta).dtype), _ptr(rows),
+                                               _ptr(weight), _ptr(out), dtype_code(out.dtype), R, H, float(eps), _stream()), "vl_add_rmsnorm")
     return out
 
 

@@ -279,6 +279,9 @@ class GqaAttention:
         bias, self.o_proj.bias = self.o_proj.bias, None
         return bias
 
+    def can_factor_norms(self, M) -> bool:
+        return not self.with_options and self.qkv_proj.can_factor_norms(M) and self.o_proj.can_factor_norms(M)
+
     def factors_norms(self, M) -> bool:
         """For M rows: the input may come as `ScaledRows` and the result may go `into_stream`."""
         return not self.with_options and self.qkv_proj.factors_norms(M) and self.o_proj.factors_norms(M)
@@ -320,7 +323,7 @@ class GqaAttention:
             ops.sigmoid_gate(out, qkv, self.gate_col)
         return self.o_proj(out, step, "attn.o")
 
-    def __call__(self, h, step, cache, sink=None):
+    def __call__(self, h, step, cache, sink=None, sums=False):
         if self.with_options:
             return self._call_with_options(h, step, cache)
         s = self.spec
@@ -349,4 +352,4 @@ class GqaAttention:
         attention_dispatch.run(qkv, out, cache, group, step, s, self.scale, fold=fold)
         if sink is not None:
             return self.o_proj.into_stream(out, sink, step, "attn.o")
-        return self.o_proj(out, step, "attn.o")
+        return self.o_proj(out, step, "attn.o", torch.float32 if sums else None)

@@ -5,7 +5,7 @@ Interfaces (duck-typed; a part is any class registered under its kind):
   every part     declare(spec) -> {relative tensor name: TensorDecl}     static
                  __init__(spec, weights, ctx)   weights: {relative name: device tensor}
   norm           __call__(x, delta, step, rows=None) -> h
-                     x float32 [T, H] residual stream; delta (activation dtype) or None is
+                     x float32 [T, H] residual stream; delta (activation dtype; float32 where the norm is `factorable`) or None is
                      added into x first (not stored when `rows` picks rows); h is new
   position       fused_rotary() -> (inv_freq, rotary_dim), or None for an encoding of its own, which then
                  offers apply(qkv, positions, num_heads, num_kv_heads, head_dim, step): it changes the
@@ -149,7 +149,7 @@ class CallCache:
 @dataclass
 class Residual:
     x: torch.Tensor                           # float32 [T, H]
-    pending: Optional[object] = None          # not yet added into x: a tensor in the activation dtype, or a `StreamSum`
+    pending: Optional[object] = None          # not yet added into x: a tensor in the activation dtype or float32, or a `StreamSum`
     normed: Optional["ScaledRows"] = None     # output of the norm `normed_for` on x, in factored form
     normed_for: object = None
     cast: Optional[torch.Tensor] = None       # x in the activation dtype, when the kernel that last wrote x left it

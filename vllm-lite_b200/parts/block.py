@@ -6,7 +6,9 @@ left pending and the next norm's kernel adds it while it reads the stream.  In a
 step of few rows the norms' kernels are saved altogether where the neighbouring
 parts can: the part before a norm adds its result into the stream itself and
 leaves the norm's output in factored form (`ScaledRows`), which the part after
-the norm takes as it is."""
+the norm takes as it is.  Where the parts can but a faster product is chosen instead,
+the part leaves its float32 sums (`sums`), so that the stream gets the same numbers
+either way."""
 from __future__ import annotations
 
 import torch
@@ -44,13 +46,13 @@ class PreNormBlock:
     chains_norms = True        # __call__ takes `next_norm`
 
     def input_norm_for_fusion(self, M):
-        """The first norm, if the block before may compute it for M rows in factored form."""
-        ok = getattr(self.norm1, "factorable", False) and _factors(self.mixer, M)
-        return self.norm1 if ok else None
+        """The first norm, if the block before may compute it for M rows in factored form, and whether it should."""
+        ok = getattr(self.norm1, "factorable", False) and _can_factor(self.mixer, M)
+        return (self.norm1, _factors(self.mixer, M)) if ok else None
 
     def __call__(self, residual, step, cache, next_norm=None):
         """next_norm: the norm that will read the stream after this block, when its reader can take
-        the factored form (`input_norm_for_fusion` of the next block)."""
+        the factored form, and whether it should (`input_norm_for_fusion` of the next block)."""
         M = step.num_tokens
         residual.cast = None                                      # this block's kernels write x without it
         if residual.normed is not None and residual.normed_for is self.norm1:
@@ -58,16 +60,23 @@ class PreNormBlock:
         else:
             h = self.norm1(residual.x, residual.pending, step, tag="norm1")
         residual.pending = residual.normed = residual.normed_for = None
-        if _factors(self.mixer, M) and getattr(self.norm2, "factorable", False) and _factors(self.ffn, M):
+        can = _can_factor(self.mixer, M) and getattr(self.norm2, "factorable", False) and _can_factor(self.ffn, M)
+        if can and _factors(self.mixer, M) and _factors(self.ffn, M):
             h = self.mixer(h, step, cache, sink=_sink(residual, self.norm2))
         else:
-            a = self.mixer(h, step, cache)
+            a = self.mixer(h, step, cache, **({"sums": True} if can else {}))
             h = self.norm2(residual.x, a, step, tag="norm2")
-        if next_norm is not None and _factors(self.ffn, M):
-            residual.normed = self.ffn(h, step, sink=_sink(residual, next_norm))
-            residual.normed_for = next_norm
+        can = next_norm is not None and _can_factor(self.ffn, M)
+        if can and next_norm[1] and _factors(self.ffn, M):
+            residual.normed = self.ffn(h, step, sink=_sink(residual, next_norm[0]))
+            residual.normed_for = next_norm[0]
         else:
-            residual.pending = self.ffn(h, step)
+            residual.pending = self.ffn(h, step, **({"sums": True} if can else {}))
+
+
+def _can_factor(part, M) -> bool:
+    f = getattr(part, "can_factor_norms", None)
+    return bool(f and f(M))
 
 
 def _factors(part, M) -> bool:

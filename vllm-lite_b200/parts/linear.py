@@ -36,14 +36,17 @@ class Linear:
         if self.bias is not None and tuple(self.bias.shape) != (self.out_features,):
             raise ValueError(f"a linear bias has out_features={self.out_features} entries, got {tuple(bias.shape)}")
 
+    def can_factor_norms(self, M) -> bool:
+        """Whether, for M rows, this layer has a kernel that takes an RMS norm's output in factored form
+        (`ScaledRows`) and adds its result into the stream (`into_stream`)."""
+        return self.bias is None and self.weight.dtype == torch.bfloat16 and ops.gemm_bf16_small_m_ok(M, self.in_features)
+
     def factors_norms(self, M) -> bool:
-        """Whether, for M rows, this layer's kernel can take an RMS norm's output in factored form
-        (`ScaledRows`) and can add its result into the stream (`into_stream`).  Not where the product that takes a tile an SM is so much
+        """Whether it should.  Not where the product that takes a tile an SM is so much
         faster that it pays for a norm's own launch (9 to 16 rows on 4,096 columns or more: a step of 12 through eight layers of
         Qwen3-8B 1,171 -> 1,130 us; with 2,048 columns the products gain 2 us each, the norm takes 3 to 4)."""
         K = self.in_features
-        return (self.bias is None and self.weight.dtype == torch.bfloat16 and ops.gemm_bf16_small_m_ok(M, K)
-                and (K < 4096 or not ops.gemm_bf16_few_ok(M, self.out_features, K)))
+        return self.can_factor_norms(M) and (K < 4096 or not ops.gemm_bf16_few_ok(M, self.out_features, K))
 
     def into_stream(self, a, sink: StreamSink, step, tag) -> ScaledRows:
         """sink.x += a W^T; returns the next norm's output on the new stream, in factored form."""

@@ -39,12 +39,15 @@ class SwiGLU:
         self.gate_up = Linear(stacked.contiguous())
         self.down = Linear(weights["down_proj.weight"])
 
+    def can_factor_norms(self, M) -> bool:
+        return self.group == ops.SWIGLU_GROUP and self.gate_up.can_factor_norms(M) and self.down.can_factor_norms(M)
+
     def factors_norms(self, M) -> bool:
         """For M rows: the input may come as `ScaledRows` and the result may go `into_stream`."""
         return self.group == ops.SWIGLU_GROUP and self.gate_up.factors_norms(M) and self.down.factors_norms(M)
 
-    def __call__(self, h, step, sink=None):
+    def __call__(self, h, step, sink=None, sums=False):
         act = self.gate_up.swiglu(h, step, "mlp.gate_up", self.group)
         if sink is not None:
             return self.down.into_stream(act, sink, step, "mlp.down")
-        return self.down(act, step, "mlp.down")
+        return self.down(act, step, "mlp.down", torch.float32 if sums else None)
