@@ -424,15 +424,19 @@ def read_ceiling(cfg, batch, context):
 KIKEPEL_SIZES = {"2k": (2048, 16, 128, 128, 768, 128, 1024, 8192, 1024, 32, 4, 65536),
                  "4k": (4096, 32, 128, 128, 1536, 128, 4096, 12288, 1408, 64, 6, 65536),
                  "4k-r256": (4096, 32, 128, 128, 1536, 256, 4096, 12288, 1408, 64, 6, 65536)}
+# every kernel that parts/matmul.py or a linear layer can hand a dense product to ("library_mm": `ops.mm`), and those of a prompt's layers
+DENSE_PRODUCTS = ("library_mm", "gemm_bf16_few", "gemm_bf16_small_m", "gemm_bf16_tc5", "gemm_bf16_tc5_pair", "gemm_f32")
+PROMPT_PRODUCTS = ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")          # (a row's head is the weight-streaming product)
 # kernels of the new design and the like kernels of the closest model, by the name of their entry in csrc/ops.py
 TIMED_OPS = ("paged_attention", "flash_prefill", "flash_prefill_tc5", "flash_decode", "gemm_heads", "gemm_grouped",
-             "gemm_grouped_fused", "gemm_grouped_tc5", "gemm_bf16_small_m", "gemm_bf16_tc5", "gemm_bf16_tc5_pair", "layernorm_add",
+             "gemm_grouped_fused", "gemm_grouped_tc5", "layernorm_add",
              "layernorm_rows", "add_rmsnorm", "latent_norm_write", "qk_norm_rope_write", "moe_route", "moe_align",
              "moe_gather", "moe_combine", "gated_act", "silu_mul", "scale_softcap", "embed", "cast", "add_bias",
              "hc_step", "dyt_rows", "short_conv", "ssd_scan", "mlstm_scan", "delta_scan", "gate_norm", "scaled_sum",
              "token_shift", "rows_norm_rope_write", "conv_rows_norm_rope_write", "rmsnorm_add", "unary_act",
              "head_norm_write", "rope_heads", "sigmoid_gate", "token_shift_multi", "decay_scan", "decay_from_raw", "head_work", "combine_maps", "linear_scan", "poly_norm", "embed_pair",
-             "stream_norm", "delta_chunks", "delta_step")
+             "stream_norm", "delta_chunks", "delta_step") + DENSE_PRODUCTS
+OP_OF = {"library_mm": "mm"}                             # the entry in csrc/ops.py, where it has another name
 
 
 def kikepel_config(size, layers):
@@ -449,7 +453,7 @@ def kikepel_config(size, layers):
 def timed_step(runner, entries, suffix=None):
     """One step with every kernel of csrc/ops.py between two CUDA events.  The launches queue up behind a
     kernel that only waits, so that the events see the kernels back to back and not the host's pace.
-    Returns {op: [launches, microseconds]} (library products through torch.mm are 'library_mm').  `suffix`(options of a
+    Returns {op: [launches, microseconds]} (library products are 'library_mm').  `suffix`(options of a
     launch) -> what is added to its name, for launches that are to be listed apart."""
     import torch
     from vllm_lite_b200.csrc import ops
@@ -468,10 +472,9 @@ def timed_step(runner, entries, suffix=None):
             return r
         return inner
     for name in TIMED_OPS:
-        saved[name] = getattr(ops, name)
-        setattr(ops, name, wrap(name, saved[name]))
-    mm = torch.mm
-    torch.mm = wrap("library_mm", mm)
+        entry = OP_OF.get(name, name)
+        saved[entry] = getattr(ops, entry)
+        setattr(ops, entry, wrap(name, saved[entry]))
     graphs, runner.decode_graphs = runner.decode_graphs, False
     try:
         torch.cuda.synchronize()
@@ -481,7 +484,6 @@ def timed_step(runner, entries, suffix=None):
     finally:
         for name, fn in saved.items():
             setattr(ops, name, fn)
-        torch.mm = mm
         runner.decode_graphs = graphs
     out = {}
     for name, e0, e1 in records:
@@ -570,11 +572,11 @@ def kikepel_bench(args):
     roof["expert_products_prefill_tflops"] = {
         "kikepel": tf(nmoe * 2.0 * T * top * 3 * W * eff, us(k, "kernels_prefill", ("gemm_grouped", "gemm_grouped_fused", "gemm_grouped_tc5"))),
         "qwen3 (all dense products of the layers)": tf(layers * 2.0 * T * q_layer,
-                                                       us(q, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+                                                       us(q, "kernels_prefill", PROMPT_PRODUCTS))}
     touched = min(E, B * top)
     roof["expert_products_decode_gbs"] = {
         "kikepel (experts that 64 tokens can reach)": gb(nmoe * touched * 3.0 * W * eff * 2, us(k, "kernels_decode_b64", ("gemm_grouped", "gemm_grouped_fused"))),
-        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", ("library_mm", "gemm_bf16_small_m")))}
+        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", DENSE_PRODUCTS))}
     roof["norm_prefill_gbs"] = {
         "kikepel layernorm_add (y in, x in and out, cast out)": gb(k["kernels_prefill"].get("layernorm_add", [0])[0] * T * W * 12.0,
                                                                   us(k, "kernels_prefill", ("layernorm_add",))),
@@ -832,11 +834,11 @@ def sodonex_bench(args):
     roof["expert_products_prefill_tflops"] = {
         "sodonex": tf(layers * 2.0 * T * top * 2 * W * eff, us(sx, "kernels_prefill", grouped)),
         "qwen3 (all dense products of the layers)": tf(layers * 2.0 * T * q_layer,
-                                                       us(q, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+                                                       us(q, "kernels_prefill", PROMPT_PRODUCTS))}
     touched = min(E, B * top)
     roof["expert_products_decode_gbs"] = {
         "sodonex (experts that 64 tokens can reach)": gb(layers * touched * 2.0 * W * eff * 2, us(sx, "kernels_decode_b64", grouped)),
-        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", ("library_mm", "gemm_bf16_small_m")))}
+        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", DENSE_PRODUCTS))}
     roof["peaks"] = {"hbm_gbs": pk["hbm_gbs"], "bf16_tflops": pk["bf16_tflops"], "source": pk["source"]}
     print(json.dumps({"sodonex_bench": size, "layers": layers, "context": context, "steps": args.steps, "warmup": warmup,
                       "dtype": "bf16", "data": "synthetic (random weights, uniform token ids)",
@@ -973,11 +975,11 @@ def puturax_bench(args):
     roof["expert_products_prefill_tflops"] = {
         "puturax": tf(n_par * 2.0 * T * top * 3 * W * eff, us(px, "kernels_prefill", grouped)),
         "qwen3 (all dense products of the layers)": tf(layers * 2.0 * T * q_layer,
-                                                       us(q, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+                                                       us(q, "kernels_prefill", PROMPT_PRODUCTS))}
     touched = min(E, B * top)
     roof["expert_products_decode_gbs"] = {
         "puturax (experts that 64 tokens can reach)": gb(n_par * touched * 3.0 * W * eff * 2, us(px, "kernels_decode_b64", grouped)),
-        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", ("library_mm", "gemm_bf16_small_m")))}
+        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", DENSE_PRODUCTS))}
     roof["peaks"] = {"hbm_gbs": pk["hbm_gbs"], "bf16_tflops": pk["bf16_tflops"], "source": pk["source"]}
     print(json.dumps({"puturax_bench": size, "layers": layers, "context": context, "steps": args.steps, "warmup": warmup,
                       "dtype": "bf16", "data": "synthetic (random weights, uniform token ids)",
@@ -1143,10 +1145,10 @@ def pafelorn_roofline(size, layers, context, results, pk):
     q_layer = (H + 2 * KV) * D * W + W * H * D + 3 * W * (top * eff + sff)
     roof["expert_products_prefill_tflops"] = {
         "pafelorn": tf(n_moe * 2.0 * T * top * share * 3 * W * eff, us(px, "kernels_prefill", grouped)),
-        "qwen3 (all dense products of the layers)": tf(layers * 2.0 * T * q_layer, us(q, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+        "qwen3 (all dense products of the layers)": tf(layers * 2.0 * T * q_layer, us(q, "kernels_prefill", PROMPT_PRODUCTS))}
     roof["expert_products_decode_gbs"] = {
         "pafelorn (experts that 64 tokens can reach)": gb(n_moe * min(E, B * top) * 3.0 * W * eff * 2, us(px, "kernels_decode_b64", grouped)),
-        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", ("library_mm", "gemm_bf16_small_m")))}
+        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", DENSE_PRODUCTS))}
     return roof
 
 
@@ -1304,12 +1306,12 @@ def vekusun_roofline(size, layers, context, results, pk):
     q_layer = (H + 2 * max(1, H // 4)) * D * W + W * H * D + 3 * W * top * eff
     roof["expert_products_prefill_tflops"] = {
         "vekusun": tf(n_moe * 2.0 * T * top * 3 * W * eff, us(vk, "kernels_prefill", grouped)),
-        "qwen3 (all dense products of the layers)": tf(len(kinds) * 2.0 * T * q_layer, us(q, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+        "qwen3 (all dense products of the layers)": tf(len(kinds) * 2.0 * T * q_layer, us(q, "kernels_prefill", PROMPT_PRODUCTS))}
     v_layers = n_delta * (C + 2 * H * D) * W + n[1] * ((qr + kr) * W + H * D * qr + H * D * W) + n[2] * ((H * (D + rot) + row2) * W + H * D * W) + n_dense * 2 * W * ff
-    roof["dense_products_prefill_tflops"] = {"vekusun": tf(2.0 * T * v_layers, us(vk, "kernels_prefill", ("gemm_bf16_tc5", "gemm_bf16_tc5_pair", "library_mm")))}
+    roof["dense_products_prefill_tflops"] = {"vekusun": tf(2.0 * T * v_layers, us(vk, "kernels_prefill", PROMPT_PRODUCTS))}
     roof["expert_products_decode_gbs"] = {
         "vekusun (experts that 64 tokens can reach)": gb(n_moe * min(E, B * top) * 3.0 * W * eff * 2, us(vk, "kernels_decode_b64", grouped)),
-        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", ("library_mm", "gemm_bf16_small_m")))}
+        "qwen3 (all products)": gb(q["weights_GB"] * 1e9 - 2.0 * vocab * W * 2, us(q, "kernels_decode_b64", DENSE_PRODUCTS))}
     return roof
 
 

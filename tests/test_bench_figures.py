@@ -35,3 +35,42 @@ def test_contract_edges_need_no_gpu():
     ref = subprocess.run([sys.executable, str(ROOT / "bench.py"), "--impl", "reference"], capture_output=True, text=True)
     line = json.loads(ref.stdout)
     assert ref.returncode == 0 and line["impl"] == "reference" and "unavailable" in line
+
+
+def test_a_timed_step_records_every_dense_product(monkeypatch):
+    """The per-kernel tables divide by what these products took: each one that the dispatcher can choose is recorded, the library's too."""
+    import re
+    from types import SimpleNamespace
+    import torch
+    from vllm_lite_b200.csrc import ops
+    from vllm_lite_b200.parts import linear, matmul
+    entries = {bench.OP_OF.get(n, n) for n in bench.DENSE_PRODUCTS}
+    chosen = {m for module in (matmul, linear) for m in re.findall(r"\bops\.(gemm_\w+|mm)\(", Path(module.__file__).read_text())}
+    assert {m for m in chosen if not m.endswith("_ok")} == entries and set(bench.DENSE_PRODUCTS) <= set(bench.TIMED_OPS)
+    assert set(bench.PROMPT_PRODUCTS) <= set(bench.DENSE_PRODUCTS) and all(hasattr(ops, bench.OP_OF.get(n, n)) for n in bench.TIMED_OPS)
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self):
+            pass
+
+        def elapsed_time(self, other):
+            return 1.0
+
+    for name, stub in (("Event", Event), ("synchronize", lambda: None), ("_sleep", lambda n: None)):
+        monkeypatch.setattr(torch.cuda, name, stub)
+    for name in entries - {"mm"}:
+        monkeypatch.setattr(ops, name, lambda *a, **k: None)
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    before = {n: getattr(ops, bench.OP_OF.get(n, n)) for n in bench.TIMED_OPS}
+
+    def step(entries):
+        for M, N in ((1, 64), (12, 64), (300, 64), (2048, 64), (2048, 40960)):
+            matmul.gemm_bf16(torch.zeros(M, 64, dtype=torch.bfloat16), torch.zeros(N, 64, dtype=torch.bfloat16),
+                             torch.zeros(M, N, dtype=torch.bfloat16) if M == 300 else None)
+
+    got = bench.timed_step(SimpleNamespace(step=step, decode_graphs=True), [])
+    assert {k: v[0] for k, v in got.items()} == {n: 1 for n in bench.DENSE_PRODUCTS if n != "gemm_f32"}
+    assert before == {n: getattr(ops, bench.OP_OF.get(n, n)) for n in bench.TIMED_OPS}
