@@ -54,11 +54,20 @@ def test_the_grouped_product_of_paired_blocks_has_no_path_to_dependent_launch():
 
 # A wait is given up by each lane at its own time.  Where the lanes then meet again (a warp's barrier, a load of tensor memory), one that left
 # by itself would let the others wait for good: whoever breaks off a loop over a wait does so by the vote of the warp.
-@pytest.mark.parametrize("name", ["gemm_tc5", "gemm_tc5_pair", "gemm_tc5_grouped", "gemm_few", "gemm_batched", "flash_tc5"])
+@pytest.mark.parametrize("name", ["gemm_tc5", "gemm_tc5_pair", "gemm_tc5_grouped", "gemm_few", "gemm_batched", "flash_tc5", "gemm_bf16"])
 def test_no_lane_leaves_a_loop_by_itself_when_a_wait_runs_out(name):
     code = re.sub(r"//[^\n]*", "", (build.CSRC / f"{name}.cu").read_text())
     assert "wait" in code and not re.search(r"if\s*\(\s*!\s*(tc5::)?mbar_wait_bounded", code)
     assert "__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))" in (build.CSRC / "tc5.cuh").read_text()
+
+
+def test_the_weight_streams_consumers_leave_together():
+    """Between two tiles the four consumer warps meet at a barrier that counts 128 threads: a warp that left alone behind a wait
+    that ran out would keep the others there."""
+    code = re.sub(r"//[^\n]*", "", (build.CSRC / "gemm_bf16.cu").read_text())
+    tiles = code[code.index("for (int n0 = r0; n0 < r1; n0 += GS_ROWS) {\n#pragma unroll"):]
+    assert 0 < tiles.index("ok = consumers_agree(ok);") < tiles.index("if (!ok) break;", tiles.index("consumers_agree"))
+    assert "bar.red.and.pred q, 1, 128, p;" in code
 
 
 def test_the_engine_is_imported_without_a_compiler(tmp_path):

@@ -64,6 +64,13 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsign
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// the same barrier, and whether all four warps say so: they leave together, since the next barrier counts all of them
+__device__ __forceinline__ bool consumers_agree(bool ok) {
+    int all;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.and.pred q, 1, 128, p;\n selp.s32 %0, 1, 0, q;\n}"
+                 : "=r"(all) : "r"((int)ok) : "memory");
+    return all != 0;
+}
 
 #define GS_CONSUMERS 4                     // consumer warps; warp 4 is the producer
 
@@ -185,7 +192,7 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
     auto multiply = [&](int it, const uint4 (&a)[STEPS][MT]) -> bool {
         const int s = git % GS_STAGES;
         const int kbase = it * GS_KC + warp * (GS_KC / GS_CONSUMERS);
-        if (!mbar_wait_bounded(&full_bar[s], (unsigned)((git / GS_STAGES) & 1))) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], (unsigned)((git / GS_STAGES) & 1)))) {
             if (lane == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_SMALL_M);
             return false;
         }
@@ -230,7 +237,7 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
         red[warp][j][g + 8][2 * t] = acc[j][2];
         red[warp][j][g + 8][2 * t + 1] = acc[j][3];
     }
-    consumer_barrier();
+    ok = consumers_agree(ok);
     if (swiglu) {
         // the tile's 16 rows of W are 8 gate rows and their 8 up rows: C[m, n0/2 + i] = silu(gate_i) * up_i
         for (int idx = tid; idx < MT * 8 * 8; idx += 32 * GS_CONSUMERS) {
