@@ -693,6 +693,18 @@ def test_unary_activation(act, dtype, n, off):
     assert bool(((out.double() - ref).abs() <= rel * ref.abs() + 1e-37).all())
 
 
+def test_gelu_of_small_float32_values():
+    """|v| <= 0.5: 1 + erff(z) to 2 ulp of erff (2^-24 here), 0.6 of that for the rounded argument and the sum's own 2^-24, relative to a sum of
+    0.61 or more, then a product.  And the same bits whether or not neighbours lie on the other side of -1.5, where the form changes."""
+    x = torch.linspace(-0.5, 0.5, 200_001, device=DEV)
+    x = x[x != 0]
+    out = ops().unary_act(x, torch.empty_like(x), "gelu")
+    ref = x.double() * 0.5 * torch.special.erfc(-x.double() / 2 ** 0.5)
+    assert bool(((out.double() - ref).abs() <= 6.2 * 2.0 ** -24 * ref.abs()).all())
+    both = torch.stack([x[:1000], x[:1000] - 3], 1).reshape(-1).contiguous()
+    assert torch.equal(ops().unary_act(both, torch.empty_like(both), "gelu")[::2], out[:1000])
+
+
 def test_gelu_beyond_numbers():
     x = torch.tensor([float("inf"), float("nan"), 3e38, -3e38], device=DEV)
     out = torch.empty_like(x)

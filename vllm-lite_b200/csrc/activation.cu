@@ -113,11 +113,15 @@ extern "C" int vl_silu_mul(const void* gu, void* out, int dtype, int T, int I, i
 #define VL_ACT_GELU 18
 // The normal distribution function at v is erfc(-v / sqrt(2)) / 2, and for z >= 0 erfc(z) = e^(-z^2) f(t), t = 1 / (1 + 0.44 z), with f(t) =
 // erfc(z) e^(z^2) smooth on (0, 1]: a polynomial of degree 8 without a constant, fitted to scipy's erfcx over z = 0 .. 10 by least
-// squares of the relative error with weights drawn to its largest places (1.8e-7).  It bounds the kernel by memory where 1 + erff(z) bound
-// it by its instructions (3,281 x 8,192 bfloat16: 39 us, 45 % more instructions), and keeps the small values for v < 0 that the sum cancels:
-// against 64 bits over -9 .. 9 1.6e-8 of the 2-norm (1 + erff: 1.7e-8), relative error at -5 .. -3 2.5e-6 (0.05).
-__device__ __forceinline__ float gelu_value(float v) {
-    const float z = fminf(fabsf(v) * 0.70710678f, 14.0f), t = __fdividef(1.0f, fmaf(0.44f, z, 1.0f));
+// squares of the relative error with weights drawn to its largest places (1.8e-7).  It keeps the small values for v < 0 that the sum 1 + erff(z)
+// cancels (relative error in float32 at -4 .. -3 1.3e-6, the sum's 5e-4), but near zero the sum is the nearer one (|v| <= 0.5: 1.4e-7 and
+// 5.7e-7 at most, 4e-8 and 1.4e-7 of the 2-norm; they cross at -1.5).  So float32 values take either form where it is the better one, with
+// the full exponential and quotient.  A bfloat16 result's rounding (2e-3) hides both: there the polynomial alone, with the fast ones, bounds the
+// kernel by memory where the sum bound it by its instructions (3,281 x 8,192: 39 us with the sum, 45 % more instructions).
+template <typename T> __device__ __forceinline__ float gelu_value(float v) {
+    constexpr bool fast = sizeof(T) == 2;
+    if (!fast && v > -1.5f) return 0.5f * v * (1.0f + erff(v * 0.70710678f));
+    const float z = fminf(fabsf(v) * 0.70710678f, 14.0f), d = fmaf(0.44f, z, 1.0f), t = fast ? __fdividef(1.0f, d) : 1.0f / d;
     float f = 0.07122346758842468f;
     f = fmaf(f, t, -0.2779480218887329f);
     f = fmaf(f, t, 0.2966874837875366f);
@@ -126,12 +130,12 @@ __device__ __forceinline__ float gelu_value(float v) {
     f = fmaf(f, t, 0.21731355786323547f);
     f = fmaf(f, t, 0.24887117743492126f);
     f = fmaf(f, t, 0.24822095036506653f);
-    const float half = 0.5f * t * f * __expf(-z * z);
+    const float half = 0.5f * t * f * (fast ? __expf(-z * z) : expf(-z * z));
     return v * (v > 0.f ? 1.0f - half : half);
 }
-template <int ACT> __device__ __forceinline__ float unary_value(float v) {
+template <typename T, int ACT> __device__ __forceinline__ float unary_value(float v) {
     if (ACT == VL_ACT_RELU2) { v = fmaxf(v, 0.f); return v * v; }
-    if (ACT == VL_ACT_GELU) return gelu_value(v);
+    if (ACT == VL_ACT_GELU) return gelu_value<T>(v);
     return tanhf(v);
 }
 // VEC = 8, 4: a thread takes eight or four neighbouring values, when the buffers allow it; eight where that still gives every SM
@@ -147,13 +151,13 @@ unary_act_kernel(const T* __restrict__ in, T* __restrict__ out, size_t n) {
         float v[8];
         load8(in + i, v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = unary_value<ACT>(v[j]);
+        for (int j = 0; j < 8; ++j) v[j] = unary_value<T, ACT>(v[j]);
         store8(out + i, v);
     } else if constexpr (VEC == 4) {
         const float4 v = Quad<T>::load(in + i);
-        Quad<T>::store(out + i, make_float4(unary_value<ACT>(v.x), unary_value<ACT>(v.y), unary_value<ACT>(v.z), unary_value<ACT>(v.w)));
+        Quad<T>::store(out + i, make_float4(unary_value<T, ACT>(v.x), unary_value<T, ACT>(v.y), unary_value<T, ACT>(v.z), unary_value<T, ACT>(v.w)));
     } else {
-        out[i] = from_f32<T>(unary_value<ACT>(to_f32(in[i])));
+        out[i] = from_f32<T>(unary_value<T, ACT>(to_f32(in[i])));
     }
 }
 
