@@ -262,3 +262,33 @@ def test_layers_of_4096_columns_leave_their_sums(monkeypatch):
     for M in (1, 8, 9, 16, 17):
         assert wide.can_factor_norms(M) is narrow.can_factor_norms(M) is (M <= 16)
         assert narrow.factors_norms(M) is (M <= 16) and wide.factors_norms(M) is (M <= 8)
+
+
+# The tcgen05 products: plain ones from 2,048 rows, the fused activation from 1,024, and from 512 where at most a quarter of the tiles is padding or
+# places without a tile (74 pairs of SMs; gate/up of 24,576 rows of W: 96 tiles for 256 rows).
+@pytest.mark.parametrize("M,N,fused,takes", [
+    (511, 24576, True, False), (512, 24576, True, True), (536, 24576, True, False), (768, 24576, True, True), (900, 24576, True, False),
+    (1023, 24576, True, True), (1024, 24576, True, True), (1024, 512, True, True), (512, 512, True, False), (768, None, True, False),
+    (1023, None, True, False), (1024, None, True, True), (1024, 24576, False, False), (2047, 24576, False, False), (2048, 64, False, True)])
+def test_which_products_run_on_tcgen05(monkeypatch, M, N, fused, takes):
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    assert ops.gemm_bf16_tc5_ok(M, 4096, fused, N) is takes
+    assert not ops.gemm_bf16_tc5_ok(M, 4100, fused, N)
+
+
+def test_a_fused_activation_is_promised_where_a_kernel_takes_it(monkeypatch):
+    """`fuses_swiglu` and the product itself ask the same rules: what is promised finds a kernel, and what is not has none."""
+    from vllm_lite_b200.parts import matmul
+    monkeypatch.setattr(ops, "sm_pairs", lambda: 74)
+    for name in ("gemm_bf16_few", "gemm_bf16_small_m", "gemm_bf16_tc5", "gemm_bf16_tc5_pair"):
+        monkeypatch.setattr(ops, name, lambda *a, _n=name, **k: _n)
+    for N in (64, 2048, 4752, 7120, 24576):
+        for K in (64, 4096, 4100):
+            w = torch.empty(N, K, dtype=torch.bfloat16, device="meta")
+            for M in (1, 8, 9, 16, 17, 32, 33, 48, 49, 64, 511, 512, 536, 768, 1023, 1024, 4096):
+                a = torch.empty(M, K, dtype=torch.bfloat16, device="meta")
+                if matmul.fuses_swiglu(M, K, N):
+                    assert matmul.gemm_bf16(a, w, None, swiglu=True).startswith("gemm_bf16_")
+                else:
+                    with pytest.raises(ValueError):
+                        matmul.gemm_bf16(a, w, None, swiglu=True)

@@ -196,3 +196,27 @@ def test_stats_report_step_counts_and_times_by_kind():
     sampled = sum(t["device_samples"] for t in eng.stats()["step_times"].values())
     assert sampled >= 2                                     # every 16th step is timed on the device
     assert all(t["device_ms_p50"] is None or t["device_ms_p50"] > 0 for t in eng.stats()["step_times"].values())
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("requests", [9, 16, 24, 48])
+def test_programmatic_launches_change_no_bit_of_a_step(requests, recorded, monkeypatch):
+    """Steps of 9 to 48 rows, whose products ask for their weights before the kernel in front has ended: the same logits, bit for bit, when
+    every kernel waits for the one before; in steps launched kernel by kernel and in recorded ones."""
+    import importlib
+    from vllm_lite_b200.engine import ModelRunner, StepEntry, random_model
+    module = importlib.import_module("vllm_lite_b200.engine.runner")
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_size=4096, num_hidden_layers=2, num_attention_heads=8,
+               num_key_value_heads=2, head_dim=128, intermediate_size=2048, vocab_size=1024, rope_theta=1e6, rms_norm_eps=1e-6,
+               tie_word_embeddings=False, max_position_embeddings=1024)
+    _, plan, weights = random_model(cfg, seed=3, dtype="bfloat16", device="cuda:0")
+
+    def run():
+        r = ModelRunner(plan, weights, num_pages=64, max_requests=64, max_context=1024, decode_graphs=recorded)
+        out = [r.step([StepEntry(i, [7 * i + s], [0]) for i in range(requests)]).clone() for s in range(6)]
+        r.check_device_errors()
+        return torch.stack(out)
+
+    overlapped = run()
+    monkeypatch.setattr(module, "launches_dependent", lambda tokens, recorded, may_pair: False)
+    assert torch.equal(run(), overlapped) and bool(overlapped.isfinite().all())

@@ -520,6 +520,73 @@ def test_experts_product_of_few_rows(groups, N, K, act):
         assert bool(((again[live].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3).all())
 
 
+# ... and where two blocks an SM would need a second round and three do not (a ring of three stages): the first and the last number of items of
+# that range, K of fewer stages than the ring's and of several rounds of it, cut at the end; every activation
+@pytest.mark.parametrize("act", [None, "silu", "relu", "capped_swish", "relu2"])
+@pytest.mark.parametrize("K", [512, 1160])
+@pytest.mark.parametrize("last,dead", [(False, 0), (True, 0), (True, 2)])
+def test_experts_product_of_few_rows_in_one_round_of_three_blocks(last, dead, K, act):
+    sms = 2 * ops().sm_pairs()
+    N, G, top, tokens = 64 * 12, 5, 2, 40
+    across, gated = N // 64, act in ("silu", "relu", "capped_swish")
+    tiles = 3 * sms // across if last else 2 * sms // across + 1
+    assert 2 * sms < tiles * across <= 3 * sms                     # the launcher's items: of all places, rows or none
+    groups = [y % G for y in range(tiles - dead)] + [-1] * dead
+    gen = torch.Generator(device=DEV).manual_seed(K + tiles)
+    cap = 16 * tiles
+    h = torch.randn(tokens, K, device=DEV, generator=gen).to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device=DEV, generator=gen) / K ** 0.5).to(torch.bfloat16)
+    rows = torch.randint(-8, tokens * top, (cap,), device=DEV, generator=gen).clamp(min=-1).to(torch.int32)
+    scale, err = torch.rand(tokens * top, device=DEV, generator=gen), torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = torch.full((cap, N // 2 if gated else N), 7.0, device=DEV, dtype=torch.bfloat16)
+    ops().gemm_grouped_fused(h, w, out, torch.tensor(groups, dtype=torch.int32, device=DEV), 16, rows, top, scale, act, 1.5, 0.8, 0.25, err)
+    assert int(err) == 0
+    for y, e in enumerate(groups):
+        at = slice(16 * y, 16 * y + 16)
+        if e < 0:
+            assert bool((out[at] == 7.0).all())
+            continue
+        r = rows[at].long()
+        a = h.double()[r.clamp(min=0) // top] * (r >= 0)[:, None]
+        s = torch.where(r >= 0, scale.double()[r.clamp(min=0)], 0.0)[:, None]
+        z, off = (a @ w[e].double().T) * s, K * 2.0 ** -24 * (a.abs() @ w[e].double().abs().T) * s          # float32 sums
+        if gated:
+            z, off = z.view(16, -1, 2, 8), off.view(16, -1, 2, 8)
+            p, u, op, ou = z[:, :, 0].reshape(16, -1), z[:, :, 1].reshape(16, -1), off[:, :, 0].reshape(16, -1), off[:, :, 1].reshape(16, -1)
+            if act == "relu":
+                z, off = p.clamp(min=0) * u, op * u.abs() + p.abs() * ou + op * ou
+            else:
+                alpha, shift = 1.0, 0.0
+                if act == "capped_swish":
+                    alpha, shift, p, u = 1.5, 0.25, p.clamp(max=0.8), u.clamp(-0.8, 0.8)
+                z = p / (1 + torch.exp(-alpha * p)) * (u + shift)          # |d/dp p sigmoid(alpha p)| <= 1.1
+                off = 1.2 * op * (u + shift).abs() + p.abs() * ou + 2.0 ** -20 * z.abs()
+        elif act == "relu2":
+            off = 2 * z.abs() * off + off * off
+            z = z.clamp(min=0) ** 2
+        assert bool(((out[at].double() - z).abs() <= 2.0 ** -8 * z.abs() + off + 1e-6).all()), y
+
+
+# the batched product of many rows: results that leave 16 bytes, two numbers and one number at a time, by the rows' alignment; tiles cut in rows and
+# columns; with an output gate (bfloat16)
+@pytest.mark.parametrize("H,N", [(2, 104), (2, 98), (3, 97), (1, 130), (2, 257)])
+@pytest.mark.parametrize("T", [512, 700])
+@pytest.mark.parametrize("out_dtype,gated", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False)])
+def test_products_per_head_of_many_rows(T, H, N, out_dtype, gated):
+    K, gen = 136, torch.Generator(device=DEV).manual_seed(T + H * N)
+    a = torch.randn(T, H * K, device=DEV, generator=gen).to(torch.bfloat16)
+    w = (torch.randn(H, N, K, device=DEV, generator=gen) / K ** 0.5).to(torch.bfloat16)
+    gate = torch.randn(T, H, device=DEV, generator=gen).to(torch.bfloat16)
+    out = torch.full((T + 1, H * N), 7.0, device=DEV, dtype=out_dtype)
+    ops().gemm_heads(a, w, out[:T], **(dict(gate=gate) if gated else {}))
+    x, v = a.double().view(T, H, K), w.double()
+    ref, size = torch.einsum("thk,hnk->thn", x, v), torch.einsum("thk,hnk->thn", x.abs(), v.abs())
+    if gated:
+        ref, size = ref * torch.sigmoid(gate.double())[:, :, None], size * torch.sigmoid(gate.double())[:, :, None]
+    bound = (K + 8) * 2.0 ** -24 * size + (2.0 ** -8 * ref.abs() if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:T].double().view(T, H, N) - ref).abs() <= bound).all()) and bool((out[T:] == 7.0).all())
+
+
 @pytest.mark.parametrize("H", [96, 1028, 2048, 4096, 8192])
 @pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
 def test_norms_of_few_and_of_many_rows_hold_the_same_bits(H, act):
