@@ -292,7 +292,8 @@ static int launch_mma_kernel(dim3 grid, cudaStream_t s, int K, Args... args) {
 
 // The same for the few rows an expert gets in a decode step (tiles of 16 rows), where the launch is one read of the reached experts'
 // weights: blocks that stay, each with a ring of NST stages (64 rows of W by TMA and the tile's 16 rows of A, 128 columns of K) that its
-// fifth warp fills as far ahead as there is room and the other four, 16 columns of the product each, work off: 14 MB of weights under way.
+// fifth warp fills as far ahead as there is room and the other four, 16 columns of the product each, work off: 4 stages x 16 KB of W x 296
+// blocks, 19 MB of weights under way (3 x 16 KB x 444: 22 MB).
 // The (tile, 64 columns) items up to the last tile that holds rows are dealt out in rounds, an item a block; a last round that would leave
 // more than half of the blocks idle is cut into items of 32 or 16 columns, as far as there are blocks for them.  (Tiles of places without rows
 // in between, which a sort leaves none of, are passed over.)  An element's sum runs over K in the same steps as above.
