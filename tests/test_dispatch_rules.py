@@ -149,6 +149,15 @@ def test_constants_that_the_chunked_time_mixing_and_its_caller_share():
         assert lib.vl_decay_chunk_floats(*sizes) == ops.decay_chunk_floats(*sizes)
 
 
+@pytest.mark.parametrize("sizes", [(1, 1, 4, 4), (7, 32, 64, 64), (3, 5, 100, 68), (4096, 16, 128, 128)])
+def test_the_delta_rules_scratch_is_what_its_caller_brings(sizes):
+    import ctypes
+    from vllm_lite_b200.csrc import build
+    floats = build.load("delta").vl_delta_chunk_floats
+    floats.restype = ctypes.c_longlong
+    assert floats(*sizes) == ops.delta_chunk_floats(*sizes)
+
+
 # where the measured times cross (148 SMs): the weight-streaming product up to 8 rows, a tile of W an SM, the library
 @pytest.mark.parametrize("M,N,K,few", [
     (8, 2048, 2048, False), (9, 2048, 2048, True), (16, 7104, 2048, True), (16, 7120, 2048, False), (17, 4736, 2048, True), (24, 4752, 8192, False),
