@@ -61,6 +61,14 @@ def test_no_lane_leaves_a_loop_by_itself_when_a_wait_runs_out(name):
     assert "__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity))" in (build.CSRC / "tc5.cuh").read_text()
 
 
+def test_capped_scores_are_scaled_and_then_capped():
+    """The two-at-a-time form of `shape_score` keeps its order: the score times the scale, that times 2 / cap.  The factors' own product first rounds
+    elsewhere, which moves last bits of every capped layer."""
+    code = re.sub(r"//[^\n]*", "", (build.CSRC / "flash_tc5.cu").read_text())
+    assert "scale_log2 * toc" not in code and "toc * scale_log2" not in code
+    assert "k2 = pair(scale_log2, scale_log2), t2 = pair(toc, toc)" in code and code.count("k2, zero2), t2, zero2)") == 1
+
+
 def test_the_weight_streams_consumers_leave_together():
     """Between two tiles the four consumer warps meet at a barrier that counts 128 threads: a warp that left alone behind a wait
     that ran out would keep the others there."""

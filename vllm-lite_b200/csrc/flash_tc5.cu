@@ -361,14 +361,15 @@ flash_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             mbar_arrive(&s_free[s]);                             // the scores are in registers: the buffer may be written again
             const int j0 = tile_of(it) * BN;
             if constexpr (SHAPED) {
-                // shape_score, two scores an instruction where there is one for two
+                // shape_score, two scores an instruction where there is one for two: its factors one after the other, as there, since
+                // their product first is another rounding (0.3 % of a prompt of 2,048 through the capped layers)
                 if (cap_l2 > 0.f) {
-                    const unsigned long long k2 = pair(scale_log2 * toc, scale_log2 * toc), zero2 = pair(0.f, 0.f);
+                    const unsigned long long k2 = pair(scale_log2, scale_log2), t2 = pair(toc, toc), zero2 = pair(0.f, 0.f);
                     const unsigned long long m2 = pair(-2.f * cap_l2, -2.f * cap_l2), c2 = pair(cap_l2, cap_l2), one2 = pair(1.f, 1.f);
 #pragma unroll
                     for (int c = 0; c < BN; c += 2) {
                         float e0, e1, r0, r1;
-                        unpair(fma2(pair(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), k2, zero2), e0, e1);
+                        unpair(fma2(fma2(pair(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), k2, zero2), t2, zero2), e0, e1);
                         unpair(add2(pair(ss_exp2(e0), ss_exp2(e1)), one2), e0, e1);
                         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(e0));
                         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(e1));
