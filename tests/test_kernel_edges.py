@@ -772,6 +772,13 @@ def test_gelu_of_small_float32_values():
     assert torch.equal(ops().unary_act(both, torch.empty_like(both), "gelu")[::2], out[:1000])
 
 
+def test_gelu_of_bfloat16_values_is_that_of_float32_rounded_once():
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    x = torch.randn(1 << 20, device=DEV, generator=gen).clamp(min=-1.49).to(torch.bfloat16)
+    wide = ops().unary_act(x.float(), torch.empty(x.shape, device=DEV), "gelu")
+    assert torch.equal(ops().unary_act(x, torch.empty_like(x), "gelu"), wide.to(torch.bfloat16))
+
+
 def test_gelu_beyond_numbers():
     x = torch.tensor([float("inf"), float("nan"), 3e38, -3e38], device=DEV)
     out = torch.empty_like(x)

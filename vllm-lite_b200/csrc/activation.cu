@@ -111,17 +111,16 @@ extern "C" int vl_silu_mul(const void* gu, void* out, int dtype, int T, int I, i
 #define VL_ACT_RELU2 16
 #define VL_ACT_TANH 17
 #define VL_ACT_GELU 18
-// The normal distribution function at v is erfc(-v / sqrt(2)) / 2, and for z >= 0 erfc(z) = e^(-z^2) f(t), t = 1 / (1 + 0.44 z), with f(t) =
-// erfc(z) e^(z^2) smooth on (0, 1]: a polynomial of degree 8 without a constant, fitted to scipy's erfcx over z = 0 .. 10 by least
-// squares of the relative error with weights drawn to its largest places (1.8e-7).  It keeps the small values for v < 0 that the sum 1 + erff(z)
-// cancels (relative error in float32 at -4 .. -3 1.3e-6, the sum's 5e-4), but near zero the sum is the nearer one (|v| <= 0.5: 1.4e-7 and
-// 5.7e-7 at most, 4e-8 and 1.4e-7 of the 2-norm; they cross at -1.5).  So float32 values take either form where it is the better one, with
-// the full exponential and quotient.  A bfloat16 result's rounding (2e-3) hides both: there the polynomial alone, with the fast ones, bounds the
-// kernel by memory where the sum bound it by its instructions (3,281 x 8,192: 39 us with the sum, 45 % more instructions).
+// v times the normal distribution function at v, (1 + erf(v / sqrt(2))) / 2.  Towards small v the sum 1 + erff(z) cancels (relative error
+// 5e-4 at -4, 5e-2 at -5), and another form takes over: the function is erfc(-v / sqrt(2)) / 2, and for z >= 0 erfc(z) = e^(-z^2) f(t),
+// t = 1 / (1 + 0.44 z), with f(t) = erfc(z) e^(z^2) smooth on (0, 1]: a polynomial of degree 8 without a constant, fitted to scipy's erfcx over
+// z = 0 .. 10 by least squares of the relative error with weights drawn to its largest places (1.8e-7; 1.3e-6 with the exponential at -4).
+// Near zero the sum is the nearer one (|v| <= 0.5: 1.4e-7 at most, the polynomial 5.7e-7), and they cross at -1.5: there float32 values change
+// over; bfloat16 results, whose own rounding is 2e-3, at -4.  (The polynomial for all bfloat16 values, with the fast exponential and
+// quotient, has 45 % fewer instructions; it gains 0.3 % of a Vekusun prompt and moves last bits.)
 template <typename T> __device__ __forceinline__ float gelu_value(float v) {
-    constexpr bool fast = sizeof(T) == 2;
-    if (!fast && v > -1.5f) return 0.5f * v * (1.0f + erff(v * 0.70710678f));
-    const float z = fminf(fabsf(v) * 0.70710678f, 14.0f), d = fmaf(0.44f, z, 1.0f), t = fast ? __fdividef(1.0f, d) : 1.0f / d;
+    if (v > (sizeof(T) == 2 ? -4.0f : -1.5f)) return 0.5f * v * (1.0f + erff(v * 0.70710678f));
+    const float z = fminf(fabsf(v) * 0.70710678f, 14.0f), t = 1.0f / fmaf(0.44f, z, 1.0f);
     float f = 0.07122346758842468f;
     f = fmaf(f, t, -0.2779480218887329f);
     f = fmaf(f, t, 0.2966874837875366f);
@@ -130,8 +129,7 @@ template <typename T> __device__ __forceinline__ float gelu_value(float v) {
     f = fmaf(f, t, 0.21731355786323547f);
     f = fmaf(f, t, 0.24887117743492126f);
     f = fmaf(f, t, 0.24822095036506653f);
-    const float half = 0.5f * t * f * (fast ? __expf(-z * z) : expf(-z * z));
-    return v * (v > 0.f ? 1.0f - half : half);
+    return v * (0.5f * t * f * expf(-z * z));                // (no number: z = 14, and v itself makes the result one as well)
 }
 template <typename T, int ACT> __device__ __forceinline__ float unary_value(float v) {
     if (ACT == VL_ACT_RELU2) { v = fmaxf(v, 0.f); return v * v; }
