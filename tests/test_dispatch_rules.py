@@ -175,6 +175,11 @@ def test_which_experts_products_run_on_tcgen05(tokens, pairs, experts, K, big):
     assert not ops.gemm_grouped_tc5_ok(torch.float32, tokens, pairs, experts, K)
 
 
+def test_few_rows_an_expert_keep_the_full_exponential():
+    assert ops.gemm_grouped_tc5_fine(1023, 4) and not ops.gemm_grouped_tc5_fine(1024, 4)
+    assert ops.gemm_grouped_tc5_fine(96 * 32 - 1, 32) and not ops.gemm_grouped_tc5_fine(96 * 32, 32)
+
+
 # Products of paired blocks never run among programmatic launches: up to 64 tokens none is chosen, beyond them a recorded step asks the model.
 def test_no_product_of_paired_blocks_among_programmatic_launches(monkeypatch):
     from vllm_lite_b200.engine.runner import PDL_MAX_TOKENS, launches_dependent

@@ -743,6 +743,29 @@ def test_experts_product_of_many_rows(sizes, N, K, act):
         assert bool(((outs[0][at].double() - z).abs() <= 2.0 ** -8 * z.abs() + off + 1e-6).all()), g
 
 
+@pytest.mark.parametrize("act", ["silu", "capped_swish"])
+def test_experts_product_with_the_full_exponential(act):
+    """Gates of -20 to -75 and ups of 1, both exact sums: what is rounded is the activation alone.  A float32 activation (exponential to 1 ulp, sum,
+    quotient: 4 x 2^-24 at most) rounds to another bfloat16 number than the exact one where it crosses the middle of a step of 2^-8 or
+    more: 6.1e-5 of the results at most.  The fast exponential, whose argument of up to 108 is rounded to 2^-18, crosses three times as many."""
+    M, K, pairs = 16384, 64, 128
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    rows = torch.zeros(M, K, device=DEV)
+    rows[:, 0] = -20 - 30 * torch.rand(M, device=DEV, generator=gen)
+    rows[:, 1], rows[:, 2] = 1.0, torch.rand(M, device=DEV, generator=gen) / 2      # (what makes every gate another one)
+    rows[:, 2] = (rows[:, 2] * 2 ** 9).round() / 2 ** 9
+    rows = rows.to(torch.bfloat16)
+    w = torch.zeros(1, 2 * pairs, K, device=DEV)
+    fine = 1 + torch.arange(pairs, device=DEV) / 256.0                       # gates: rows[:, 0] times these, products of two 8-bit numbers
+    w.view(-1, 2, 8, K)[:, 0, :, 0], w.view(-1, 2, 8, K)[:, 0, :, 2], w.view(-1, 2, 8, K)[:, 1, :, 1] = fine.to(torch.bfloat16).float().view(-1, 8), 1.0, 1.0
+    err, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty(M, pairs, device=DEV, dtype=torch.bfloat16)
+    starts = torch.tensor([0, M], dtype=torch.int32, device=DEV)
+    ops().gemm_grouped_tc5(rows, w.to(torch.bfloat16), out, starts, err, act=act, alpha=1.0, limit=1e9, shift=0.0, fine=True)
+    g = rows[:, :1].double() * fine.to(torch.bfloat16).double() + rows[:, 2:3].double()
+    exact = (g / (1 + torch.exp(-g))).float()                                # (one rounding to float32 first: 2^-15 of a bfloat16 step)
+    assert float((out != exact.to(torch.bfloat16)).float().mean()) <= 6.1e-5 and int(err) == 0
+
+
 # functions of one argument: eight, four and single values a thread, and buffers that begin anywhere
 @pytest.mark.parametrize("act", ["gelu", "tanh", "relu2"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -126,7 +126,7 @@ _SIGNATURES = {
                               c_void_p, c_void_p, c_void_p, c_void_p],
     ("gemm_batched", "vl_gemm_rows_f32w"): [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("gemm_tc5_grouped", "vl_gemm_bf16_tc5_grouped"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                                       c_void_p, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
+                                                       c_void_p, c_int, c_float, c_float, c_float, c_int, c_void_p, c_void_p],
     ("moe", "vl_moe_align"): [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     ("moe", "vl_moe_gather"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ("moe", "vl_moe_combine"): [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1291,11 +1291,18 @@ def gemm_grouped_tc5_ok(dtype, tokens, pairs, num_experts, K) -> bool:
     return dtype == torch.bfloat16 and K % 8 == 0 and tokens > 64 and pairs >= 6 * num_experts
 
 
-def gemm_grouped_tc5(rows, w, out, starts, err, row_index=None, row_scale=None, act=None, alpha=1.0, limit=0.0, shift=0.0):
+def gemm_grouped_tc5_fine(pairs, num_experts) -> bool:
+    """Whether that product's activation takes the full exponential: below 96 rows an expert, where `gemm_grouped_fused` served before it and takes
+    it too.  Both are far inside a bfloat16 result's rounding and cost the same; beyond, the fast one keeps the bits that prompts have
+    always had."""
+    return pairs < max(1024, 96 * num_experts)
+
+
+def gemm_grouped_tc5(rows, w, out, starts, err, row_index=None, row_scale=None, act=None, alpha=1.0, limit=0.0, shift=0.0, fine=False):
     """The grouped product on the tcgen05 tensor cores: rows [cap, K] sorted by group, group g's rows are
     starts[g] .. starts[g + 1] (int32 [G + 1], `moe_align`), w [G, N, K], out [cap, N] or, with `act` (w then interleaves 8 gate rows
     with their 8 up rows), [cap, N / 2] = act(gate, up).
-    row_scale: the float32 sums of row m are multiplied by row_scale[row_index[m]] first."""
+    row_scale: the float32 sums of row m are multiplied by row_scale[row_index[m]] first.  fine: the activation's exponential is the full one."""
     _need(rows, torch.bfloat16, "rows", 2); _need(w, torch.bfloat16, "w", 3); _need(out, torch.bfloat16, "out", 2)
     _need(starts, torch.int32, "starts", 1)
     G, N, K = w.shape
@@ -1310,7 +1317,7 @@ def gemm_grouped_tc5(rows, w, out, starts, err, row_index=None, row_scale=None, 
         _need(row_scale, torch.float32, "row_scale")
     _check(_fn("gemm_tc5_grouped", "vl_gemm_bf16_tc5_grouped")(
         _ptr(rows), _ptr(w), _ptr(out), cap, N, K, G, _ptr(starts), _ptr(row_index), _ptr(row_scale),
-        _act_code(act), float(alpha), float(limit), float(shift), _ptr(err), _stream()),
+        _act_code(act), float(alpha), float(limit), float(shift), int(fine), _ptr(err), _stream()),
         "vl_gemm_bf16_tc5_grouped")
     return out
 

@@ -153,7 +153,8 @@ class RoutedExperts:
             # many rows: both products on the tcgen05 tensor cores, from a sorted copy of the tokens' rows
             rows = ops.moe_gather(h, sorted_rows, weights, top, ws.get(tag + "moe.rows", (cap, H), self.dtype), False)
             ops.gemm_grouped_tc5(rows, self.gate_up, act, starts, step.err, sorted_rows,
-                                 weights if s.scale_input else None, s.activation, s.alpha, s.limit, s.up_shift)
+                                 weights if s.scale_input else None, s.activation, s.alpha, s.limit, s.up_shift,
+                                 ops.gemm_grouped_tc5_fine(pairs, E))
             res = ops.gemm_grouped_tc5(act, self.down, ws.get(tag + "moe.down", (cap, H), self.dtype), starts, step.err)
             return ops.moe_combine(res, place, weights, top, ws.get(tag + "moe.out", (T, H), self.dtype), not s.scale_input,
                                    add=self._shared(h, step), **last)
