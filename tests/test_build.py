@@ -70,12 +70,16 @@ def test_capped_scores_are_scaled_and_then_capped():
 
 
 def test_the_weight_streams_consumers_leave_together():
-    """Between two tiles the four consumer warps meet at a barrier that counts 128 threads: a warp that left alone behind a wait
-    that ran out would keep the others there."""
+    """Between two tiles the four consumer warps meet at barriers that count 128 threads, and their lanes behind every stage: one that left
+    alone behind a wait that ran out would keep the others there.  So a wait notes for the block that it gave up, no loop over stages is left, and
+    all ask between the tile's two barriers."""
     code = re.sub(r"//[^\n]*", "", (build.CSRC / "gemm_bf16.cu").read_text())
-    tiles = code[code.index("for (int n0 = r0; n0 < r1; n0 += GS_ROWS) {\n#pragma unroll"):]
-    assert 0 < tiles.index("ok = consumers_agree(ok);") < tiles.index("if (!ok) break;", tiles.index("consumers_agree"))
-    assert "bar.red.and.pred q, 1, 128, p;" in code
+    stages = code[code.index("auto multiply = "):code.index("for (int n0 = r0; n0 < r1; n0 += GS_ROWS) {\n#pragma unroll")]
+    assert "mbar_wait_or_note(" in stages and "return" not in stages
+    tile = code[code.index("for (int n0 = r0; n0 < r1; n0 += GS_ROWS) {\n#pragma unroll"):]
+    first = tile.index("consumer_barrier();")
+    asked, second, left = tile.index("const bool ok = !s_gave_up;"), tile.index("consumer_barrier();", first + 1), tile.index("if (!ok) {")
+    assert first < asked < second < left and tile[:left].count("break;") == 1            # (the last of an odd number of stages)
 
 
 def test_the_engine_is_imported_without_a_compiler(tmp_path):

@@ -58,19 +58,24 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
     }
     return false;
 }
+// The same for consumers, whose lanes meet again behind it: who gives up notes that for the block and goes on as if the stage were there, and from
+// then on nobody waits long.  No lane leaves a loop by itself.  (A decode step of 8 rows through eight layers 979 -> 981 us; a vote of the warp
+// at every stage 5 us, a thread's own note of it 7.)
+__device__ __forceinline__ void mbar_wait_or_note(unsigned long long* bar, unsigned parity, volatile int* gave_up) {
+    if (mbar_try_wait(bar, parity)) return;
+    const long long t0 = clock64();
+    for (int i = 0; i < VL_WAIT_POLL_LIMIT; ++i) {
+        if (mbar_try_wait(bar, parity)) return;
+        if ((i & 31) == 31 && (*gave_up || vl_wait_gave_up(i, t0))) break;
+    }
+    *gave_up = 1;
+}
 // Both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-// the same barrier, and whether all four warps say so: they leave together, since the next barrier counts all of them
-__device__ __forceinline__ bool consumers_agree(bool ok) {
-    int all;
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.and.pred q, 1, 128, p;\n selp.s32 %0, 1, 0, q;\n}"
-                 : "=r"(all) : "r"((int)ok) : "memory");
-    return all != 0;
-}
 
 #define GS_CONSUMERS 4                     // consumer warps; warp 4 is the producer
 
@@ -101,6 +106,7 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
     constexpr int GS_ROWB = GS_KC * 2 + 16;    // bytes of a padded row of a stage: rows 16 bytes apart modulo 128
     extern __shared__ __align__(128) unsigned char gs_smem[];               // [GS_STAGES][16][GS_ROWB]
     __shared__ float red[GS_CONSUMERS][MT][GS_ROWS][8];
+    __shared__ volatile int s_gave_up;                                      // a consumer's wait ran out
     __shared__ float s_inv[16];                                             // row scales of a fused input norm
     __shared__ __align__(8) unsigned long long full_bar[GS_STAGES], empty_bar[GS_STAGES];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -111,6 +117,7 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
     const int iters = (K + GS_KC - 1) / GS_KC;
     pdl_launch_dependents();
     if (tid == 0) {
+        s_gave_up = 0;
         for (int i = 0; i < GS_STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], GS_CONSUMERS); }
         mbar_fence_init();
     }
@@ -189,14 +196,10 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
         }
     };
     int git = 0;                                                           // stages consumed so far, over all tiles
-    // A wait that runs out ends no loop, since the lanes of a warp meet again behind it: the thread remembers, waits for nothing more, hands no
-    // stage back and works on with what lies there (in bounds, never stored), and at the tile's end all four warps leave together.
-    // (A vote of the warp at every stage costs a decode step of 8 rows 0.3 %.)
-    bool ok = true;
     auto multiply = [&](int it, const uint4 (&a)[STEPS][MT]) {
         const int s = git % GS_STAGES;
         const int kbase = it * GS_KC + warp * (GS_KC / GS_CONSUMERS);
-        if (ok) ok = mbar_wait_bounded(&full_bar[s], (unsigned)((git / GS_STAGES) & 1));
+        mbar_wait_or_note(&full_bar[s], (unsigned)((git / GS_STAGES) & 1), &s_gave_up);
         const unsigned char* stage = gs_smem + (size_t)s * GS_ROWS * GS_ROWB + (size_t)warp * (GS_KC / GS_CONSUMERS) * 2;
 #pragma unroll
         for (int u = 0; u < STEPS; ++u) {
@@ -212,7 +215,7 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
             }
         }
         __syncwarp();
-        if (lane == 0 && ok) mbar_arrive(&empty_bar[s]);
+        if (lane == 0) mbar_arrive(&empty_bar[s]);
         ++git;
     };
     for (int n0 = r0; n0 < r1; n0 += GS_ROWS) {
@@ -236,8 +239,8 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
         red[warp][j][g + 8][2 * t] = acc[j][2];
         red[warp][j][g + 8][2 * t + 1] = acc[j][3];
     }
-    if (!ok && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_SMALL_M);
-    ok = consumers_agree(ok);
+    consumer_barrier();
+    const bool ok = !s_gave_up;                                            // the same for all: whoever gave up did so before the barrier
     if (swiglu) {
         // the tile's 16 rows of W are 8 gate rows and their 8 up rows: C[m, n0/2 + i] = silu(gate_i) * up_i
         for (int idx = tid; idx < MT * 8 * 8; idx += 32 * GS_CONSUMERS) {
@@ -283,7 +286,12 @@ gemm_bf16_small_m_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W,
         }
     }
     consumer_barrier();                                                    // `red` is free for the next tile
-    if (!ok) break;                                                        // a wait ran out: the error word says so
+    if (!ok) {                                                             // a wait ran out: copies in flight get time to land
+        if (tid == 0 && err) atomicOr(err, VL_DEV_WAIT_EXPIRED | VL_DEV_IN_GEMM_SMALL_M);
+        const long long t0 = clock64();
+        while (clock64() - t0 < VL_WAIT_CYCLE_LIMIT) {}
+        break;
+    }
     }
     if (nf.ss_out && (tid & 15) == 0) {
 #pragma unroll
