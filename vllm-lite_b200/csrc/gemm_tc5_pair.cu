@@ -235,9 +235,10 @@ extern "C" int vl_gemm_bf16_tc5_pair(const void* A, const void* W, void* C, int 
     if (((uintptr_t)A | (uintptr_t)W) & 15) return VL_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     // Which width.  A K block of a tile of 512 columns costs 1.93 of one of 256, and its epilogue, which nothing hides, 6.5 more: it wins
-    // where it saves a round of the pairs of SMs and K is long (us, 256 / 512): 2,048 rows x 12,288 -> 4,096 147.8 / 150.5 with the
-    // clocks down, 3,000 x 8,192 -> 2,048 83.9 / 81.3, 4,096 x 12,288 -> 4,096 281.6 / 271.4; 2,048 x 2,048 -> 8,192 49.5 / 51.5, 2,048 x 4,096 -> 4,096
-    // 49.0 / 48.7, 2,048 x 4,096 -> 6,144 70.1 / 88.2.
+    // where it saves a round of the pairs of SMs and K is long.  Inside a pass of eight layers of Qwen3-8B, where the clocks are down and only the
+    // down product (x 12,288 -> 4,096) takes it (us a pass, 256 / 512, means of three runs in turn): 2,048 rows 6,087 / 6,025, 4,096 rows 12,262 /
+    // 12,126.  Alone (us, 256 / 512): 3,000 x 8,192 -> 2,048 83.9 / 81.3, and where the rule says 256: 2,048 x 2,048 -> 8,192 49.5 / 51.5, 2,048 x
+    // 4,096 -> 4,096 49.0 / 48.7, 2,048 x 4,096 -> 6,144 70.1 / 88.2.
     static int pairs = 0;
     if (!pairs) {
         int dev = 0, sms = 0;
